@@ -5,7 +5,7 @@
 // This is the kv_bits == 8 route of the dispatcher; the decode loop spends its bytes on codes
 // (D bytes per token and head for each of K and V), so the kernels stay simple: a warp owns a
 // token row, a lane D/32 channels.
-#include "fq_common.cuh"
+#include "fq_quant_pages.cuh"
 
 namespace fq {
 
@@ -464,6 +464,15 @@ extern "C" int fq_quantize_kv_int8(
     FQ_CHECK_ARG(!V || (V_uint8 && V_scale && V_mn), FQ_ERR_ARG, "%s: V given without its outputs", fn);
     FQ_CHECK_ARG((int64_t)B * H * S <= 0x7fffffffLL * 4, FQ_ERR_ARG, "%s: too many tokens for one launch", fn);
     if (S == 0) return FQ_OK;
+    {   // whole pages of 16-bit rows: the register-resident kernel (V alone: any multiple of 16 tokens)
+        QuantPagesParams f{};
+        f.K_new = K; f.V_new = V; f.nw_sb = in_sb; f.nw_sh = in_sh; f.nw_ss = in_ss;
+        f.n_new = S; f.n_quant = S; f.B = B; f.H = H; f.D = D; f.page = page; f.bits = 8;
+        f.K_codes = K ? K_uint8 : nullptr; f.V_codes = V ? V_uint8 : nullptr; f.cd_sb = c_sb; f.cd_sh = c_sh; f.cd_ss = c_ss;
+        f.K_scale = K ? static_cast<uint16_t*>(K_scale) : nullptr; f.K_mn = static_cast<uint16_t*>(K_mn); f.km_sb = km_sb; f.km_sh = km_sh; f.km_sp = km_sp;
+        f.V_scale = static_cast<uint16_t*>(V_scale); f.V_mn = static_cast<uint16_t*>(V_mn); f.vm_sb = vm_sb; f.vm_sh = vm_sh; f.vm_ss = 1;
+        if (quant_pages_supported(f, dtype)) return quant_pages_launch(f, dtype, stream, fn);
+    }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint16_t *ks = static_cast<uint16_t*>(K_scale), *km = static_cast<uint16_t*>(K_mn), *vs = static_cast<uint16_t*>(V_scale), *vm = static_cast<uint16_t*>(V_mn);
     if (dtype == FQ_F32) launch_quant_int8<float>(K, V, in_sb, in_sh, in_ss, B, H, S, D, page, K_uint8, V_uint8, c_sb, c_sh, c_ss, ks, km, km_sb, km_sh, km_sp, vs, vm, vm_sb, vm_sh, st);

@@ -6,7 +6,7 @@
 // code can be produced, so the page is read twice (the second read is served by L1/L2);
 // V is per token and needs one read.  HBM traffic per page: 2*page*D*sizeof(T) in,
 // page*D (codes) + 2*D*2 (K metadata) + page*4 (V metadata) out.
-#include "fq_common.cuh"
+#include "fq_quant_pages.cuh"
 
 namespace fq {
 
@@ -312,6 +312,19 @@ int quantize_kv_int4_launch(
     FQ_CHECK_ARG(km_sb % 8 == 0 && km_sh % 8 == 0 && km_sp % 8 == 0 && aligned(K_scale, 16) && aligned(K_mn, 16),
                  FQ_ERR_ALIGN, "%s: K metadata rows must be 16-byte aligned", fn);
 
+    // whole pages of a prompt: the register-resident kernel.  The general one below takes ragged last pages, other
+    // page sizes, head dimensions and fp32, appends that complete no page, and positions read on the device.
+    if (dp.pos == nullptr && n_quant > 0) {
+        QuantPagesParams f{};
+        f.K_head = K_head; f.V_head = V_head; f.K_new = K_new; f.V_new = V_new;
+        f.hd_sb = hd_sb; f.hd_sh = hd_sh; f.hd_ss = hd_ss; f.nw_sb = nw_sb; f.nw_sh = nw_sh; f.nw_ss = nw_ss;
+        f.n_head = n_head; f.n_new = n_new; f.n_quant = n_quant; f.B = B; f.H = H; f.D = D; f.page = page; f.bits = 4;
+        f.K_codes = K_packed; f.V_codes = V_packed; f.cd_sb = pk_sb; f.cd_sh = pk_sh; f.cd_ss = pk_ss;
+        f.K_scale = static_cast<uint16_t*>(K_scale); f.K_mn = static_cast<uint16_t*>(K_mn); f.km_sb = km_sb; f.km_sh = km_sh; f.km_sp = km_sp;
+        f.V_scale = static_cast<uint16_t*>(V_scale); f.V_mn = static_cast<uint16_t*>(V_mn); f.vm_sb = vm_sb; f.vm_sh = vm_sh; f.vm_ss = vm_ss;
+        f.stage_K = stage_K; f.stage_V = stage_V; f.st_sb = st_sb; f.st_sh = st_sh; f.st_ss = st_ss;
+        if (quant_pages_supported(f, dtype)) return quant_pages_launch(f, dtype, stream, fn);
+    }
     QuantParams p;
     p.K_head = K_head; p.V_head = V_head; p.K_new = K_new; p.V_new = V_new;
     p.hd_sb = hd_sb; p.hd_sh = hd_sh; p.hd_ss = hd_ss; p.nw_sb = nw_sb; p.nw_sh = nw_sh; p.nw_ss = nw_ss;
