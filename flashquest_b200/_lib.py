@@ -13,6 +13,7 @@ import torch
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libflashquest_b200.so")
+BIND_PATH = os.path.join(_PKG, "lib", "_fq_bind.so")
 
 FQ_F32, FQ_F16, FQ_BF16 = 0, 1, 2
 _DTYPE_CODE = {torch.float32: FQ_F32, torch.float16: FQ_F16, torch.bfloat16: FQ_BF16}
@@ -157,6 +158,9 @@ _PROTOTYPES["fq_sparse_decode_int8"] = (I, [P, I, L, L, P, P, L, L, L, P, P, L, 
 _PROTOTYPES["fq_sparse_decode_int8_counted"] = (I, [P, I, L, L, P, P, L, L, L, P, P, L, L, L, P, P, L, L, P, L, L, I, P,
                                                    P, P, I, L, L, L, I, I, I, I, I, I, I, I, F, P, P, P, Z, I, P])
 _PROTOTYPES["fq_prefill_attention"] = (I, [P, L, L, L, P, L, L, L, P, L, L, L, I, I, I, I, I, I, I, F, P, L, L, L, P])
+_PROTOTYPES["fq_append_kv_int8"] = (I, [ctypes.POINTER(Int4CacheDesc), I, I, P, P, L, L, L, I, P])
+_PROTOTYPES["fq_decode_layer_int8"] = _PROTOTYPES["fq_decode_layer_int4"]
+_PROTOTYPES["fq_rope_qkv"] = (I, [P, L, P, L, P, L, I, P, L, P, L, I, I, I, I, P, P, P, I, P])
 
 # entry points added by later sources register themselves here (name -> (restype, argtypes))
 EXTRA_PROTOTYPES: dict = {}
@@ -180,6 +184,25 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+_bind = None
+
+
+def bind():
+    """The CPython module over the C ABI (csrc/fq_bind.cpp): step calls without per-argument ctypes conversions."""
+    global _bind
+    if _bind is None:
+        import importlib.util
+        if not os.path.exists(BIND_PATH):
+            raise FlashQuestError(f"{BIND_PATH} is missing: build it with `python -m flashquest_b200.build`.")
+        lib()
+        ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)          # the module's C ABI symbols resolve against it
+        spec = importlib.util.spec_from_file_location("_fq_bind", BIND_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _bind = module
+    return _bind
 
 
 def exported_symbols():

@@ -15,6 +15,8 @@ CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIB_DIR, "libflashquest_b200.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
+BIND_SRC = os.path.join(CSRC, "fq_bind.cpp")
+BIND = os.path.join(LIB_DIR, "_fq_bind.so")       # CPython module over the C ABI (see fq_bind.cpp)
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -41,6 +43,29 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_bind(force: bool = False) -> str:
+    """The CPython module: host code only, resolved against the running torch and the library beside it."""
+    if not force and not _stale(BIND, [BIND_SRC, os.path.join(INCLUDE, "flashquest_b200.h")]):
+        return BIND
+    import sysconfig
+
+    import torch
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda, "include")]
+    for inc in ("include", os.path.join("include", "torch", "csrc", "api", "include")):
+        cmd += ["-isystem", os.path.join(tdir, inc)]
+    tlib = os.path.join(tdir, "lib")
+    cmd += [BIND_SRC, "-o", BIND + ".tmp", "-L", tlib, f"-Wl,-rpath,{tlib}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {BIND_SRC}:\n{r.stdout}\n{r.stderr}")
+    os.replace(BIND + ".tmp", BIND)
+    return BIND
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(LIB_DIR, exist_ok=True)
     headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(INCLUDE, "*.h"))
@@ -58,6 +83,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError(f"nvcc failed for {src}:\n{r.stdout}\n{r.stderr}")
         return r.stderr
 
+    bind = ThreadPoolExecutor(max_workers=1).submit(build_bind, force)
     with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
         logs = list(ex.map(compile_one, zip(srcs, objs)))
     if verbose:
@@ -69,6 +95,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    bind.result()
     return LIB
 
 

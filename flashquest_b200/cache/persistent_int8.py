@@ -2,9 +2,12 @@
 same constructor keywords, attributes, view keys and error behaviour."""
 from __future__ import annotations
 
+import ctypes
+
 import torch
 from transformers.cache_utils import Cache
 
+from .._lib import Int4CacheDesc, check, dtype_code, lib, ptr, require_cuda, stream_ptr
 from ..kernel.kv_quant import quantize_kv_int8_into
 
 
@@ -37,6 +40,22 @@ class PersistentInt8KVCache(Cache):
         self.V_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self._seen_tokens = [0] * num_layers
 
+        # the one-launch append (fq_append_kv_int8): 16-bit staging, head_dim 64 / 128, pages of 16, 32 or 64 tokens
+        self._one_launch = dtype in (torch.float16, torch.bfloat16) and D in (64, 128) and page_size in (16, 32, 64)
+        self._desc = None
+
+    def desc(self) -> Int4CacheDesc:
+        """struct fq_int4_cache of this cache (code rows of D bytes)."""
+        if self._desc is None or self._desc.K_packed != self.K_uint8.data_ptr() or self._desc.K_partial != self.K_partial.data_ptr():
+            self._desc = Int4CacheDesc(
+                self.K_uint8.data_ptr(), self.V_uint8.data_ptr(), *self.K_uint8.stride()[:4],
+                self.K_scale.data_ptr(), self.K_mn.data_ptr(), *self.K_scale.stride()[:4],
+                self.V_scale.data_ptr(), self.V_mn.data_ptr(), *self.V_scale.stride()[:3],
+                self.K_partial.data_ptr(), self.V_partial.data_ptr(), *self.K_partial.stride()[:4],
+                dtype_code(self.K_partial), self.num_layers, self.batch_size, self.num_kv_heads, self.head_dim, self.page_size,
+                self.max_seq_len)
+        return self._desc
+
     def get_seq_length(self, layer_idx: int = 0) -> int:
         return self._seen_tokens[layer_idx]
 
@@ -58,6 +77,17 @@ class PersistentInt8KVCache(Cache):
             raise RuntimeError(f"PersistentInt8KVCache: seen+new={seen + S_new} exceeds max_seq_len={self.max_seq_len}")
         page = self.page_size
         li = layer_idx
+        if S_new > 0 and self._one_launch:
+            if K_new.dtype != self.dtype or V_new.dtype != self.dtype:
+                K_new, V_new = K_new.to(self.dtype), V_new.to(self.dtype)
+            if K_new.stride(3) != 1 or V_new.stride() != K_new.stride() or any(s % 8 for s in K_new.stride()[:3]) \
+                    or K_new.data_ptr() % 16 or V_new.data_ptr() % 16:
+                K_new, V_new = K_new.contiguous(), V_new.contiguous()
+            require_cuda(K_new, V_new)
+            check(lib().fq_append_kv_int8(ctypes.byref(self.desc()), li, seen, ptr(K_new), ptr(V_new), *K_new.stride()[:3], S_new,
+                                          stream_ptr(self.K_uint8.device)))
+            self._seen_tokens[layer_idx] = seen + S_new
+            return
         partial_len = seen % page
         K_stream = torch.cat([self.K_partial[li, :, :, :partial_len], K_new.to(self.dtype)], dim=2)
         V_stream = torch.cat([self.V_partial[li, :, :, :partial_len], V_new.to(self.dtype)], dim=2)

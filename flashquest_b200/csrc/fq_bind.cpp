@@ -1,0 +1,158 @@
+// Native step calls for the Python layer: unpacks the tensors of one decode step and calls the C ABI.
+//
+// A ctypes call with forty arguments costs about 20 us of host time (one conversion object per pointer, stride
+// and size), more than the kernels of a short decode step take; here a step is one METH_FASTCALL function that
+// reads pointers and strides from the tensors directly.  A `plan` (capsule) holds what does not change between
+// steps: the cache descriptor, the parameters and the addresses of the engine's preallocated buffers.
+//
+// A call returns 0 (done), 1 (the tensors are not in a form the native path takes: the caller prepares them and
+// calls again through the general path) or a negative FQ_ERR_* code.
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/flashquest_b200.h"
+
+namespace {
+
+struct Plan {
+    int kind;                       // 4, 8: fq_int4_cache; 3: fq_turbo_cache
+    fq_int4_cache c4;
+    fq_turbo_cache c3;
+    fq_decode_params prm;
+    int device, cache_dtype, n_layers;
+    float* scores; int64_t sc_sl;
+    int32_t* compact; int64_t cp_sl;
+    char* O; int64_t o_sl;          // bytes
+    float* lse; int64_t lse_sl;
+    char* ws; size_t ws_sl, ws_bytes;
+    char* scratch; size_t scratch_bytes;
+    char *q_rot, *k_rot, *v_rot;    // rotated q / k and cast v of the patched forward, dense, cache dtype
+};
+
+const char* kPlanName = "flashquest_b200.plan";
+
+void free_plan(PyObject* cap) { delete static_cast<Plan*>(PyCapsule_GetPointer(cap, kPlanName)); }
+
+Plan* plan_of(PyObject* o) { return static_cast<Plan*>(PyCapsule_GetPointer(o, kPlanName)); }
+
+inline void* as_ptr(PyObject* o) { return reinterpret_cast<void*>(PyLong_AsUnsignedLongLong(o)); }
+
+int dtype_of(const at::Tensor& t) {
+    switch (t.scalar_type()) {
+        case at::kHalf: return FQ_F16;
+        case at::kBFloat16: return FQ_BF16;
+        case at::kFloat: return FQ_F32;
+        default: return -1;
+    }
+}
+
+inline const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream(); }
+
+// plan(kind, cache_desc, params, device, n_layers, scores, sc_sl, compact, cp_sl, O, o_sl_bytes, lse, lse_sl,
+//      ws, ws_sl, ws_bytes, scratch, scratch_bytes, q_rot, k_rot, v_rot): addresses and sizes as integers
+PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 21) { PyErr_SetString(PyExc_TypeError, "plan() takes 21 arguments"); return nullptr; }
+    Plan* p = new Plan();
+    p->kind = static_cast<int>(PyLong_AsLong(a[0]));
+    if (p->kind == 3) { p->c3 = *static_cast<const fq_turbo_cache*>(as_ptr(a[1])); p->cache_dtype = p->c3.kv_dtype; }
+    else { p->c4 = *static_cast<const fq_int4_cache*>(as_ptr(a[1])); p->cache_dtype = p->c4.kv_dtype; }
+    p->prm = *static_cast<const fq_decode_params*>(as_ptr(a[2]));
+    p->device = static_cast<int>(PyLong_AsLong(a[3]));
+    p->n_layers = static_cast<int>(PyLong_AsLong(a[4]));
+    p->scores = static_cast<float*>(as_ptr(a[5])); p->sc_sl = PyLong_AsLongLong(a[6]);
+    p->compact = static_cast<int32_t*>(as_ptr(a[7])); p->cp_sl = PyLong_AsLongLong(a[8]);
+    p->O = static_cast<char*>(as_ptr(a[9])); p->o_sl = PyLong_AsLongLong(a[10]);
+    p->lse = static_cast<float*>(as_ptr(a[11])); p->lse_sl = PyLong_AsLongLong(a[12]);
+    p->ws = static_cast<char*>(as_ptr(a[13])); p->ws_sl = PyLong_AsSize_t(a[14]); p->ws_bytes = PyLong_AsSize_t(a[15]);
+    p->scratch = static_cast<char*>(as_ptr(a[16])); p->scratch_bytes = PyLong_AsSize_t(a[17]);
+    p->q_rot = static_cast<char*>(as_ptr(a[18])); p->k_rot = static_cast<char*>(as_ptr(a[19])); p->v_rot = static_cast<char*>(as_ptr(a[20]));
+    if (PyErr_Occurred()) { delete p; return nullptr; }
+    return PyCapsule_New(p, kPlanName, free_plan);
+}
+
+int run_layer(const Plan* p, int layer, int seen, const void* k, const void* v, int64_t sb, int64_t sh, int64_t ss, int n_new,
+              const void* q, int q_dtype, int64_t q_sb, int64_t q_sh, const fq_decode_params* prm, void* stream) {
+    float* sc = p->scores + layer * p->sc_sl;
+    int32_t* cp = p->compact + layer * p->cp_sl;
+    char* O = p->O + layer * p->o_sl;
+    float* lse = p->lse + layer * p->lse_sl;
+    char* ws = p->ws + static_cast<size_t>(layer) * p->ws_sl;
+    if (p->kind == 3)
+        return fq_decode_layer_turbo(&p->c3, layer, seen, k, v, sb, sh, ss, n_new, q, q_dtype, q_sb, q_sh, prm, sc, cp,
+                                     p->scratch, p->scratch_bytes, O, lse, ws, p->ws_bytes, stream);
+    if (p->kind == 8)
+        return fq_decode_layer_int8(&p->c4, layer, seen, k, v, sb, sh, ss, n_new, q, q_dtype, q_sb, q_sh, prm, sc, cp,
+                                    O, lse, ws, p->ws_bytes, stream);
+    return fq_decode_layer_int4(&p->c4, layer, seen, k, v, sb, sh, ss, n_new, q, q_dtype, q_sb, q_sh, prm, sc, cp,
+                                O, lse, ws, p->ws_bytes, stream);
+}
+
+// step(plan, layer, seen, k, v, q, params | 0): k, v (B,H_kv,n,D) of the cache's dtype, q (B,H_q,1,D) or (B,H_q,D)
+PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 7) { PyErr_SetString(PyExc_TypeError, "step() takes 7 arguments"); return nullptr; }
+    const Plan* p = plan_of(a[0]);
+    if (!p) return nullptr;
+    const int layer = static_cast<int>(PyLong_AsLong(a[1])), seen = static_cast<int>(PyLong_AsLong(a[2]));
+    const at::Tensor *k = tensor_of(a[3]), *v = tensor_of(a[4]), *q = tensor_of(a[5]);
+    const fq_decode_params* prm = static_cast<const fq_decode_params*>(as_ptr(a[6]));
+    if (PyErr_Occurred()) return nullptr;
+    if (!k || !v || !q) return PyLong_FromLong(1);
+    const int B = p->kind == 3 ? p->c3.B : p->c4.B, Hkv = p->kind == 3 ? p->c3.Hkv : p->c4.Hkv, D = p->kind == 3 ? p->c3.D : p->c4.D;
+    const int Hq = p->prm.Hq;
+    const int qd = static_cast<int>(q->dim());
+    const bool ok = k->dim() == 4 && v->dim() == 4 && (qd == 3 || (qd == 4 && q->size(2) == 1)) && k->is_cuda() && v->is_cuda() && q->is_cuda() &&
+                    dtype_of(*k) == p->cache_dtype && dtype_of(*v) == p->cache_dtype && dtype_of(*q) >= 0 &&
+                    k->sizes() == v->sizes() && k->strides() == v->strides() && k->size(0) == B && k->size(1) == Hkv && k->size(3) == D &&
+                    k->stride(3) == 1 && q->size(0) == B && q->size(1) == Hq && q->size(qd - 1) == D && q->stride(qd - 1) == 1 &&
+                    (p->kind != 3 || (q->stride(1) == D && q->stride(0) == static_cast<int64_t>(Hq) * D));
+    if (!ok) return PyLong_FromLong(1);
+    const int rc = run_layer(p, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), static_cast<int>(k->size(2)),
+                             q->data_ptr(), dtype_of(*q), q->stride(0), q->stride(1), prm ? prm : &p->prm, stream_of(p->device));
+    return PyLong_FromLong(rc);
+}
+
+// forward(plan, layer, seen, q, k, v, cos, sin, params | 0): one new token of the patched attention forward.
+// q (B,1,H_q*D), k, v (B,1,H_kv*D): the projections as the linears return them; cos, sin (B or 1,1,D) of the same dtype.
+PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 9) { PyErr_SetString(PyExc_TypeError, "forward() takes 9 arguments"); return nullptr; }
+    const Plan* p = plan_of(a[0]);
+    if (!p) return nullptr;
+    const int layer = static_cast<int>(PyLong_AsLong(a[1])), seen = static_cast<int>(PyLong_AsLong(a[2]));
+    const at::Tensor* t[5];
+    for (int i = 0; i < 5; ++i) t[i] = tensor_of(a[3 + i]);
+    const fq_decode_params* prm = static_cast<const fq_decode_params*>(as_ptr(a[8]));
+    if (PyErr_Occurred()) return nullptr;
+    const int B = p->kind == 3 ? p->c3.B : p->c4.B, Hkv = p->kind == 3 ? p->c3.Hkv : p->c4.Hkv, D = p->kind == 3 ? p->c3.D : p->c4.D;
+    const int Hq = p->prm.Hq;
+    const int dt = t[0] ? dtype_of(*t[0]) : -1;
+    if (dt != FQ_F16 && dt != FQ_BF16) return PyLong_FromLong(1);
+    for (int i = 0; i < 5; ++i) {
+        if (!t[i] || !t[i]->is_cuda() || dtype_of(*t[i]) != dt || t[i]->dim() != 3 || t[i]->size(1) != 1 || t[i]->stride(2) != 1) return PyLong_FromLong(1);
+        const int64_t width = i == 0 ? static_cast<int64_t>(Hq) * D : i < 3 ? static_cast<int64_t>(Hkv) * D : D;
+        if (t[i]->size(2) != width || !(t[i]->size(0) == B || (i >= 3 && t[i]->size(0) == 1))) return PyLong_FromLong(1);
+    }
+    const int64_t cs = t[3]->size(0) == 1 ? 0 : t[3]->stride(0), ss = t[4]->size(0) == 1 ? 0 : t[4]->stride(0);
+    void* st = stream_of(p->device);
+    int rc = fq_rope_qkv(t[0]->data_ptr(), t[0]->stride(0), t[1]->data_ptr(), t[1]->stride(0), t[2]->data_ptr(), t[2]->stride(0), dt,
+                         t[3]->data_ptr(), cs, t[4]->data_ptr(), ss, B, Hq, Hkv, D, p->q_rot, p->k_rot, p->v_rot, p->cache_dtype, st);
+    if (rc == 0)
+        rc = run_layer(p, layer, seen, p->k_rot, p->v_rot, static_cast<int64_t>(Hkv) * D, D, D, 1, p->q_rot, p->cache_dtype,
+                       static_cast<int64_t>(Hq) * D, D, prm ? prm : &p->prm, st);
+    return PyLong_FromLong(rc);
+}
+
+PyMethodDef kMethods[] = {
+    {"plan", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(make_plan)), METH_FASTCALL, nullptr},
+    {"step", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(step)), METH_FASTCALL, nullptr},
+    {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(forward)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_fq_bind", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__fq_bind(void) { return PyModule_Create(&kModule); }

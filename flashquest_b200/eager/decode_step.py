@@ -14,10 +14,94 @@ import math
 
 import torch
 
-from .._lib import DecodeParams, Int4CacheDesc, TurboCacheDesc, check, dtype_code, lib, ptr, stream_ptr
+from .._lib import DecodeParams, Int4CacheDesc, TurboCacheDesc, bind, check, dtype_code, lib, ptr, stream_ptr
 
 
-class QuestDecodeInt4:
+class _NativeSteps:
+    """step() and forward_token() over the CPython module (csrc/fq_bind.cpp): one call that reads pointers and strides
+    from the tensors itself.  The subclass has set the cache descriptor, the parameters and the preallocated buffers."""
+
+    def _build_plan(self, kind, scores, compact, workspace, scratch=None):
+        """scores, compact, workspace: with a leading layer dimension, or shared by the layers (stride 0)."""
+        per = lambda t, nd: t.stride(0) if t.dim() == nd else 0
+        B, D, dt = self.B, self.D, self.cache.dtype
+        # what the patched forward's rotary embedding writes: q, k, v of the new token in the cache's dtype
+        self.q_rot = torch.empty(B, self.Hq, 1, D, dtype=dt, device=self.device)
+        self.k_rot = torch.empty(B, self.Hkv, 1, D, dtype=dt, device=self.device)
+        self.v_rot = torch.empty_like(self.k_rot)
+        ws_bytes = workspace.shape[-1]
+        self._plan_ = bind().plan(
+            kind, ctypes.addressof(self._cdesc), ctypes.addressof(self._prm), self.device.index or 0, self.cache.num_layers,
+            scores.data_ptr(), per(scores, 4), compact.data_ptr(), per(compact, 4),
+            self.O.data_ptr(), self.O.stride(0) * self.O.element_size(), self.lse.data_ptr(), self.lse.stride(0),
+            workspace.data_ptr(), per(workspace, 2), ws_bytes,
+            scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
+            self.q_rot.data_ptr(), self.k_rot.data_ptr(), self.v_rot.data_ptr())
+        self._outs = [(self.O[i].unsqueeze(2), self.lse[i].unsqueeze(2)) for i in range(self.cache.num_layers)]
+        self._step, self._forward = bind().step, bind().forward
+
+    def _seen_checked(self, layer_idx, n_new):
+        c = self.cache
+        if layer_idx < 0 or layer_idx >= c.num_layers:
+            raise IndexError(f"layer_idx {layer_idx} out of range [0, {c.num_layers})")
+        seen = c._seen_tokens[layer_idx]
+        if seen + n_new > c.max_seq_len:
+            raise RuntimeError(f"{type(c).__name__}: seen+new={seen + n_new} exceeds max_seq_len={c.max_seq_len}")
+        return seen
+
+    def step(self, k_new: torch.Tensor, v_new: torch.Tensor, q: torch.Tensor, layer_idx: int, prm=None):
+        """Append k_new, v_new (B,H_kv,n,D) to the layer and attend with q (B,H_q,1,D) in ONE foreign call: what
+        cache.update_quantized followed by the decode branch does.  `prm`: a per-layer fq_decode_params
+        (params_for) instead of the engine's own.  Returns views (O (B,H_q,1,D), lse (B,H_q,1)) of
+        preallocated per-layer buffers."""
+        n_new = k_new.shape[2]
+        seen = self._seen_checked(layer_idx, n_new)
+        addr = 0 if prm is None else ctypes.addressof(prm)
+        rc = self._step(self._plan_, layer_idx, seen, k_new, v_new, q, addr)
+        if rc == 1:            # another dtype, or strides the kernels do not take: prepare and call again
+            dt = self.cache.dtype
+            k_new, v_new = k_new.to(dt), v_new.to(dt)
+            if k_new.stride(3) != 1 or v_new.stride() != k_new.stride():
+                k_new, v_new = k_new.contiguous(), v_new.contiguous()
+            q = q.reshape(self.B, self.Hq, self.D).contiguous()
+            rc = self._step(self._plan_, layer_idx, seen, k_new, v_new, q, addr)
+            if rc == 1:
+                raise ValueError(f"step: k, v must be (B={self.B}, H_kv={self.Hkv}, n, D={self.D}) and q (B, H_q={self.Hq}, 1, D) CUDA tensors")
+        if rc:
+            check(rc)
+        self.cache._seen_tokens[layer_idx] = seen + n_new
+        self.launches += self.LAUNCHES
+        return self._outs[layer_idx]
+
+    def forward_token(self, q, k, v, cos, sin, layer_idx: int, prm=None):
+        """One new token from the projections: rotary embedding (Hugging Face's roundings), cast to the cache's dtype and
+        step(), in one call.  q (B,1,H_q*D), k, v (B,1,H_kv*D), cos, sin (B,1,D), one 16-bit dtype.  Returns O (B,H_q,1,D),
+        or None when the tensors are not of that form (nothing has been done)."""
+        seen = self._seen_checked(layer_idx, 1)
+        rc = self._forward(self._plan_, layer_idx, seen, q, k, v, cos, sin, 0 if prm is None else ctypes.addressof(prm))
+        if rc == 1:
+            return None
+        if rc:
+            check(rc)
+        self.cache._seen_tokens[layer_idx] = seen + 1
+        self.launches += self.LAUNCHES + 1
+        return self._outs[layer_idx][0]
+
+    def params_for(self, head_pattern_layer: torch.Tensor):
+        """fq_decode_params of one layer whose retrieval / streaming KV heads are given by
+        head_pattern_layer (H_kv,) bool: retrieval heads keep `retention`, streaming heads 0
+        (eager/llama_persistent_patch.py:214-219).  Returns (struct, tensor kept alive by the caller)."""
+        n_rep = self.Hq // self.Hkv
+        pat = head_pattern_layer.to(self.device).bool().repeat_interleave(n_rep)
+        r = torch.where(pat, torch.full((self.Hq,), self.retention, device=self.device),
+                        torch.zeros(self.Hq, device=self.device)).float().contiguous()
+        return DecodeParams(self.Hq, r.data_ptr(), self.retention, self.k_max_static, self.num_sinks, self.window_pages,
+                            self.bucket, self.sm_scale, self.n_split), r
+
+
+class QuestDecodeInt4(_NativeSteps):
+    LAUNCHES = 4
+
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4,
                  window_pages: int = 2, head_pattern_layer: torch.Tensor | None = None,
                  q_dtype=torch.bfloat16, n_split: int | None = None):
@@ -74,45 +158,7 @@ class QuestDecodeInt4:
         self._prm = DecodeParams(
             self.Hq, self.retention_per_q.data_ptr() if self.retention_per_q is not None else None, self.retention,
             self.k_max_static, self.num_sinks, self.window_pages, self.bucket, self.sm_scale, self.n_split)
-
-    def params_for(self, head_pattern_layer: torch.Tensor):
-        """fq_decode_params of one layer whose retrieval / streaming KV heads are given by
-        head_pattern_layer (H_kv,) bool: retrieval heads keep `retention`, streaming heads 0
-        (eager/llama_persistent_patch.py:214-219).  Returns (struct, tensor kept alive by the caller)."""
-        n_rep = self.Hq // self.Hkv
-        pat = head_pattern_layer.to(self.device).bool().repeat_interleave(n_rep)
-        r = torch.where(pat, torch.full((self.Hq,), self.retention, device=self.device),
-                        torch.zeros(self.Hq, device=self.device)).float().contiguous()
-        return DecodeParams(self.Hq, r.data_ptr(), self.retention, self.k_max_static, self.num_sinks, self.window_pages,
-                            self.bucket, self.sm_scale, self.n_split), r
-
-    def step(self, k_new: torch.Tensor, v_new: torch.Tensor, q: torch.Tensor, layer_idx: int, prm=None):
-        """Append k_new, v_new (B,H_kv,n,D) to the layer and attend with q (B,H_q,1,D) in ONE
-        foreign call (fq_decode_layer_int4): what cache.update_quantized followed by attend()
-        does, without the per-call slicing.  Tensors must have the cache's dtype.  `prm`: a
-        per-layer fq_decode_params (params_for) instead of the engine's own."""
-        c = self.cache
-        if layer_idx < 0 or layer_idx >= c.num_layers:
-            raise IndexError(f"layer_idx {layer_idx} out of range [0, {c.num_layers})")
-        seen = c._seen_tokens[layer_idx]
-        n_new = k_new.shape[2]
-        if seen + n_new > c.max_seq_len:
-            raise RuntimeError(f"PersistentInt4KVCache: seen+new={seen + n_new} exceeds max_seq_len={c.max_seq_len}")
-        if k_new.dtype != c.dtype or v_new.dtype != c.dtype:
-            k_new, v_new = k_new.to(c.dtype), v_new.to(c.dtype)
-        if k_new.stride(3) != 1 or v_new.stride() != k_new.stride():
-            k_new, v_new = k_new.contiguous(), v_new.contiguous()
-        q3 = q.reshape(self.B, self.Hq, self.D)
-        O, lse = self.O[layer_idx], self.lse[layer_idx]
-        check(lib().fq_decode_layer_int4(
-            ctypes.byref(self._cdesc), layer_idx, seen,
-            ptr(k_new), ptr(v_new), k_new.stride(0), k_new.stride(1), k_new.stride(2), n_new,
-            ptr(q3), dtype_code(q3), q3.stride(0), q3.stride(1), ctypes.byref(prm if prm is not None else self._prm),
-            ptr(self.scores[layer_idx]), ptr(self.compact[layer_idx]), ptr(O), ptr(lse),
-            ptr(self.workspace[layer_idx]), self.workspace.shape[1], stream_ptr(self.device)))
-        c._seen_tokens[layer_idx] = seen + n_new
-        self.launches += 4
-        return O.unsqueeze(2), lse.unsqueeze(2)
+        self._build_plan(4, self.scores, self.compact, self.workspace)
 
     def step_all(self, k_new: torch.Tensor, v_new: torch.Tensor, q: torch.Tensor):
         """step() for every layer in ONE foreign call (fq_decode_step_int4): k_new, v_new
@@ -240,12 +286,13 @@ class QuestDecodeInt4:
         return O.unsqueeze(2), lse.unsqueeze(2)
 
 
-class QuestDecodeTurbo:
+class QuestDecodeTurbo(_NativeSteps):
     """Decode-branch dispatcher for the persistent TurboQuant (K3-V3) cache: the kv_bits == 3 route of
     make_quest_persistent_forward (flashquest/eager/llama_persistent_patch.py:93-115,202-245) as ONE
     foreign call per layer (fq_decode_layer_turbo): append, page scores from the raw page metadata,
     top-k + compact index, rotation of Q, sparse attention in the rotated basis, rotation of O, tail
     attention and LSE merge.  All buffers are preallocated."""
+    LAUNCHES = 10
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,
                  q_dtype=torch.bfloat16, n_split: int | None = None):
@@ -287,30 +334,43 @@ class QuestDecodeTurbo:
         self._prm = DecodeParams(self.Hq, None, self.retention, self.k_max_static, self.num_sinks, self.window_pages,
                                  self.bucket, self.sm_scale, self.n_split)
         self.launches = 0
+        self._build_plan(3, self.scores, self.compact, self.workspace, self.scratch)
 
-    params_for = QuestDecodeInt4.params_for
 
-    def step(self, k_new: torch.Tensor, v_new: torch.Tensor, q: torch.Tensor, layer_idx: int, prm=None):
-        """Append k_new, v_new (B,H_kv,n,D) and attend with q (B,H_q,1,D) (raw basis): (O (B,H_q,1,D), lse (B,H_q,1))."""
-        c = self.cache
-        if layer_idx < 0 or layer_idx >= c.num_layers:
-            raise IndexError(f"layer_idx {layer_idx} out of range [0, {c.num_layers})")
-        seen = c._seen_tokens[layer_idx]
-        n_new = k_new.shape[2]
-        if seen + n_new > c.max_seq_len:
-            raise RuntimeError(f"PersistentTurboKVCache: seen+new={seen + n_new} exceeds max_seq_len={c.max_seq_len}")
-        if k_new.dtype != c.dtype or v_new.dtype != c.dtype:
-            k_new, v_new = k_new.to(c.dtype), v_new.to(c.dtype)
-        if k_new.stride(3) != 1 or v_new.stride() != k_new.stride():
-            k_new, v_new = k_new.contiguous(), v_new.contiguous()
-        q3 = q.reshape(self.B, self.Hq, self.D).contiguous()
-        O, lse = self.O[layer_idx], self.lse[layer_idx]
-        check(lib().fq_decode_layer_turbo(
-            ctypes.byref(self._cdesc), layer_idx, seen,
-            ptr(k_new), ptr(v_new), k_new.stride(0), k_new.stride(1), k_new.stride(2), n_new,
-            ptr(q3), dtype_code(q3), q3.stride(0), q3.stride(1), ctypes.byref(prm if prm is not None else self._prm),
-            ptr(self.scores), ptr(self.compact), ptr(self.scratch), self.scratch.numel(), ptr(O), ptr(lse),
-            ptr(self.workspace), self.workspace.numel(), stream_ptr(self.device)))
-        c._seen_tokens[layer_idx] = seen + n_new
-        self.launches += 10
-        return O.unsqueeze(2), lse.unsqueeze(2)
+class QuestDecodeInt8(_NativeSteps):
+    """Decode-branch dispatcher for the persistent INT8 cache: the kv_bits == 8 route of make_quest_persistent_forward
+    (flashquest/eager/llama_persistent_patch.py:202-245) as ONE foreign call per layer (fq_decode_layer_int8): append, page
+    scores, top-k with compact index, attention with the staged tail in the same softmax."""
+    LAUNCHES = 5
+
+    def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,
+                 q_dtype=torch.bfloat16, n_split: int | None = None):
+        if getattr(cache, "kv_bits", None) != 8:
+            raise NotImplementedError(f"QuestDecodeInt8 only supports kv_bits=8; got {getattr(cache, 'kv_bits', None)}")
+        if not (0.0 <= float(retention) <= 1.0):
+            raise ValueError(f"scalar retention must be in [0, 1]; got {retention}")
+        self.cache = cache
+        self.Hq, self.Hkv = num_q_heads, cache.num_kv_heads
+        if self.Hq % self.Hkv != 0:
+            raise ValueError(f"H_q={self.Hq} must be divisible by H_kv={self.Hkv}")
+        self.D, self.page, self.B = cache.head_dim, cache.page_size, cache.batch_size
+        self.retention, self.num_sinks, self.window_pages = float(retention), int(num_sinks), int(window_pages)
+        P_max = cache.max_seq_len // self.page
+        self.k_max_static = math.ceil(self.retention * P_max)
+        self.bucket = max(1, self.k_max_static + self.num_sinks + self.window_pages)
+        dev = cache.K_uint8.device
+        self.device, self.q_dtype = dev, q_dtype
+        self.sm_scale = 1.0 / math.sqrt(self.D)
+        self.scores = torch.empty(self.B, self.Hq, max(P_max, 1), dtype=torch.float32, device=dev)
+        self.compact = torch.empty(self.B, self.Hq, self.bucket, dtype=torch.int32, device=dev)
+        self.O = torch.empty(cache.num_layers, self.B, self.Hq, self.D, dtype=q_dtype, device=dev)
+        self.lse = torch.empty(cache.num_layers, self.B, self.Hq, dtype=torch.float32, device=dev)
+        # a warp should walk six pages at least, and about sixteen 128-thread CTAs per SM fill the GPU
+        self.n_split = n_split or max(1, min(64, self.bucket // 24, (16 * 148) // (self.B * self.Hq)))
+        self.workspace = torch.empty(lib().fq_sparse_decode_int8_workspace_bytes(self.B, self.Hq, self.D, self.n_split),
+                                     dtype=torch.uint8, device=dev)
+        self._cdesc = cache.desc()
+        self._prm = DecodeParams(self.Hq, None, self.retention, self.k_max_static, self.num_sinks, self.window_pages,
+                                 self.bucket, self.sm_scale, self.n_split)
+        self.launches = 0
+        self._build_plan(8, self.scores, self.compact, self.workspace)

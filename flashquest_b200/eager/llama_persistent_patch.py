@@ -10,11 +10,11 @@ embedding, appends k/v to the persistent cache and attends:
   * decode (S_q == 1, reference :202-245): page scores from the quantised metadata, static-k_max
     top-k with per-head retention from the head pattern, sparse attention over the selected
     pages, tail attention over the staged tokens and the LSE merge.
-      kv_bits == 4 or 8, use_compact_kernel=False: the reference's own sequence of steps — bool
-        mask, sparse kernel, separate tail attention, two-way merge of bf16 partial results;
-      kv_bits == 4, use_compact_kernel=True: ONE foreign call per layer (fq_decode_layer_int4:
-        append + scores + top-k with compact index + attention with the tail in the same softmax);
-      kv_bits == 3: ONE foreign call per layer (fq_decode_layer_turbo).
+    The whole branch is ONE foreign call per layer and token for every kv_bits: rotary embedding, append, scores,
+    top-k with compact index, attention with the tail in the same fp32 softmax (Turbo: tail attention and merge apart).
+    use_compact_kernel=False selects the same pages and differs from the reference's mask sequence only in that the
+    partial results are never rounded to bf16.  An INT8 cache whose pages the one-launch append does not take (page
+    size other than 16, 32, 64) runs the reference's own sequence: bool mask, sparse kernel, tail attention, merge.
     An empty cache (no completed page) and a cache without tail take the reference's branches
     (:206-209, :236-237).
 """
@@ -30,9 +30,8 @@ from ..kernel.kv_quant import (dequantize_k, dequantize_k_int4, dequantize_k_tur
                                dequantize_v_turbo)
 from ..kernel.prefill_attn import prefill_causal_attention
 from ..kernel.sparse_fwd import flash_attn_sparse_fwd
-from ..kernel.sparse_int4_fwd import flash_attn_sparse_int4_fwd
-from .criticality import page_scores_int4_fast, page_scores_int8_fast
-from .decode_step import QuestDecodeInt4, QuestDecodeTurbo
+from .criticality import page_scores_int8_fast
+from .decode_step import QuestDecodeInt4, QuestDecodeInt8, QuestDecodeTurbo
 from .selection import select_pages_vectorized
 from .tail_merge import _bf16_dense_attn_with_lse, _merge_two_attentions
 
@@ -47,7 +46,7 @@ def _engine(cache, kind, num_q_heads, retention, num_sinks, window_pages):
     key = (kind, num_q_heads, float(retention), int(num_sinks), int(window_pages))
     store = cache.__dict__.setdefault("_fq_engines", {})
     if key not in store:
-        cls = QuestDecodeInt4 if kind == 4 else QuestDecodeTurbo
+        cls = {3: QuestDecodeTurbo, 4: QuestDecodeInt4, 8: QuestDecodeInt8}[kind]
         store[key] = cls(cache, num_q_heads=num_q_heads, retention=retention, num_sinks=num_sinks,
                          window_pages=window_pages, q_dtype=cache.dtype)
     return store[key]
@@ -102,12 +101,18 @@ def make_quest_persistent_forward(
         raise ValueError(f"unsupported cache.kv_bits={kv_bits!r}")
     if page_size != cache.page_size:
         raise ValueError(f"page_size={page_size} differs from the cache's page_size={cache.page_size}")
-    state = {}       # per-layer fq_decode_params (+ the retention tensor it points to), built on first use
+    # The native decode route (one foreign call per token and layer).  With use_compact_kernel=False it computes the same
+    # selection as the reference's mask sequence and attends the staged tail in the same fp32 softmax.  An INT8 cache
+    # outside the one-launch append keeps the reference's own sequence of steps below.
+    native = kv_bits in (3, 4) or cache._one_launch
+    state = {}       # H_q -> (engine, fq_decode_params, the retention tensor it points to), built on first use
 
-    def _layer_params(engine, device):
-        if "prm" not in state:
-            state["prm"] = engine.params_for(head_pattern_layer.to(device))
-        return state["prm"][0]
+    def _native(H_q, device):
+        got = state.get(H_q)
+        if got is None:
+            engine = _engine(cache, kv_bits, H_q, retention, num_sinks, window_pages)
+            got = state[H_q] = (engine,) + engine.params_for(head_pattern_layer.to(device))
+        return got
 
     def forward(
         self,
@@ -120,23 +125,36 @@ def make_quest_persistent_forward(
     ) -> tuple[torch.Tensor, Optional[torch.Tensor]]:
         input_shape = hidden_states.shape[:-1]
         hidden_shape = (*input_shape, -1, self.head_dim)
+        li = self.layer_idx
 
-        q = self.q_proj(hidden_states).view(hidden_shape).transpose(1, 2)
-        k = self.k_proj(hidden_states).view(hidden_shape).transpose(1, 2)
-        v = self.v_proj(hidden_states).view(hidden_shape).transpose(1, 2)
+        q, k, v = self.q_proj(hidden_states), self.k_proj(hidden_states), self.v_proj(hidden_states)
+        model_dtype = q.dtype
+        if native and len(input_shape) == 2 and input_shape[1] == 1:
+            engine, prm, _ = _native(q.shape[-1] // head_dim, q.device)
+            cos, sin = position_embeddings
+            O = engine.forward_token(q, k, v, cos, sin, li, prm=prm)
+            if O is not None:
+                if TRACE is not None:
+                    TRACE(li, engine.q_rot, engine.k_rot, engine.v_rot, O)
+                attn_output = O.view(*input_shape, -1)
+                if O.dtype != model_dtype:
+                    attn_output = attn_output.to(model_dtype)
+                return self.o_proj(attn_output), None
+
+        q = q.view(hidden_shape).transpose(1, 2)
+        k = k.view(hidden_shape).transpose(1, 2)
+        v = v.view(hidden_shape).transpose(1, 2)
 
         cos, sin = position_embeddings
         q, k = apply_rotary_pos_emb(q, k, cos, sin)
 
         # the kernels and the cache work in the cache's staging dtype (bf16 in the reference);
         # AWQ models are fp16: cast in, cast back before o_proj (reference :182-190)
-        model_dtype = q.dtype
-        if model_dtype != cache.dtype:
+        if q.dtype != cache.dtype:
             q, k, v = q.to(cache.dtype), k.to(cache.dtype), v.to(cache.dtype)
 
         S_q = q.shape[2]
         H_q = q.shape[1]
-        li = self.layer_idx
 
         if S_q > 1:
             cache.update_quantized(k, v, layer_idx=li)
@@ -150,9 +168,9 @@ def make_quest_persistent_forward(
             attn_output = prefill_causal_attention(q, K_full, V_full, out_bshd=True)            # (B,S_q,H_q,D)
             if TRACE is not None:
                 attn_bhsd = attn_output.transpose(1, 2)
-        elif kv_bits == 3 or use_compact_kernel:
-            engine = _engine(cache, kv_bits, H_q, retention, num_sinks, window_pages)
-            O, _ = engine.step(k, v, q, li, prm=_layer_params(engine, q.device))
+        elif native:
+            engine, prm, _ = _native(H_q, q.device)
+            O, _ = engine.step(k, v, q, li, prm=prm)
             attn_bhsd = O
             attn_output = O.transpose(1, 2)
         else:
@@ -171,20 +189,13 @@ def make_quest_persistent_forward(
                     torch.full((H_q,), retention, device=q.device),
                     torch.zeros(H_q, device=q.device),
                 )
-                score_fn = page_scores_int4_fast if kv_bits == 4 else page_scores_int8_fast
-                scores = score_fn(q, views["K_scale"], views["K_mn"])
+                scores = page_scores_int8_fast(q, views["K_scale"], views["K_mn"])
                 sel = select_pages_vectorized(scores, retention=retention_per_q, num_sinks=num_sinks,
                                               window_pages=window_pages, k_max_static=k_max_static)
-                if kv_bits == 4:
-                    O_sparse, lse_sparse = flash_attn_sparse_int4_fwd(
-                        q, views["K_packed"], views["K_scale"], views["K_mn"],
-                        views["V_packed"], views["V_scale"], views["V_mn"],
-                        selection_mask=sel, page_size=page_size, return_lse=True)
-                else:
-                    O_sparse, lse_sparse = flash_attn_sparse_fwd(
-                        q, views["K_uint8"], views["K_scale"], views["K_mn"],
-                        views["V_uint8"], views["V_scale"], views["V_mn"],
-                        selection_mask=sel, page_size=page_size, return_lse=True)
+                O_sparse, lse_sparse = flash_attn_sparse_fwd(
+                    q, views["K_uint8"], views["K_scale"], views["K_mn"],
+                    views["V_uint8"], views["V_scale"], views["V_mn"],
+                    selection_mask=sel, page_size=page_size, return_lse=True)
                 if partial_len == 0:
                     attn_bhsd = O_sparse
                 else:

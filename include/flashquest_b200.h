@@ -538,6 +538,27 @@ int fq_decode_layer_int4(
     float* scores, int32_t* compact, void* O, float* lse,
     void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same for an INT8 cache: the fq_int4_cache record with code rows of D bytes.  scores / compact / O / lse as above;
+ * workspace of fq_sparse_decode_int8_workspace_bytes(B, Hq, D, params->n_split) bytes, n_split >= 1.  The append takes
+ * head_dim 64 or 128 and pages of 16, 32 or 64 tokens (FQ_ERR_UNSUPPORTED otherwise); fq_append_kv_int8 is that append
+ * alone (persistent_int8.py:72-141), any number of tokens. */
+int fq_append_kv_int8(const fq_int4_cache* cache, int layer, int seen, const void* K_new, const void* V_new,
+                      int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new, void* stream);
+int fq_decode_layer_int8(
+    const fq_int4_cache* cache, int layer, int seen,
+    const void* K_new, const void* V_new, int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new,
+    const void* Q, int q_dtype, int64_t q_sb, int64_t q_sh,
+    const fq_decode_params* params,
+    float* scores, int32_t* compact, void* O, float* lse,
+    void* workspace, size_t workspace_bytes, void* stream);
+
+/* Rotary embedding of one new token as Hugging Face's apply_rotary_pos_emb computes it (x*cos + rotate_half(x)*sin, each
+ * product and the sum rounded to `dtype`), then cast to out_dtype; v is only cast.  q (B,Hq*D), k, v (B,Hkv*D) with batch
+ * strides, cos, sin (B,D) with batch strides (0: shared); outputs dense.  D even, at most 128; fp16 / bf16. */
+int fq_rope_qkv(const void* q, int64_t q_sb, const void* k, int64_t k_sb, const void* v, int64_t v_sb, int dtype,
+                const void* cosv, int64_t cos_sb, const void* sinv, int64_t sin_sb, int B, int Hq, int Hkv, int D,
+                void* q_out, void* k_out, void* v_out, int out_dtype, void* stream);
+
 /* One decode step of one layer on a persistent TurboQuant K3-V3 cache, in one host call: what the
  * reference's patched forward does for cache.kv_bits == 3 (eager/llama_persistent_patch.py:93-115,
  * 193-245): PersistentTurboKVCache.update_quantized (cache/persistent_turbo.py:83-147),

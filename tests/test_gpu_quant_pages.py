@@ -1,0 +1,71 @@
+"""Bulk packing kernel (csrc/fq_quant_pages.cu) against the CPU oracle, bit for bit: every page size, head dimension and code
+width it takes, staged heads, left-over tokens, values on rounding ties, constant and extreme rows."""
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(B, H, S, D, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(B, H, S, D, generator=g)
+    x[..., 5:: D // 4] *= 8
+    x[:, :, 3] = 0.25                                                     # a constant row
+    x[:, :, : S // 2, 7] = torch.arange(S // 2) % 16 * 0.5 - 2             # quotients on and next to half-integers
+    x[:, :, 6] = torch.linspace(-7.5, 7.5, D)
+    x[:, :, 9] *= 1e-6
+    x[:, :, 11] *= 3e3
+    return x.to(dtype)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("page", [16, 32, 64])
+@pytest.mark.parametrize("D,dtype,B,S,first", [(128, torch.float16, 2, 64 * 3 + 5, 0), (128, torch.bfloat16, 1, 64 * 5, 13),
+                                              (64, torch.bfloat16, 2, 64 * 2 + 63, 7), (64, torch.float16, 1, 64, 15)])
+def test_bulk_append_matches_oracle(bits, page, D, dtype, B, S, first):
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    H = 3
+    K, V = _data(B, H, S, D, dtype, 1), _data(B, H, S, D, dtype, 2)
+    cache = (PersistentInt4KVCache if bits == 4 else PersistentInt8KVCache)(
+        batch_size=B, num_layers=2, num_kv_heads=H, head_dim=D, max_seq_len=S + page, page_size=page, dtype=dtype)
+    if first:                                                              # a staged head in front of the bulk
+        cache.update_quantized(K[:, :, :first].cuda(), V[:, :, :first].cuda(), 1)
+    cache.update_quantized(K[:, :, first:].cuda(), V[:, :, first:].cuda(), 1)
+    n = S // page * page
+    views = cache.get_views(1)
+    qk, qv = (oracle.quantize_k_int4, oracle.quantize_v_int4) if bits == 4 else (oracle.quantize_k, oracle.quantize_v)
+    names = ("K_packed", "V_packed") if bits == 4 else ("K_uint8", "V_uint8")
+    for got, want in zip((views[names[0]], views["K_scale"], views["K_mn"]), qk(K[:, :, :n], page)):
+        assert torch.equal(got.cpu(), want)
+    for got, want in zip((views[names[1]], views["V_scale"], views["V_mn"]), qv(V[:, :, :n])):
+        assert torch.equal(got.cpu(), want)
+    assert torch.equal(views["K_partial"].cpu(), K[:, :, n:]) and torch.equal(views["V_partial"].cpu(), V[:, :, n:])
+    if bits == 8:
+        assert not cache.K_partial[1, :, :, S - n:].any() and not cache.V_partial[1, :, :, S - n:].any()
+
+
+@pytest.mark.parametrize("model,stage", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.bfloat16), (torch.float16, torch.float16)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_rope_of_the_patched_forward_matches_hugging_face(model, stage, D):
+    """q, k, v that go into the cache: the bits of apply_rotary_pos_emb followed by the cast."""
+    from transformers.models.llama.modeling_llama import apply_rotary_pos_emb
+
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.eager.decode_step import QuestDecodeInt8
+    B, Hq, Hkv = 3, 6, 2
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).to(model)
+    cache = PersistentInt8KVCache(batch_size=B, num_layers=1, num_kv_heads=Hkv, head_dim=D, max_seq_len=64, page_size=16, dtype=stage)
+    engine = QuestDecodeInt8(cache, num_q_heads=Hq, q_dtype=stage)
+    q, k, v, cos, sin = r(B, 1, Hq * D), r(B, 1, Hkv * D), r(B, 1, Hkv * D), r(B, 1, D), r(B, 1, D)
+    O = engine.forward_token(q, k, v, cos, sin, 0)
+    want_q, want_k = apply_rotary_pos_emb(q.view(B, 1, Hq, D).transpose(1, 2), k.view(B, 1, Hkv, D).transpose(1, 2), cos, sin)
+    assert torch.equal(engine.q_rot, want_q.to(stage)) and torch.equal(engine.k_rot, want_k.to(stage))
+    want_v = v.view(B, 1, Hkv, D).transpose(1, 2).to(stage)
+    assert torch.equal(cache.K_partial[0, :, :, :1], want_k.to(stage)) and torch.equal(cache.V_partial[0, :, :, :1], want_v)
+    # one staged token: its value is the output
+    assert torch.allclose(O.float(), want_v.float().repeat_interleave(Hq // Hkv, 1), atol=1e-3)
+    assert cache.get_seq_length() == 1
