@@ -100,6 +100,8 @@ class LlamaScratchDesc(ctypes.Structure):
 
 _PROTOTYPES["fq_llama_decode_step"] = (I, [ctypes.POINTER(LlamaModelDesc), ctypes.POINTER(Int4CacheDesc),
                                           ctypes.POINTER(DecodeParams), P, P, I, ctypes.POINTER(LlamaScratchDesc), P])
+_PROTOTYPES["fq_llama_prefill_workspace_bytes"] = (Z, [ctypes.POINTER(LlamaModelDesc), I])
+_PROTOTYPES["fq_llama_prefill"] = (I, [ctypes.POINTER(LlamaModelDesc), ctypes.POINTER(Int4CacheDesc), P, I, F, P, Z, P, P, P])
 _PROTOTYPES["fq_llama_decode_step_dev"] = _PROTOTYPES["fq_llama_decode_step"]
 
 

@@ -688,6 +688,14 @@ typedef struct fq_llama_scratch {
     void* attn_ws; size_t attn_ws_sl, attn_ws_bytes;   /* per layer split-K scratch of the attention, tickets zero */
 } fq_llama_scratch;
 
+/* Prefill of ONE prompt of S tokens into an empty cache (B == 1) in one call: add+RMSNorm -> q/k/v -> rotary embedding ->
+ * bulk INT4 append -> dense causal attention over the dequantised pages and the staged tail -> o -> add+RMSNorm ->
+ * gate/up -> SwiGLU -> down per layer; after the last layer's attention only the last token: final norm, lm_head, argmax.
+ * x (S,hidden) fp16: the embedded prompt.  workspace: 256-byte aligned, fq_llama_prefill_workspace_bytes(model, S). */
+size_t fq_llama_prefill_workspace_bytes(const fq_llama_model* model, int S);
+int fq_llama_prefill(const fq_llama_model* model, const fq_int4_cache* cache, const void* x, int S, float sm_scale,
+                     void* workspace, size_t workspace_bytes, void* logits, int32_t* next_id, void* stream);
+
 /* x (B, hidden) fp16: the embedding rows of this step's tokens; seen[layer] tokens already cached
  * (all sequences of the batch are at the same position).  Writes scratch->logits and next_ids. */
 int fq_llama_decode_step(const fq_llama_model* model, const fq_int4_cache* cache, const fq_decode_params* params,
