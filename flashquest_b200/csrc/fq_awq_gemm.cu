@@ -23,7 +23,7 @@
 // word instead of spinning forever.
 #include <cuda.h>
 
-#include "fq_common.cuh"
+#include "fq_awq_skinny.cuh"
 
 namespace fq {
 
@@ -379,6 +379,14 @@ extern "C" int fq_awq_gemm(
     FQ_CHECK_ARG(n_proj >= 1 && n_proj <= GM_MAX_PROJ, FQ_ERR_ARG, "%s: 1..%d projections per call, got %d", fn, GM_MAX_PROJ, n_proj);
     FQ_CHECK_ARG(x && qweight && scales && qzeros && N && y, FQ_ERR_ARG, "%s: null pointer", fn);
     FQ_CHECK_ARG(aligned(x, 16), FQ_ERR_ALIGN, "%s: x must be 16-byte aligned", fn);
+    if (M <= 1024) {
+        SkinnyCall c{};
+        c.x = x; c.M = M; c.K = K; c.group = group; c.n_proj = n_proj; c.interleaved = interleaved ? 1 : 0;
+        for (int i = 0; i < n_proj; ++i) {
+            c.qweight[i] = qweight[i]; c.scales[i] = scales[i]; c.qzeros[i] = qzeros[i]; c.bias[i] = bias ? bias[i] : nullptr; c.N[i] = N[i]; c.y[i] = y[i];
+        }
+        if (awq_skinny_supported(c)) return awq_skinny_launch(c, stream, fn);
+    }
     EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) return fail(FQ_ERR_CUDA, "%s: the driver does not export cuTensorMapEncodeTiled", fn);
     GemmParams p{};
