@@ -32,6 +32,7 @@ constexpr int GM_BN = 256;          // columns per tile: one MMA of N = 256 per 
 constexpr int GM_BK = 64;
 constexpr int GM_TMEM_COLS = 512;   // all of an SM's tensor memory: MT = 1: two accumulator sets, MT = 2: one
 constexpr int GM_DEQ_WARPS = 8;
+constexpr int GM_DEQ_GROUP = 4;     // warps that convert one k block
 constexpr int GM_EPI_WARPS = 4;
 constexpr int GM_THREADS = (2 + GM_DEQ_WARPS + GM_EPI_WARPS) * 32;     // TMA warp, MMA warp, dequantise warps, epilogue warps
 
@@ -40,15 +41,19 @@ constexpr unsigned GM_SPIN_LIMIT = 1u << 26;
 constexpr int GM_A_BYTES = GM_BM * GM_BK * 2;             // 16 KiB per M tile
 constexpr int GM_RAW_BYTES = GM_BK * (GM_BN / 8) * 4;     // 8 KiB
 constexpr int GM_B_BYTES = GM_BK * GM_BN * 2;             // 32 KiB
-// MT = accumulators (M tiles of 128 rows) per CTA tile.  MT = 2 (256 x 256 tiles, 3 stages): every byte fetched from L2
-// feeds twice the MMAs, the tile for long M; MT = 1 (128 x 256 tiles, 4 stages, two accumulator sets so that a
+// MT = accumulators (M tiles of 128 rows) per CTA tile.  MT = 2 (256 x 256 tiles): every byte fetched from L2
+// feeds twice the MMAs, the tile for long M; MT = 1 (128 x 256 tiles, two accumulator sets so that a
 // finished tile is drained while the next one is multiplied): more tiles, the one for short M.
 template <int MT> struct GmCfg {
-    static constexpr int STAGES = MT == 2 ? 3 : 4;
+    // a ring for each kind of data, as deep as its latency asks: x tiles and raw codes come about 1 us after their request,
+    // a dequantised tile only has to bridge the MMAs of one block
+    static constexpr int X_STAGES = MT == 2 ? 3 : 4;
+    static constexpr int B_STAGES = MT == 2 ? 2 : 3;
+    static constexpr int RAW_STAGES = MT == 2 ? 4 : 6;
     static constexpr int ACC_SETS = GM_TMEM_COLS / (MT * GM_BN);
-    static constexpr int STAGE_BYTES = MT * GM_A_BYTES + GM_B_BYTES + GM_RAW_BYTES;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers, tmem address */;
-    static_assert((3 * STAGES + 2 * ACC_SETS) * 8 + 4 <= 256, "barrier block");
+    static constexpr int X_BYTES = MT * GM_A_BYTES;
+    static constexpr int SMEM = X_STAGES * X_BYTES + B_STAGES * GM_B_BYTES + RAW_STAGES * GM_RAW_BYTES + 1024 /* alignment slack */ + 256 /* barriers, tmem address */;
+    static_assert((2 * (X_STAGES + B_STAGES + RAW_STAGES) + 2 * ACC_SETS) * 8 + 4 <= 256, "barrier block");
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
 
@@ -87,6 +92,13 @@ __device__ __forceinline__ bool gm_wait(uint64_t* bar, unsigned parity) {
     }
     return true;
 }
+// the same for a whole warp; true = gave up
+__device__ __forceinline__ bool gm_timeout(uint64_t* bar, unsigned parity) { return __any_sync(0xffffffffu, !gm_wait(bar, parity)); }
+__device__ __forceinline__ bool gm_elect() {
+    uint32_t pred;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+    return pred != 0;
+}
 __device__ __forceinline__ void gm_tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(gm_smem(dst)), "l"(map), "r"(gm_smem(bar)), "r"(x), "r"(y) : "memory");
@@ -110,28 +122,32 @@ template <bool INTERLEAVED, int GM_MT>
 __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
     const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
     const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_w3, const GemmParams p) {
-    constexpr int GM_STAGES = GmCfg<GM_MT>::STAGES, GM_ACC_SETS = GmCfg<GM_MT>::ACC_SETS, GM_STAGE_BYTES = GmCfg<GM_MT>::STAGE_BYTES;
+    using C = GmCfg<GM_MT>;
+    constexpr int GM_ACC_SETS = C::ACC_SETS, XS = C::X_STAGES, BS = C::B_STAGES, RS = C::RAW_STAGES;
     extern __shared__ unsigned char gm_raw_smem[];
-    // stage s: [A tiles | B (dequantised) | raw codes]; every tile 1024-byte aligned
+    // x tiles | dequantised weights | raw codes; every tile 1024-byte aligned
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gm_raw_smem) + 1023) & ~(uintptr_t)1023);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(base + GM_STAGES * GM_STAGE_BYTES);
-    uint64_t* full_raw = bars;                       // [stages] TMA bytes landed (x tiles + raw codes)
-    uint64_t* b_ready = bars + GM_STAGES;            // [stages] dequantised tile written (256 arrivals)
-    uint64_t* empty = bars + 2 * GM_STAGES;          // [stages] the MMAs that read the stage have completed
-    uint64_t* acc_ready = bars + 3 * GM_STAGES;      // [sets] all MMAs of a tile have completed
+    unsigned char* sX = base;
+    unsigned char* sB = sX + XS * C::X_BYTES;
+    unsigned char* sRaw = sB + BS * GM_B_BYTES;
+    uint64_t* x_full = reinterpret_cast<uint64_t*>(sRaw + RS * GM_RAW_BYTES);
+    uint64_t* x_empty = x_full + XS;                 // [x stages] the MMAs that read the tile have completed
+    uint64_t* raw_full = x_empty + XS;
+    uint64_t* raw_empty = raw_full + RS;             // [raw stages] read by the four warps of its group
+    uint64_t* b_ready = raw_empty + RS;              // [B stages] dequantised tile written
+    uint64_t* b_empty = b_ready + BS;
+    uint64_t* acc_ready = b_empty + BS;              // [sets] all MMAs of a tile have completed
     uint64_t* acc_empty = acc_ready + GM_ACC_SETS;   // [sets] the epilogue has drained the set (128 arrivals)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + GM_ACC_SETS);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int num_kb = p.K / GM_BK;
     const int total_tiles = p.n_tiles * p.m_tiles;
 
     if (tid == 0) {
-        for (int s = 0; s < GM_STAGES; ++s) {
-            gm_mbar_init(&full_raw[s], 1);
-            gm_mbar_init(&b_ready[s], GM_DEQ_WARPS * 32);
-            gm_mbar_init(&empty[s], 1);
-        }
+        for (int s = 0; s < XS; ++s) { gm_mbar_init(&x_full[s], 1); gm_mbar_init(&x_empty[s], 1); }
+        for (int s = 0; s < RS; ++s) { gm_mbar_init(&raw_full[s], 1); gm_mbar_init(&raw_empty[s], GM_DEQ_GROUP); }
+        for (int s = 0; s < BS; ++s) { gm_mbar_init(&b_ready[s], GM_DEQ_GROUP); gm_mbar_init(&b_empty[s], 1); }
         for (int a = 0; a < GM_ACC_SETS; ++a) {
             gm_mbar_init(&acc_ready[a], 1);
             gm_mbar_init(&acc_empty[a], GM_EPI_WARPS * 32);
@@ -159,135 +175,160 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
         m0 = (tile / p.n_tiles) * (GM_BM * GM_MT);
     };
 
+    // The producer and issuer warps walk their loops as whole warps and one elected lane issues: operands that are
+    // uniform over the warp then stay in uniform registers (inside a branch on lane == 0 an MMA issue took 90 cycles).
     if (warp == 0) {
         // =========================== TMA producer ===========================
-        if (lane == 0) {
-            int g = 0;                                  // k blocks issued so far, over all tiles
-            for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
-                int pj, n0, m0;
-                locate(tile, pj, n0, m0);
-                const CUtensorMap* map_w = pj == 0 ? &map_w0 : (pj == 1 ? &map_w1 : (pj == 2 ? &map_w2 : &map_w3));
-                for (int kb = 0; kb < num_kb; ++kb, ++g) {
-                    const int s = g % GM_STAGES;
-                    if (g >= GM_STAGES && !gm_wait(&empty[s], (unsigned)(g / GM_STAGES - 1) & 1u)) { failed = true; break; }
-                    unsigned char* st = base + s * GM_STAGE_BYTES;
-                    gm_mbar_expect_tx(&full_raw[s], GM_MT * GM_A_BYTES + GM_RAW_BYTES);
-#pragma unroll
-                    for (int mt = 0; mt < GM_MT; ++mt) gm_tma_2d(st + mt * GM_A_BYTES, &map_x, kb * GM_BK, m0 + mt * GM_BM, &full_raw[s]);
-                    gm_tma_2d(st + GM_MT * GM_A_BYTES + GM_B_BYTES, map_w, n0 / 8, kb * GM_BK, &full_raw[s]);
+        // raw codes run RS blocks ahead of the dequantisation, x tiles XS blocks ahead of the MMAs
+        const int my_tiles = total_tiles > (int)blockIdx.x ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+        const int blocks = my_tiles * num_kb;
+        int rt = blockIdx.x, rk = 0, xt = blockIdx.x, xk = 0;       // tile and k block of the next raw / x request
+        int rpj = 0, rn0 = 0, rm0 = 0, xpj = 0, xn0 = 0, xm0 = 0;
+        int rs = 0, xs = 0;
+        unsigned rph = 1u, xph = 1u;                                // the first pass finds every stage free
+        for (int g = 0, r = 0; g < blocks && !failed; ++g) {
+            for (; r < blocks && r < g + RS; ++r) {
+                if (rk == 0) locate(rt, rpj, rn0, rm0);
+                if (gm_timeout(&raw_empty[rs], rph)) { failed = true; break; }
+                const CUtensorMap* map_w = rpj == 0 ? &map_w0 : (rpj == 1 ? &map_w1 : (rpj == 2 ? &map_w2 : &map_w3));
+                if (gm_elect()) {
+                    gm_mbar_expect_tx(&raw_full[rs], GM_RAW_BYTES);
+                    gm_tma_2d(sRaw + rs * GM_RAW_BYTES, map_w, rn0 / 8, rk * GM_BK, &raw_full[rs]);
                 }
+                __syncwarp();
+                if (++rs == RS) { rs = 0; rph ^= 1u; }
+                if (++rk == num_kb) { rk = 0; rt += gridDim.x; }
+                if (r >= RS) { ++r; break; }                        // steady state: one raw request per x request
             }
+            if (failed) break;
+            if (xk == 0) locate(xt, xpj, xn0, xm0);
+            if (gm_timeout(&x_empty[xs], xph)) { failed = true; break; }
+            if (gm_elect()) {
+                gm_mbar_expect_tx(&x_full[xs], C::X_BYTES);
+#pragma unroll
+                for (int mt = 0; mt < GM_MT; ++mt) gm_tma_2d(sX + xs * C::X_BYTES + mt * GM_A_BYTES, &map_x, xk * GM_BK, xm0 + mt * GM_BM, &x_full[xs]);
+            }
+            __syncwarp();
+            if (++xs == XS) { xs = 0; xph ^= 1u; }
+            if (++xk == num_kb) { xk = 0; xt += gridDim.x; }
         }
     } else if (warp == 1) {
         // =========================== MMA issuer ===========================
-        if (lane == 0) {
-            // instruction descriptor: fp32 accumulate, fp16 A (K-major) and B (MN-major), N = 128, M = 128
-            const uint32_t idesc = (1u << 4) | (0u << 7) | (0u << 10) | (0u << 15) | (1u << 16) | ((uint32_t)(GM_BN >> 3) << 17) |
+        // instruction descriptor: fp32 accumulate, fp16 A (K-major) and B (MN-major), N = 256, M = 128
+        constexpr uint32_t idesc = (1u << 4) | (0u << 7) | (0u << 10) | (0u << 15) | (1u << 16) | ((uint32_t)(GM_BN >> 3) << 17) |
                                    ((uint32_t)(GM_BM >> 4) << 24);
-            int g = 0, it = 0;
-            for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++it) {
-                const int set = it % GM_ACC_SETS, use = it / GM_ACC_SETS;
-                // the set must have been drained by the epilogue of the tile that used it last
-                if (use >= 1 && !gm_wait(&acc_empty[set], (unsigned)(use - 1) & 1u)) { failed = true; break; }
+        // A: K-major; 8 rows x 64 k = one 1 KiB atom; 16 k = 32 B further inside the swizzled row.  B: MN-major; 64 columns x
+        // 8 k = one 1 KiB atom; atoms 1 KiB apart along K, BK*128 B apart along N (4 atoms)
+        const uint64_t da0 = gm_desc(gm_smem(sX), 16, 1024), db0 = gm_desc(gm_smem(sB), GM_BK * 128, 1024);
+        int g = 0, it = 0;
+        for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++it) {
+            const int set = it % GM_ACC_SETS, use = it / GM_ACC_SETS;
+            // the set must have been drained by the epilogue of the tile that used it last
+            if (use >= 1 && gm_timeout(&acc_empty[set], (unsigned)(use - 1) & 1u)) { failed = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem_base + (uint32_t)(set * GM_MT * GM_BN);
+            for (int kb = 0; kb < num_kb; ++kb, ++g) {
+                const int xs = g % XS, bs = g % BS;
+                if (gm_timeout(&x_full[xs], (unsigned)(g / XS) & 1u) || gm_timeout(&b_ready[bs], (unsigned)(g / BS) & 1u)) { failed = true; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem_base + (uint32_t)(set * GM_MT * GM_BN);
-                for (int kb = 0; kb < num_kb; ++kb, ++g) {
-                    const int s = g % GM_STAGES;
-                    const unsigned ph = (unsigned)(g / GM_STAGES) & 1u;
-                    if (!gm_wait(&full_raw[s], ph) || !gm_wait(&b_ready[s], ph)) { failed = true; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = gm_smem(base + s * GM_STAGE_BYTES);
-                    const uint32_t b_addr = a_addr + GM_MT * GM_A_BYTES;
+                const uint64_t da = da0 + (uint64_t)(xs * (C::X_BYTES >> 4)), db = db0 + (uint64_t)(bs * (GM_B_BYTES >> 4));
+                if (gm_elect()) {
 #pragma unroll
-                    for (int k = 0; k < GM_BK / 16; ++k) {
-                        // B: MN-major; 64 columns x 8 k = one 1 KiB atom; atoms 1 KiB apart along K, BK*128 B apart along N (4 atoms)
-                        const uint64_t db = gm_desc(b_addr + k * 2048, GM_BK * 128, 1024);
+                    for (int k = 0; k < GM_BK / 16; ++k)
 #pragma unroll
-                        for (int mt = 0; mt < GM_MT; ++mt) {
-                            // A: K-major; 8 rows x 64 k = one 1 KiB atom; 16 k = 32 B further inside the swizzled row
-                            const uint64_t da = gm_desc(a_addr + mt * GM_A_BYTES + k * 32, 16, 1024);
-                            gm_mma(acc + mt * GM_BN, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-                        }
-                    }
-                    gm_commit(&empty[s]);          // arrives when the MMAs issued so far have read their operands
+                        for (int mt = 0; mt < GM_MT; ++mt)
+                            gm_mma(acc + mt * GM_BN, da + mt * (GM_A_BYTES >> 4) + k * (32 >> 4), db + k * (2048 >> 4), idesc, (kb | k) != 0 ? 1u : 0u);
+                    gm_commit(&x_empty[xs]);           // arrive when the MMAs issued so far have read their operands
+                    gm_commit(&b_empty[bs]);
+                    if (kb + 1 == num_kb) gm_commit(&acc_ready[set]);
                 }
-                if (!failed) gm_commit(&acc_ready[set]);
+                __syncwarp();
             }
         }
     } else if (warp < 2 + GM_DEQ_WARPS) {
         // =========================== dequantise ===========================
-        const int t = tid - 64;                       // 0..255
+        // two groups of four warps alternate: one block is converted while the other's is multiplied
+        const int grp = (warp - 2) / GM_DEQ_GROUP;
+        const int t = (tid - 64) % (GM_DEQ_GROUP * 32);
         const int c = t & 31;                         // int32 column of the raw tile = 8 output columns n0 + 8c ..
-        const int kr0 = t >> 5;                       // first k row of this thread; it takes rows kr0 + 8 i
+        const int kr0 = t >> 5;                       // first k row of this thread; it takes rows kr0 + 4 i
         const int gpk = p.group / GM_BK;              // k blocks per quantisation group
-        uint32_t zsub[4];                             // (1024 + zero) for the four column pairs, half2 bits
-        __half2 sc2[4];                               // scales of the four column pairs
         const int a_n = c >> 3, chunk = c & 7;        // 64-column atom and 16-byte chunk inside its rows
-        const int n_grp = (num_kb + gpk - 1) / gpk;
-        int g = 0;
-        for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+        const __half2 sixteenth = __float2half2_rn(0.0625f);
+        // block g of this CTA = k block kb of tile `tile`; the scale and zero words of a group's next block are requested one
+        // block ahead, across tiles
+        int tile = blockIdx.x, kb = grp;
+        auto settle = [&]() { while (kb >= num_kb && tile < total_tiles) { kb -= num_kb; tile += gridDim.x; } };
+        auto load_meta = [&](uint32_t& zw, uint4& s4) {
+            zw = 0; s4 = make_uint4(0, 0, 0, 0);
+            if (tile >= total_tiles) return;
             int pj, n0, m0;
             locate(tile, pj, n0, m0);
             const GemmProj& P = p.proj[pj];
-            // scale and zero words of the NEXT group are requested one group ahead
-            const bool col_ok = n0 + 8 * c < P.N;      // a projection of 128 (mod 256) columns ends inside its last tile
-            auto load_meta = [&](int gi, uint32_t& zw, uint4& s4) {
-                zw = 0; s4 = make_uint4(0, 0, 0, 0);
-                if (col_ok) {
-                    zw = (uint32_t)__ldg(P.qzeros + (int64_t)gi * (P.N / 8) + n0 / 8 + c);
-                    s4 = __ldg(reinterpret_cast<const uint4*>(P.scales + (int64_t)gi * P.N + n0 + 8 * c));
+            const int gi = kb / gpk;
+            if (n0 + 8 * c < P.N) {                   // a projection of 128 (mod 256) columns ends inside its last tile
+                zw = (uint32_t)__ldg(P.qzeros + (int64_t)gi * (P.N / 8) + n0 / 8 + c);
+                s4 = __ldg(reinterpret_cast<const uint4*>(P.scales + (int64_t)gi * P.N + n0 + 8 * c));
+            }
+        };
+        uint32_t zw_nx;
+        uint4 s4_nx;
+        settle();
+        load_meta(zw_nx, s4_nx);
+        for (int g = grp; tile < total_tiles; g += GM_DEQ_WARPS / GM_DEQ_GROUP) {
+            const int bs = g % BS, rs = g % RS;
+            const uint32_t zw = zw_nx, sw[4] = {s4_nx.x, s4_nx.y, s4_nx.z, s4_nx.w};
+            kb += GM_DEQ_WARPS / GM_DEQ_GROUP;
+            settle();
+            load_meta(zw_nx, s4_nx);
+            // per column pair: even nibbles h = 1024 + code, minus (1024 + zero); odd ones h = 1024 + 16 code, times 1/16 minus
+            // (64 + zero): both exact; then the scale, rounded once
+            __half2 zs[4], sc2[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t z = ((zw >> (4 * q)) & 0x000f000fu) | 0x64006400u;
+                zs[q] = __hsub2((q & 1) ? __float2half2_rn(960.0f) : __float2half2_rn(0.0f), *reinterpret_cast<const __half2*>(&z));
+                if constexpr (INTERLEAVED) sc2[q] = *reinterpret_cast<const __half2*>(&sw[q]);      // columns (2q, 2q+1)
+                else {                                                                              // columns (q, q+4)
+                    const __half* sh = reinterpret_cast<const __half*>(sw);
+                    sc2[q] = __halves2half2(sh[q], sh[q + 4]);
                 }
-            };
-            uint32_t zw_nx = 0; uint4 s4_nx = make_uint4(0, 0, 0, 0);
-            load_meta(0, zw_nx, s4_nx);
-            for (int kb = 0; kb < num_kb; ++kb, ++g) {
-                const int s = g % GM_STAGES;
-                if (kb % gpk == 0) {                      // new group: scale and zero of this thread's 8 columns
-                    const int gi = kb / gpk;
-                    const uint32_t zw = zw_nx;
-                    const uint4 s4 = s4_nx;
-                    if (gi + 1 < n_grp) load_meta(gi + 1, zw_nx, s4_nx);
-                    const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w};
+            }
+            if (gm_timeout(&raw_full[rs], (unsigned)(g / RS) & 1u)) { failed = true; break; }
+            const uint32_t* raw = reinterpret_cast<const uint32_t*>(sRaw + rs * GM_RAW_BYTES) + kr0 * (GM_BN / 8) + c;
+            uint32_t w[GM_BK / 4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) zsub[q] = ((zw >> (4 * q)) & 0x000f000fu) | 0x64006400u;
-                    if constexpr (INTERLEAVED) {
+            for (int i = 0; i < GM_BK / 4; ++i) w[i] = raw[4 * i * (GM_BN / 8)];
+            if (g >= BS && gm_timeout(&b_empty[bs], (unsigned)(g / BS - 1) & 1u)) { failed = true; break; }
+            unsigned char* bt = sB + bs * GM_B_BYTES + a_n * (GM_BK * 128);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) sc2[q] = *reinterpret_cast<const __half2*>(&sw[q]);      // columns (2q, 2q+1)
-                    } else {
-                        // word q of the codes pairs columns (q, q+4)
-                        const __half* sh = reinterpret_cast<const __half*>(sw);
+            for (int i = 0; i < GM_BK / 4; ++i) {
+                const int kr = kr0 + 4 * i;
+                const uint32_t w8 = w[i] >> 8;
+                uint32_t o[4] = {(w[i] & 0x000f000fu) | 0x64006400u, (w[i] & 0x00f000f0u) | 0x64006400u,
+                                 (w8 & 0x000f000fu) | 0x64006400u, (w8 & 0x00f000f0u) | 0x64006400u};
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) sc2[q] = __halves2half2(sh[q], sh[q + 4]);
-                    }
+                for (int q = 0; q < 4; ++q) {
+                    const __half2 h = *reinterpret_cast<const __half2*>(&o[q]);
+                    const __half2 r = __hmul2((q & 1) ? __hfma2(h, sixteenth, zs[q]) : __hadd2(h, zs[q]), sc2[q]);
+                    o[q] = *reinterpret_cast<const uint32_t*>(&r);
                 }
-                if (!gm_wait(&full_raw[s], (unsigned)(g / GM_STAGES) & 1u)) { failed = true; break; }
-                unsigned char* st = base + s * GM_STAGE_BYTES;
-                const uint32_t* raw = reinterpret_cast<const uint32_t*>(st + GM_MT * GM_A_BYTES + GM_B_BYTES);
-                unsigned char* bt = st + GM_MT * GM_A_BYTES + a_n * (GM_BK * 128);
-#pragma unroll
-                for (int i = 0; i < GM_BK / 8; ++i) {
-                    const int kr = kr0 + 8 * i;
-                    const uint32_t w = raw[kr * (GM_BN / 8) + c];
-                    uint32_t o[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const uint32_t h = ((w >> (4 * q)) & 0x000f000fu) | 0x64006400u;                   // (1024 + code) pairs
-                        const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&h), *reinterpret_cast<const __half2*>(&zsub[q]));
-                        const __half2 r = __hmul2(d, sc2[q]);
-                        o[q] = *reinterpret_cast<const uint32_t*>(&r);
-                    }
-                    uint4 out;
-                    if constexpr (INTERLEAVED) {
-                        out = make_uint4(o[0], o[1], o[2], o[3]);
-                    } else {      // pairs (q, q+4) -> column order
-                        out = make_uint4(__byte_perm(o[0], o[1], 0x5410), __byte_perm(o[2], o[3], 0x5410),
-                                         __byte_perm(o[0], o[1], 0x7632), __byte_perm(o[2], o[3], 0x7632));
-                    }
-                    // row kr of the atom column a_n: 128 B per row, 16-byte chunks swizzled by the row index
-                    *reinterpret_cast<uint4*>(bt + kr * 128 + ((chunk ^ (kr & 7)) << 4)) = out;
+                uint4 out;
+                if constexpr (INTERLEAVED) {
+                    out = make_uint4(o[0], o[1], o[2], o[3]);
+                } else {      // pairs (q, q+4) -> column order
+                    out = make_uint4(__byte_perm(o[0], o[1], 0x5410), __byte_perm(o[2], o[3], 0x5410),
+                                     __byte_perm(o[0], o[1], 0x7632), __byte_perm(o[2], o[3], 0x7632));
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy stores -> visible to the tensor core
-                gm_mbar_arrive(&b_ready[s]);
+                // row kr of the atom column a_n: 128 B per row, 16-byte chunks swizzled by the row index
+                *reinterpret_cast<uint4*>(bt + kr * 128 + ((chunk ^ (kr & 7)) << 4)) = out;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy stores -> visible to the tensor core
+            __syncwarp();
+            if (lane == 0) {
+                gm_mbar_arrive(&b_ready[bs]);
+                // not earlier: an arrival right behind the loads let the refill overtake them (wrong tiles, about 1 launch in 10)
+                gm_mbar_arrive(&raw_empty[rs]);
             }
         }
     } else {
@@ -379,7 +420,11 @@ extern "C" int fq_awq_gemm(
     FQ_CHECK_ARG(n_proj >= 1 && n_proj <= GM_MAX_PROJ, FQ_ERR_ARG, "%s: 1..%d projections per call, got %d", fn, GM_MAX_PROJ, n_proj);
     FQ_CHECK_ARG(x && qweight && scales && qzeros && N && y, FQ_ERR_ARG, "%s: null pointer", fn);
     FQ_CHECK_ARG(aligned(x, 16), FQ_ERR_ALIGN, "%s: x must be 16-byte aligned", fn);
-    if (M <= 1024) {
+    // Up to 384 tiles of 128 x 128 (2.6 waves of the SMs): the split-K kernel.  Measured at 3072 x 16384: 59 us against 74 at
+    // 384 rows (384 tiles), 79 against 75 at 512 (512 tiles); at 3072 x 3072: 37 against 42 at 1024 rows (192 tiles).
+    int64_t tiles128 = 0;
+    for (int i = 0; i < n_proj; ++i) tiles128 += (N[i] + 127) / 128;
+    if (tiles128 * ((M + 127) / 128) <= 384) {
         SkinnyCall c{};
         c.x = x; c.M = M; c.K = K; c.group = group; c.n_proj = n_proj; c.interleaved = interleaved ? 1 : 0;
         for (int i = 0; i < n_proj; ++i) {

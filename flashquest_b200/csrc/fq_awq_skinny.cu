@@ -258,10 +258,6 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
             uint32_t w[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) w[i] = raw[128 * i];
-            __syncwarp();
-            if (lane == 0) sk_arrive(&empty_raw[r]);
-            for (int i = 0; i < SK_DEQ_WARPS / SK_DEQ_GROUP; ++i)
-                if (++r == p.raw_stages) { r = 0; rph ^= 1u; }
             if (kb >= AS && sk_any_timeout(&a_empty[s], (unsigned)(kb / AS - 1) & 1u)) { failed = true; break; }
             unsigned char* at = sW + s * SK_A + (c >> 3) * (SK_BK * 128);
 #pragma unroll
@@ -287,7 +283,9 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) sk_arrive(&a_ready[s]);
+            if (lane == 0) { sk_arrive(&a_ready[s]); sk_arrive(&empty_raw[r]); }      // (the raw tile not before its values have been used)
+            for (int i = 0; i < SK_DEQ_WARPS / SK_DEQ_GROUP; ++i)
+                if (++r == p.raw_stages) { r = 0; rph ^= 1u; }
         }
         // ---- the accumulator ----
         if (ng > 0 && sk_any_timeout(&acc_ready, 0u)) failed = true;

@@ -1,0 +1,56 @@
+"""The AWQ GEMM at the edges of its row tiles and K splits (csrc/fq_awq_skinny.cu, csrc/fq_awq_gemm.cu) against a plain
+PyTorch product of the fp16-rounded weights, and equal to itself over repeated launches."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _linear(K, N, group, interleaved, bias, g):
+    from flashquest_b200.quant import AWQLinear
+    ri = lambda *s: torch.randint(-2 ** 31, 2 ** 31 - 1, s, dtype=torch.int32, device="cuda", generator=g)
+    sc = (torch.rand(K // group, N, device="cuda", generator=g) * 0.019 + 0.001).half()
+    b = torch.randn(N, device="cuda", generator=g).half() if bias else None
+    return AWQLinear(ri(K, N // 8), sc, ri(K // group, N // 8), b, group_size=group, interleaved=interleaved)
+
+
+def _weights(lin):
+    order = [0, 2, 4, 6, 1, 3, 5, 7] if lin.interleaved else list(range(8))
+
+    def unpack(q):
+        out = torch.empty(q.shape[0], q.shape[1] * 8, device=q.device)
+        for i in range(8):
+            out[:, order[i]::8] = ((q >> (4 * i)) & 15).float()
+        return out
+    rep = lambda t: t.repeat_interleave(lin.group_size, 0)
+    return ((unpack(lin.qweight) - rep(unpack(lin.qzeros))) * rep(lin.scales.float())).half().float()
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 33, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("K,Ns,group,interleaved,bias", [(512, (128, 384), 128, True, False), (3072, (256, 128, 128), 128, True, True),
+                                                         (1536, (256,), 256, False, True)])
+def test_rows_and_splits(M, K, Ns, group, interleaved, bias):
+    from flashquest_b200.kernel.fused_proj import awq_gemm_fused
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    lins = [_linear(K, N, group, interleaved, bias, g) for N in Ns]
+    x = torch.randn(M, K, device="cuda", generator=g).half()
+    got = awq_gemm_fused(x, lins)
+    for y, lin in zip(got, lins):
+        want = x.float() @ _weights(lin) + (lin.bias.float() if bias else 0)
+        assert (y.float() - want).abs().max().item() <= 2e-3 * want.abs().max().item() + 1e-3
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(got, awq_gemm_fused(x, lins)))
+
+
+@pytest.mark.parametrize("M", [1100, 2048])
+def test_large_tiles_repeat(M):
+    """More tiles than SMs: a CTA's second tile overlaps the epilogue of its first."""
+    from flashquest_b200.kernel.fused_proj import awq_gemm_fused
+    g = torch.Generator(device="cuda").manual_seed(M)
+    lin = _linear(3072, 5120, 128, True, False, g)
+    x = torch.randn(M, 3072, device="cuda", generator=g).half()
+    (first,) = awq_gemm_fused(x, (lin,))
+    want = x.float() @ _weights(lin)
+    assert (first.float() - want).abs().max().item() <= 2e-3 * want.abs().max().item() + 1e-3
+    for _ in range(30):
+        assert torch.equal(first, awq_gemm_fused(x, (lin,))[0])
