@@ -4,10 +4,10 @@
 // (query i sees keys 0..i), fp16 or bf16 operands, fp32 accumulation and softmax.
 //
 // One CTA = 128 queries of one query head, walking key tiles of 128:
-//   warp 0      : two threads issue the TMA loads (4-D tensor maps over Q, K, V; 128-byte swizzle): Q once, then one
-//                 thread the K tiles and one the V tiles, each into its own two-deep ring (a K stage is free again as
-//                 soon as S has been computed, long before the V stage of the same tile);
-//   warp 1      : one thread issues tcgen05.mma: S = Q K^T (M 128, N 128, K 16 x 8) into one of two S buffers in
+//   warp 0      : issues the TMA loads (4-D tensor maps over Q, K, V; 128-byte swizzle): Q once, then the K tiles one
+//                 ahead of the V tiles, each into its own two-deep ring (a K stage is free again as soon as S has been
+//                 computed, long before the V stage of the same tile);
+//   warp 1      : issues tcgen05.mma: S = Q K^T (M 128, N 128, K 16 x 8) into one of two S buffers in
 //                 tensor memory, and O += P V into the one O accumulator in tensor memory, with P read from tensor
 //                 memory as the A operand and V from shared memory as the MN-major B operand; S runs up to two key
 //                 tiles ahead of P V;
@@ -64,6 +64,13 @@ __device__ __forceinline__ bool pt_wait(uint64_t* bar, unsigned parity) {
         if (++spins > PT_SPIN_LIMIT) return false;
     }
     return true;
+}
+// the same for a whole warp; true = gave up
+__device__ __forceinline__ bool pt_timeout(uint64_t* bar, unsigned parity) { return __any_sync(0xffffffffu, !pt_wait(bar, parity)); }
+__device__ __forceinline__ bool pt_elect() {
+    uint32_t pred;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+    return pred != 0;
 }
 __device__ __forceinline__ void pt_tma_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
@@ -146,7 +153,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(
     // the tile maxima as bf16 [tile parity][column half][lane], at the end the denominators as fp32 [column half][lane]
     __shared__ __align__(16) unsigned char s_xch[4 * 256];
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     // the heaviest query tiles (most keys under the causal mask) are scheduled first
     const int qt = gridDim.x - 1 - blockIdx.x, hq = blockIdx.y, b = blockIdx.z;
     const int hkv = hq / (p.Hq / p.Hkv);
@@ -174,75 +181,91 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(
     const uint32_t tmem_base = *tmem_slot;
     bool failed = false;
 
+    // The producer and issuer warps walk their loops as whole warps and one elected lane issues: descriptors and addresses
+    // that are uniform over the warp then stay in uniform registers.  Inside a branch on lane == 0 an MMA issue took about 90
+    // cycles, 1440 for the 16 of a tile whose MMAs take 1024.
     if (warp == 0) {
         // =========================== TMA producer ===========================
-        if (lane == 0 && n_tiles > 0) {           // Q, then the K tiles
+        // Q, then K one tile ahead of V: a K stage is free as soon as S has been computed
+        if (n_tiles > 0 && pt_elect()) {
             pt_mbar_expect_tx(q_full, PT_TILE_BYTES);
             pt_tma_4d(sQ, &map_q, 0, q0, hq, b, q_full);
             pt_tma_4d(sQ + PT_HALF_BYTES, &map_q, 64, q0, hq, b, q_full);
-            for (int j = 0; j < n_tiles; ++j) {
-                const int s = j & 1;
-                if (j >= 2 && !pt_wait(&k_empty[s], (unsigned)((j >> 1) - 1) & 1u)) { failed = true; break; }
-                pt_mbar_expect_tx(&k_full[s], PT_TILE_BYTES);
-                pt_tma_4d(sK + s * PT_TILE_BYTES, &map_k, 0, j * PT_BN, hkv, b, &k_full[s]);
-                pt_tma_4d(sK + s * PT_TILE_BYTES + PT_HALF_BYTES, &map_k, 64, j * PT_BN, hkv, b, &k_full[s]);
+        }
+        __syncwarp();
+        for (int j = 0; j <= n_tiles; ++j) {
+            const int s = j & 1, sv = s ^ 1;
+            if (j < n_tiles) {
+                if (j >= 2 && pt_timeout(&k_empty[s], (unsigned)((j >> 1) - 1) & 1u)) { failed = true; break; }
+                if (pt_elect()) {
+                    pt_mbar_expect_tx(&k_full[s], PT_TILE_BYTES);
+                    pt_tma_4d(sK + s * PT_TILE_BYTES, &map_k, 0, j * PT_BN, hkv, b, &k_full[s]);
+                    pt_tma_4d(sK + s * PT_TILE_BYTES + PT_HALF_BYTES, &map_k, 64, j * PT_BN, hkv, b, &k_full[s]);
+                }
+                __syncwarp();
             }
-        } else if (lane == 1 && n_tiles > 0) {    // the V tiles
-            for (int j = 0; j < n_tiles; ++j) {
-                const int s = j & 1;
-                if (j >= 2 && !pt_wait(&v_empty[s], (unsigned)((j >> 1) - 1) & 1u)) { failed = true; break; }
-                pt_mbar_expect_tx(&v_full[s], PT_TILE_BYTES);
-                pt_tma_4d(sV + s * PT_TILE_BYTES, &map_v, 0, j * PT_BN, hkv, b, &v_full[s]);
-                pt_tma_4d(sV + s * PT_TILE_BYTES + PT_HALF_BYTES, &map_v, 64, j * PT_BN, hkv, b, &v_full[s]);
+            if (j >= 1) {
+                const int jv = j - 1;
+                if (jv >= 2 && pt_timeout(&v_empty[sv], (unsigned)((jv >> 1) - 1) & 1u)) { failed = true; break; }
+                if (pt_elect()) {
+                    pt_mbar_expect_tx(&v_full[sv], PT_TILE_BYTES);
+                    pt_tma_4d(sV + sv * PT_TILE_BYTES, &map_v, 0, jv * PT_BN, hkv, b, &v_full[sv]);
+                    pt_tma_4d(sV + sv * PT_TILE_BYTES + PT_HALF_BYTES, &map_v, 64, jv * PT_BN, hkv, b, &v_full[sv]);
+                }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
         // =========================== MMA issuer ===========================
-        if (lane == 0 && n_tiles > 0) {
-            const uint32_t fmt = p.bf16 ? 1u : 0u;
-            // fp32 accumulate; A K-major; B K-major (S = Q K^T) or MN-major (O = P V); N = 128, M = 128
-            const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | (0u << 15) | (0u << 16) | ((uint32_t)(PT_BN >> 3) << 17) |
-                                     ((uint32_t)(PT_BM >> 4) << 24);
-            const uint32_t idesc_o = idesc_s | (1u << 16);
-            const uint32_t q_addr = pt_smem(sQ);
-            auto issue_s = [&](int j) -> bool {           // S[j & 1] = Q K_j^T; the buffer was read by the softmax of tile j-2
-                const int s = j & 1;
-                if (!pt_wait(&k_full[s], (unsigned)(j >> 1) & 1u)) return false;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t k_addr = pt_smem(sK + s * PT_TILE_BYTES);
+        const uint32_t fmt = p.bf16 ? 1u : 0u;
+        // fp32 accumulate; A K-major; B K-major (S = Q K^T) or MN-major (O = P V); N = 128, M = 128
+        const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | (0u << 15) | (0u << 16) | ((uint32_t)(PT_BN >> 3) << 17) |
+                                 ((uint32_t)(PT_BM >> 4) << 24);
+        const uint32_t idesc_o = idesc_s | (1u << 16);
+        // K-major, 128-byte swizzle: 8 rows x 64 elements = one 1 KiB atom; 16 k = 32 B inside the row; second half 16 KiB on
+        const uint64_t dq0 = pt_desc(pt_smem(sQ), 16, 1024), dk0 = pt_desc(pt_smem(sK), 16, 1024);
+        // V, MN-major: 64 channels x 8 keys = one atom, 16 keys = 2 KiB, channel halves 16 KiB apart
+        const uint64_t dv0 = pt_desc(pt_smem(sV), PT_HALF_BYTES, 1024);
+        auto issue_s = [&](int j) -> bool {           // S[j & 1] = Q K_j^T; the buffer was read by the softmax of tile j-2
+            const int s = j & 1;
+            if (pt_timeout(&k_full[s], (unsigned)(j >> 1) & 1u)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t dk = dk0 + (uint64_t)(s * (PT_TILE_BYTES >> 4));
+            const uint32_t acc = tmem_base + (uint32_t)(s * PT_BN);
+            if (pt_elect()) {
 #pragma unroll
                 for (int kk = 0; kk < PT_D / 16; ++kk) {
-                    // K-major, 128-byte swizzle: 8 rows x 64 elements = one 1 KiB atom; 16 k = 32 B inside the row; second half 16 KiB on
-                    const uint32_t off = (uint32_t)(kk >> 2) * PT_HALF_BYTES + (uint32_t)(kk & 3) * 32;
-                    pt_mma(tmem_base + (uint32_t)(s * PT_BN), pt_desc(q_addr + off, 16, 1024), pt_desc(k_addr + off, 16, 1024), idesc_s, kk != 0 ? 1u : 0u);
+                    const uint32_t off = ((uint32_t)(kk >> 2) * PT_HALF_BYTES + (uint32_t)(kk & 3) * 32) >> 4;
+                    pt_mma(acc, dq0 + off, dk + off, idesc_s, kk != 0 ? 1u : 0u);
                 }
                 pt_commit(&s_ready[s]);
                 pt_commit(&k_empty[s]);
-                return true;
-            };
-            if (!pt_wait(q_full, 0u) || !issue_s(0)) failed = true;
-            if (!failed && n_tiles > 1 && !issue_s(1)) failed = true;
-            for (int j = 0; j < n_tiles && !failed; ++j) {
-                const int s = j & 1;
-                const unsigned ph = (unsigned)(j >> 1) & 1u;
-                // p_ready also says that the softmax threads have rescaled O where a row's maximum moved
-                if (!pt_wait(&p_ready[s], ph) || !pt_wait(&v_full[s], ph)) { failed = true; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t v_addr = pt_smem(sV + s * PT_TILE_BYTES);
+            }
+            __syncwarp();
+            return true;
+        };
+        if (n_tiles > 0 && (pt_timeout(q_full, 0u) || !issue_s(0))) failed = true;
+        if (!failed && n_tiles > 1 && !issue_s(1)) failed = true;
+        for (int j = 0; j < n_tiles && !failed; ++j) {
+            const int s = j & 1;
+            const unsigned ph = (unsigned)(j >> 1) & 1u;
+            // p_ready also says that the softmax threads have rescaled O where a row's maximum moved
+            if (pt_timeout(&p_ready[s], ph) || pt_timeout(&v_full[s], ph)) { failed = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t dv = dv0 + (uint64_t)(s * (PT_TILE_BYTES >> 4));
+            const uint32_t p0 = tmem_base + (uint32_t)(s * PT_BN), acc = tmem_base + (uint32_t)(2 * PT_BN);
+            if (pt_elect()) {
 #pragma unroll
-                for (int kk = 0; kk < PT_BN / 16; ++kk) {
+                for (int kk = 0; kk < PT_BN / 16; ++kk)
                     // A = P of tile j in tensor memory, written over the S buffer it came from: keys 0..63 in columns 0..31
-                    // of the buffer, keys 64..127 in columns 64..95 (each half under the S columns its writer owns);
-                    // B = V, MN-major: 64 channels x 8 keys = one atom, 16 keys = 2 KiB, channel halves 16 KiB apart
-                    const uint32_t p_taddr = tmem_base + (uint32_t)(s * PT_BN + (kk >> 2) * 64 + (kk & 3) * 8);
-                    pt_mma_ta(tmem_base + (uint32_t)(2 * PT_BN), p_taddr,
-                              pt_desc(v_addr + (uint32_t)kk * 2048, PT_HALF_BYTES, 1024), idesc_o, (kk != 0 || j != 0) ? 1u : 0u);
-                }
+                    // of the buffer, keys 64..127 in columns 64..95 (each half under the S columns its writer owns)
+                    pt_mma_ta(acc, p0 + (uint32_t)((kk >> 2) * 64 + (kk & 3) * 8), dv + (uint64_t)(kk * (2048 >> 4)), idesc_o, (kk != 0 || j != 0) ? 1u : 0u);
                 pt_commit(&pv_done[s]);
                 pt_commit(&v_empty[s]);
-                // S two tiles ahead: its buffer has just been released by p_ready of tile j
-                if (j + 2 < n_tiles && !issue_s(j + 2)) { failed = true; break; }
             }
+            __syncwarp();
+            // S two tiles ahead: its buffer has just been released by p_ready of tile j
+            if (j + 2 < n_tiles && !issue_s(j + 2)) { failed = true; break; }
         }
     } else {
         // =========================== softmax and output ===========================
