@@ -1,4 +1,5 @@
-"""The AWQ GEMM at the edges of its row tiles and K splits (csrc/fq_awq_skinny.cu, csrc/fq_awq_gemm.cu) against a plain
+"""The AWQ GEMM at the edges of its row tiles and K splits (csrc/fq_awq_skinny.cu, csrc/fq_awq_gemm.cu), and the GEMV
+over its K splits, passes and tiles per CTA (csrc/fq_awq_regv.cu), against a plain
 PyTorch product of the fp16-rounded weights, and equal to itself over repeated launches."""
 import pytest
 import torch
@@ -54,3 +55,18 @@ def test_large_tiles_repeat(M):
     assert (first.float() - want).abs().max().item() <= 2e-3 * want.abs().max().item() + 1e-3
     for _ in range(30):
         assert torch.equal(first, awq_gemm_fused(x, (lin,))[0])
+
+
+@pytest.mark.parametrize("M", [1, 3, 8])
+@pytest.mark.parametrize("K,Ns,interleaved,bias", [(128, (128,), True, True), (1152, (384, 128), False, False), (8320, (256,), True, False),
+                                                   (4096, (9600, 128), True, True)])
+def test_gemv_splits_and_tiles(M, K, Ns, interleaved, bias):
+    from flashquest_b200.kernel.fused_proj import awq_gemv_fused
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    lins = [_linear(K, N, 128, interleaved, bias, g) for N in Ns]
+    x = torch.randn(M, K, device="cuda", generator=g).half()
+    got = awq_gemv_fused(x, lins)
+    for y, lin in zip(got, lins):
+        want = x.float() @ _weights(lin) + (lin.bias.float() if bias else 0)
+        assert (y.float() - want).abs().max().item() <= 2e-3 * want.abs().max().item() + 1e-3
+    assert all(torch.equal(a, b) for a, b in zip(got, awq_gemv_fused(x, lins)))
