@@ -225,54 +225,84 @@ __global__ void __launch_bounds__(GEMVH_WARPS * 32) gemv_f16_kernel(const __half
     }
 }
 
-// The same product for 2..8 rows on the tensor cores (mma.sync m16n8k16, fp32 accumulation): on the CUDA cores every
-// weight costs one fma per row and a shared-memory read of x, which for 8 rows is several times the HBM time of W.
-// A warp owns 16 output rows (A = 16 rows of W, straight from global memory with 16-byte loads), B = the rows of x
-// (staged once per CTA as fp16, padded to 8 rows); lane (g, t) reads W[n0+g][k0+8t .. +7] and W[n0+g+8][...], i.e. the
-// k index inside an MMA is permuted the same way for A and B.  CTAs are persistent over tiles of 128 output rows.
-constexpr int GEMVM_WARPS = 8;
+// The same product on the tensor cores (mma.sync m16n8k16, fp32 accumulation), K a multiple of 32: HBM bound, so what counts
+// is bytes in flight.  A CTA owns 16 output rows at a time (A = W, B = the rows of x, staged once as fp16 and padded to 8
+// rows); its eight warps interleave 32-wide k steps, so a step of the CTA reads 512 contiguous bytes of each row.  A lane
+// keeps GEMVM_DEPTH steps (two 16-byte loads each) in registers and refills a slot as soon as it is used, across the end of
+// a tile too: 16 KiB per warp, 128 KiB per SM on the way at any time.  Lane (g, t) reads W[n0+g][k0+8t .. +7] and
+// W[n0+g+8][...], i.e. the k index inside an MMA is permuted the same way for A and B.  The warps' sums meet in shared
+// memory, in warp order, one barrier per tile (two buffers).  788 MB of W (128256 x 3072): 118 us at 1 row (one warp per row
+// on the CUDA cores: 139), 120 us = 6.6 TB/s at 8 (four steps in flight and a tile per warp: 259).
+constexpr int GEMVM_WARPS = 8, GEMVM_ROWS = 16, GEMVM_DEPTH = 8;
 constexpr int GEMVM_XPAD = 32;      // fp16 elements: row stride = 16 words mod 32, conflict-free 16-byte fragment loads
 
-__global__ void __launch_bounds__(GEMVM_WARPS * 32) gemv_f16_mma_kernel(const __half* __restrict__ x, const __half* __restrict__ W,
-                                                                        int Mrows, int K, int N, __half* __restrict__ y) {
+__device__ __forceinline__ uint4 gemvm_ldg(const __half* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+__global__ void __launch_bounds__(GEMVM_WARPS * 32, 2) gemv_f16_mma_kernel(const __half* __restrict__ x, const __half* __restrict__ W,
+                                                                           int Mrows, int K, int N, __half* __restrict__ y) {
     extern __shared__ __align__(16) __half s_xh[];      // [8][K + XPAD]
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int xs = K + GEMVM_XPAD;
+    __shared__ float s_part[2][GEMVM_WARPS][8][GEMVM_ROWS + 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int xs = K + GEMVM_XPAD, k_steps = K >> 5;
+    const int tiles = (N + GEMVM_ROWS - 1) / GEMVM_ROWS;
+    const int steps = (k_steps + GEMVM_WARPS - 1) / GEMVM_WARPS;       // of every warp; past k_steps they load nothing
+    // the load cursor runs GEMVM_DEPTH steps ahead of the products
+    int lt = blockIdx.x, ls = 0;
+    uint4 wa[GEMVM_DEPTH], wb[GEMVM_DEPTH];
+    auto load = [&](int d) {
+        const int ks = ls * GEMVM_WARPS + warp;
+        if (lt < tiles && ks < k_steps) {
+            const int64_t k = 32 * ks + 8 * t;
+            wa[d] = gemvm_ldg(W + (int64_t)min(lt * GEMVM_ROWS + g, N - 1) * K + k);
+            wb[d] = gemvm_ldg(W + (int64_t)min(lt * GEMVM_ROWS + g + 8, N - 1) * K + k);
+        }
+        if (++ls == steps) { ls = 0; lt += gridDim.x; }
+    };
+#pragma unroll
+    for (int d = 0; d < GEMVM_DEPTH; ++d) load(d);                     // weights never change: before the dependency wait
     pdl_wait();
     pdl_trigger();
-    for (int i = threadIdx.x; i < 8 * (K / 8); i += GEMVM_WARPS * 32) {
+    for (int i = tid; i < 8 * (K / 8); i += GEMVM_WARPS * 32) {
         const int m = i / (K / 8), kk = (i - m * (K / 8)) * 8;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (m < Mrows) v = __ldcg(reinterpret_cast<const uint4*>(x + (int64_t)m * K + kk));
         *reinterpret_cast<uint4*>(s_xh + m * xs + kk) = v;
     }
     __syncthreads();
-    const int tiles = (N + 16 * GEMVM_WARPS - 1) / (16 * GEMVM_WARPS);
-    const __half* xrow = s_xh + g * xs + 8 * t;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int n0 = tile * 16 * GEMVM_WARPS + warp * 16;
-        if (n0 >= N) continue;
-        const __half* wa = W + (int64_t)min(n0 + g, N - 1) * K + 8 * t;
-        const __half* wb = W + (int64_t)min(n0 + g + 8, N - 1) * K + 8 * t;
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-        for (int k0 = 0; k0 < K; k0 += 32) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(wa + k0));
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(wb + k0));
-            const uint4 xv = *reinterpret_cast<const uint4*>(xrow + k0);
-            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a.x), "r"(b.x), "r"(a.y), "r"(b.y), "r"(xv.x), "r"(xv.y));
-            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a.z), "r"(b.z), "r"(a.w), "r"(b.w), "r"(xv.z), "r"(xv.w));
-        }
-        // c0, c1: output row n0+g for x rows 2t, 2t+1; c2, c3: output row n0+g+8
-        if (2 * t < Mrows) {
-            if (n0 + g < N) y[(int64_t)(2 * t) * N + n0 + g] = __float2half_rn(c[0]);
-            if (n0 + g + 8 < N) y[(int64_t)(2 * t) * N + n0 + g + 8] = __float2half_rn(c[2]);
-        }
-        if (2 * t + 1 < Mrows) {
-            if (n0 + g < N) y[(int64_t)(2 * t + 1) * N + n0 + g] = __float2half_rn(c[1]);
-            if (n0 + g + 8 < N) y[(int64_t)(2 * t + 1) * N + n0 + g + 8] = __float2half_rn(c[3]);
+    const __half* xrow = s_xh + g * xs + 8 * t + 32 * warp;
+    int tile = blockIdx.x, s = 0, buf = 0;
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    while (tile < tiles) {
+#pragma unroll
+        for (int d = 0; d < GEMVM_DEPTH; ++d) {
+            if (tile >= tiles) break;
+            if (s * GEMVM_WARPS + warp < k_steps) {
+                const uint4 a = wa[d], b = wb[d], xv = *reinterpret_cast<const uint4*>(xrow + s * (32 * GEMVM_WARPS));
+                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                             : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a.x), "r"(b.x), "r"(a.y), "r"(b.y), "r"(xv.x), "r"(xv.y));
+                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                             : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a.z), "r"(b.z), "r"(a.w), "r"(b.w), "r"(xv.z), "r"(xv.w));
+            }
+            load(d);
+            if (++s == steps) {
+                // c0, c1: output row g for x rows 2t, 2t+1; c2, c3: output row g + 8
+                float(*P)[GEMVM_ROWS + 1] = s_part[buf][warp];
+                P[2 * t][g] = c[0]; P[2 * t + 1][g] = c[1]; P[2 * t][g + 8] = c[2]; P[2 * t + 1][g + 8] = c[3];
+                __syncthreads();
+                const int m = tid >> 4, n = tid & 15;
+                if (m < Mrows && tile * GEMVM_ROWS + n < N) {
+                    float v = 0.f;
+#pragma unroll
+                    for (int w = 0; w < GEMVM_WARPS; ++w) v += s_part[buf][w][m][n];
+                    y[(int64_t)m * N + tile * GEMVM_ROWS + n] = __float2half_rn(v);
+                }
+                c[0] = c[1] = c[2] = c[3] = 0.f;
+                s = 0; buf ^= 1; tile += gridDim.x;
+            }
         }
     }
 }
@@ -425,13 +455,13 @@ extern "C" int fq_gemv_f16(const void* x, const void* W, int M, int K, int N, vo
     FQ_CHECK_ARG(M >= 1 && M <= 8, FQ_ERR_UNSUPPORTED, "%s: M=%d rows; 1..8 are built", fn, M);
     FQ_CHECK_ARG(K % 8 == 0 && aligned(W, 16) && aligned(x, 2), FQ_ERR_ALIGN, "%s: K must be a multiple of 8 and W 16-byte aligned", fn);
     cudaStream_t st0 = static_cast<cudaStream_t>(stream);
-    if (M >= 2 && K % 32 == 0 && (size_t)8 * (K + GEMVM_XPAD) * 2 <= 100 * 1024) {
+    if (K % 32 == 0 && aligned(x, 16) && (size_t)8 * (K + GEMVM_XPAD) * 2 <= 100 * 1024) {
         const size_t smem_m = (size_t)8 * (K + GEMVM_XPAD) * 2;
         if (smem_m > 40 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(gemv_f16_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_m);
             if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: %s", fn, cudaGetErrorString(e));
         }
-        const int tiles = (N + 16 * GEMVM_WARPS - 1) / (16 * GEMVM_WARPS);
+        const int tiles = (N + GEMVM_ROWS - 1) / GEMVM_ROWS;
         launch_k(PDL_GEMV, gemv_f16_mma_kernel, dim3((unsigned)(tiles < 2 * 148 ? tiles : 2 * 148)), dim3(GEMVM_WARPS * 32), smem_m, st0,
                  static_cast<const __half*>(x), static_cast<const __half*>(W), M, K, N, static_cast<__half*>(y));
         FQ_CHECK_LAUNCH(fn);
