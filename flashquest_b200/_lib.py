@@ -160,6 +160,8 @@ _PROTOTYPES["fq_sparse_decode_int8"] = (I, [P, I, L, L, P, P, L, L, L, P, P, L, 
 _PROTOTYPES["fq_sparse_decode_int8_counted"] = (I, [P, I, L, L, P, P, L, L, L, P, P, L, L, L, P, P, L, L, P, L, L, I, P,
                                                    P, P, I, L, L, L, I, I, I, I, I, I, I, I, F, P, P, P, Z, I, P])
 _PROTOTYPES["fq_prefill_attention"] = (I, [P, L, L, L, P, L, L, L, P, L, L, L, I, I, I, I, I, I, I, F, P, L, L, L, P])
+_PROTOTYPES["fq_append_kv_int4"] = (I, [ctypes.POINTER(Int4CacheDesc), I, I, P, P, L, L, L, I, P])
+_PROTOTYPES["fq_append_kv_turbo"] = (I, [ctypes.POINTER(TurboCacheDesc), I, I, P, P, L, L, L, I, P])
 _PROTOTYPES["fq_append_kv_int8"] = (I, [ctypes.POINTER(Int4CacheDesc), I, I, P, P, L, L, L, I, P])
 _PROTOTYPES["fq_decode_layer_int8"] = _PROTOTYPES["fq_decode_layer_int4"]
 _PROTOTYPES["fq_rope_qkv"] = (I, [P, L, P, L, P, L, I, P, L, P, L, I, I, I, I, P, P, P, I, P])

@@ -8,9 +8,12 @@ constructor argument (default bf16 as in the reference).
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 from transformers.cache_utils import Cache
 
+from .._lib import Int4CacheDesc, bind, check, dtype_code
 from ..kernel.kv_quant import quantize_kv_int4_into
 
 
@@ -47,6 +50,20 @@ class PersistentInt4KVCache(Cache):
         self.K_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self.V_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self._seen_tokens = [0] * num_layers
+        self._desc = None
+
+    def desc(self) -> Int4CacheDesc:
+        """struct fq_int4_cache of this cache."""
+        d = self._desc
+        if d is None or d.K_packed != self.K_packed.data_ptr() or d.K_partial != self.K_partial.data_ptr():
+            d = self._desc = Int4CacheDesc(
+                self.K_packed.data_ptr(), self.V_packed.data_ptr(), *self.K_packed.stride()[:4],
+                self.K_scale.data_ptr(), self.K_mn.data_ptr(), *self.K_scale.stride()[:4],
+                self.V_scale.data_ptr(), self.V_mn.data_ptr(), *self.V_scale.stride()[:3],
+                self.K_partial.data_ptr(), self.V_partial.data_ptr(), *self.K_partial.stride()[:4],
+                dtype_code(self.K_partial), self.num_layers, self.batch_size, self.num_kv_heads, self.head_dim, self.page_size,
+                self.max_seq_len)
+        return d
 
     def get_seq_length(self, layer_idx: int = 0) -> int:
         return self._seen_tokens[layer_idx]
@@ -69,6 +86,12 @@ class PersistentInt4KVCache(Cache):
                 f"PersistentInt4KVCache: seen+new={seen + S_new} exceeds max_seq_len={self.max_seq_len}")
         if S_new == 0:
             return
+        if K_new.is_cuda and self.K_packed.is_cuda:      # one native call where the tensors are of the cache's dtype and form
+            rc = bind().append(4, ctypes.addressof(self.desc()), self.K_packed.get_device(), layer_idx, seen, K_new, V_new)
+            if rc <= 0:
+                check(rc)
+                self._seen_tokens[layer_idx] = seen + S_new
+                return
         if K_new.dtype != self.dtype:
             K_new = K_new.to(self.dtype)
         if V_new.dtype != self.dtype:

@@ -10,6 +10,7 @@
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -111,6 +112,7 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
                     k->stride(3) == 1 && q->size(0) == B && q->size(1) == Hq && q->size(qd - 1) == D && q->stride(qd - 1) == 1 &&
                     (p->kind != 3 || (q->stride(1) == D && q->stride(0) == static_cast<int64_t>(Hq) * D));
     if (!ok) return PyLong_FromLong(1);
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
     const int rc = run_layer(p, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), static_cast<int>(k->size(2)),
                              q->data_ptr(), dtype_of(*q), q->stride(0), q->stride(1), prm ? prm : &p->prm, stream_of(p->device));
     return PyLong_FromLong(rc);
@@ -137,6 +139,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (t[i]->size(2) != width || !(t[i]->size(0) == B || (i >= 3 && t[i]->size(0) == 1))) return PyLong_FromLong(1);
     }
     const int64_t cs = t[3]->size(0) == 1 ? 0 : t[3]->stride(0), ss = t[4]->size(0) == 1 ? 0 : t[4]->stride(0);
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
     void* st = stream_of(p->device);
     int rc = fq_rope_qkv(t[0]->data_ptr(), t[0]->stride(0), t[1]->data_ptr(), t[1]->stride(0), t[2]->data_ptr(), t[2]->stride(0), dt,
                          t[3]->data_ptr(), cs, t[4]->data_ptr(), ss, B, Hq, Hkv, D, p->q_rot, p->k_rot, p->v_rot, p->cache_dtype, st);
@@ -146,7 +149,32 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return PyLong_FromLong(rc);
 }
 
+// append(kv_bits, cache descriptor, device, layer, seen, k, v): k, v (B,H_kv,n,D) of the cache's dtype
+PyObject* append(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 7) { PyErr_SetString(PyExc_TypeError, "append() takes 7 arguments"); return nullptr; }
+    const int kind = static_cast<int>(PyLong_AsLong(a[0])), device = static_cast<int>(PyLong_AsLong(a[2]));
+    const void* desc = as_ptr(a[1]);
+    const int layer = static_cast<int>(PyLong_AsLong(a[3])), seen = static_cast<int>(PyLong_AsLong(a[4]));
+    const at::Tensor *k = tensor_of(a[5]), *v = tensor_of(a[6]);
+    if (PyErr_Occurred()) return nullptr;
+    const auto* c3 = static_cast<const fq_turbo_cache*>(desc);
+    const auto* c4 = static_cast<const fq_int4_cache*>(desc);
+    const int B = kind == 3 ? c3->B : c4->B, Hkv = kind == 3 ? c3->Hkv : c4->Hkv, D = kind == 3 ? c3->D : c4->D;
+    const int dt = kind == 3 ? c3->kv_dtype : c4->kv_dtype;
+    if (!k || !v || (dt != FQ_F16 && dt != FQ_BF16) || k->dim() != 4 || !k->is_cuda() || !v->is_cuda() || k->get_device() != device ||
+        v->get_device() != device || dtype_of(*k) != dt || dtype_of(*v) != dt || k->sizes() != v->sizes() || k->strides() != v->strides() ||
+        k->size(0) != B || k->size(1) != Hkv || k->size(3) != D || k->stride(3) != 1 || k->size(2) < 1)
+        return PyLong_FromLong(1);
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+    const int nn = static_cast<int>(k->size(2));
+    void* st = stream_of(device);
+    const int rc = kind == 3 ? fq_append_kv_turbo(c3, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), nn, st)
+                             : fq_append_kv_int4(c4, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), nn, st);
+    return PyLong_FromLong(rc);
+}
+
 PyMethodDef kMethods[] = {
+    {"append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(append)), METH_FASTCALL, nullptr},
     {"plan", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(make_plan)), METH_FASTCALL, nullptr},
     {"step", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(step)), METH_FASTCALL, nullptr},
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(forward)), METH_FASTCALL, nullptr},

@@ -4,6 +4,25 @@
 // per layer instead of four plus the slicing arithmetic.
 #include "fq_common.cuh"
 
+extern "C" int fq_append_kv_int4(const fq_int4_cache* c, int layer, int seen, const void* K_new, const void* V_new,
+                                 int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new, void* stream) {
+    using namespace fq;
+    const char* fn = "fq_append_kv_int4";
+    FQ_CHECK_ARG(c && K_new && V_new, FQ_ERR_ARG, "%s: null pointer", fn);
+    FQ_CHECK_ARG(layer >= 0 && layer < c->L, FQ_ERR_ARG, "%s: layer_idx %d out of range [0, %d)", fn, layer, c->L);
+    FQ_CHECK_ARG(seen >= 0 && n_new > 0 && seen + n_new <= c->max_seq_len, FQ_ERR_ARG, "%s: seen+new=%d exceeds max_seq_len=%d", fn, seen + n_new, c->max_seq_len);
+    const int page = c->page, partial = seen % page, n_quant = (partial + n_new) / page * page, tok0 = seen - partial;
+    char* Kt = static_cast<char*>(c->K_partial) + layer * c->pt_sl * 2;
+    char* Vt = static_cast<char*>(c->V_partial) + layer * c->pt_sl * 2;
+    const int64_t co = layer * c->pk_sl + (int64_t)tok0 * c->pk_ss, mo = layer * c->km_sl + (int64_t)(tok0 / page) * c->km_sp, vo = layer * c->vm_sl + tok0;
+    return fq_quantize_kv_int4(
+        Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, partial, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, c->kv_dtype, c->B, c->Hkv, c->D, page, n_quant,
+        c->K_packed + co, c->V_packed + co, c->pk_sb, c->pk_sh, c->pk_ss,
+        static_cast<uint16_t*>(c->K_scale) + mo, static_cast<uint16_t*>(c->K_mn) + mo, c->km_sb, c->km_sh, c->km_sp,
+        static_cast<uint16_t*>(c->V_scale) + vo, static_cast<uint16_t*>(c->V_mn) + vo, c->vm_sb, c->vm_sh, 1,
+        Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, stream);
+}
+
 extern "C" int fq_decode_layer_int4(
     const fq_int4_cache* c, int layer, int seen,
     const void* K_new, const void* V_new, int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new,
@@ -20,12 +39,6 @@ extern "C" int fq_decode_layer_int4(
     FQ_CHECK_ARG(c->kv_dtype == FQ_F16 || c->kv_dtype == FQ_BF16, FQ_ERR_DTYPE, "%s: cache dtype code %d", fn, c->kv_dtype);
     const int page = c->page, D = c->D, B = c->B, Hkv = c->Hkv, Hq = prm->Hq;
     const size_t esz = 2;
-    const int partial_len = seen % page;
-    const int total = partial_len + n_new;
-    const int n_quant = (total / page) * page;
-    const int tok_start = seen - partial_len;
-    const int pg_start = tok_start / page;
-
     uint8_t* Kp = c->K_packed + layer * c->pk_sl;
     uint8_t* Vp = c->V_packed + layer * c->pk_sl;
     uint16_t* Ks = static_cast<uint16_t*>(c->K_scale) + layer * c->km_sl;
@@ -37,14 +50,7 @@ extern "C" int fq_decode_layer_int4(
 
     int rc;
     if (n_new > 0) {
-        rc = fq_quantize_kv_int4(
-            Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, partial_len,
-            K_new, V_new, nw_sb, nw_sh, nw_ss, n_new,
-            c->kv_dtype, B, Hkv, D, page, n_quant,
-            Kp + (int64_t)tok_start * c->pk_ss, Vp + (int64_t)tok_start * c->pk_ss, c->pk_sb, c->pk_sh, c->pk_ss,
-            Ks + (int64_t)pg_start * c->km_sp, Km + (int64_t)pg_start * c->km_sp, c->km_sb, c->km_sh, c->km_sp,
-            Vs + tok_start, Vm + tok_start, c->vm_sb, c->vm_sh, 1,
-            Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, stream);
+        rc = fq_append_kv_int4(c, layer, seen, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, stream);
         if (rc != FQ_OK) return rc;
     }
     const int now = seen + n_new;

@@ -1,5 +1,5 @@
 // Host-side chaining of one decode step of one layer on a persistent TurboQuant (K3-V3) cache:
-// pack-on-append (K planes, V planes, raw page metadata + staging), page scores from the raw
+// pack-on-append, page scores from the raw
 // metadata, top-k + compact index, rotation of Q, sparse attention over the selected planes in
 // the rotated basis, rotation of O back, tail attention over the staged tokens and the LSE merge.
 // No device code of its own: it exists so that a caller pays one foreign call per layer.
@@ -31,10 +31,6 @@ extern "C" int fq_decode_layer_turbo(
                  "%s: scratch of %zu B needed, %zu given", fn, fq_decode_layer_turbo_scratch_bytes(B, Hq, D), scratch_bytes);
     FQ_CHECK_ARG(q_sh == D && q_sb == (int64_t)Hq * D, FQ_ERR_ARG, "%s: Q must be dense (B,H_q,D)", fn);
     const size_t esz = 2;
-    const int partial_len = seen % page;
-    const int n_quant = ((partial_len + n_new) / page) * page;
-    const int tok_start = seen - partial_len;
-    const int pg_start = tok_start / page;
     uint8_t* Kms = c->K_msb + layer * c->ms_sl; uint8_t* Kls = c->K_lsb + layer * c->ls_sl;
     uint8_t* Vms = c->V_msb + layer * c->ms_sl; uint8_t* Vls = c->V_lsb + layer * c->ls_sl;
     uint16_t* Kst = static_cast<uint16_t*>(c->K_scale_turbo) + layer * c->st_sl;
@@ -45,24 +41,7 @@ extern "C" int fq_decode_layer_turbo(
     char* Vt = static_cast<char*>(c->V_partial) + layer * c->pt_sl * esz;
     int rc;
     if (n_new > 0) {
-        if (n_quant > 0) {
-            rc = fq_quantize_turbo(Kt, c->pt_sb, c->pt_sh, c->pt_ss, partial_len, K_new, nw_sb, nw_sh, nw_ss, n_new, c->kv_dtype, B, Hkv, D, n_quant,
-                                   Kms + (int64_t)tok_start * c->ms_ss, c->ms_sb, c->ms_sh, c->ms_ss,
-                                   Kls + (int64_t)tok_start * c->ls_ss, c->ls_sb, c->ls_sh, c->ls_ss,
-                                   Kst + tok_start, c->st_sb, c->st_sh, 1, stream);
-            if (rc != FQ_OK) return rc;
-            rc = fq_quantize_turbo(Vt, c->pt_sb, c->pt_sh, c->pt_ss, partial_len, V_new, nw_sb, nw_sh, nw_ss, n_new, c->kv_dtype, B, Hkv, D, n_quant,
-                                   Vms + (int64_t)tok_start * c->ms_ss, c->ms_sb, c->ms_sh, c->ms_ss,
-                                   Vls + (int64_t)tok_start * c->ls_ss, c->ls_sb, c->ls_sh, c->ls_ss,
-                                   Vst + tok_start, c->st_sb, c->st_sh, 1, stream);
-            if (rc != FQ_OK) return rc;
-        }
-        // raw per-page K metadata (for scoring) + staging of the left-over tokens, after the launches
-        // above have read the staged head
-        rc = fq_quantize_kv_int4(Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, partial_len, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new,
-                                 c->kv_dtype, B, Hkv, D, page, n_quant, nullptr, nullptr, 0, 0, 0,
-                                 Ksr + (int64_t)pg_start * c->km_sp, Kmr + (int64_t)pg_start * c->km_sp, c->km_sb, c->km_sh, c->km_sp,
-                                 nullptr, nullptr, 0, 0, 0, Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, stream);
+        rc = fq_append_kv_turbo(c, layer, seen, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, stream);
         if (rc != FQ_OK) return rc;
     }
     const int now = seen + n_new;

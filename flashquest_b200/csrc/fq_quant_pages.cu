@@ -18,22 +18,6 @@
 
 namespace fq {
 
-template <typename T> struct Q2;
-template <> struct Q2<__half> {
-    using type = __half2;
-    __device__ static float2 f2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
-    __device__ static uint32_t mn(uint32_t a, uint32_t b) { uint32_t r; asm("min.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
-    __device__ static uint32_t mx(uint32_t a, uint32_t b) { uint32_t r; asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
-    static constexpr uint32_t POS_INF = 0x7c007c00u;
-};
-template <> struct Q2<__nv_bfloat16> {
-    using type = __nv_bfloat162;
-    __device__ static float2 f2(uint32_t u) { return make_float2(bf16_lo(u), bf16_hi(u)); }
-    __device__ static uint32_t mn(uint32_t a, uint32_t b) { uint32_t r; asm("min.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
-    __device__ static uint32_t mx(uint32_t a, uint32_t b) { uint32_t r; asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
-    static constexpr uint32_t POS_INF = 0x7f807f80u;
-};
-
 __device__ __forceinline__ float rcp_approx(float x) { float y; asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 // max(|a|, |b|, c), NaN if any is NaN
 __device__ __forceinline__ float absmax_nan(float a, float b, float c) {
@@ -175,17 +159,7 @@ __global__ void __launch_bounds__(128, 4) quant_pages_kernel(QuantPagesParams p)
             for (int j = 0; j < 4; ++j) {
                 m2[j] = Q2<T>::f2(mn[j]);
                 const float2 hi = Q2<T>::f2(mx[j]);
-                // scale arithmetic in the input dtype.  The quotient of a T value by 15 or 255, rounded to T, from the
-                // product with the rounded reciprocal and one residual step: equal for every T value (checked
-                // exhaustively on the host); an infinite range takes the division
-                float d[2] = {Dt<T>::rn(__fsub_rn(hi.x, m2[j].x)), Dt<T>::rn(__fsub_rn(hi.y, m2[j].y))}, s[2];
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const float q0 = __fmul_rn(d[e], RTOP);
-                    float q = __fmaf_rn(__fmaf_rn(-q0, TOP, d[e]), RTOP, q0);
-                    if (!(d[e] <= 3.0e38f)) q = d[e];
-                    s[e] = fmaxf(Dt<T>::rn(q), eps);
-                }
+                const float s[2] = {page_scale<T>(hi.x, m2[j].x, TOP, RTOP, eps), page_scale<T>(hi.y, m2[j].y, TOP, RTOP, eps)};
                 sc[j] = make_float2(s[0], s[1]);
                 rs[j] = make_float2(rcp_approx(s[0]), rcp_approx(s[1]));
             }

@@ -18,6 +18,33 @@ struct QuantPagesParams {
     int zero_rest;                           // also zero the staging rows behind them
 };
 
+template <typename T> struct Q2;
+template <> struct Q2<__half> {
+    using type = __half2;
+    __device__ static float2 f2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
+    __device__ static uint32_t mn(uint32_t a, uint32_t b) { uint32_t r; asm("min.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+    __device__ static uint32_t mx(uint32_t a, uint32_t b) { uint32_t r; asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+    static constexpr uint32_t POS_INF = 0x7c007c00u;
+};
+template <> struct Q2<__nv_bfloat16> {
+    using type = __nv_bfloat162;
+    __device__ static float2 f2(uint32_t u) { return make_float2(bf16_lo(u), bf16_hi(u)); }
+    __device__ static uint32_t mn(uint32_t a, uint32_t b) { uint32_t r; asm("min.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+    __device__ static uint32_t mx(uint32_t a, uint32_t b) { uint32_t r; asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+    static constexpr uint32_t POS_INF = 0x7f807f80u;
+};
+
+// Scale of a page's channel, in the input dtype: max(rn(rn(hi - lo) / top), eps).  The quotient of a T value by 15 or 255,
+// rounded to T, from the product with the rounded reciprocal and one residual step: equal for every T value (checked
+// exhaustively on the host); an infinite range takes the division.
+template <typename T>
+__device__ __forceinline__ float page_scale(float hi, float lo, float top, float rtop, float eps) {
+    const float d = Dt<T>::rn(__fsub_rn(hi, lo)), q0 = __fmul_rn(d, rtop);
+    float q = __fmaf_rn(__fmaf_rn(-q0, top, d), rtop, q0);
+    if (!(d <= 3.0e38f)) q = d;
+    return fmaxf(Dt<T>::rn(q), eps);
+}
+
 // Whether the kernel takes this call (else: the general kernels).
 bool quant_pages_supported(const QuantPagesParams& p, int dtype);
 int quant_pages_launch(const QuantPagesParams& p, int dtype, void* stream, const char* fn);

@@ -6,7 +6,7 @@
 // exchange with lane ^ (stride / values-per-lane) by shuffle.  Every stage is rounded to the
 // tensor's dtype exactly as the reference's eager ops do (kernel/wht.py:26-41), so results are
 // bit-identical.  HBM-bound: D*sizeof(T) in, 3*D/8 + 2 bytes out per token.
-#include "fq_common.cuh"
+#include "fq_quant_pages.cuh"
 
 namespace fq {
 
@@ -142,13 +142,19 @@ __global__ void __launch_bounds__(128) wht_kernel(const T* __restrict__ x, T* __
 }
 
 struct TurboParams {
-    const void *head, *nw;                       // token stream: head[0:n_head] ++ new
+    // token streams head[0:n_head] ++ new; the packed kernel takes K and V in one launch (n_streams 2), the other one stream 0
+    const void *head[2], *nw[2];
     int64_t hd_sb, hd_sh, hd_ss, nw_sb, nw_sh, nw_ss;
-    int n_head, n_quant, D;
-    uint8_t *msb, *lsb;                          // (B,H,n,D/8), (B,H,n,D/4)
+    int n_streams, n_head, n_quant, D;
+    uint8_t *msb[2], *lsb[2];                    // (B,H,n,D/8), (B,H,n,D/4)
     int64_t ms_sb, ms_sh, ms_ss, ls_sb, ls_sh, ls_ss;
-    uint16_t* scale;                             // (B,H,n) bf16
+    uint16_t* scale[2];                          // (B,H,n) bf16
     int64_t sc_sb, sc_sh, sc_ss;
+    // with pages of 16 tokens: minimum and scale of stream 0 per page and channel (null: none), and the rows
+    // behind n_quant written to the head buffers
+    uint16_t *raw_scale, *raw_mn;
+    int64_t km_sb, km_sh, km_sp;
+    int n_stage;
 };
 
 // quantize_k_turbo / quantize_v_turbo without the raw page metadata
@@ -167,8 +173,8 @@ __global__ void __launch_bounds__(128) turbo_quant_kernel(TurboParams p) {
     if (t >= p.n_quant) return;
     const int D = p.D;
     const T* row = t < p.n_head
-        ? static_cast<const T*>(p.head) + b * p.hd_sb + h * p.hd_sh + (int64_t)t * p.hd_ss
-        : static_cast<const T*>(p.nw) + b * p.nw_sb + h * p.nw_sh + (int64_t)(t - p.n_head) * p.nw_ss;
+        ? static_cast<const T*>(p.head[0]) + b * p.hd_sb + h * p.hd_sh + (int64_t)t * p.hd_ss
+        : static_cast<const T*>(p.nw[0]) + b * p.nw_sb + h * p.nw_sh + (int64_t)(t - p.n_head) * p.nw_ss;
     float v[EPL];
     load_row<T, EPL>(row, lane, D, v);
     wht_lanes<T, EPL>(v, lane, D);
@@ -197,8 +203,8 @@ __global__ void __launch_bounds__(128) turbo_quant_kernel(TurboParams p) {
         const int k = nearest(__fdiv_rn(v[j], s), d0, d1);
         idx[j] = (unsigned)(k + (d1 < d0 ? 1 : 0));
     }
-    uint8_t* msb = p.msb + b * p.ms_sb + h * p.ms_sh + (int64_t)t * p.ms_ss;
-    uint8_t* lsb = p.lsb + b * p.ls_sb + h * p.ls_sh + (int64_t)t * p.ls_ss;
+    uint8_t* msb = p.msb[0] + b * p.ms_sb + h * p.ms_sh + (int64_t)t * p.ms_ss;
+    uint8_t* lsb = p.lsb[0] + b * p.ls_sb + h * p.ls_sh + (int64_t)t * p.ls_ss;
     if constexpr (EPL == 4) {
         // lane = channels 4l..4l+3: exactly one byte of the 2-bit plane, half a byte of the 1-bit plane
         unsigned l8 = 0, m4 = 0;
@@ -228,7 +234,7 @@ __global__ void __launch_bounds__(128) turbo_quant_kernel(TurboParams p) {
             lsb[k] = (uint8_t)m;
         }
     }
-    if (lane == 0) p.scale[b * p.sc_sb + h * p.sc_sh + (int64_t)t * p.sc_ss] = f32_to_bf16_bits(s);
+    if (lane == 0) p.scale[0][b * p.sc_sb + h * p.sc_sh + (int64_t)t * p.sc_ss] = f32_to_bf16_bits(s);
 }
 
 // The same coding for the shape that matters (head_dim 128, 16-bit values, 8-byte aligned rows); results are bit-identical
@@ -247,6 +253,7 @@ __global__ void __launch_bounds__(128) turbo_quant_kernel(TurboParams p) {
 //  * a token whose two signs disagree at a threshold (an exact tie of the fp32 distances), or whose scale is not finite,
 //    takes the value-by-value path.
 // 32 768 tokens x 8 heads (67 MB of fp16): 77 us with a warp per token, 34 us so (2.3 TB/s).
+// In an append K, V, the page extrema and the staged rows are one launch: 32 768 tokens 113 -> 75 us (three launches read K twice).
 
 // The reference's own decision (kernel/kv_quant.py:253-279): fp32 quotient, fp32 distances, first index on ties.
 // Out of line: it runs for a few values in 10^4 and should not lengthen the loop body.
@@ -294,17 +301,18 @@ __global__ void __launch_bounds__(TQ_WARPS * 32, 6) turbo_quant128_kernel(TurboP
     __shared__ __align__(16) uint8_t s_m[TQ_WARPS][TQ_TOK][16], s_l[TQ_WARPS][TQ_TOK][32];
     __shared__ uint32_t s_x[TQ_WARPS][16][32];     // the value-by-value path's copy of a warp's packed values
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 3, r = lane >> 2;
-    const int b = blockIdx.z, h = blockIdx.y;
+    const int which = p.n_streams == 2 ? blockIdx.z & 1 : 0, b = p.n_streams == 2 ? blockIdx.z >> 1 : blockIdx.z, h = blockIdx.y;
     const int t0 = (blockIdx.x * TQ_WARPS + warp) * TQ_TOK * iters;
-    const T* head = static_cast<const T*>(p.head) + b * p.hd_sb + h * p.hd_sh;
-    const T* nw = static_cast<const T*>(p.nw) + b * p.nw_sb + h * p.nw_sh;
-    uint8_t* msb = p.msb + b * p.ms_sb + h * p.ms_sh;
-    uint8_t* lsb = p.lsb + b * p.ls_sb + h * p.ls_sh;
-    uint16_t* scale = p.scale + b * p.sc_sb + h * p.sc_sh;
+    const T* head = static_cast<const T*>(p.head[which]) + b * p.hd_sb + h * p.hd_sh;
+    const T* nw = static_cast<const T*>(p.nw[which]) + b * p.nw_sb + h * p.nw_sh;
+    uint8_t* msb = p.msb[which] + b * p.ms_sb + h * p.ms_sh;
+    uint8_t* lsb = p.lsb[which] + b * p.ls_sb + h * p.ls_sh;
+    uint16_t* scale = p.scale[which] + b * p.sc_sb + h * p.sc_sh;
 
+    auto row_of = [&](int tok) { return tok < p.n_head ? head + (int64_t)tok * p.hd_ss : nw + (int64_t)(tok - p.n_head) * p.nw_ss; };
     auto load_row = [&](int tok, uint4 (&raw)[4]) {
         tok = min(tok, p.n_quant - 1);
-        const T* row = (tok < p.n_head ? head + (int64_t)tok * p.hd_ss : nw + (int64_t)(tok - p.n_head) * p.nw_ss) + 8 * t;
+        const T* row = row_of(tok) + 8 * t;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (vec_in) raw[j] = __ldg(reinterpret_cast<const uint4*>(row + 32 * j));
@@ -315,6 +323,36 @@ __global__ void __launch_bounds__(TQ_WARPS * 32, 6) turbo_quant128_kernel(TurboP
         }
     };
     if (t0 >= p.n_quant) return;
+    if (p.raw_scale != nullptr && which == 0 && t0 % 16 == 0) {
+        // the page's extrema, as quant_pages_kernel computes them; these reads bring the rows in for the coding below
+        const int half = lane >> 4, c = lane & 15;
+        uint4 u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) u[i] = __ldg(reinterpret_cast<const uint4*>(row_of(t0 + 2 * i + half)) + c);
+        uint32_t mn[4] = {u[0].x, u[0].y, u[0].z, u[0].w}, mx[4] = {u[0].x, u[0].y, u[0].z, u[0].w};
+#pragma unroll
+        for (int i = 1; i < 8; ++i) {
+            const uint32_t w[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { mn[j] = Q2<T>::mn(mn[j], w[j]); mx[j] = Q2<T>::mx(mx[j], w[j]); }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            mn[j] = Q2<T>::mn(mn[j], __shfl_xor_sync(0xffffffffu, mn[j], 16));
+            mx[j] = Q2<T>::mx(mx[j], __shfl_xor_sync(0xffffffffu, mx[j], 16));
+        }
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                              // lanes 0..15 the scales, 16..31 the minima
+            const float2 lo = Q2<T>::f2(mn[j]), hi = Q2<T>::f2(mx[j]);
+            const float eps = Dt<T>::rn(1e-6f);
+            const float ox = half ? lo.x : page_scale<T>(hi.x, lo.x, 15.0f, 1.0f / 15.0f, eps);
+            const float oy = half ? lo.y : page_scale<T>(hi.y, lo.y, 15.0f, 1.0f / 15.0f, eps);
+            o[j] = f32_to_bf16_bits(ox) | ((uint32_t)f32_to_bf16_bits(oy) << 16);
+        }
+        const int64_t mo = b * p.km_sb + h * p.km_sh + (int64_t)(t0 >> 4) * p.km_sp + 8 * c;
+        *reinterpret_cast<uint4*>((half ? p.raw_mn : p.raw_scale) + mo) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
     uint4 raw[4];
     load_row(t0 + r, raw);
     const uint32_t one = IS_HALF ? 0x3c003c00u : 0x3f803f80u;
@@ -441,6 +479,39 @@ __global__ void __launch_bounds__(TQ_WARPS * 32, 6) turbo_quant128_kernel(TurboP
             }
         }
     }
+    if (p.n_stage > 0 && blockIdx.x == 0 && warp < 2) {
+        // the rows behind the last page become the staged ones, once the first page's warps have read those before
+        if (iters == 1) asm volatile("bar.sync 1, 64;" ::: "memory");
+        if (warp == 0) {
+            T* st = const_cast<T*>(head);
+            for (int i = lane >> 4; i < p.n_stage; i += 2)
+                *(reinterpret_cast<uint4*>(st + (int64_t)i * p.hd_ss) + (lane & 15)) = *(reinterpret_cast<const uint4*>(nw + (int64_t)(p.n_quant - p.n_head + i) * p.nw_ss) + (lane & 15));
+        }
+    }
+}
+
+// The packed kernel, where it takes the rows: head_dim 128, 16-bit values, 8-byte aligned rows (16 bytes for the page
+// extrema and the staging).  Returns false if it does not.
+static bool turbo_launch128(const TurboParams& p, int dtype, int B, int H, cudaStream_t st) {
+    auto vec = [](const void* q, int64_t m, int64_t n, int64_t a, int64_t b, int64_t c) { return q == nullptr || (aligned(q, m) && a % n == 0 && b % n == 0 && c % n == 0); };
+    bool in8 = true, in16 = true, out16 = true;
+    for (int i = 0; i < p.n_streams; ++i) {
+        in8 = in8 && vec(p.head[i], 8, 4, p.hd_sb, p.hd_sh, p.hd_ss) && vec(p.nw[i], 8, 4, p.nw_sb, p.nw_sh, p.nw_ss);
+        in16 = in16 && vec(p.head[i], 16, 8, p.hd_sb, p.hd_sh, p.hd_ss) && vec(p.nw[i], 16, 8, p.nw_sb, p.nw_sh, p.nw_ss);
+        out16 = out16 && vec(p.msb[i], 16, 16, p.ms_sb, p.ms_sh, p.ms_ss) && vec(p.lsb[i], 16, 16, p.ls_sb, p.ls_sh, p.ls_ss);
+    }
+    const bool pages = p.raw_scale != nullptr || p.n_stage > 0;
+    if (p.D != 128 || dtype == FQ_F32 || !in8 || (pages && !(in16 && vec(p.raw_scale, 16, 8, p.km_sb, p.km_sh, p.km_sp) && aligned(p.raw_mn, 16)))) return false;
+    if ((int64_t)B * p.n_streams > 65535) return false;
+    // tiles of 8 tokens per warp: one until every warp slot of the chip is taken, then two (the second one's rows are
+    // in flight while the first is coded; with four the last wave costs more: 34.2 against 36.3 us at 262 144 rows)
+    const int64_t tiles = (int64_t)((p.n_quant + TQ_TOK - 1) / TQ_TOK) * B * H * p.n_streams;
+    const int iters = tiles > 148 * 24 ? 2 : 1;
+    const int per_cta = TQ_WARPS * TQ_TOK * iters;
+    dim3 grid((unsigned)((p.n_quant + per_cta - 1) / per_cta), (unsigned)H, (unsigned)(B * p.n_streams));
+    if (dtype == FQ_F16) turbo_quant128_kernel<__half><<<grid, TQ_WARPS * 32, 0, st>>>(p, iters, in16, out16);
+    else turbo_quant128_kernel<__nv_bfloat16><<<grid, TQ_WARPS * 32, 0, st>>>(p, iters, in16, out16);
+    return true;
 }
 
 // dequantize_k_turbo / dequantize_v_turbo (kernel/kv_quant.py:366-378, :408-420):
@@ -544,30 +615,15 @@ extern "C" int fq_quantize_turbo(
     if (n_quant == 0) return FQ_OK;
     FQ_CHECK_ARG(msb && lsb && scale && (nw || n_new == 0) && (head || n_head == 0), FQ_ERR_ARG, "%s: null pointer", fn);
     FQ_CHECK_ARG(B <= 65535 && H <= 65535, FQ_ERR_ARG, "%s: B and H must be <= 65535", fn);
-    TurboParams p;
-    p.head = head; p.nw = nw; p.hd_sb = hd_sb; p.hd_sh = hd_sh; p.hd_ss = hd_ss;
+    TurboParams p{};
+    p.n_streams = 1; p.head[0] = head; p.nw[0] = nw; p.hd_sb = hd_sb; p.hd_sh = hd_sh; p.hd_ss = hd_ss;
     p.nw_sb = nw_sb; p.nw_sh = nw_sh; p.nw_ss = nw_ss; p.n_head = n_head; p.n_quant = n_quant; p.D = D;
-    p.msb = msb; p.lsb = lsb; p.ms_sb = ms_sb; p.ms_sh = ms_sh; p.ms_ss = ms_ss; p.ls_sb = ls_sb; p.ls_sh = ls_sh; p.ls_ss = ls_ss;
-    p.scale = static_cast<uint16_t*>(scale); p.sc_sb = sc_sb; p.sc_sh = sc_sh; p.sc_ss = sc_ss;
+    p.msb[0] = msb; p.lsb[0] = lsb; p.ms_sb = ms_sb; p.ms_sh = ms_sh; p.ms_ss = ms_ss; p.ls_sb = ls_sb; p.ls_sh = ls_sh; p.ls_ss = ls_ss;
+    p.scale[0] = static_cast<uint16_t*>(scale); p.sc_sb = sc_sb; p.sc_sh = sc_sh; p.sc_ss = sc_ss;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    {
-        // head_dim 128, 16-bit values, every row 8-byte aligned: the packed kernel (eight tokens per warp)
-        auto rows8 = [](const void* q, int64_t a, int64_t b2, int64_t c) { return q == nullptr || (aligned(q, 8) && a % 4 == 0 && b2 % 4 == 0 && c % 4 == 0); };
-        if (D == 128 && dtype != FQ_F32 && rows8(head, hd_sb, hd_sh, hd_ss) && rows8(nw, nw_sb, nw_sh, nw_ss)) {
-            auto vec = [](const void* q, int64_t m, int64_t a, int64_t b2, int64_t c) { return q == nullptr || (aligned(q, 16) && a % m == 0 && b2 % m == 0 && c % m == 0); };
-            const int vec_in = vec(head, 8, hd_sb, hd_sh, hd_ss) && vec(nw, 8, nw_sb, nw_sh, nw_ss);
-            const int vec_out = vec(msb, 16, ms_sb, ms_sh, ms_ss) && vec(lsb, 16, ls_sb, ls_sh, ls_ss);
-            // tiles of 8 tokens per warp: one until every warp slot of the chip is taken, then two (the second one's rows are
-            // in flight while the first is coded; with four the last wave costs more: 34.2 against 36.3 us at 262 144 rows)
-            const int64_t tiles = (int64_t)((n_quant + TQ_TOK - 1) / TQ_TOK) * B * H;
-            const int iters = tiles > 148 * 24 ? 2 : 1;
-            const int per_cta = TQ_WARPS * TQ_TOK * iters;
-            dim3 grid8((unsigned)((n_quant + per_cta - 1) / per_cta), (unsigned)H, (unsigned)B);
-            if (dtype == FQ_F16) turbo_quant128_kernel<__half><<<grid8, TQ_WARPS * 32, 0, st>>>(p, iters, vec_in, vec_out);
-            else turbo_quant128_kernel<__nv_bfloat16><<<grid8, TQ_WARPS * 32, 0, st>>>(p, iters, vec_in, vec_out);
-            FQ_CHECK_LAUNCH(fn);
-            return FQ_OK;
-        }
+    if (turbo_launch128(p, dtype, B, H, st)) {
+        FQ_CHECK_LAUNCH(fn);
+        return FQ_OK;
     }
     dim3 grid((unsigned)((n_quant + 3) / 4), (unsigned)H, (unsigned)B);
     if (dtype == FQ_F32) launch_turbo<float>(p, grid, st);
@@ -575,6 +631,52 @@ extern "C" int fq_quantize_turbo(
     else launch_turbo<__nv_bfloat16>(p, grid, st);
     FQ_CHECK_LAUNCH(fn);
     return FQ_OK;
+}
+
+extern "C" int fq_append_kv_turbo(const fq_turbo_cache* c, int layer, int seen, const void* K_new, const void* V_new,
+                                  int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new, void* stream) {
+    using namespace fq;
+    const char* fn = "fq_append_kv_turbo";
+    FQ_CHECK_ARG(c && K_new && V_new, FQ_ERR_ARG, "%s: null pointer", fn);
+    FQ_CHECK_ARG(layer >= 0 && layer < c->L, FQ_ERR_ARG, "%s: layer_idx %d out of range [0, %d)", fn, layer, c->L);
+    FQ_CHECK_ARG(seen >= 0 && n_new > 0 && seen + n_new <= c->max_seq_len, FQ_ERR_ARG, "%s: seen+new=%d exceeds max_seq_len=%d", fn, seen + n_new, c->max_seq_len);
+    const int page = c->page, D = c->D, B = c->B, H = c->Hkv;
+    const int partial = seen % page, n_quant = (partial + n_new) / page * page, tok0 = seen - partial;
+    char* Kt = static_cast<char*>(c->K_partial) + layer * c->pt_sl * 2;
+    char* Vt = static_cast<char*>(c->V_partial) + layer * c->pt_sl * 2;
+    uint16_t* Ksr = static_cast<uint16_t*>(c->K_scale_raw) + layer * c->km_sl + (int64_t)(tok0 / page) * c->km_sp;
+    uint16_t* Kmr = static_cast<uint16_t*>(c->K_mn_raw) + layer * c->km_sl + (int64_t)(tok0 / page) * c->km_sp;
+    if (n_quant > 0) {
+        TurboParams p{};
+        p.n_streams = 2; p.head[0] = Kt; p.head[1] = Vt; p.nw[0] = K_new; p.nw[1] = V_new;
+        p.hd_sb = c->pt_sb; p.hd_sh = c->pt_sh; p.hd_ss = c->pt_ss; p.nw_sb = nw_sb; p.nw_sh = nw_sh; p.nw_ss = nw_ss;
+        p.n_head = partial; p.n_quant = n_quant; p.D = D;
+        const int64_t mo = layer * c->ms_sl + (int64_t)tok0 * c->ms_ss, lo = layer * c->ls_sl + (int64_t)tok0 * c->ls_ss;
+        p.msb[0] = c->K_msb + mo; p.msb[1] = c->V_msb + mo; p.ms_sb = c->ms_sb; p.ms_sh = c->ms_sh; p.ms_ss = c->ms_ss;
+        p.lsb[0] = c->K_lsb + lo; p.lsb[1] = c->V_lsb + lo; p.ls_sb = c->ls_sb; p.ls_sh = c->ls_sh; p.ls_ss = c->ls_ss;
+        p.scale[0] = static_cast<uint16_t*>(c->K_scale_turbo) + layer * c->st_sl + tok0;
+        p.scale[1] = static_cast<uint16_t*>(c->V_scale_turbo) + layer * c->st_sl + tok0;
+        p.sc_sb = c->st_sb; p.sc_sh = c->st_sh; p.sc_ss = 1;
+        if (page == 16) {
+            p.raw_scale = Ksr; p.raw_mn = Kmr; p.km_sb = c->km_sb; p.km_sh = c->km_sh; p.km_sp = c->km_sp;
+            p.n_stage = partial + n_new - n_quant;
+        }
+        if (turbo_launch128(p, c->kv_dtype, B, H, static_cast<cudaStream_t>(stream))) {
+            FQ_CHECK_LAUNCH(fn);
+            if (page == 16) return FQ_OK;
+        } else {
+            for (int i = 0; i < 2; ++i) {
+                const int rc = fq_quantize_turbo(p.head[i], c->pt_sb, c->pt_sh, c->pt_ss, partial, p.nw[i], nw_sb, nw_sh, nw_ss, n_new, c->kv_dtype, B, H, D, n_quant,
+                                                 p.msb[i], c->ms_sb, c->ms_sh, c->ms_ss, p.lsb[i], c->ls_sb, c->ls_sh, c->ls_ss, p.scale[i], c->st_sb, c->st_sh, 1, stream);
+                if (rc != FQ_OK) return rc;
+            }
+        }
+    }
+    // raw per-page K metadata (for scoring) + staging of the left-over tokens, after the launches
+    // above have read the staged head
+    return fq_quantize_kv_int4(Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, partial, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new,
+                               c->kv_dtype, B, H, D, page, n_quant, nullptr, nullptr, 0, 0, 0, Ksr, Kmr, c->km_sb, c->km_sh, c->km_sp,
+                               nullptr, nullptr, 0, 0, 0, Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, stream);
 }
 
 extern "C" int fq_dequantize_turbo(

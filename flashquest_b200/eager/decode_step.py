@@ -14,7 +14,7 @@ import math
 
 import torch
 
-from .._lib import DecodeParams, Int4CacheDesc, TurboCacheDesc, bind, check, dtype_code, lib, ptr, stream_ptr
+from .._lib import DecodeParams, bind, check, dtype_code, lib, ptr, stream_ptr
 
 
 class _NativeSteps:
@@ -148,13 +148,7 @@ class QuestDecodeInt4(_NativeSteps):
         self.workspace = torch.zeros(L, max(self.ws_bytes, 256), dtype=torch.uint8, device=dev)
         self.launches = 0
         # descriptors for the one-call-per-layer entry point
-        c = cache
-        self._cdesc = Int4CacheDesc(
-            c.K_packed.data_ptr(), c.V_packed.data_ptr(), *c.K_packed.stride()[:4],
-            c.K_scale.data_ptr(), c.K_mn.data_ptr(), *c.K_scale.stride()[:4],
-            c.V_scale.data_ptr(), c.V_mn.data_ptr(), *c.V_scale.stride()[:3],
-            c.K_partial.data_ptr(), c.V_partial.data_ptr(), *c.K_partial.stride()[:4],
-            dtype_code(c.K_partial), c.num_layers, self.B, self.Hkv, self.D, self.page, c.max_seq_len)
+        self._cdesc = cache.desc()
         self._prm = DecodeParams(
             self.Hq, self.retention_per_q.data_ptr() if self.retention_per_q is not None else None, self.retention,
             self.k_max_static, self.num_sinks, self.window_pages, self.bucket, self.sm_scale, self.n_split)
@@ -323,14 +317,7 @@ class QuestDecodeTurbo(_NativeSteps):
             self.scratch = torch.empty(lib().fq_decode_layer_turbo_scratch_bytes(self.B, self.Hq, self.D), dtype=torch.uint8, device=dev)
             self.workspace = torch.zeros(max(lib().fq_sparse_decode_workspace_bytes(self.B, self.Hq, self.D, self.n_split), 256),
                                          dtype=torch.uint8, device=dev)
-        c = cache
-        self._cdesc = TurboCacheDesc(
-            c.K_msb.data_ptr(), c.K_lsb.data_ptr(), c.V_msb.data_ptr(), c.V_lsb.data_ptr(),
-            *c.K_msb.stride()[:4], *c.K_lsb.stride()[:4],
-            c.K_scale_turbo.data_ptr(), c.V_scale_turbo.data_ptr(), *c.K_scale_turbo.stride()[:3],
-            c.K_scale_raw.data_ptr(), c.K_mn_raw.data_ptr(), *c.K_scale_raw.stride()[:4],
-            c.K_partial.data_ptr(), c.V_partial.data_ptr(), *c.K_partial.stride()[:4],
-            dtype_code(c.K_partial), c.num_layers, self.B, self.Hkv, self.D, self.page, c.max_seq_len)
+        self._cdesc = cache.desc()
         self._prm = DecodeParams(self.Hq, None, self.retention, self.k_max_static, self.num_sinks, self.window_pages,
                                  self.bucket, self.sm_scale, self.n_split)
         self.launches = 0

@@ -552,6 +552,11 @@ int fq_decode_layer_int8(
     float* scores, int32_t* compact, void* O, float* lse,
     void* workspace, size_t workspace_bytes, void* stream);
 
+/* The append of an INT4 cache alone (cache/persistent_int4.py:69-132): any number of tokens behind the `seen` ones; whole
+ * pages are coded, the rest is staged.  fq_append_kv_turbo is the same for a TurboQuant cache (persistent_turbo.py:83-147). */
+int fq_append_kv_int4(const fq_int4_cache* cache, int layer, int seen, const void* K_new, const void* V_new,
+                      int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new, void* stream);
+
 /* Rotary embedding of one new token as Hugging Face's apply_rotary_pos_emb computes it (x*cos + rotate_half(x)*sin, each
  * product and the sum rounded to `dtype`), then cast to out_dtype; v is only cast.  q (B,Hq*D), k, v (B,Hkv*D) with batch
  * strides, cos, sin (B,D) with batch strides (0: shared); outputs dense.  D even, at most 128; fp16 / bf16. */
@@ -585,6 +590,8 @@ typedef struct fq_turbo_cache {
     int kv_dtype;                                  /* FQ_F16 | FQ_BF16 */
     int L, B, Hkv, D, page, max_seq_len;
 } fq_turbo_cache;
+int fq_append_kv_turbo(const fq_turbo_cache* cache, int layer, int seen, const void* K_new, const void* V_new,
+                       int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new, void* stream);
 size_t fq_decode_layer_turbo_scratch_bytes(int B, int Hq, int D);
 int fq_decode_layer_turbo(
     const fq_turbo_cache* cache, int layer, int seen,

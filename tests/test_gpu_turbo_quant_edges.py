@@ -39,3 +39,30 @@ def test_equals_warp_per_token(dtype, n, offset, stride_out):
     odd.copy_(x)
     for a, b in zip(_quant(fast, stride_out), _quant(odd)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("page", [16, 32])
+@pytest.mark.parametrize("pieces", [(1, 15, 16, 1), (5, 30, 300), (20, 12, 3, 2049)])
+def test_append_pieces(page, pieces):
+    """The one-launch append (planes, page metadata, staging), piece by piece, against the whole stream through the general kernels."""
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    from flashquest_b200.kernel.kv_quant import quantize_k_turbo
+    g = torch.Generator(device="cuda").manual_seed(sum(pieces))
+    c = PersistentTurboKVCache(batch_size=2, num_layers=2, num_kv_heads=3, head_dim=128, max_seq_len=4096, page_size=page, dtype=torch.float16)
+    K, V = (torch.randn(2, 3, sum(pieces), 128, device="cuda", generator=g).half() for _ in range(2))
+    at = 0
+    for n in pieces:
+        c.update_quantized(K[:, :, at:at + n], V[:, :, at:at + n], 1)
+        at += n
+        done = at // page * page
+        w = c.get_views(1)
+        assert torch.equal(w["K_partial"], K[:, :, done:at]) and torch.equal(w["V_partial"], V[:, :, done:at])
+        if not done:
+            continue
+        odd = torch.empty(2, 2, 3, done, 129, dtype=torch.float16, device="cuda")[..., 1:]
+        odd[0].copy_(K[:, :, :done]), odd[1].copy_(V[:, :, :done])
+        for name, x in (("K", odd[0]), ("V", odd[1])):
+            m, l, sc = _quant(x)
+            assert torch.equal(w[name + "_msb"], m) and torch.equal(w[name + "_lsb"], l) and torch.equal(w[name + "_scale_turbo"][..., 0], sc)
+        _, _, _, sr, mr = quantize_k_turbo(K[:, :, :done].contiguous(), page)
+        assert torch.equal(w["K_scale_raw"], sr) and torch.equal(w["K_mn_raw"], mr)
