@@ -35,10 +35,10 @@ int fail(int code, const char* fmt, ...);
 // previous kernel) and block in pdl_wait() until the previous kernel has completed and its
 // writes are visible.  pdl_trigger() comes right after the wait in every kernel, so at most
 // two kernels of a chain overlap and whatever a kernel reads before its wait must have been
-// written at least two kernels earlier.  All kernels get the attribute but the selection kernel,
-// which measured 3 us slower per launch when it was made resident early beside the scoring kernel.
-enum { PDL_SCORES = 1, PDL_SELECT = 2, PDL_ATTN = 4, PDL_QUANT = 8, PDL_GEMV = 16 };
-constexpr bool pdl_enabled(int kind) { return kind != PDL_SELECT; }
+// written at least two kernels earlier.  All kernels get the attribute but the selection of rows of
+// more than 8192 pages, whose CTAs of 1024 threads and up to 192 KB, resident early, took the scoring kernel's place (3 us).
+enum { PDL_SCORES = 1, PDL_SELECT = 2, PDL_ATTN = 4, PDL_QUANT = 8, PDL_GEMV = 16, PDL_SELECT_LONG = 32 };
+constexpr bool pdl_enabled(int kind) { return kind != PDL_SELECT_LONG; }
 
 template <typename... KP, typename... A>
 inline cudaError_t launch_k(int kind, void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
