@@ -108,13 +108,92 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_early_kernel(
     }
 }
 
+// page_scores_kernel for many pages (thousands per SM): CTAs stay and stream.  Each warp runs its own cp.async ring of
+// SCORE_RING units of four pages (2 KiB at head_dim 128), so 16 warps keep 64 KiB and more per SM on the way while q stays
+// in registers; the short-lived CTAs of the kernel above start with two latencies in a row (37 us against 20 of HBM time for 134 MB).
+// 16 x 8 rows of 2048 pages 35.0 -> 24.6 us, of
+// 8191 133.9 -> 88.0 (6.1 TB/s); a ring of 4 or 6 units is no faster (25.2, 26.2).
+constexpr int SCORE_RING = 3, SCORE_STREAM_CTAS = 4 * 148;
+
+template <typename QT, int NR, int CH>
+__global__ void __launch_bounds__(SCORE_THREADS, NR > 3 ? 3 : 4) page_scores_stream_kernel(
+    const QT* __restrict__ Q, int64_t q_sb, int64_t q_sh,
+    const uint16_t* __restrict__ K_scale, const uint16_t* __restrict__ K_mn,
+    int64_t km_sb, int64_t km_sh, int64_t km_sp,
+    int Hq, int Hkv, int P, int head_off,
+    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, const int* __restrict__ pos, int pos_new, int pos_page, float levels) {
+    constexpr int CHUNKS = 8 * CH;                         // 16-byte chunks per metadata row
+    __shared__ __align__(16) uint4 ring[SCORE_THREADS / 32][SCORE_RING][4][2][CHUNKS];
+    const int b = blockIdx.z, hkv = blockIdx.y;
+    const int n_rep = Hq / Hkv;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int l = lane & 7, qw = lane >> 3;
+    const int nr = min(NR, n_rep - head_off);
+    pdl_wait();        // Q and the newest metadata row come from the kernels before this one
+    pdl_trigger();
+    if (pos) P = min(P, (*pos + pos_new) / pos_page);
+    const int units = (P + 3) >> 2, per = (units + gridDim.x - 1) / gridDim.x;
+    const int u_end = min(units, (int)(blockIdx.x + 1) * per);
+    int u = blockIdx.x * per + warp;
+    const uint16_t* sc_base = K_scale + b * km_sb + hkv * km_sh + 8 * l;
+    const uint16_t* mn_base = K_mn + b * km_sb + hkv * km_sh + 8 * l;
+    auto issue = [&](int unit, int slot) {
+        const int p = 4 * unit + qw;
+        if (unit < u_end && p < P) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&ring[warp][slot][qw][0][l + 8 * c])), "l"(mn_base + (int64_t)p * km_sp + 64 * c) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&ring[warp][slot][qw][1][l + 8 * c])), "l"(sc_base + (int64_t)p * km_sp + 64 * c) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < SCORE_RING - 1; ++i) issue(u + 4 * i, i);
+    float q[NR][CH][8];
+    score_load_q<QT, NR, CH>(Q + b * q_sb, q_sh, hkv * n_rep + head_off, nr, l, CHUNKS, q);
+    float* srow = scores + b * sc_sb + (hkv * n_rep + head_off + min(l, nr - 1)) * sc_sh;
+    int slot = 0;
+    for (; u < u_end; u += 4) {
+        issue(u + 4 * (SCORE_RING - 1), (slot + SCORE_RING - 1) % SCORE_RING);
+        asm volatile("cp.async.wait_group %0;" ::"n"(SCORE_RING - 1) : "memory");     // a lane reads only what it copied itself
+        uint4 m4[CH], s4[CH];
+#pragma unroll
+        for (int c = 0; c < CH; ++c) { m4[c] = ring[warp][slot][qw][0][l + 8 * c]; s4[c] = ring[warp][slot][qw][1][l + 8 * c]; }
+        const float v = score_page<NR, CH>(q, m4, s4, l, levels);
+        const int p = 4 * u + qw;
+        if (p < P && l < nr) srow[p] = v;
+        slot = (slot + 1) % SCORE_RING;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// CTAs per (batch, kv head) row of the streaming kernel: whole waves of resident CTAs, at least 64 pages each
+static int score_stream_ctas(int rows, int P) {
+    int best = 1;
+    double best_t = 1e30;
+    for (int c = 1; c <= 64 && c * 64 <= P; ++c) {
+        const double t = (double)((rows * (int64_t)c + SCORE_STREAM_CTAS - 1) / SCORE_STREAM_CTAS) / c * (1.0 + 0.004 * c);
+        if (t < best_t) { best_t = t; best = c; }
+    }
+    return best;
+}
+
 template <typename QT, int NR>
 static void launch_scores(int CH, dim3 grid, cudaStream_t st, const void* Q, int64_t q_sb, int64_t q_sh,
                           const void* K_scale, const void* K_mn, int64_t km_sb, int64_t km_sh, int64_t km_sp,
                           int Hq, int Hkv, int P, int D, int head_off, float* scores, int64_t sc_sb, int64_t sc_sh, const DynPos& dp, float levels) {
+    // 64 pages per resident CTA and more: below that the ring never fills and the short CTAs start sooner
+    const int rows = (int)(grid.y * grid.z);
+    const int stream_ctas = (D == 128 || D == 64) && (int64_t)rows * P >= (int64_t)SCORE_STREAM_CTAS * 64 ? score_stream_ctas(rows, P) : 0;
 #define FQ_LAUNCH_SC(CHV)                                                                              \
     do {                                                                                               \
-        if (dp.pos != nullptr && dp.early)                                                             \
+        if (stream_ctas > 0)                                                                           \
+            launch_k(PDL_SCORES, page_scores_stream_kernel<QT, NR, (CHV > 2 ? 2 : CHV)>, dim3((unsigned)stream_ctas, grid.y, grid.z), dim3(SCORE_THREADS), 0, st, \
+                     static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale),     \
+                     static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P, head_off, scores, sc_sb, sc_sh, \
+                     dp.pos, dp.n_new, dp.page, levels);                                               \
+        else if (dp.pos != nullptr && dp.early)                                                             \
             launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV>, grid, dim3(SCORE_THREADS), 0, st,              \
                      static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale),     \
                      static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P, D, head_off, scores, sc_sb, sc_sh, \
