@@ -56,7 +56,7 @@ __device__ __forceinline__ void rv_pairs(uint32_t wa, uint32_t wb, uint32_t (&h)
 template <bool INTERLEAVED>
 __global__ void __launch_bounds__(RV_THREADS, 2) awq_regv_kernel(const __grid_constant__ RvParams p) {
     extern __shared__ __align__(16) unsigned char rv_smem[];
-    __shared__ float s_red[RV_WARPS];
+    __shared__ float s_red[8][RV_WARPS];                        // sums of squares: CTA of the cluster, warp
     __shared__ __half2 s_cs[64];                                 // (cos, sin) of channel pair i
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int rank = blockIdx.x, tile_first = blockIdx.y * p.tiles_per_cta, n_tiles = min(p.tiles_per_cta, p.tiles_total - tile_first);
@@ -118,12 +118,17 @@ __global__ void __launch_bounds__(RV_THREADS, 2) awq_regv_kernel(const __grid_co
     // ---- the CTA's k range of the input, through the operator in front of the linear ----
     union V8 { uint4 u; __half2 h[4]; };
     if (p.pro_kind == FQ_GEMV_ADD_RMSNORM) {
-        // wr warps per row: h = x (+ b), its sum of squares over the whole row; h of the own range goes to shared memory
-        const int wr = M == 1 ? 8 : M == 2 ? 4 : M <= 4 ? 2 : 1, m = warp / wr, ws = warp - m * wr, n8 = p.K >> 3;
+        // wr warps per row: h = x (+ b) of the CTA's own k range goes to shared memory; the sum of squares covers the whole
+        // row.  From three rows on each CTA of the cluster sums its own range and they exchange the sums: reading whole rows
+        // everywhere is 44 MB of L2 traffic per launch at 8 rows of 3072 (a batch-8 token 2497 -> 2406 us), while for one
+        // row the exchange costs more than the 12 KB it saves (a single-row token 1983 -> 2020 us).
+        const bool share = p.ks > 1 && M > 2;
+        const int wr = M == 1 ? 8 : M == 2 ? 4 : M <= 4 ? 2 : 1, m = warp / wr, ws = warp - m * wr;
+        const int k_lo = share ? k_first : 0, n8 = (share ? k_len : p.K) >> 3;
         float ss = 0.f;
         if (m < M) {
-            const uint4* xa = reinterpret_cast<const uint4*>(p.x + (int64_t)m * p.K);
-            const uint4* xb = p.pro_b ? reinterpret_cast<const uint4*>(p.pro_b + (int64_t)m * p.K) : nullptr;
+            const uint4* xa = reinterpret_cast<const uint4*>(p.x + (int64_t)m * p.K + k_lo);
+            const uint4* xb = p.pro_b ? reinterpret_cast<const uint4*>(p.pro_b + (int64_t)m * p.K + k_lo) : nullptr;
 #pragma unroll 4
             for (int k8 = ws * 32 + lane; k8 < n8; k8 += 32 * wr) {
                 V8 a;
@@ -134,10 +139,10 @@ __global__ void __launch_bounds__(RV_THREADS, 2) awq_regv_kernel(const __grid_co
 #pragma unroll
                     for (int j = 0; j < 4; ++j) a.h[j] = __hadd2(a.h[j], b.h[j]);
                 }
-                const int kk = 8 * k8 - k_first;
+                const int kk = k_lo + 8 * k8 - k_first;
                 if (kk >= 0 && kk < k_len) {
                     *reinterpret_cast<uint4*>(s_x + m * xstride + kk) = a.u;
-                    if (p.pro_out && blockIdx.y == 0) *reinterpret_cast<uint4*>(p.pro_out + (int64_t)m * p.K + 8 * k8) = a.u;
+                    if (p.pro_out && blockIdx.y == 0) *reinterpret_cast<uint4*>(p.pro_out + (int64_t)m * p.K + k_first + kk) = a.u;
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { const float2 f = __half22float2(a.h[j]); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss); }
@@ -145,12 +150,24 @@ __global__ void __launch_bounds__(RV_THREADS, 2) awq_regv_kernel(const __grid_co
         }
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-        if (lane == 0) s_red[warp] = ss;
-        __syncthreads();
+        if (share) {
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster runs
+            if (lane < p.ks) {
+                uint32_t at = (uint32_t)__cvta_generic_to_shared(&s_red[rank][warp]);
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(at), "r"(lane));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(ss) : "memory");
+            }
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else {
+            if (lane == 0) s_red[0][warp] = ss;
+            __syncthreads();
+        }
         for (int i = tid; i < M * (k_len / 8); i += RV_THREADS) {
             const int r = i / (k_len / 8), k8 = i - r * (k_len / 8);
             float tot = 0.f;
-            for (int j = 0; j < wr; ++j) tot += s_red[r * wr + j];
+            for (int c = 0; c < (share ? p.ks : 1); ++c)
+                for (int j = 0; j < wr; ++j) tot += s_red[c][r * wr + j];
             const float inv = rsqrtf(tot / (float)p.K + p.eps);
             V8 a, wt;
             a.u = *reinterpret_cast<const uint4*>(s_x + r * xstride + 8 * k8);
@@ -188,7 +205,7 @@ __global__ void __launch_bounds__(RV_THREADS, 2) awq_regv_kernel(const __grid_co
         }
     }
     __syncthreads();
-    if (p.ks > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // every CTA of the cluster runs
+    if (p.ks > 1 && !(p.pro_kind == FQ_GEMV_ADD_RMSNORM && M > 2)) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // every CTA of the cluster runs
 
     float* part = s_part + (size_t)warp * M * RV_TOK;
     for (int u = 0; u < n_tiles; ++u) {
