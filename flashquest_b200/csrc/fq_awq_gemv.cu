@@ -24,7 +24,7 @@
 // column of its partial tile into the shared memory of the CTA that finishes that column, which adds
 // the partial sums in rank order after one cluster barrier — no global round trip, no atomics, a
 // fixed summation order, and the epilogue (bias, rounding, rotary embedding) spread over the cluster.
-#include "fq_awq_regv.cuh"
+#include "fq_common.cuh"
 
 #include <cooperative_groups.h>
 
@@ -507,14 +507,6 @@ extern "C" int fq_awq_gemv_fused(
     FQ_CHECK_ARG(aligned(x, 16), FQ_ERR_ALIGN, "%s: x must be 16-byte aligned", fn);
     FQ_CHECK_ARG(k_split >= 1 && k_split <= GEMV_MAX_CLUSTER && (k_split & (k_split - 1)) == 0, FQ_ERR_ARG,
                  "%s: k_split=%d must be 1, 2, 4 or 8 (the CTAs of one thread-block cluster)", fn, k_split);
-    {
-        RegvCall c{};
-        c.x = x; c.M = M; c.K = K; c.group = group; c.n_proj = n_proj; c.interleaved = interleaved ? 1 : 0; c.pro = pro; c.rope = rope;
-        for (int i = 0; i < n_proj; ++i) {
-            c.qweight[i] = qweight[i]; c.scales[i] = scales[i]; c.qzeros[i] = qzeros[i]; c.bias[i] = bias ? bias[i] : nullptr; c.N[i] = N[i]; c.y[i] = y[i];
-        }
-        if (awq_regv_supported(c)) return awq_regv_launch(c, stream, fn);
-    }
     GemvParams p;
     p.x = static_cast<const __half*>(x); p.M = M; p.K = K; p.group = group; p.n_groups = K / group;
     p.n_proj = n_proj; p.interleaved = interleaved ? 1 : 0;

@@ -1,5 +1,5 @@
 """The AWQ GEMM at the edges of its row tiles and K splits (csrc/fq_awq_skinny.cu, csrc/fq_awq_gemm.cu), and the GEMV
-over its K splits, passes and tiles per CTA (csrc/fq_awq_regv.cu), against a plain
+over its K splits and rows (csrc/fq_awq_gemv.cu), against a plain
 PyTorch product of the fp16-rounded weights, and equal to itself over repeated launches."""
 import pytest
 import torch
@@ -70,3 +70,19 @@ def test_gemv_splits_and_tiles(M, K, Ns, interleaved, bias):
         want = x.float() @ _weights(lin) + (lin.bias.float() if bias else 0)
         assert (y.float() - want).abs().max().item() <= 2e-3 * want.abs().max().item() + 1e-3
     assert all(torch.equal(a, b) for a, b in zip(got, awq_gemv_fused(x, lins)))
+
+
+@pytest.mark.parametrize("rows,H", [(3, 128), (8, 3072), (8, 8192)])
+def test_norm_apart_from_gemv(rows, H):
+    """A decode step's RMSNorm as its own launch in front of the GEMV gives the bits of the one folded into it."""
+    from flashquest_b200._lib import check, lib, ptr, stream_ptr
+    from flashquest_b200.kernel.fused_proj import awq_gemv_fused
+    g = torch.Generator(device="cuda").manual_seed(H)
+    lin = _linear(H, 128, 128, True, False, g)
+    x, d = (torch.randn(rows, H, device="cuda", generator=g).half() for _ in range(2))
+    w = torch.rand(H, device="cuda", generator=g).half()
+    folded = awq_gemv_fused(x, (lin,), add=d, norm_weight=w, eps=1e-5)[0]
+    normed, total = torch.empty_like(x), torch.empty_like(x)
+    check(lib().fq_add_rmsnorm(ptr(x), ptr(d), ptr(w), 1e-5, rows, H, ptr(total), ptr(normed), stream_ptr(x.device)))
+    assert torch.equal(total, x + d)
+    assert torch.equal(awq_gemv_fused(normed, (lin,))[0], folded)
