@@ -1,21 +1,24 @@
-// AWQ W4A16 linears for 1 .. a few hundred rows on tcgen05: decode batches and short prompts.
+// AWQ W4A16 linears for 9 .. a few hundred rows on tcgen05: short prompts.
 //
 // y[M,N] = x[M,K] @ W with W in AutoAWQ's GEMM format.  The work is reading the weights (0.5 byte each) once; the grid of
 // 256-column tiles of the large GEMM leaves most SMs idle at few rows (12 of 148 for 3072 columns) and its three or four
-// stages wait for the TMA latency.  Here a CTA owns 128 columns and up to 128 rows, the K range of a tile is split over a
-// thread-block cluster so that about one CTA per SM is busy, and every kind of data has a ring as deep as its latency asks:
+// stages wait for the TMA latency.  Here a CTA owns 128 columns and up to 128 rows, and every kind of data has a ring as deep
+// as its latency asks:
 //   warp 0       raw weight tiles (128 k x 128 columns = 8 KiB) by TMA, the first ones before the dependency wait (weights
-//                never change); scales and zeros of the whole range by bulk copies
+//                never change); scales and zeros by bulk copies
 //   warp 2       x tiles by TMA (only the live rows are fetched; the MMA reads whatever lies behind them into rows that
 //                nobody looks at, so stages of few rows overlap)
 //   warp 1       tcgen05.mma M 128 (rows) x N 128 x K 16 into one TMEM accumulator
-//   warps 4..11  weights to fp16, (code - zero) * scale rounded once like the large GEMM: one shift, four three-input logic
+//   warps 4 ..   weights to fp16, (code - zero) * scale rounded once like the large GEMM: one shift, four three-input logic
 //                operations, four exact subtractions (an odd nibble's factor of 16 goes with an fma) and four products per
-//                8 weights; two groups of four warps alternate.  Then the accumulator, the cluster's reduce-scatter through
-//                distributed shared memory (partial sums added in rank order), bias, fp16, 16-byte stores.
+//                8 weights; groups of four warps take turns.  Then the accumulator, bias, fp16, 16-byte stores.
+// The K range is not split: one chain of products in k order gives the bits of the large GEMM, so a prompt's cache does not
+// depend on which kernel its length picks.  (Split over a cluster the 16-row linears took 48 us a layer instead of 82, but a
+// last-bit difference moves 4-bit codes of the cache a few layers on.)  Bound by the chain
+// itself: 8 MMAs of 64 cycles and their waits per block of 128 k.
+// 3072 -> 5120 / 3072 / 16384 and 8192 -> 3072, 16 rows, us: large GEMM 43 / 43 / 50 / 115, here 15 / 14 / 19 / 35.
 #include "fq_awq_skinny.cuh"
 
-#include <cooperative_groups.h>
 #include <cuda.h>
 
 namespace fq {
@@ -23,15 +26,13 @@ namespace fq {
 constexpr int SK_BN = 128, SK_BK = 128;            // k block: the synchronisation of a block costs about 600 cycles whatever its length
 constexpr int SK_RAW = SK_BK * SK_BN / 2;          // 8 KiB of codes per k block
 constexpr int SK_A = SK_BK * SK_BN * 2;            // 32 KiB dequantised
-constexpr int SK_DEQ_WARPS = 8;
-constexpr int SK_MAX_RAW = 8;                     // ring depth limit
+constexpr int SK_MAX_RAW = 9;                     // ring depth limit
 constexpr unsigned SK_SPIN_LIMIT = 1u << 26;
 
 struct SkProj { const __half* scales; const int32_t* qzeros; const __half* bias; __half* y; int N, tile0; };
 struct SkParams {
     SkProj proj[SK_MAX_PROJ];
-    int n_proj, M, K, group, n_groups, ks, groups_per_rank, raw_stages;
-    int recv_off;                      // offset of the reduce-scatter buffer (0: over the pipeline buffers)
+    int n_proj, M, K, group, n_groups, raw_stages;
     int* status;
 };
 
@@ -78,29 +79,21 @@ __device__ __forceinline__ void sk_ld8(uint32_t taddr, uint32_t* v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
 }
-__device__ __forceinline__ uint32_t sk_map(uint32_t local_addr, int rank) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-    return remote;
-}
-__device__ __forceinline__ void sk_st_cluster4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void sk_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void sk_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 // TN: rows of x per CTA (16 .. 128)
 template <int TN> struct SkCfg {
     static constexpr int COLS = SK_BN / 2;                          // columns per epilogue thread
-    static constexpr int THREADS = (4 + SK_DEQ_WARPS) * 32;
     static constexpr int STAGES = TN > 64 ? 2 : 3;                  // dequantised weights
+    // Groups of four warps that dequantise, one k block each in turn: as many as stages.  With more, a group could come back to
+    // a stage two of its phases ahead, which a parity wait cannot see; the raw ring is a multiple of it for the same reason.
+    static constexpr int GROUPS = STAGES;
+    static constexpr int THREADS = (4 + 4 * GROUPS) * 32;
     static constexpr int X_STAGES = 3;                              // an x tile arrives about 1 us after its request
     static constexpr int X_HALF = TN * 64 * 2;                      // bytes per 64 k (one 128-byte row per row of x)
     static constexpr int X_TILE = 2 * X_HALF;                       // bytes per k block
     static constexpr int X_BYTES = (2 * X_STAGES - 1) * X_HALF + 128 * 64 * 2;
     static constexpr int TMEM_COLS = SK_BN;
 };
-constexpr int SK_DEQ_GROUP = 4;                    // warps that dequantise one k block; two groups alternate
+constexpr int SK_DEQ_GROUP = 4;                    // warps that dequantise one k block
 
 template <bool INTERLEAVED, int TN>
 __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
@@ -115,21 +108,20 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
     unsigned char* sX = sW + AS * SK_A;
     unsigned char* sRaw = sX + C::X_BYTES;
     unsigned char* sMeta = sRaw + p.raw_stages * SK_RAW;            // per group: 128 scales fp16, 16 zero words
-    float* sRecv = reinterpret_cast<float*>(base + p.recv_off);     // [source rank][row][128] fp32, then the fp16 rows
+    float* sOut = reinterpret_cast<float*>(base);                   // [row][128] fp32, over the pipeline buffers at the end
     __shared__ uint64_t full_raw[SK_MAX_RAW], empty_raw[SK_MAX_RAW], a_ready[AS], a_empty[AS], x_full[XS], x_empty[XS], acc_ready, meta_full;
     __shared__ uint32_t tmem_slot;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int rank = blockIdx.x, row0 = blockIdx.z * TN;
+    const int row0 = blockIdx.y * TN;
     const int gpk = p.group / SK_BK;                                 // k blocks per group
-    const int g0 = min(p.n_groups, rank * p.groups_per_rank), g1 = min(p.n_groups, g0 + p.groups_per_rank);
-    const int ng = g1 - g0, nkb = ng * gpk, kb0 = g0 * gpk;
+    const int ng = p.n_groups, nkb = ng * gpk;
     int pj = 0;
 #pragma unroll
     for (int i = 1; i < SK_MAX_PROJ; ++i)
-        if (i < p.n_proj && (int)blockIdx.y >= p.proj[i].tile0) pj = i;
+        if (i < p.n_proj && (int)blockIdx.x >= p.proj[i].tile0) pj = i;
     const SkProj& P = p.proj[pj];
-    const int n0 = ((int)blockIdx.y - P.tile0) * SK_BN;
+    const int n0 = ((int)blockIdx.x - P.tile0) * SK_BN;
     const int rows = min(TN, p.M - row0);                            // live rows of this tile
     bool failed = false;
 
@@ -149,7 +141,6 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    if (p.ks > 1) sk_cluster_arrive();                               // matched by the wait before the first remote store
 
     if (warp == 0) {
         // =========================== weight producer ===========================
@@ -158,14 +149,14 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
         if (sk_elect()) {
             for (int kb = 0; kb < depth; ++kb) {
                 sk_expect(&full_raw[kb], SK_RAW);
-                sk_tma(sRaw + kb * SK_RAW, map_w, nb, (kb0 + kb) * SK_BK, &full_raw[kb]);
+                sk_tma(sRaw + kb * SK_RAW, map_w, nb, kb * SK_BK, &full_raw[kb]);
             }
-            if (ng > 0) sk_expect(&meta_full, (unsigned)ng * 320u);
+            sk_expect(&meta_full, (unsigned)ng * 320u);
         }
         __syncwarp();
         for (int g = lane; g < ng; g += 32) {
-            sk_bulk(sMeta + g * 320, P.scales + (int64_t)(g0 + g) * P.N + n0, 256, &meta_full);
-            sk_bulk(sMeta + g * 320 + 256, P.qzeros + ((int64_t)(g0 + g) * P.N + n0) / 8, 64, &meta_full);
+            sk_bulk(sMeta + g * 320, P.scales + (int64_t)g * P.N + n0, 256, &meta_full);
+            sk_bulk(sMeta + g * 320 + 256, P.qzeros + ((int64_t)g * P.N + n0) / 8, 64, &meta_full);
         }
         __syncwarp();
         int s = 0;
@@ -178,7 +169,7 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
             }
             if (sk_elect()) {
                 sk_expect(&full_raw[s], SK_RAW);
-                sk_tma(sRaw + s * SK_RAW, map_w, nb, (kb0 + kb) * SK_BK, &full_raw[s]);
+                sk_tma(sRaw + s * SK_RAW, map_w, nb, kb * SK_BK, &full_raw[s]);
             }
             __syncwarp();
             if (++s == p.raw_stages) { s = 0; ph ^= 1u; }
@@ -218,8 +209,8 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
             if (kb >= XS && sk_any_timeout(&x_empty[s], (unsigned)(kb / XS - 1) & 1u)) { failed = true; break; }
             if (sk_elect()) {
                 sk_expect(&x_full[s], C::X_TILE);
-                sk_tma(sX + s * C::X_TILE, &map_x, (kb0 + kb) * SK_BK, row0, &x_full[s]);
-                sk_tma(sX + s * C::X_TILE + C::X_HALF, &map_x, (kb0 + kb) * SK_BK + 64, row0, &x_full[s]);
+                sk_tma(sX + s * C::X_TILE, &map_x, kb * SK_BK, row0, &x_full[s]);
+                sk_tma(sX + s * C::X_TILE + C::X_HALF, &map_x, kb * SK_BK + 64, row0, &x_full[s]);
             }
             __syncwarp();
         }
@@ -228,10 +219,10 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
         const int grp = (warp - DEQ0) / SK_DEQ_GROUP, t = (tid - DEQ0 * 32) % (SK_DEQ_GROUP * 32);
         const int c = t & 15, kr0 = t >> 4;                           // pack of 8 columns; k rows kr0 + 8 i
         const int chunk = c & 7;
-        if (ng > 0 && sk_any_timeout(&meta_full, 0u)) failed = true;
+        if (sk_any_timeout(&meta_full, 0u)) failed = true;
         int r = grp % p.raw_stages;
         unsigned rph = (unsigned)(grp / p.raw_stages) & 1u;
-        for (int kb = grp; kb < nkb && !failed; kb += SK_DEQ_WARPS / SK_DEQ_GROUP) {
+        for (int kb = grp; kb < nkb && !failed; kb += C::GROUPS) {
             const int s = kb % AS;
             // per column pair: even nibbles h = 1024 + code, minus (1024 + zero); odd ones h = 1024 + 16 code, times 1/16 minus
             // (64 + zero): both exact; then the scale, rounded once
@@ -284,76 +275,46 @@ __global__ void __launch_bounds__(SkCfg<TN>::THREADS, 1) awq_skinny_kernel(
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) { sk_arrive(&a_ready[s]); sk_arrive(&empty_raw[r]); }      // (the raw tile not before its values have been used)
-            for (int i = 0; i < SK_DEQ_WARPS / SK_DEQ_GROUP; ++i)
+            for (int i = 0; i < C::GROUPS; ++i)
                 if (++r == p.raw_stages) { r = 0; rph ^= 1u; }
         }
         // ---- the accumulator ----
-        if (ng > 0 && sk_any_timeout(&acc_ready, 0u)) failed = true;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // ---- reduce-scatter over the cluster, output ----
-        const int lq = warp & 3, part = (warp - DEQ0) >> 2, row = lq * 32 + lane;      // TMEM lane quarter (rows), half of the columns
-        const int tpr = (rows + p.ks - 1) / p.ks;                    // rows finished by each CTA of the cluster
-        const int my0 = rank * tpr, mine = max(0, min(tpr, rows - my0));
-        constexpr int RS = SK_BN + 4;                                // row stride (floats): 16-byte stores of 8 lanes hit all banks
-        __syncwarp();
-        if (p.ks > 1) {
-            sk_cluster_wait();                                       // every CTA of the cluster has started
-            if (p.recv_off == 0) { sk_cluster_arrive(); sk_cluster_wait(); }     // ... and is done with its pipeline buffers
-        }
-        if (lq * 32 < rows) {
-            uint32_t acc[C::COLS];
+        if (warp < DEQ0 + 8) {
+            if (sk_any_timeout(&acc_ready, 0u)) failed = true;       // every product is done, so the pipeline buffers are free
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int lq = warp & 3, part = (warp - DEQ0) >> 2, row = lq * 32 + lane;      // TMEM lane quarter (rows), half of the columns
+            constexpr int RS = SK_BN + 4;                            // row stride (floats): 16-byte stores of 8 lanes hit all banks
+            __syncwarp();
+            if (lq * 32 < rows) {
+                uint32_t acc[C::COLS];
 #pragma unroll
-            for (int c = 0; c < C::COLS / 8; ++c) sk_ld8(tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(part * C::COLS + c * 8), acc + 8 * c);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (ng == 0)
+                for (int c = 0; c < C::COLS / 8; ++c) sk_ld8(tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(part * C::COLS + c * 8), acc + 8 * c);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (row < rows) {
 #pragma unroll
-                for (int i = 0; i < C::COLS; ++i) acc[i] = 0u;
-          if (row < rows) {
-            const int dst = row / tpr;
-            const uint32_t local = sk_smem(sRecv + (rank * tpr + row - dst * tpr) * RS + part * C::COLS);
-            const uint32_t at = p.ks > 1 ? sk_map(local, dst) : local;
-            if (p.ks > 1) {
-#pragma unroll
-                for (int i = 0; i < C::COLS; i += 4) sk_st_cluster4(at + 4 * i, acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < C::COLS; i += 4)
-                    *reinterpret_cast<uint4*>(sRecv + row * RS + part * C::COLS + i) = make_uint4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+                    for (int i = 0; i < C::COLS; i += 4)
+                        *reinterpret_cast<uint4*>(sOut + row * RS + part * C::COLS + i) = make_uint4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+                }
             }
-          }
-        }
-        __syncwarp();
-        if (p.ks > 1) { sk_cluster_arrive(); sk_cluster_wait(); }
-        else asm volatile("bar.sync 1, %0;" ::"n"(SK_DEQ_WARPS * 32) : "memory");
-        __half* yb = P.y + (int64_t)(row0 + my0) * P.N + n0;
-        for (int i = tid - DEQ0 * 32; i < mine * 16; i += SK_DEQ_WARPS * 32) {
-            const int r = i >> 4, c8 = (i & 15) * 8;
-            float v[8];
+            __syncwarp();
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            __half* yb = P.y + (int64_t)row0 * P.N + n0;
+            for (int i = tid - DEQ0 * 32; i < rows * 16; i += 256) {
+                const int r = i >> 4, c8 = (i & 15) * 8;
+                const float4 a = *reinterpret_cast<const float4*>(sOut + r * RS + c8), b = *reinterpret_cast<const float4*>(sOut + r * RS + c8 + 4);
+                float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                if (P.bias) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = 0.f;
-            for (int sr = 0; sr < p.ks; ++sr) {
-                const float4 a = *reinterpret_cast<const float4*>(sRecv + (sr * tpr + r) * RS + c8), b = *reinterpret_cast<const float4*>(sRecv + (sr * tpr + r) * RS + c8 + 4);
-                v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+                    for (int e = 0; e < 8; ++e) v[e] += __half2float(P.bias[n0 + c8 + e]);
+                }
+                uint32_t o[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { const __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]); o[e] = *reinterpret_cast<const uint32_t*>(&h); }
+                *reinterpret_cast<uint4*>(yb + (int64_t)r * P.N + c8) = make_uint4(o[0], o[1], o[2], o[3]);
             }
-            if (P.bias) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] += __half2float(P.bias[n0 + c8 + e]);
-            }
-            uint32_t o[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { const __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]); o[e] = *reinterpret_cast<const uint32_t*>(&h); }
-            *reinterpret_cast<uint4*>(yb + (int64_t)r * P.N + c8) = make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
 
-    // the epilogue warps' exchange above meets every warp of the cluster at its barriers
-    if (p.ks > 1 && warp < DEQ0) {
-        __syncwarp();
-        sk_cluster_wait();
-        if (p.recv_off == 0) { sk_cluster_arrive(); sk_cluster_wait(); }
-        sk_cluster_arrive();
-        sk_cluster_wait();
-    }
     if (failed) atomicExch(p.status, FQ_ERR_TIMEOUT);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -373,22 +334,9 @@ static SkEncodeFn sk_encode_fn() {
     return reinterpret_cast<SkEncodeFn>(fn);
 }
 
-// K ranges of a column tile: as many as keep about one CTA per SM (the pipeline of the next kernel needs the other half of
-// every SM), at most one portable cluster, at least two groups each.
-// Clusters that fit at one CTA per SM, by cluster size, as cudaOccupancyMaxActiveClusters reports them for a B200 (its
-// GPCs differ in size); one cluster too many would run as a second wave.
-static int sk_splits(int tiles, int n_groups) {
-    static const int fit[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
-    int ks = 8;
-    while (ks > 1 && fit[ks] < tiles) --ks;
-    while (ks > 1 && (n_groups + ks - 1) / ks < 2) --ks;
-    const int per = (n_groups + ks - 1) / ks;
-    return (n_groups + per - 1) / per;                               // no empty rank
-}
-
 bool awq_skinny_supported(const SkinnyCall& c) {
     if (!(c.group == 128 || c.group == 256) || c.K <= 0 || c.K % c.group || c.n_proj < 1 || c.n_proj > SK_MAX_PROJ || c.M < 1) return false;
-    if (!aligned(c.x, 16) || (int64_t)(c.K / c.group) * 320 > 48 * 1024) return false;
+    if (!aligned(c.x, 16) || (int64_t)(c.K / c.group) * 320 > 40 * 1024) return false;
     for (int i = 0; i < c.n_proj; ++i)
         if (c.N[i] % SK_BN || !aligned(c.qweight[i], 16) || !aligned(c.scales[i], 16) || !aligned(c.qzeros[i], 16) || !aligned(c.y[i], 16)) return false;
     return true;
@@ -398,19 +346,13 @@ template <bool IL, int TN>
 static int sk_launch(const SkinnyCall& c, SkParams& p, const CUtensorMap* maps, int tiles, cudaStream_t st, const char* fn) {
     using C = SkCfg<TN>;
     const int m_tiles = (c.M + TN - 1) / TN;
-    p.ks = sk_splits(tiles * m_tiles, p.n_groups);
-    p.groups_per_rank = (p.n_groups + p.ks - 1) / p.ks;
-    const int nkb = p.groups_per_rank * (p.group / SK_BK);
-    const int rows = c.M < TN ? c.M : TN, tpr = (rows + p.ks - 1) / p.ks;
-    const int fixed = C::STAGES * SK_A + C::X_BYTES + p.groups_per_rank * 320;
-    const int recv = p.ks * tpr * (SK_BN + 4) * 4;
-    const bool over = p.ks == 1 || recv > 24 * 1024;                 // the exchange lies over the pipeline buffers (one cluster barrier more)
-    int raw = (220 * 1024 - fixed - (over ? 0 : recv)) / SK_RAW;
-    raw = raw > SK_MAX_RAW ? SK_MAX_RAW : raw;
+    const int nkb = p.n_groups * (p.group / SK_BK), rows = c.M < TN ? c.M : TN;
+    const int fixed = C::STAGES * SK_A + C::X_BYTES + p.n_groups * 320;
+    int raw = (220 * 1024 - fixed) / SK_RAW;
+    raw = (raw > SK_MAX_RAW ? SK_MAX_RAW : raw) / C::GROUPS * C::GROUPS;      // at least one per group: awq_skinny_supported bounds K
     p.raw_stages = raw > nkb ? nkb : raw;
-    const int pipe = (fixed + p.raw_stages * SK_RAW + 127) & ~127;
-    p.recv_off = over ? 0 : pipe;
-    const int smem = (over ? (recv > pipe ? recv : pipe) : pipe + recv) + 1024;
+    const int pipe = fixed + p.raw_stages * SK_RAW, out = rows * (SK_BN + 4) * 4;
+    const int smem = (out > pipe ? out : pipe) + 1024;
     static std::atomic<uint64_t> reserved{0};                        // per instantiation, one bit per device
     int dev = 0;
     cudaGetDevice(&dev);
@@ -421,14 +363,12 @@ static int sk_launch(const SkinnyCall& c, SkParams& p, const CUtensorMap* maps, 
         reserved.fetch_or(bit, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)p.ks, (unsigned)tiles, (unsigned)m_tiles); cfg.blockDim = dim3(C::THREADS);
+    cfg.gridDim = dim3((unsigned)tiles, (unsigned)m_tiles); cfg.blockDim = dim3(C::THREADS);
     cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cudaLaunchAttribute at[2]{};
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = p.ks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = 2;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at; cfg.numAttrs = 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, awq_skinny_kernel<IL, TN>, maps[0], maps[1], maps[2], maps[3], maps[4], p);
     if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: launch failed: %s", fn, cudaGetErrorString(e));
     FQ_CHECK_LAUNCH(fn);

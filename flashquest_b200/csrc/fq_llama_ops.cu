@@ -53,13 +53,17 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(
 }
 
 // The same with the row held in registers, 16 bytes per access: rows of H <= 8 * NORM_THREADS * NORM_CHUNKS halves (H a
-// multiple of 8, 16-byte aligned).  HBM/L2-bound; 4099 rows of 3072: 20.9 -> 11 us.
+// multiple of 8, 16-byte aligned).  The squares are added in one of two orders, so that a row gives the same bits whichever
+// kernel takes it: STRIDED as add_rmsnorm_kernel does (a thread owns every 256th value; through shared memory), else as the
+// prologue of awq_gemv_kernel does (every 256th piece of eight).  HBM/L2-bound; 4099 rows of 3072: 20.9 -> 18 us (11 without STRIDED).
 constexpr int NORM_CHUNKS = 4;
 constexpr int NORM_ROWS = 3;        // rows from which a GEMV's RMSNorm is a launch of its own
+template <bool STRIDED>
 __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_vec_kernel(
     const __half* __restrict__ a, const __half* __restrict__ b, const __half* __restrict__ weight, float eps,
     int H, __half* __restrict__ sum_out, __half* __restrict__ y) {
     __shared__ float s_red[NORM_THREADS / 32];
+    __shared__ __align__(16) __half s_row[STRIDED ? 8 * NORM_THREADS * NORM_CHUNKS : 8];
     const int64_t row = blockIdx.x;
     const int n8 = H >> 3;
     union V { uint4 u; __half2 h[4]; };
@@ -79,9 +83,18 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_vec_kernel(
                 for (int j = 0; j < 4; ++j) x[i].h[j] = __hadd2(x[i].h[j], t.h[j]);
             }
             if (sum_out) reinterpret_cast<uint4*>(sum_out + row * H)[c] = x[i].u;
+            if constexpr (STRIDED) {
+                reinterpret_cast<uint4*>(s_row)[c] = x[i].u;
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { const float2 f = __half22float2(x[i].h[j]); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss); }
+                for (int j = 0; j < 4; ++j) { const float2 f = __half22float2(x[i].h[j]); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss); }
+            }
         }
+    }
+    if constexpr (STRIDED) {
+        __syncthreads();
+#pragma unroll 4
+        for (int i = threadIdx.x; i < H; i += NORM_THREADS) { const float f = __half2float(s_row[i]); ss = fmaf(f, f, ss); }
     }
     const float r = rsqrtf(block_sum(ss, s_red) / (float)H + eps);
 #pragma unroll
@@ -372,15 +385,16 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_f16_kernel(const __half
 
 }  // namespace fq
 
-extern "C" int fq_add_rmsnorm(const void* a, const void* b, const void* weight, float eps, int64_t rows, int H,
-                              void* sum_out, void* y, void* stream) {
-    using namespace fq;
+namespace fq {
+// piecewise: the summation order of the GEMV's prologue (rows of up to 8 * NORM_THREADS * NORM_CHUNKS aligned halves)
+static int add_rmsnorm_launch(const void* a, const void* b, const void* weight, float eps, int64_t rows, int H,
+                              void* sum_out, void* y, bool piecewise, void* stream) {
     const char* fn = "fq_add_rmsnorm";
     FQ_CHECK_ARG(a && weight && y && rows >= 0 && H > 0, FQ_ERR_ARG, "%s: bad arguments", fn);
     FQ_CHECK_ARG((size_t)H * 2 <= 96 * 1024, FQ_ERR_UNSUPPORTED, "%s: hidden size %d too large", fn, H);
     if (rows == 0) return FQ_OK;
     if (H % 8 == 0 && H <= 8 * NORM_THREADS * NORM_CHUNKS && aligned(a, 16) && aligned(b, 16) && aligned(weight, 16) && aligned(sum_out, 16) && aligned(y, 16)) {
-        launch_k(PDL_GEMV, add_rmsnorm_vec_kernel, dim3((unsigned)rows), dim3(NORM_THREADS), 0, static_cast<cudaStream_t>(stream),
+        launch_k(PDL_GEMV, piecewise ? add_rmsnorm_vec_kernel<false> : add_rmsnorm_vec_kernel<true>, dim3((unsigned)rows), dim3(NORM_THREADS), 0, static_cast<cudaStream_t>(stream),
                  static_cast<const __half*>(a), static_cast<const __half*>(b), static_cast<const __half*>(weight), eps, H,
                  static_cast<__half*>(sum_out), static_cast<__half*>(y));
         FQ_CHECK_LAUNCH(fn);
@@ -396,6 +410,12 @@ extern "C" int fq_add_rmsnorm(const void* a, const void* b, const void* weight, 
              static_cast<__half*>(sum_out), static_cast<__half*>(y));
     FQ_CHECK_LAUNCH(fn);
     return FQ_OK;
+}
+}  // namespace fq
+
+extern "C" int fq_add_rmsnorm(const void* a, const void* b, const void* weight, float eps, int64_t rows, int H,
+                              void* sum_out, void* y, void* stream) {
+    return fq::add_rmsnorm_launch(a, b, weight, eps, rows, H, sum_out, y, false, stream);
 }
 
 namespace fq {
@@ -536,13 +556,13 @@ static int llama_step_impl(const fq_llama_model* m, const fq_int4_cache* cache, 
     // goes to.  From NORM_ROWS rows on a launch of its own: folded, every CTA of the GEMV reads all the rows whole (44 MB through
     // L2 at 8 rows of 3072), which cost 7 us of 17 at 8 rows; the launch is 3 us, under which the GEMV's weights arrive.
     // Same arithmetic and order, same bits.  A token of 8 sequences over 4k: 3154 -> 2773 us, of 3: 2482 -> 2405, of 2: even.
-    const bool norm_apart = B >= NORM_ROWS && H % 8 == 0 && H <= 8 * NORM_THREADS * NORM_CHUNKS;
+    const bool norm_apart = B >= NORM_ROWS && H % 8 == 0 && H <= 8 * NORM_THREADS * NORM_CHUNKS && aligned(x, 16);
     auto norm_prologue = [&](const void* w, fq_gemv_prologue& pro, const void** src) -> int {
         pro.kind = FQ_GEMV_ADD_RMSNORM; pro.b = delta; pro.weight = w; pro.eps = m->rms_eps; pro.out = nullptr;
         *src = xin;
         if (delta) { pro.out = flip ? s->resid1 : s->resid0; flip ^= 1; xin = pro.out; }
         if (!norm_apart) return FQ_OK;
-        const int r = fq_add_rmsnorm(*src, pro.b, w, m->rms_eps, B, H, pro.out, s->normed, stream);
+        const int r = add_rmsnorm_launch(*src, pro.b, w, m->rms_eps, B, H, pro.out, s->normed, true, stream);
         pro.kind = FQ_GEMV_PLAIN;
         *src = s->normed;
         return r;

@@ -72,17 +72,18 @@ def test_gemv_splits_and_tiles(M, K, Ns, interleaved, bias):
     assert all(torch.equal(a, b) for a, b in zip(got, awq_gemv_fused(x, lins)))
 
 
-@pytest.mark.parametrize("rows,H", [(3, 128), (8, 3072), (8, 8192)])
-def test_norm_apart_from_gemv(rows, H):
-    """A decode step's RMSNorm as its own launch in front of the GEMV gives the bits of the one folded into it."""
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (8, 3072), (2, 8192)])
+def test_norm_equals_general_kernel(rows, H):
+    """Rows 16 bytes at a time give the bits of the value-by-value kernel, which unaligned rows take."""
     from flashquest_b200._lib import check, lib, ptr, stream_ptr
-    from flashquest_b200.kernel.fused_proj import awq_gemv_fused
     g = torch.Generator(device="cuda").manual_seed(H)
-    lin = _linear(H, 128, 128, True, False, g)
     x, d = (torch.randn(rows, H, device="cuda", generator=g).half() for _ in range(2))
     w = torch.rand(H, device="cuda", generator=g).half()
-    folded = awq_gemv_fused(x, (lin,), add=d, norm_weight=w, eps=1e-5)[0]
-    normed, total = torch.empty_like(x), torch.empty_like(x)
-    check(lib().fq_add_rmsnorm(ptr(x), ptr(d), ptr(w), 1e-5, rows, H, ptr(total), ptr(normed), stream_ptr(x.device)))
-    assert torch.equal(total, x + d)
-    assert torch.equal(awq_gemv_fused(normed, (lin,))[0], folded)
+    odd = torch.empty(rows * H + 1, dtype=torch.float16, device="cuda")[1:].view(rows, H)
+    odd.copy_(x)
+    out = []
+    for a in (x, odd):
+        normed, total = torch.empty_like(x), torch.empty_like(x)
+        check(lib().fq_add_rmsnorm(ptr(a), ptr(d), ptr(w), 1e-5, rows, H, ptr(total), ptr(normed), stream_ptr(x.device)))
+        out.append((normed, total))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
