@@ -399,6 +399,8 @@ __global__ void __launch_bounds__(128) lse_merge_kernel(const T* __restrict__ O_
                                                         int n, int64_t rows, int D, T* __restrict__ O, float* __restrict__ lse) {
     const int lane = threadIdx.x & 31;
     const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_trigger();
     if (r >= rows) return;
     float m = -INFINITY;
     for (int i = 0; i < n; ++i) m = fmaxf(m, lse_parts[(int64_t)i * rows + r]);
@@ -504,9 +506,9 @@ extern "C" int fq_lse_merge(const void* O_parts, const float* lse_parts, int dty
     FQ_CHECK_ARG(O_parts && lse_parts && O, FQ_ERR_ARG, "%s: null pointer", fn);
     const unsigned blocks = (unsigned)((rows + 3) / 4);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dtype == FQ_F32) lse_merge_kernel<float><<<blocks, 128, 0, st>>>(static_cast<const float*>(O_parts), lse_parts, n, rows, D, static_cast<float*>(O), lse);
-    else if (dtype == FQ_F16) lse_merge_kernel<__half><<<blocks, 128, 0, st>>>(static_cast<const __half*>(O_parts), lse_parts, n, rows, D, static_cast<__half*>(O), lse);
-    else if (dtype == FQ_BF16) lse_merge_kernel<__nv_bfloat16><<<blocks, 128, 0, st>>>(static_cast<const __nv_bfloat16*>(O_parts), lse_parts, n, rows, D, static_cast<__nv_bfloat16*>(O), lse);
+    if (dtype == FQ_F32) launch_k(PDL_ATTN, lse_merge_kernel<float>, dim3(blocks), dim3(128), 0, st, static_cast<const float*>(O_parts), lse_parts, n, rows, D, static_cast<float*>(O), lse);
+    else if (dtype == FQ_F16) launch_k(PDL_ATTN, lse_merge_kernel<__half>, dim3(blocks), dim3(128), 0, st, static_cast<const __half*>(O_parts), lse_parts, n, rows, D, static_cast<__half*>(O), lse);
+    else if (dtype == FQ_BF16) launch_k(PDL_ATTN, lse_merge_kernel<__nv_bfloat16>, dim3(blocks), dim3(128), 0, st, static_cast<const __nv_bfloat16*>(O_parts), lse_parts, n, rows, D, static_cast<__nv_bfloat16*>(O), lse);
     else return fail(FQ_ERR_DTYPE, "%s: dtype code %d", fn, dtype);
     FQ_CHECK_LAUNCH(fn);
     return FQ_OK;
