@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_kernel(Int8AttnParams 
     const int hkv = hq / (p.Hq / p.Hkv);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float c = p.sm_scale * I8_LOG2E;
+    pdl_trigger();     // the merge may become resident
     float q[CPL];
 #pragma unroll
     for (int j = 0; j < CPL; ++j) q[j] = i8_ld(p.Q, p.q_dtype, b * p.q_sb + hq * p.q_sh + CPL * lane + j) * c;
@@ -267,6 +268,7 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int l = lane & 7, qw = lane >> 3;
     const float c = p.sm_scale * I8_LOG2E;
+    pdl_trigger();     // the merge may become resident
     float q[DPL];
 #pragma unroll
     for (int j = 0; j < DPL; ++j) q[j] = i8_ld(p.Q, p.q_dtype, b * p.q_sb + hq * p.q_sh + DPL * l + j) * c;
@@ -415,17 +417,36 @@ __global__ void __launch_bounds__(128) int8_merge_kernel(const float* __restrict
                                                          int64_t rows, int D, void* __restrict__ O, int q_dtype, float* __restrict__ lse) {
     const int lane = threadIdx.x & 31;
     const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_trigger();
     if (r >= rows) return;
+    // Latency-bound.  A lane holds the weight of every 32nd split, the sums run over the splits in order with eight rows in
+    // flight; with the early launch an INT8 step of 4 x 20k goes from 56.7 to 52.9 us, of 1 x 4k from 26.1 to 23.5.
     float m = -INFINITY;
-    for (int i = 0; i < n_split; ++i) m = fmaxf(m, part_lse[i * rows + r]);
-    float wsum = 0.f;
-    if (m != -INFINITY)
-        for (int i = 0; i < n_split; ++i) wsum += expf(part_lse[i * rows + r] - m);
-    for (int d = lane; d < D; d += 32) {
-        float a = 0.f;
-        if (m != -INFINITY)
-            for (int i = 0; i < n_split; ++i) a = fmaf(expf(part_lse[i * rows + r] - m), part_o[(i * rows + r) * D + d], a);
-        const float v = m != -INFINITY ? a / wsum : 0.f;
+    for (int i = lane; i < n_split; i += 32) m = fmaxf(m, part_lse[i * rows + r]);
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    float wsum = 0.f, a[4] = {0.f, 0.f, 0.f, 0.f};              // head_dim <= 128
+    if (m != -INFINITY) {
+        for (int i0 = 0; i0 < n_split; i0 += 32) {
+            const float wl = i0 + lane < n_split ? expf(part_lse[(i0 + lane) * rows + r] - m) : 0.f;
+            const int cnt = min(32, n_split - i0);
+#pragma unroll 8
+            for (int j = 0; j < cnt; ++j) {
+                const float w = __shfl_sync(0xffffffffu, wl, j);
+                const float* row = part_o + ((i0 + j) * rows + r) * D;
+                wsum += w;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (lane + 32 * k < D) a[k] = fmaf(w, row[lane + 32 * k], a[k]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int d = lane + 32 * k;
+        if (d >= D) break;
+        const float v = m != -INFINITY ? a[k] / wsum : 0.f;
         if (q_dtype == FQ_F16) static_cast<__half*>(O)[r * D + d] = __float2half_rn(v);
         else static_cast<__nv_bfloat16*>(O)[r * D + d] = __float2bfloat16_rn(v);
     }
@@ -549,6 +570,8 @@ extern "C" int fq_sparse_decode_int8_counted(
     // 16-byte aligned code and metadata rows: the quarter-warp-per-token kernel
     const bool vec16 = have_pages && aligned(K_uint8, 16) && aligned(V_uint8, 16) && kv_sb % 16 == 0 && kv_sh % 16 == 0 && kv_ss % 16 == 0 &&
                        aligned(K_scale, 16) && aligned(K_mn, 16) && km_sb % 8 == 0 && km_sh % 8 == 0 && km_sp % 8 == 0;
+    // (An ordinary launch: one wave of CTAs that started early would settle unevenly around the selection's, 59 against 53 us for
+    // a step of 4 x 20k.  The merge behind it starts early.)
     if (vec16) {
         if (D == 128) sparse_decode_int8_q_kernel<128><<<grid, 128, 0, st>>>(p);
         else sparse_decode_int8_q_kernel<64><<<grid, 128, 0, st>>>(p);
@@ -558,7 +581,7 @@ extern "C" int fq_sparse_decode_int8_counted(
     }
     FQ_CHECK_LAUNCH(fn);
     const int64_t rows = (int64_t)B * Hq;
-    int8_merge_kernel<<<(unsigned)((rows + 3) / 4), 128, 0, st>>>(p.part_o, p.part_lse, n_split, rows, D, O, q_dtype, lse);
+    launch_k(PDL_ATTN, int8_merge_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), 0, st, p.part_o, p.part_lse, n_split, rows, D, O, q_dtype, lse);
     FQ_CHECK_LAUNCH(fn);
     return FQ_OK;
 }
