@@ -1,6 +1,7 @@
 // Bulk packing of whole pages (fq_quant_pages.cu), shared by the INT4, INT8 and TurboQuant append paths.
 #pragma once
 #include "fq_common.cuh"
+#include "fq_exact_div.cuh"
 
 namespace fq {
 
@@ -34,15 +35,10 @@ template <> struct Q2<__nv_bfloat16> {
     static constexpr uint32_t POS_INF = 0x7f807f80u;
 };
 
-// Scale of a page's channel, in the input dtype: max(rn(rn(hi - lo) / top), eps).  The quotient of a T value by 15 or 255,
-// rounded to T, from the product with the rounded reciprocal and one residual step: equal for every T value (checked
-// exhaustively on the host); an infinite range takes the division.
+// Scale of a page's channel, in the input dtype: max(rn(rn(hi - lo) / top), eps).
 template <typename T>
 __device__ __forceinline__ float page_scale(float hi, float lo, float top, float rtop, float eps) {
-    const float d = Dt<T>::rn(__fsub_rn(hi, lo)), q0 = __fmul_rn(d, rtop);
-    float q = __fmaf_rn(__fmaf_rn(-q0, top, d), rtop, q0);
-    if (!(d <= 3.0e38f)) q = d;
-    return fmaxf(Dt<T>::rn(q), eps);
+    return fmaxf(Dt<T>::rn(div_by_top(Dt<T>::rn(__fsub_rn(hi, lo)), top, rtop)), eps);
 }
 
 // Whether the kernel takes this call (else: the general kernels).

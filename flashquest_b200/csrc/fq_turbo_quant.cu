@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(128) turbo_quant_kernel(TurboParams p) {
 // packed 16-bit pairs and shared by four lanes: lane t of a row's quad holds channels 32j + 8t .. + 7, so four of the seven
 // butterflies stay inside a lane and a warp codes eight tokens at a time.
 //  * a butterfly with a partner lane is one shuffle and one packed fma(mine, +-1, other), which rounds once like the add;
-//  * x / fp32(sqrt(128)) rounded to the dtype equals x * TURBO_RCD rounded to the dtype, TURBO_RCD two ulps above
-//    fp32(1 / sqrt(128)), for every one of the 65 536 bit patterns of either dtype (checked exhaustively on the host);
+//  * x / fp32(sqrt(128)) rounded to the dtype equals x * TURBO_RCD rounded to the dtype for every one of the 65 536 bit
+//    patterns of either dtype (fq_exact_div.cuh);
 //  * the sum of squares adds in turbo_quant_kernel's order: groups of four channels, then groups 16, 8, 4, 2, 1 apart;
 //  * the code of v depends on the nearest entry of v / s, which is monotone in |v|.  So a token needs four 16-bit numbers:
 //    the smallest |v| that reaches the second, third and fourth magnitude, and the smallest v > 0 that counts as positive
@@ -272,7 +272,6 @@ __device__ __noinline__ unsigned turbo_idx_exact(float v, float s) {
 
 // midpoints between neighbouring codebook magnitudes
 constexpr float TURBO_M0 = 0.50055f, TURBO_M1 = 1.04995f, TURBO_M2 = 1.7479f;
-constexpr float TURBO_RCD = 0.0883883610367775f;
 
 // one value of the value-by-value path: |v| against the midpoints, the exact decision near them or near zero
 __device__ __noinline__ unsigned turbo_idx_value(float v, float s) {

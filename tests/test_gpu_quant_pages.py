@@ -47,6 +47,36 @@ def test_bulk_append_matches_oracle(bits, page, D, dtype, B, S, first):
         assert not cache.K_partial[1, :, :, S - n:].any() and not cache.V_partial[1, :, :, S - n:].any()
 
 
+@pytest.mark.parametrize("bits", [3, 4, 8])
+@pytest.mark.parametrize("page", [16, 64])
+def test_page_range_at_the_top_of_bf16(bits, page):
+    """Ranges of 3.0e38 up to the largest finite bf16 value and beyond it: the scale is the rounded quotient, not the range."""
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    D, S = 128, 2 * page
+    K = _data(1, 2, S, D, torch.bfloat16, 3).float()
+    top = torch.linspace(2.9e38, 3.38e38, 64)                               # every range that the old limit of 3.0e38 cut off
+    K[:, :, 0::2, 64:], K[:, :, 1::2, 64:] = top / 2, -top / 2
+    K[:, :, :page, 0], K[:, :, page - 1, 0] = 3.3e38, -3.3e38               # an infinite range
+    K = K.bfloat16()
+    V = _data(1, 2, S, D, torch.bfloat16, 4)
+    cache = {3: PersistentTurboKVCache, 4: PersistentInt4KVCache, 8: PersistentInt8KVCache}[bits](
+        batch_size=1, num_layers=1, num_kv_heads=2, head_dim=D, max_seq_len=S, page_size=page, dtype=torch.bfloat16)
+    cache.update_quantized(K.cuda(), V.cuda(), 0)
+    views = cache.get_views(0)
+    if bits == 8:
+        want = oracle.quantize_k(K, page)
+        got = views["K_uint8"], views["K_scale"], views["K_mn"]
+    else:
+        want = oracle.quantize_k_int4(K, page)
+        got = (views["K_packed"], views["K_scale"], views["K_mn"]) if bits == 4 else (None, views["K_scale_raw"], views["K_mn_raw"])
+    assert torch.isfinite(want[1][..., 64:].float()).all() and want[1][..., 64:].float().max() < 3e37
+    assert torch.equal(got[1].cpu(), want[1]) and torch.equal(got[2].cpu(), want[2])
+    if bits != 3:
+        assert torch.equal(got[0].cpu()[..., (bits * 64) // 8:], want[0][..., (bits * 64) // 8:])       # the channels of finite range
+
+
 @pytest.mark.parametrize("model,stage", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.bfloat16), (torch.float16, torch.float16)])
 @pytest.mark.parametrize("D", [64, 128])
 def test_rope_of_the_patched_forward_matches_hugging_face(model, stage, D):
