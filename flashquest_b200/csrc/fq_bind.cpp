@@ -54,6 +54,13 @@ inline const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? 
 
 void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream(); }
 
+// The native calls run without the GIL, as ctypes calls do: a launch blocks while the stream's queue is full, and other
+// Python threads go on meanwhile.  What comes from Python objects has been read before.
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 // plan(kind, cache_desc, params, device, n_layers, scores, sc_sl, compact, cp_sl, O, o_sl_bytes, lse, lse_sl,
 //      ws, ws_sl, ws_bytes, scratch, scratch_bytes, q_rot, k_rot, v_rot): addresses and sizes as integers
 PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -112,9 +119,14 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
                     k->stride(3) == 1 && q->size(0) == B && q->size(1) == Hq && q->size(qd - 1) == D && q->stride(qd - 1) == 1 &&
                     (p->kind != 3 || (q->stride(1) == D && q->stride(0) == static_cast<int64_t>(Hq) * D));
     if (!ok) return PyLong_FromLong(1);
-    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
-    const int rc = run_layer(p, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), static_cast<int>(k->size(2)),
-                             q->data_ptr(), dtype_of(*q), q->stride(0), q->stride(1), prm ? prm : &p->prm, stream_of(p->device));
+    const fq_decode_params par = prm ? *prm : p->prm;
+    int rc;
+    {
+        const NoGil released;
+        const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
+        rc = run_layer(p, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), static_cast<int>(k->size(2)),
+                       q->data_ptr(), dtype_of(*q), q->stride(0), q->stride(1), &par, stream_of(p->device));
+    }
     return PyLong_FromLong(rc);
 }
 
@@ -139,13 +151,18 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (t[i]->size(2) != width || !(t[i]->size(0) == B || (i >= 3 && t[i]->size(0) == 1))) return PyLong_FromLong(1);
     }
     const int64_t cs = t[3]->size(0) == 1 ? 0 : t[3]->stride(0), ss = t[4]->size(0) == 1 ? 0 : t[4]->stride(0);
-    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
-    void* st = stream_of(p->device);
-    int rc = fq_rope_qkv(t[0]->data_ptr(), t[0]->stride(0), t[1]->data_ptr(), t[1]->stride(0), t[2]->data_ptr(), t[2]->stride(0), dt,
+    const fq_decode_params par = prm ? *prm : p->prm;
+    int rc;
+    {
+        const NoGil released;
+        const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
+        void* st = stream_of(p->device);
+        rc = fq_rope_qkv(t[0]->data_ptr(), t[0]->stride(0), t[1]->data_ptr(), t[1]->stride(0), t[2]->data_ptr(), t[2]->stride(0), dt,
                          t[3]->data_ptr(), cs, t[4]->data_ptr(), ss, B, Hq, Hkv, D, p->q_rot, p->k_rot, p->v_rot, p->cache_dtype, st);
-    if (rc == 0)
-        rc = run_layer(p, layer, seen, p->k_rot, p->v_rot, static_cast<int64_t>(Hkv) * D, D, D, 1, p->q_rot, p->cache_dtype,
-                       static_cast<int64_t>(Hq) * D, D, prm ? prm : &p->prm, st);
+        if (rc == 0)
+            rc = run_layer(p, layer, seen, p->k_rot, p->v_rot, static_cast<int64_t>(Hkv) * D, D, D, 1, p->q_rot, p->cache_dtype,
+                           static_cast<int64_t>(Hq) * D, D, &par, st);
+    }
     return PyLong_FromLong(rc);
 }
 
@@ -165,11 +182,15 @@ PyObject* append(PyObject*, PyObject* const* a, Py_ssize_t n) {
         v->get_device() != device || dtype_of(*k) != dt || dtype_of(*v) != dt || k->sizes() != v->sizes() || k->strides() != v->strides() ||
         k->size(0) != B || k->size(1) != Hkv || k->size(3) != D || k->stride(3) != 1 || k->size(2) < 1)
         return PyLong_FromLong(1);
-    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
     const int nn = static_cast<int>(k->size(2));
-    void* st = stream_of(device);
-    const int rc = kind == 3 ? fq_append_kv_turbo(c3, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), nn, st)
-                             : fq_append_kv_int4(c4, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), nn, st);
+    int rc;
+    {
+        const NoGil released;
+        const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+        void* st = stream_of(device);
+        rc = kind == 3 ? fq_append_kv_turbo(c3, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), nn, st)
+                       : fq_append_kv_int4(c4, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), nn, st);
+    }
     return PyLong_FromLong(rc);
 }
 
