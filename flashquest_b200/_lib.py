@@ -229,9 +229,17 @@ def dtype_code(t: torch.Tensor) -> int:
 
 
 def require_cuda(*tensors):
+    """All on one GPU: a kernel takes addresses, and one of another GPU would be a bad address, not an error."""
+    device = None
     for t in tensors:
-        if t is not None and not t.is_cuda:
+        if t is None:
+            continue
+        if not t.is_cuda:
             raise FlashQuestError("flashquest_b200 operators take CUDA tensors (no CPU path)")
+        if device is None:
+            device = t.get_device()
+        elif t.get_device() != device:
+            raise FlashQuestError(f"tensors on different GPUs: cuda:{device} and cuda:{t.get_device()}")
 
 
 def ptr(t):

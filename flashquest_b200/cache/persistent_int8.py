@@ -83,7 +83,7 @@ class PersistentInt8KVCache(Cache):
             if K_new.stride(3) != 1 or V_new.stride() != K_new.stride() or any(s % 8 for s in K_new.stride()[:3]) \
                     or K_new.data_ptr() % 16 or V_new.data_ptr() % 16:
                 K_new, V_new = K_new.contiguous(), V_new.contiguous()
-            require_cuda(K_new, V_new)
+            require_cuda(K_new, V_new, self.K_uint8)
             check(lib().fq_append_kv_int8(ctypes.byref(self.desc()), li, seen, ptr(K_new), ptr(V_new), *K_new.stride()[:3], S_new,
                                           stream_ptr(self.K_uint8.device)))
             self._seen_tokens[layer_idx] = seen + S_new

@@ -52,6 +52,9 @@ int dtype_of(const at::Tensor& t) {
 
 inline const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 
+// on the GPU whose buffers the plan or cache holds: an address of another one would be read there
+inline bool on_device(const at::Tensor& t, int device) { return t.is_cuda() && t.get_device() == device; }
+
 void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream(); }
 
 // The native calls run without the GIL, as ctypes calls do: a launch blocks while the stream's queue is full, and other
@@ -113,7 +116,7 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int B = p->kind == 3 ? p->c3.B : p->c4.B, Hkv = p->kind == 3 ? p->c3.Hkv : p->c4.Hkv, D = p->kind == 3 ? p->c3.D : p->c4.D;
     const int Hq = p->prm.Hq;
     const int qd = static_cast<int>(q->dim());
-    const bool ok = k->dim() == 4 && v->dim() == 4 && (qd == 3 || (qd == 4 && q->size(2) == 1)) && k->is_cuda() && v->is_cuda() && q->is_cuda() &&
+    const bool ok = k->dim() == 4 && v->dim() == 4 && (qd == 3 || (qd == 4 && q->size(2) == 1)) && on_device(*k, p->device) && on_device(*v, p->device) && on_device(*q, p->device) &&
                     dtype_of(*k) == p->cache_dtype && dtype_of(*v) == p->cache_dtype && dtype_of(*q) >= 0 &&
                     k->sizes() == v->sizes() && k->strides() == v->strides() && k->size(0) == B && k->size(1) == Hkv && k->size(3) == D &&
                     k->stride(3) == 1 && q->size(0) == B && q->size(1) == Hq && q->size(qd - 1) == D && q->stride(qd - 1) == 1 &&
@@ -146,7 +149,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int dt = t[0] ? dtype_of(*t[0]) : -1;
     if (dt != FQ_F16 && dt != FQ_BF16) return PyLong_FromLong(1);
     for (int i = 0; i < 5; ++i) {
-        if (!t[i] || !t[i]->is_cuda() || dtype_of(*t[i]) != dt || t[i]->dim() != 3 || t[i]->size(1) != 1 || t[i]->stride(2) != 1) return PyLong_FromLong(1);
+        if (!t[i] || !on_device(*t[i], p->device) || dtype_of(*t[i]) != dt || t[i]->dim() != 3 || t[i]->size(1) != 1 || t[i]->stride(2) != 1) return PyLong_FromLong(1);
         const int64_t width = i == 0 ? static_cast<int64_t>(Hq) * D : i < 3 ? static_cast<int64_t>(Hkv) * D : D;
         if (t[i]->size(2) != width || !(t[i]->size(0) == B || (i >= 3 && t[i]->size(0) == 1))) return PyLong_FromLong(1);
     }
@@ -178,8 +181,8 @@ PyObject* append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const auto* c4 = static_cast<const fq_int4_cache*>(desc);
     const int B = kind == 3 ? c3->B : c4->B, Hkv = kind == 3 ? c3->Hkv : c4->Hkv, D = kind == 3 ? c3->D : c4->D;
     const int dt = kind == 3 ? c3->kv_dtype : c4->kv_dtype;
-    if (!k || !v || (dt != FQ_F16 && dt != FQ_BF16) || k->dim() != 4 || !k->is_cuda() || !v->is_cuda() || k->get_device() != device ||
-        v->get_device() != device || dtype_of(*k) != dt || dtype_of(*v) != dt || k->sizes() != v->sizes() || k->strides() != v->strides() ||
+    if (!k || !v || (dt != FQ_F16 && dt != FQ_BF16) || k->dim() != 4 || !on_device(*k, device) || !on_device(*v, device) ||
+        dtype_of(*k) != dt || dtype_of(*v) != dt || k->sizes() != v->sizes() || k->strides() != v->strides() ||
         k->size(0) != B || k->size(1) != Hkv || k->size(3) != D || k->stride(3) != 1 || k->size(2) < 1)
         return PyLong_FromLong(1);
     const int nn = static_cast<int>(k->size(2));

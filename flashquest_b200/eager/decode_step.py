@@ -14,7 +14,7 @@ import math
 
 import torch
 
-from .._lib import DecodeParams, bind, check, dtype_code, lib, ptr, stream_ptr
+from .._lib import DecodeParams, bind, check, dtype_code, lib, ptr, require_cuda, stream_ptr
 
 
 class _NativeSteps:
@@ -66,7 +66,7 @@ class _NativeSteps:
             q = q.reshape(self.B, self.Hq, self.D).contiguous()
             rc = self._step(self._plan_, layer_idx, seen, k_new, v_new, q, addr)
             if rc == 1:
-                raise ValueError(f"step: k, v must be (B={self.B}, H_kv={self.Hkv}, n, D={self.D}) and q (B, H_q={self.Hq}, 1, D) CUDA tensors")
+                raise ValueError(f"step: k, v must be (B={self.B}, H_kv={self.Hkv}, n, D={self.D}) and q (B, H_q={self.Hq}, 1, D) tensors on {self.device}")
         if rc:
             check(rc)
         self.cache._seen_tokens[layer_idx] = seen + n_new
@@ -163,6 +163,7 @@ class QuestDecodeInt4(_NativeSteps):
         n_new = k_new.shape[3]
         if k_new.shape[0] != Ln or q.shape[0] != Ln:
             raise ValueError(f"expected {Ln} layers, got {k_new.shape[0]} / {q.shape[0]}")
+        require_cuda(k_new, v_new, q, self.O)
         for li in range(Ln):
             if c._seen_tokens[li] + n_new > c.max_seq_len:
                 raise RuntimeError(f"PersistentInt4KVCache: seen+new={c._seen_tokens[li] + n_new} exceeds max_seq_len={c.max_seq_len}")
@@ -199,6 +200,7 @@ class QuestDecodeInt4(_NativeSteps):
         n_new = k_new.shape[3]
         if not (1 <= n_new < self.page):
             raise ValueError(f"n_new={n_new} must be in [1, page_size)")
+        require_cuda(k_new, v_new, q, self.O)
         if k_new.dtype != c.dtype or v_new.dtype != c.dtype or k_new.stride(4) != 1 or v_new.stride() != k_new.stride():
             raise ValueError("k_new / v_new must be dense tensors of the cache's dtype with equal strides")
         q4 = q.view(Ln, self.B, self.Hq, self.D)
@@ -244,6 +246,7 @@ class QuestDecodeInt4(_NativeSteps):
         partial_len = seen % page
         completed = seen - partial_len
         P = completed // page
+        require_cuda(q, self.O)
         q3 = q.reshape(self.B, self.Hq, self.D)
         li = layer_idx
         L = lib()

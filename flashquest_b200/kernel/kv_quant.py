@@ -24,7 +24,7 @@ def quantize_kv_int4_into(K_new, V_new, page_size, n_quant, *, K_packed=None, K_
     the left-over tokens into the staging views.  This is the page-flush step of
     PersistentInt4KVCache.update_quantized (cache/persistent_int4.py:94-130) as one kernel."""
     ref = K_new if K_new is not None else V_new
-    require_cuda(ref)
+    require_cuda(K_new, V_new, K_packed, V_packed, K_scale, V_scale, K_head, V_head, stage_K, stage_V)
     B, H, n_new, D = ref.shape
     if D % 2 != 0:
         raise ValueError(f"quantize_k_int4 requires even head_dim; got {D}")
@@ -126,7 +126,7 @@ def dequantize_v_int4(V_packed, scale, mn) -> torch.Tensor:
 def quantize_kv_int8_into(K, V, page_size, *, K_uint8=None, K_scale=None, K_mn=None, V_uint8=None, V_scale=None, V_mn=None):
     """One call of fq_quantize_kv_int8 writing into (possibly strided) output views; K or V may be None."""
     ref = K if K is not None else V
-    require_cuda(ref)
+    require_cuda(K, V, K_uint8, V_uint8)
     B, H, S, D = ref.shape
     K = inner_contiguous(K) if K is not None else None
     V = inner_contiguous(V) if V is not None else None
@@ -206,7 +206,7 @@ K_TURBO_CODEBOOK_VALUES = (-2.1519, -1.3439, -0.7560, -0.2451, 0.2451, 0.7560, 1
 def quantize_turbo_into(x_new, n_quant, *, msb, lsb, scale, head=None, n_head=0):
     """One launch of fq_quantize_turbo over the stream head[:n_head] ++ x_new, writing planes
     and scales into (possibly strided) views."""
-    require_cuda(x_new)
+    require_cuda(x_new, head, msb)
     B, H, n_new, D = x_new.shape
     x_new = inner_contiguous(x_new)
     z3 = (0, 0, 0)
