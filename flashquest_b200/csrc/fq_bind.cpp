@@ -55,6 +55,14 @@ inline const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? 
 // on the GPU whose buffers the plan or cache holds: an address of another one would be read there
 inline bool on_device(const at::Tensor& t, int device) { return t.is_cuda() && t.get_device() == device; }
 
+// equal strides wherever a stride is used: that of an axis of length 1 can be anything, also after contiguous()
+bool same_layout(const at::Tensor& a, const at::Tensor& b) {
+    if (a.sizes() != b.sizes()) return false;
+    for (int64_t i = 0; i < a.dim(); ++i)
+        if (a.size(i) != 1 && a.stride(i) != b.stride(i)) return false;
+    return true;
+}
+
 void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream(); }
 
 // The native calls run without the GIL, as ctypes calls do: a launch blocks while the stream's queue is full, and other
@@ -118,17 +126,18 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int qd = static_cast<int>(q->dim());
     const bool ok = k->dim() == 4 && v->dim() == 4 && (qd == 3 || (qd == 4 && q->size(2) == 1)) && on_device(*k, p->device) && on_device(*v, p->device) && on_device(*q, p->device) &&
                     dtype_of(*k) == p->cache_dtype && dtype_of(*v) == p->cache_dtype && dtype_of(*q) >= 0 &&
-                    k->sizes() == v->sizes() && k->strides() == v->strides() && k->size(0) == B && k->size(1) == Hkv && k->size(3) == D &&
+                    same_layout(*k, *v) && k->size(0) == B && k->size(1) == Hkv && k->size(3) == D &&
                     k->stride(3) == 1 && q->size(0) == B && q->size(1) == Hq && q->size(qd - 1) == D && q->stride(qd - 1) == 1 &&
-                    (p->kind != 3 || (q->stride(1) == D && q->stride(0) == static_cast<int64_t>(Hq) * D));
+                    (p->kind != 3 || ((Hq == 1 || q->stride(1) == D) && (B == 1 || q->stride(0) == static_cast<int64_t>(Hq) * D)));
     if (!ok) return PyLong_FromLong(1);
+    const int64_t q_sb = p->kind == 3 ? static_cast<int64_t>(Hq) * D : q->stride(0), q_sh = p->kind == 3 ? D : q->stride(1);
     const fq_decode_params par = prm ? *prm : p->prm;
     int rc;
     {
         const NoGil released;
         const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
         rc = run_layer(p, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), static_cast<int>(k->size(2)),
-                       q->data_ptr(), dtype_of(*q), q->stride(0), q->stride(1), &par, stream_of(p->device));
+                       q->data_ptr(), dtype_of(*q), q_sb, q_sh, &par, stream_of(p->device));
     }
     return PyLong_FromLong(rc);
 }
@@ -182,7 +191,7 @@ PyObject* append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int B = kind == 3 ? c3->B : c4->B, Hkv = kind == 3 ? c3->Hkv : c4->Hkv, D = kind == 3 ? c3->D : c4->D;
     const int dt = kind == 3 ? c3->kv_dtype : c4->kv_dtype;
     if (!k || !v || (dt != FQ_F16 && dt != FQ_BF16) || k->dim() != 4 || !on_device(*k, device) || !on_device(*v, device) ||
-        dtype_of(*k) != dt || dtype_of(*v) != dt || k->sizes() != v->sizes() || k->strides() != v->strides() ||
+        dtype_of(*k) != dt || dtype_of(*v) != dt || !same_layout(*k, *v) ||
         k->size(0) != B || k->size(1) != Hkv || k->size(3) != D || k->stride(3) != 1 || k->size(2) < 1)
         return PyLong_FromLong(1);
     const int nn = static_cast<int>(k->size(2));

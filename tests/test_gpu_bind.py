@@ -56,3 +56,32 @@ def test_other_threads_run_while_the_launch_queue_is_full(call):
     torch.cuda.synchronize()
     assert took > 0.3, "the launch queue did not fill: nothing was tested"
     assert max(gaps) < 0.1, max(gaps)
+
+
+def _restride(t, axis, by):
+    """The same tensor with another stride on an axis of length 1."""
+    assert t.shape[axis] == 1
+    strides = list(t.stride())
+    strides[axis] += by
+    return t.as_strided(t.shape, strides)
+
+
+@pytest.mark.parametrize("kind,Hq,Hkv", [(4, 4, 2), (3, 4, 2), (8, 4, 2), (3, 1, 1), (4, 1, 1)])
+def test_strides_of_axes_of_length_one_do_not_matter(kind, Hq, Hkv):
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    from flashquest_b200.eager.decode_step import QuestDecodeInt4, QuestDecodeInt8, QuestDecodeTurbo
+    cls, eng = {3: (PersistentTurboKVCache, QuestDecodeTurbo), 4: (PersistentInt4KVCache, QuestDecodeInt4), 8: (PersistentInt8KVCache, QuestDecodeInt8)}[kind]
+    g = torch.Generator(device="cuda").manual_seed(6)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).half()
+    cache = cls(batch_size=1, num_layers=1, num_kv_heads=Hkv, head_dim=64, max_seq_len=128, page_size=16, dtype=torch.float16)
+    cache.update_quantized(r(1, Hkv, 70, 64), r(1, Hkv, 70, 64), 0)
+    engine = eng(cache, num_q_heads=Hq, retention=0.5, num_sinks=1, window_pages=1, q_dtype=torch.float16)
+    k, v, q = r(1, Hkv, 1, 64), r(1, Hkv, 1, 64), r(1, Hq, 1, 64)
+    want = [t.clone() for t in engine.step(k, v, q, 0)]
+    odd = [_restride(_restride(t, 0, by), 2, by) for t, by in ((k, 8), (v, 24), (q, 40))]
+    if Hq == 1:
+        odd = [_restride(t, 1, 16) for t in odd]
+    cache._seen_tokens[0] = 70
+    assert all(torch.equal(a, b) for a, b in zip(want, engine.step(*odd, 0)))

@@ -186,3 +186,41 @@ def test_patch_argument_errors():
     with pytest.raises(NotImplementedError, match="kv_bits=4"):
         lpp.make_quest_persistent_forward(cache=Fake(), head_pattern_layer=torch.ones(2, dtype=torch.bool), retention=0.5,
                                           num_sinks=2, window_pages=1, page_size=16, use_compact_kernel=True)
+
+
+def _oracle_checked_run(kv_bits, page, head_dim=64, model_dtype=torch.bfloat16, compact=False, n_steps=None, fused=True):
+    """Prefill and decode steps across a page end, every attention call replayed on the oracle; returns (cache, patched model)."""
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    from flashquest_b200.eager import llama_persistent_patch as lpp
+    from transformers import AutoConfig
+    from transformers.models.llama.modeling_llama import LlamaModel
+    cfg = AutoConfig.for_model("llama", hidden_size=256, num_attention_heads=4, num_key_value_heads=2, num_hidden_layers=2,
+                               intermediate_size=256, max_position_embeddings=512, vocab_size=128, head_dim=head_dim)
+    torch.manual_seed(7)
+    model = LlamaModel(cfg).cuda().to(model_dtype).eval()
+    S, n_steps = 4 * page - 3, n_steps or 7
+    cache = {3: PersistentTurboKVCache, 4: PersistentInt4KVCache, 8: PersistentInt8KVCache}[kv_bits](
+        num_layers=2, batch_size=1, num_kv_heads=2, head_dim=head_dim, page_size=page, max_seq_len=8 * page)
+    pattern = torch.tensor([[True, True], [True, False]])
+    retention, sinks, window = 0.5, 2, 1
+    lpp.patch_llama_for_quest_persistent(model, cache=cache, head_pattern=pattern, retention=retention, num_sinks=sinks, window_pages=window,
+                                         page_size=page, use_compact_kernel=compact)
+    rows = [torch.where(pattern[l].repeat_interleave(2), torch.tensor(retention), torch.tensor(0.0)).float() for l in range(2)]
+    g = torch.Generator(device="cuda").manual_seed(8)
+    ids = torch.randint(0, 128, (1, S + n_steps), device="cuda", generator=g)
+    check = _OracleCheck(kv_bits, page, 2, 4, rows, sinks, window, math.ceil(retention * 8), fused_tail=fused)
+    lpp.TRACE = check
+    try:
+        _run(model, cache, ids[:, :S], ids[:, S:])
+    finally:
+        lpp.TRACE = None
+    assert check.calls == 2 * (1 + n_steps) and cache.get_seq_length() == S + n_steps
+    return cache, model
+
+
+@pytest.mark.parametrize("kv_bits,compact", [(3, False), (4, False), (4, True), (8, False)])
+def test_fp32_model_on_a_16_bit_cache(kv_bits, compact):
+    """Outside the dtypes of the one-call route: Hugging Face's rotary embedding, then the native step."""
+    _oracle_checked_run(kv_bits, 16, model_dtype=torch.float32, compact=compact)
