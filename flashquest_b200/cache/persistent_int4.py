@@ -92,6 +92,9 @@ class PersistentInt4KVCache(Cache):
                 check(rc)
                 self._seen_tokens[layer_idx] = seen + S_new
                 return
+        if K_new.shape != V_new.shape or K_new.shape[0] > self.batch_size or K_new.shape[1] > self.num_kv_heads or K_new.shape[3] != self.head_dim:
+            raise ValueError(f"PersistentInt4KVCache: K_new and V_new must be (B={self.batch_size}, H_kv={self.num_kv_heads}, n, D={self.head_dim}); "
+                             f"got {tuple(K_new.shape)} and {tuple(V_new.shape)}")
         if K_new.dtype != self.dtype:
             K_new = K_new.to(self.dtype)
         if V_new.dtype != self.dtype:

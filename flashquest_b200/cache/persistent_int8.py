@@ -75,6 +75,9 @@ class PersistentInt8KVCache(Cache):
         S_new = K_new.shape[2]
         if seen + S_new > self.max_seq_len:
             raise RuntimeError(f"PersistentInt8KVCache: seen+new={seen + S_new} exceeds max_seq_len={self.max_seq_len}")
+        want = (self.batch_size, self.num_kv_heads, S_new, self.head_dim)
+        if K_new.shape != want or V_new.shape != want:       # the launch takes addresses: it would read past a smaller tensor
+            raise RuntimeError(f"PersistentInt8KVCache: K_new and V_new must be {want}; got {tuple(K_new.shape)} and {tuple(V_new.shape)}")
         page = self.page_size
         li = layer_idx
         if S_new > 0 and self._one_launch:
