@@ -85,7 +85,8 @@ class PersistentInt8KVCache(Cache):
                 K_new, V_new = K_new.to(self.dtype), V_new.to(self.dtype)
             if K_new.stride(3) != 1 or V_new.stride() != K_new.stride() or any(s % 8 for s in K_new.stride()[:3]) \
                     or K_new.data_ptr() % 16 or V_new.data_ptr() % 16:
-                K_new, V_new = K_new.contiguous(), V_new.contiguous()
+                # copies, not contiguous(): that hands back a dense tensor off a 16-byte boundary as it is
+                K_new, V_new = (t.clone(memory_format=torch.contiguous_format) for t in (K_new, V_new))
             require_cuda(K_new, V_new, self.K_uint8)
             check(lib().fq_append_kv_int8(ctypes.byref(self.desc()), li, seen, ptr(K_new), ptr(V_new), *K_new.stride()[:3], S_new,
                                           stream_ptr(self.K_uint8.device)))

@@ -55,6 +55,14 @@ inline const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? 
 // on the GPU whose buffers the plan or cache holds: an address of another one would be read there
 inline bool on_device(const at::Tensor& t, int device) { return t.is_cuda() && t.get_device() == device; }
 
+// every row of a 16-bit tensor on a 16-byte boundary
+bool rows_aligned(const at::Tensor& t) {
+    if (reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) return false;
+    for (int64_t i = 0; i + 1 < t.dim(); ++i)
+        if (t.stride(i) % 8) return false;
+    return true;
+}
+
 // equal strides wherever a stride is used: that of an axis of length 1 can be anything, also after contiguous()
 bool same_layout(const at::Tensor& a, const at::Tensor& b) {
     if (a.sizes() != b.sizes()) return false;
@@ -129,7 +137,8 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
                     same_layout(*k, *v) && k->size(0) == B && k->size(1) == Hkv && k->size(3) == D &&
                     k->stride(3) == 1 && q->size(0) == B && q->size(1) == Hq && q->size(qd - 1) == D && q->stride(qd - 1) == 1 &&
                     (p->kind != 3 || ((Hq == 1 || q->stride(1) == D) && (B == 1 || q->stride(0) == static_cast<int64_t>(Hq) * D)));
-    if (!ok) return PyLong_FromLong(1);
+    // the INT8 append takes 16-byte aligned rows only (the other two refuse the rest themselves)
+    if (!ok || (p->kind == 8 && k->size(2) > 0 && !(rows_aligned(*k) && rows_aligned(*v)))) return PyLong_FromLong(1);
     const int64_t q_sb = p->kind == 3 ? static_cast<int64_t>(Hq) * D : q->stride(0), q_sh = p->kind == 3 ? D : q->stride(1);
     const fq_decode_params par = prm ? *prm : p->prm;
     int rc;

@@ -20,6 +20,7 @@ from .._lib import DecodeParams, bind, check, dtype_code, lib, ptr, require_cuda
 class _NativeSteps:
     """step() and forward_token() over the CPython module (csrc/fq_bind.cpp): one call that reads pointers and strides
     from the tensors itself.  The subclass has set the cache descriptor, the parameters and the preallocated buffers."""
+    COPY_ROWS = False        # rows off a 16-byte boundary are copied before the append (a dense tensor can be off it)
 
     def _build_plan(self, kind, scores, compact, workspace, scratch=None):
         """scores, compact, workspace: with a leading layer dimension, or shared by the layers (stride 0)."""
@@ -61,7 +62,9 @@ class _NativeSteps:
         if rc == 1:            # another dtype, or strides the kernels do not take: prepare and call again
             dt = self.cache.dtype
             k_new, v_new = k_new.to(dt), v_new.to(dt)
-            if k_new.stride(3) != 1 or v_new.stride() != k_new.stride():
+            if self.COPY_ROWS:
+                k_new, v_new = (t.clone(memory_format=torch.contiguous_format) for t in (k_new, v_new))
+            elif k_new.stride(3) != 1 or v_new.stride() != k_new.stride():
                 k_new, v_new = k_new.contiguous(), v_new.contiguous()
             q = q.reshape(self.B, self.Hq, self.D).contiguous()
             rc = self._step(self._plan_, layer_idx, seen, k_new, v_new, q, addr)
@@ -332,6 +335,7 @@ class QuestDecodeInt8(_NativeSteps):
     (flashquest/eager/llama_persistent_patch.py:202-245) as ONE foreign call per layer (fq_decode_layer_int8): append, page
     scores, top-k with compact index, attention with the staged tail in the same softmax."""
     LAUNCHES = 5
+    COPY_ROWS = True
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,
                  q_dtype=torch.bfloat16, n_split: int | None = None):

@@ -85,3 +85,29 @@ def test_strides_of_axes_of_length_one_do_not_matter(kind, Hq, Hkv):
         odd = [_restride(t, 1, 16) for t in odd]
     cache._seen_tokens[0] = 70
     assert all(torch.equal(a, b) for a, b in zip(want, engine.step(*odd, 0)))
+
+
+@pytest.mark.parametrize("form", ["dense", "rows"])
+@pytest.mark.parametrize("n", [1, 37])
+def test_int8_takes_rows_off_a_16_byte_boundary(form, n):
+    """As its torch.cat form did: a dense tensor two bytes off, and rows of D + 1 values."""
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.eager.decode_step import QuestDecodeInt8
+    g = torch.Generator(device="cuda").manual_seed(9)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).half()
+
+    def off(t):
+        if form == "dense":
+            out = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape)
+        else:
+            out = torch.empty(*t.shape[:-1], t.shape[-1] + 1, dtype=t.dtype, device="cuda")[..., :-1]
+        return out.copy_(t)
+    k0, v0, k, v, q = r(2, 2, 30, 64), r(2, 2, 30, 64), r(2, 2, n, 64), r(2, 2, n, 64), r(2, 4, 1, 64)
+    results = []
+    for f in (lambda t: t, off):
+        cache = PersistentInt8KVCache(batch_size=2, num_layers=1, num_kv_heads=2, head_dim=64, max_seq_len=128, page_size=16, dtype=torch.float16)
+        engine = QuestDecodeInt8(cache, num_q_heads=4, retention=0.5, num_sinks=1, window_pages=1, q_dtype=torch.float16)
+        cache.update_quantized(f(k0), f(v0), 0)
+        out = [t.clone() for t in engine.step(f(k), f(v), q, 0)]
+        results.append(out + [t.clone() for t in cache.get_views(0).values() if torch.is_tensor(t)])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
