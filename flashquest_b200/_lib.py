@@ -165,6 +165,7 @@ _PROTOTYPES["fq_append_kv_turbo"] = (I, [ctypes.POINTER(TurboCacheDesc), I, I, P
 _PROTOTYPES["fq_append_kv_int8"] = (I, [ctypes.POINTER(Int4CacheDesc), I, I, P, P, L, L, L, I, P])
 _PROTOTYPES["fq_decode_layer_int8"] = _PROTOTYPES["fq_decode_layer_int4"]
 _PROTOTYPES["fq_rope_qkv"] = (I, [P, L, P, L, P, L, I, P, L, P, L, I, I, I, I, P, P, P, I, P])
+_PROTOTYPES["fq_rope_qkv_pattern"] = (I, [P, L, P, L, P, L, I, P, L, P, L, I, I, I, I, P, P, P, I, P, L, F, P, P])
 
 # entry points added by later sources register themselves here (name -> (restype, argtypes))
 EXTRA_PROTOTYPES: dict = {}

@@ -31,6 +31,7 @@ struct Plan {
     char* ws; size_t ws_sl, ws_bytes;
     char* scratch; size_t scratch_bytes;
     char *q_rot, *k_rot, *v_rot;    // rotated q / k and cast v of the patched forward, dense, cache dtype
+    float* retention;               // (n_layers, H_q): written by the patched forward from the head pattern
 };
 
 const char* kPlanName = "flashquest_b200.plan";
@@ -81,9 +82,9 @@ struct NoGil {
 };
 
 // plan(kind, cache_desc, params, device, n_layers, scores, sc_sl, compact, cp_sl, O, o_sl_bytes, lse, lse_sl,
-//      ws, ws_sl, ws_bytes, scratch, scratch_bytes, q_rot, k_rot, v_rot): addresses and sizes as integers
+//      ws, ws_sl, ws_bytes, scratch, scratch_bytes, q_rot, k_rot, v_rot, retention): addresses and sizes as integers
 PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 21) { PyErr_SetString(PyExc_TypeError, "plan() takes 21 arguments"); return nullptr; }
+    if (n != 22) { PyErr_SetString(PyExc_TypeError, "plan() takes 22 arguments"); return nullptr; }
     Plan* p = new Plan();
     p->kind = static_cast<int>(PyLong_AsLong(a[0]));
     if (p->kind == 3) { p->c3 = *static_cast<const fq_turbo_cache*>(as_ptr(a[1])); p->cache_dtype = p->c3.kv_dtype; }
@@ -98,6 +99,7 @@ PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p->ws = static_cast<char*>(as_ptr(a[13])); p->ws_sl = PyLong_AsSize_t(a[14]); p->ws_bytes = PyLong_AsSize_t(a[15]);
     p->scratch = static_cast<char*>(as_ptr(a[16])); p->scratch_bytes = PyLong_AsSize_t(a[17]);
     p->q_rot = static_cast<char*>(as_ptr(a[18])); p->k_rot = static_cast<char*>(as_ptr(a[19])); p->v_rot = static_cast<char*>(as_ptr(a[20]));
+    p->retention = static_cast<float*>(as_ptr(a[21]));
     if (PyErr_Occurred()) { delete p; return nullptr; }
     return PyCapsule_New(p, kPlanName, free_plan);
 }
@@ -151,10 +153,11 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return PyLong_FromLong(rc);
 }
 
-// forward(plan, layer, seen, q, k, v, cos, sin, params | 0): one new token of the patched attention forward.
-// q (B,1,H_q*D), k, v (B,1,H_kv*D): the projections as the linears return them; cos, sin (B or 1,1,D) of the same dtype.
+// forward(plan, layer, seen, q, k, v, cos, sin, params | 0, pattern | None): one new token of the patched attention forward.
+// q (B,1,H_q*D), k, v (B,1,H_kv*D): the projections as the linears return them; cos, sin (B or 1,1,D) of the same dtype;
+// pattern (H_kv,) bool, read by the launch: retrieval heads keep the parameters' retention, streaming heads 0.
 PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 9) { PyErr_SetString(PyExc_TypeError, "forward() takes 9 arguments"); return nullptr; }
+    if (n != 10) { PyErr_SetString(PyExc_TypeError, "forward() takes 10 arguments"); return nullptr; }
     const Plan* p = plan_of(a[0]);
     if (!p) return nullptr;
     const int layer = static_cast<int>(PyLong_AsLong(a[1])), seen = static_cast<int>(PyLong_AsLong(a[2]));
@@ -171,15 +174,21 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const int64_t width = i == 0 ? static_cast<int64_t>(Hq) * D : i < 3 ? static_cast<int64_t>(Hkv) * D : D;
         if (t[i]->size(2) != width || !(t[i]->size(0) == B || (i >= 3 && t[i]->size(0) == 1))) return PyLong_FromLong(1);
     }
+    const at::Tensor* pat = a[9] == Py_None ? nullptr : tensor_of(a[9]);
+    if (a[9] != Py_None && (!pat || !on_device(*pat, p->device) || pat->scalar_type() != at::kBool || pat->dim() != 1 || pat->size(0) != Hkv))
+        return PyLong_FromLong(1);
     const int64_t cs = t[3]->size(0) == 1 ? 0 : t[3]->stride(0), ss = t[4]->size(0) == 1 ? 0 : t[4]->stride(0);
-    const fq_decode_params par = prm ? *prm : p->prm;
+    fq_decode_params par = prm ? *prm : p->prm;
+    float* ret = p->retention + static_cast<int64_t>(layer) * Hq;
+    if (pat) par.retention_per_head = ret;
     int rc;
     {
         const NoGil released;
         const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
         void* st = stream_of(p->device);
-        rc = fq_rope_qkv(t[0]->data_ptr(), t[0]->stride(0), t[1]->data_ptr(), t[1]->stride(0), t[2]->data_ptr(), t[2]->stride(0), dt,
-                         t[3]->data_ptr(), cs, t[4]->data_ptr(), ss, B, Hq, Hkv, D, p->q_rot, p->k_rot, p->v_rot, p->cache_dtype, st);
+        rc = fq_rope_qkv_pattern(t[0]->data_ptr(), t[0]->stride(0), t[1]->data_ptr(), t[1]->stride(0), t[2]->data_ptr(), t[2]->stride(0), dt,
+                         t[3]->data_ptr(), cs, t[4]->data_ptr(), ss, B, Hq, Hkv, D, p->q_rot, p->k_rot, p->v_rot, p->cache_dtype,
+                                 pat ? static_cast<const uint8_t*>(pat->data_ptr()) : nullptr, pat ? pat->stride(0) : 0, par.retention, ret, st);
         if (rc == 0)
             rc = run_layer(p, layer, seen, p->k_rot, p->v_rot, static_cast<int64_t>(Hkv) * D, D, D, 1, p->q_rot, p->cache_dtype,
                            static_cast<int64_t>(Hq) * D, D, &par, st);

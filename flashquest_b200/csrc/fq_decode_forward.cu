@@ -9,15 +9,19 @@ namespace fq {
 // q*cos + rotate_half(q)*sin, every product and the sum rounded to the model's dtype TM, then cast to the cache's
 // dtype TC; v is only cast.  One CTA per (head, batch), a thread per channel pair (i, i + D/2).  Latency-bound: it
 // replaces eleven element-wise launches of a few hundred values each.
+// `pattern` (one byte per KV head, not 0: a retrieval head) is turned into the retention of every query head here, at each
+// call: the caller's tensor may have changed since the last one.  The selection, three launches on, reads the result.
 template <typename TM, typename TC>
 __global__ void __launch_bounds__(64) rope_qkv_kernel(const TM* __restrict__ q, int64_t q_sb, const TM* __restrict__ k, int64_t k_sb,
                                                       const TM* __restrict__ v, int64_t v_sb, const TM* __restrict__ cosv, int64_t c_sb,
                                                       const TM* __restrict__ sinv, int64_t s_sb, int Hq, int Hkv, int D,
-                                                      TC* __restrict__ q_out, TC* __restrict__ k_out, TC* __restrict__ v_out) {
+                                                      TC* __restrict__ q_out, TC* __restrict__ k_out, TC* __restrict__ v_out,
+                                                      const uint8_t* __restrict__ pattern, int64_t pt_s, float retention, float* __restrict__ ret_out) {
     const int head = blockIdx.x, b = blockIdx.y, half = D / 2, i = threadIdx.x;
     pdl_wait();
     pdl_trigger();
     if (i >= half) return;
+    if (pattern != nullptr && i == 0 && b == 0 && head < Hq) ret_out[head] = pattern[(head / (Hq / Hkv)) * pt_s] ? retention : 0.0f;
     const bool is_q = head < Hq, is_v = head >= Hq + Hkv;
     const int hh = is_q ? head : is_v ? head - Hq - Hkv : head - Hq;
     const TM* src = (is_q ? q + b * q_sb : is_v ? v + b * v_sb : k + b * k_sb) + (int64_t)hh * D;
@@ -36,11 +40,12 @@ __global__ void __launch_bounds__(64) rope_qkv_kernel(const TM* __restrict__ q, 
 
 template <typename TM, typename TC>
 static void launch_rope_qkv(const void* q, int64_t q_sb, const void* k, int64_t k_sb, const void* v, int64_t v_sb, const void* c, int64_t c_sb,
-                            const void* s, int64_t s_sb, int B, int Hq, int Hkv, int D, void* qo, void* ko, void* vo, cudaStream_t st) {
+                            const void* s, int64_t s_sb, int B, int Hq, int Hkv, int D, void* qo, void* ko, void* vo,
+                            const uint8_t* pattern, int64_t pt_s, float retention, float* ret_out, cudaStream_t st) {
     launch_k(PDL_QUANT, rope_qkv_kernel<TM, TC>, dim3((unsigned)(Hq + 2 * Hkv), (unsigned)B), dim3(64), 0, st,
              static_cast<const TM*>(q), q_sb, static_cast<const TM*>(k), k_sb, static_cast<const TM*>(v), v_sb,
              static_cast<const TM*>(c), c_sb, static_cast<const TM*>(s), s_sb, Hq, Hkv, D,
-             static_cast<TC*>(qo), static_cast<TC*>(ko), static_cast<TC*>(vo));
+             static_cast<TC*>(qo), static_cast<TC*>(ko), static_cast<TC*>(vo), pattern, pt_s, retention, ret_out);
 }
 
 }  // namespace fq
@@ -48,8 +53,17 @@ static void launch_rope_qkv(const void* q, int64_t q_sb, const void* k, int64_t 
 extern "C" int fq_rope_qkv(const void* q, int64_t q_sb, const void* k, int64_t k_sb, const void* v, int64_t v_sb, int dtype,
                            const void* cosv, int64_t cos_sb, const void* sinv, int64_t sin_sb, int B, int Hq, int Hkv, int D,
                            void* q_out, void* k_out, void* v_out, int out_dtype, void* stream) {
+    return fq_rope_qkv_pattern(q, q_sb, k, k_sb, v, v_sb, dtype, cosv, cos_sb, sinv, sin_sb, B, Hq, Hkv, D, q_out, k_out, v_out, out_dtype,
+                               nullptr, 0, 0.0f, nullptr, stream);
+}
+
+extern "C" int fq_rope_qkv_pattern(const void* q, int64_t q_sb, const void* k, int64_t k_sb, const void* v, int64_t v_sb, int dtype,
+                                   const void* cosv, int64_t cos_sb, const void* sinv, int64_t sin_sb, int B, int Hq, int Hkv, int D,
+                                   void* q_out, void* k_out, void* v_out, int out_dtype,
+                                   const uint8_t* pattern, int64_t pattern_stride, float retention, float* retention_per_head, void* stream) {
     using namespace fq;
     const char* fn = "fq_rope_qkv";
+    FQ_CHECK_ARG(!pattern || (retention_per_head && Hkv > 0 && Hq % Hkv == 0), FQ_ERR_ARG, "%s: a head pattern needs H_q a multiple of H_kv and an output", fn);
     FQ_CHECK_ARG(q && k && v && cosv && sinv && q_out && k_out && v_out, FQ_ERR_ARG, "%s: null pointer", fn);
     FQ_CHECK_ARG(B > 0 && Hq > 0 && Hkv > 0 && D > 0 && D % 2 == 0 && D <= 128 && B <= 65535, FQ_ERR_ARG, "%s: bad sizes", fn);
     FQ_CHECK_ARG((dtype == FQ_F16 || dtype == FQ_BF16) && (out_dtype == FQ_F16 || out_dtype == FQ_BF16), FQ_ERR_DTYPE, "%s: fp16 or bf16 only", fn);
@@ -57,7 +71,7 @@ extern "C" int fq_rope_qkv(const void* q, int64_t q_sb, const void* k, int64_t k
     using hf = __half; using bf = __nv_bfloat16;
     auto go = dtype == FQ_F16 ? (out_dtype == FQ_F16 ? launch_rope_qkv<hf, hf> : launch_rope_qkv<hf, bf>)
                               : (out_dtype == FQ_F16 ? launch_rope_qkv<bf, hf> : launch_rope_qkv<bf, bf>);
-    go(q, q_sb, k, k_sb, v, v_sb, cosv, cos_sb, sinv, sin_sb, B, Hq, Hkv, D, q_out, k_out, v_out, st);
+    go(q, q_sb, k, k_sb, v, v_sb, cosv, cos_sb, sinv, sin_sb, B, Hq, Hkv, D, q_out, k_out, v_out, pattern, pattern_stride, retention, retention_per_head, st);
     FQ_CHECK_LAUNCH(fn);
     return FQ_OK;
 }

@@ -30,6 +30,7 @@ class _NativeSteps:
         self.q_rot = torch.empty(B, self.Hq, 1, D, dtype=dt, device=self.device)
         self.k_rot = torch.empty(B, self.Hkv, 1, D, dtype=dt, device=self.device)
         self.v_rot = torch.empty_like(self.k_rot)
+        self.pattern_retention = torch.zeros(self.cache.num_layers, self.Hq, dtype=torch.float32, device=self.device)
         ws_bytes = workspace.shape[-1]
         self._plan_ = bind().plan(
             kind, ctypes.addressof(self._cdesc), ctypes.addressof(self._prm), self.device.index or 0, self.cache.num_layers,
@@ -37,7 +38,8 @@ class _NativeSteps:
             self.O.data_ptr(), self.O.stride(0) * self.O.element_size(), self.lse.data_ptr(), self.lse.stride(0),
             workspace.data_ptr(), per(workspace, 2), ws_bytes,
             scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
-            self.q_rot.data_ptr(), self.k_rot.data_ptr(), self.v_rot.data_ptr())
+            self.q_rot.data_ptr(), self.k_rot.data_ptr(), self.v_rot.data_ptr(),
+            self.pattern_retention.data_ptr())
         self._outs = [(self.O[i].unsqueeze(2), self.lse[i].unsqueeze(2)) for i in range(self.cache.num_layers)]
         self._step, self._forward = bind().step, bind().forward
 
@@ -76,12 +78,13 @@ class _NativeSteps:
         self.launches += self.LAUNCHES
         return self._outs[layer_idx]
 
-    def forward_token(self, q, k, v, cos, sin, layer_idx: int, prm=None):
+    def forward_token(self, q, k, v, cos, sin, layer_idx: int, prm=None, pattern=None):
         """One new token from the projections: rotary embedding (Hugging Face's roundings), cast to the cache's dtype and
-        step(), in one call.  q (B,1,H_q*D), k, v (B,1,H_kv*D), cos, sin (B,1,D), one 16-bit dtype.  Returns O (B,H_q,1,D),
+        step(), in one call.  q (B,1,H_q*D), k, v (B,1,H_kv*D), cos, sin (B,1,D), one 16-bit dtype.  `pattern` (H_kv,) bool on
+        the cache's GPU, read at every call: retrieval heads keep `retention`, streaming heads 0.  Returns O (B,H_q,1,D),
         or None when the tensors are not of that form (nothing has been done)."""
         seen = self._seen_checked(layer_idx, 1)
-        rc = self._forward(self._plan_, layer_idx, seen, q, k, v, cos, sin, 0 if prm is None else ctypes.addressof(prm))
+        rc = self._forward(self._plan_, layer_idx, seen, q, k, v, cos, sin, 0 if prm is None else ctypes.addressof(prm), pattern)
         if rc == 1:
             return None
         if rc:

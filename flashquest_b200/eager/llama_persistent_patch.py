@@ -105,14 +105,22 @@ def make_quest_persistent_forward(
     # selection as the reference's mask sequence and attends the staged tail in the same fp32 softmax.  An INT8 cache
     # outside the one-launch append keeps the reference's own sequence of steps below.
     native = kv_bits in (3, 4) or cache._one_launch
-    state = {}       # H_q -> (engine, fq_decode_params, the retention tensor it points to), built on first use
+    state = {}       # H_q -> engine, built on first use
 
-    def _native(H_q, device):
-        got = state.get(H_q)
-        if got is None:
-            engine = _engine(cache, kv_bits, H_q, retention, num_sinks, window_pages)
-            got = state[H_q] = (engine,) + engine.params_for(head_pattern_layer.to(device))
-        return got
+    def _native(H_q):
+        engine = state.get(H_q)
+        if engine is None:
+            engine = state[H_q] = _engine(cache, kv_bits, H_q, retention, num_sinks, window_pages)
+        return engine
+
+    def _pattern(device):
+        """head_pattern_layer as it is now, in the form the launch reads: the caller may change it between calls."""
+        p = head_pattern_layer
+        if p.device != device:
+            p = p.to(device)
+        if p.dtype != torch.bool:
+            p = p.bool()
+        return p if p.dim() == 1 else p.reshape(-1)
 
     def forward(
         self,
@@ -130,9 +138,9 @@ def make_quest_persistent_forward(
         q, k, v = self.q_proj(hidden_states), self.k_proj(hidden_states), self.v_proj(hidden_states)
         model_dtype = q.dtype
         if native and len(input_shape) == 2 and input_shape[1] == 1:
-            engine, prm, _ = _native(q.shape[-1] // head_dim, q.device)
+            engine = _native(q.shape[-1] // head_dim)
             cos, sin = position_embeddings
-            O = engine.forward_token(q, k, v, cos, sin, li, prm=prm)
+            O = engine.forward_token(q, k, v, cos, sin, li, pattern=_pattern(q.device))
             if O is not None:
                 if TRACE is not None:
                     TRACE(li, engine.q_rot, engine.k_rot, engine.v_rot, O)
@@ -169,7 +177,8 @@ def make_quest_persistent_forward(
             if TRACE is not None:
                 attn_bhsd = attn_output.transpose(1, 2)
         elif native:
-            engine, prm, _ = _native(H_q, q.device)
+            engine = _native(H_q)
+            prm, retention_per_q = engine.params_for(head_pattern_layer)     # the struct points into the tensor
             O, _ = engine.step(k, v, q, li, prm=prm)
             attn_bhsd = O
             attn_output = O.transpose(1, 2)

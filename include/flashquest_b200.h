@@ -563,6 +563,13 @@ int fq_append_kv_int4(const fq_int4_cache* cache, int layer, int seen, const voi
 int fq_rope_qkv(const void* q, int64_t q_sb, const void* k, int64_t k_sb, const void* v, int64_t v_sb, int dtype,
                 const void* cosv, int64_t cos_sb, const void* sinv, int64_t sin_sb, int B, int Hq, int Hkv, int D,
                 void* q_out, void* k_out, void* v_out, int out_dtype, void* stream);
+/* The same, and from `pattern` (one byte per KV head, `pattern_stride` apart, device memory, may be NULL) the retention of
+ * every query head for the selection behind it: retention_per_head[h] = pattern[h / (Hq/Hkv)] ? retention : 0
+ * (eager/llama_persistent_patch.py:214-219). */
+int fq_rope_qkv_pattern(const void* q, int64_t q_sb, const void* k, int64_t k_sb, const void* v, int64_t v_sb, int dtype,
+                        const void* cosv, int64_t cos_sb, const void* sinv, int64_t sin_sb, int B, int Hq, int Hkv, int D,
+                        void* q_out, void* k_out, void* v_out, int out_dtype,
+                        const uint8_t* pattern, int64_t pattern_stride, float retention, float* retention_per_head, void* stream);
 
 /* One decode step of one layer on a persistent TurboQuant K3-V3 cache, in one host call: what the
  * reference's patched forward does for cache.kv_bits == 3 (eager/llama_persistent_patch.py:93-115,

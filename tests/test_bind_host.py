@@ -19,7 +19,7 @@ SETUP = """
     B, HQ, HKV, D = 1, 4, 2, 64
     c = _lib.Int4CacheDesc(kv_dtype=_lib.FQ_F16, L=1, B=B, Hkv=HKV, D=D, page=16, max_seq_len=64)
     prm = _lib.DecodeParams(Hq=HQ)
-    plan = mod.plan(4, ctypes.addressof(c), ctypes.addressof(prm), 0, 1, *[0] * 16)
+    plan = mod.plan(4, ctypes.addressof(c), ctypes.addressof(prm), 0, 1, *[0] * 17)
     fake = FakeTensorMode()
 
     def calls(device):
@@ -29,7 +29,7 @@ SETUP = """
             flat = [t.view(B, 1, -1) for t in (q, k, v)]
         return {"append": lambda: mod.append(4, ctypes.addressof(c), 0, 0, 0, k, v),
                 "step": lambda: mod.step(plan, 0, 0, k, v, q, 0),
-                "forward": lambda: mod.forward(plan, 0, 0, *flat, cs, cs, 0)}
+                "forward": lambda: mod.forward(plan, 0, 0, *flat, cs, cs, 0, None)}
 """
 
 

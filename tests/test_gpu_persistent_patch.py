@@ -224,3 +224,51 @@ def _oracle_checked_run(kv_bits, page, head_dim=64, model_dtype=torch.bfloat16, 
 def test_fp32_model_on_a_16_bit_cache(kv_bits, compact):
     """Outside the dtypes of the one-call route: Hugging Face's rotary embedding, then the native step."""
     _oracle_checked_run(kv_bits, 16, model_dtype=torch.float32, compact=compact)
+
+
+@pytest.mark.parametrize("kv_bits,page,compact,model_dtype,where", [
+    (4, 16, False, torch.bfloat16, "cuda"), (4, 16, True, torch.bfloat16, "cuda"), (8, 16, False, torch.bfloat16, "cuda"),
+    (8, 8, False, torch.bfloat16, "cuda"), (3, 16, False, torch.bfloat16, "cuda"), (4, 16, False, torch.float32, "cuda"),
+    (4, 16, False, torch.bfloat16, "cpu"), (4, 16, False, torch.bfloat16, "column")])
+def test_head_pattern_changed_between_tokens(kv_bits, page, compact, model_dtype, where):
+    """head_pattern_layer is read at every call: changed in place between two requests it gives what a forward made with the
+    new pattern gives."""
+    from types import SimpleNamespace
+
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    from flashquest_b200.eager.llama_persistent_patch import make_quest_persistent_forward
+    Hq, Hkv, D, n = 4, 2, 64, 20 * page + 3
+    g = torch.Generator(device="cuda").manual_seed(10)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    cache = {3: PersistentTurboKVCache, 4: PersistentInt4KVCache, 8: PersistentInt8KVCache}[kv_bits](
+        batch_size=1, num_layers=1, num_kv_heads=Hkv, head_dim=D, max_seq_len=24 * page, page_size=page)
+    cache.update_quantized(r(1, Hkv, n, D).bfloat16(), r(1, Hkv, n, D).bfloat16(), 0)
+    linear = lambda w: lambda x: torch.nn.functional.linear(x, w)
+    module = SimpleNamespace(head_dim=D, layer_idx=0, q_proj=linear(r(Hq * D, 32).to(model_dtype)), k_proj=linear(r(Hkv * D, 32).to(model_dtype)),
+                             v_proj=linear(r(Hkv * D, 32).to(model_dtype)), o_proj=linear(torch.eye(Hq * D, device="cuda").to(model_dtype)))
+    hidden, angle = r(1, 1, 32).to(model_dtype), r(1, 1, D)
+    rope = (angle.cos().to(model_dtype), angle.sin().to(model_dtype))
+
+    def pattern(*rows):
+        t = torch.tensor(rows, device="cpu" if where == "cpu" else "cuda")
+        return torch.stack([t, ~t], 1)[:, 0] if where == "column" else t
+
+    def make(p):
+        f = make_quest_persistent_forward(cache=cache, head_pattern_layer=p, retention=0.5, num_sinks=1, window_pages=1, page_size=page,
+                                          use_compact_kernel=compact)
+
+        def call():
+            cache._seen_tokens[0] = n
+            return f(module, hidden, rope, past_key_values=cache)[0].clone()
+        return call
+    live = pattern(True, False)
+    call = make(live)
+    first = call()
+    assert torch.equal(first, make(pattern(True, False))())
+    for rows in ((False, True), (True, True), (False, False), (True, False)):
+        live.copy_(torch.tensor(rows))
+        want = make(pattern(*rows))()
+        assert torch.equal(call(), want)
+        assert rows == (True, False) or not torch.equal(want, first)
