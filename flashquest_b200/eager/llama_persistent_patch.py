@@ -110,7 +110,10 @@ def make_quest_persistent_forward(
     def _native(H_q):
         engine = state.get(H_q)
         if engine is None:
-            engine = state[H_q] = _engine(cache, kv_bits, H_q, retention, num_sinks, window_pages)
+            r = float(retention)
+            if not (kv_bits == 3 or use_compact_kernel):
+                r = min(r, 1.0)          # the mask sequence keeps every page for a retention above 1; the other routes refuse it
+            engine = state[H_q] = _engine(cache, kv_bits, H_q, r, num_sinks, window_pages)
         return engine
 
     def _pattern(device):

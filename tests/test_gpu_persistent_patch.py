@@ -272,3 +272,41 @@ def test_head_pattern_changed_between_tokens(kv_bits, page, compact, model_dtype
         want = make(pattern(*rows))()
         assert torch.equal(call(), want)
         assert rows == (True, False) or not torch.equal(want, first)
+
+
+def _small(kv_bits, page, D=64, dtype=torch.bfloat16, **kw):
+    """A layer with a few pages cached and its patched forward: (call, cache)."""
+    from types import SimpleNamespace
+
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    from flashquest_b200.eager.llama_persistent_patch import make_quest_persistent_forward
+    g = torch.Generator(device="cuda").manual_seed(11)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    Hq, Hkv, n = 4, 2, 9 * page + 3
+    cache = {3: PersistentTurboKVCache, 4: PersistentInt4KVCache, 8: PersistentInt8KVCache}[kv_bits](
+        batch_size=1, num_layers=1, num_kv_heads=Hkv, head_dim=D, max_seq_len=12 * page, page_size=page, dtype=dtype)
+    cache.update_quantized(r(1, Hkv, n, D).to(dtype), r(1, Hkv, n, D).to(dtype), 0)
+    linear = lambda w: lambda x: torch.nn.functional.linear(x, w)
+    module = SimpleNamespace(head_dim=D, layer_idx=0, q_proj=linear(r(Hq * D, 32)), k_proj=linear(r(Hkv * D, 32)), v_proj=linear(r(Hkv * D, 32)),
+                             o_proj=linear(r(32, Hq * D)))
+    hidden, rope = r(1, 1, 32), (r(1, 1, D), r(1, 1, D))
+    kw = dict(dict(head_pattern_layer=torch.tensor([True, False], device="cuda"), retention=0.5, num_sinks=1, window_pages=1, page_size=page), **kw)
+    forward = make_quest_persistent_forward(cache=cache, **kw)
+
+    def call():
+        cache._seen_tokens[0] = n
+        return forward(module, hidden, rope, past_key_values=cache)[0].clone()
+    return call, cache
+
+
+@pytest.mark.parametrize("kv_bits,page", [(4, 16), (8, 16), (8, 8)])
+def test_mask_route_keeps_every_page_for_a_retention_above_one(kv_bits, page):
+    assert torch.equal(_small(kv_bits, page, retention=1.5)[0](), _small(kv_bits, page, retention=1.0)[0]())
+
+
+@pytest.mark.parametrize("kv_bits,compact", [(4, True), (3, False)])
+def test_other_routes_refuse_a_retention_above_one(kv_bits, compact):
+    with pytest.raises(ValueError, match="retention must be in"):
+        _small(kv_bits, 16, retention=1.5, use_compact_kernel=compact)[0]()
