@@ -119,6 +119,8 @@ def make_quest_persistent_forward(
     def _pattern(device):
         """head_pattern_layer as it is now, in the form the launch reads: the caller may change it between calls."""
         p = head_pattern_layer
+        if p.dtype not in (torch.bool, torch.uint8) and not (kv_bits == 3 or use_compact_kernel):
+            raise RuntimeError(f"head_pattern_layer must be a boolean tensor, but has dtype {p.dtype}")     # as torch.where does
         if p.device != device:
             p = p.to(device)
         if p.dtype != torch.bool:
@@ -181,7 +183,7 @@ def make_quest_persistent_forward(
                 attn_bhsd = attn_output.transpose(1, 2)
         elif native:
             engine = _native(H_q)
-            prm, retention_per_q = engine.params_for(head_pattern_layer)     # the struct points into the tensor
+            prm, retention_per_q = engine.params_for(_pattern(q.device))     # the struct points into the tensor
             O, _ = engine.step(k, v, q, li, prm=prm)
             attn_bhsd = O
             attn_output = O.transpose(1, 2)

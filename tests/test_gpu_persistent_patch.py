@@ -310,3 +310,16 @@ def test_mask_route_keeps_every_page_for_a_retention_above_one(kv_bits, page):
 def test_other_routes_refuse_a_retention_above_one(kv_bits, compact):
     with pytest.raises(ValueError, match="retention must be in"):
         _small(kv_bits, 16, retention=1.5, use_compact_kernel=compact)[0]()
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.float32])
+def test_pattern_dtypes(dtype):
+    """torch.where takes a boolean pattern in the mask sequence; the other routes convert theirs."""
+    pattern = torch.tensor([1, 0], device="cuda", dtype=dtype)
+    for kv_bits, page in ((4, 16), (8, 16), (8, 8)):
+        call, cache = _small(kv_bits, page, head_pattern_layer=pattern)
+        with pytest.raises(RuntimeError, match="boolean tensor"):
+            call()
+    for kw in (dict(kv_bits=4, use_compact_kernel=True), dict(kv_bits=3)):
+        assert torch.equal(_small(page=16, head_pattern_layer=pattern, **kw)[0](), _small(page=16, **kw)[0]())
+    assert torch.equal(_small(4, 16, head_pattern_layer=pattern.to(torch.uint8))[0](), _small(4, 16)[0]())
