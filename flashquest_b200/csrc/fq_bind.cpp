@@ -168,7 +168,8 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int B = p->kind == 3 ? p->c3.B : p->c4.B, Hkv = p->kind == 3 ? p->c3.Hkv : p->c4.Hkv, D = p->kind == 3 ? p->c3.D : p->c4.D;
     const int Hq = p->prm.Hq;
     const int dt = t[0] ? dtype_of(*t[0]) : -1;
-    if (dt != FQ_F16 && dt != FQ_BF16) return PyLong_FromLong(1);
+    // outside the rotary launch's dtypes and sizes the caller's general path says what is not supported
+    if ((dt != FQ_F16 && dt != FQ_BF16) || (p->cache_dtype != FQ_F16 && p->cache_dtype != FQ_BF16) || D > 128 || D % 2) return PyLong_FromLong(1);
     for (int i = 0; i < 5; ++i) {
         if (!t[i] || !on_device(*t[i], p->device) || dtype_of(*t[i]) != dt || t[i]->dim() != 3 || t[i]->size(1) != 1 || t[i]->stride(2) != 1) return PyLong_FromLong(1);
         const int64_t width = i == 0 ? static_cast<int64_t>(Hq) * D : i < 3 ? static_cast<int64_t>(Hkv) * D : D;

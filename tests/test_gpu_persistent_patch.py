@@ -323,3 +323,12 @@ def test_pattern_dtypes(dtype):
     for kw in (dict(kv_bits=4, use_compact_kernel=True), dict(kv_bits=3)):
         assert torch.equal(_small(page=16, head_pattern_layer=pattern, **kw)[0](), _small(page=16, **kw)[0]())
     assert torch.equal(_small(4, 16, head_pattern_layer=pattern.to(torch.uint8))[0](), _small(4, 16)[0]())
+
+
+@pytest.mark.parametrize("kv_bits,compact", [(3, False), (4, False), (4, True)])
+def test_unsupported_forms_raise_what_the_kernels_say(kv_bits, compact):
+    """head_dim 256 and fp32 caches: the attention's own errors, not those of the rotary launch in front of it."""
+    with pytest.raises(NotImplementedError, match="head_dim=256 not in"):
+        _small(kv_bits, 16, D=256, use_compact_kernel=compact)[0]()
+    with pytest.raises(RuntimeError, match="cache dtype code 0"):
+        _small(kv_bits, 16, dtype=torch.float32, use_compact_kernel=compact)[0]()
