@@ -6,12 +6,14 @@
 // steps: the cache descriptor, the parameters and the addresses of the engine's preallocated buffers.
 //
 // A call returns 0 (done), 1 (the tensors are not in a form the native path takes: the caller prepares them and
-// calls again through the general path) or a negative FQ_ERR_* code.
+// calls again through the general path) or a negative FQ_ERR_* code.  What torch throws on the way (a tensor without storage
+// has no address) becomes a Python exception.
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/flashquest_b200.h"
@@ -84,6 +86,7 @@ struct NoGil {
 // plan(kind, cache_desc, params, device, n_layers, scores, sc_sl, compact, cp_sl, O, o_sl_bytes, lse, lse_sl,
 //      ws, ws_sl, ws_bytes, scratch, scratch_bytes, q_rot, k_rot, v_rot, retention): addresses and sizes as integers
 PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (n != 22) { PyErr_SetString(PyExc_TypeError, "plan() takes 22 arguments"); return nullptr; }
     Plan* p = new Plan();
     p->kind = static_cast<int>(PyLong_AsLong(a[0]));
@@ -102,6 +105,7 @@ PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p->retention = static_cast<float*>(as_ptr(a[21]));
     if (PyErr_Occurred()) { delete p; return nullptr; }
     return PyCapsule_New(p, kPlanName, free_plan);
+    END_HANDLE_TH_ERRORS
 }
 
 int run_layer(const Plan* p, int layer, int seen, const void* k, const void* v, int64_t sb, int64_t sh, int64_t ss, int n_new,
@@ -123,6 +127,7 @@ int run_layer(const Plan* p, int layer, int seen, const void* k, const void* v, 
 
 // step(plan, layer, seen, k, v, q, params | 0): k, v (B,H_kv,n,D) of the cache's dtype, q (B,H_q,1,D) or (B,H_q,D)
 PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (n != 7) { PyErr_SetString(PyExc_TypeError, "step() takes 7 arguments"); return nullptr; }
     const Plan* p = plan_of(a[0]);
     if (!p) return nullptr;
@@ -151,12 +156,14 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
                        q->data_ptr(), dtype_of(*q), q_sb, q_sh, &par, stream_of(p->device));
     }
     return PyLong_FromLong(rc);
+    END_HANDLE_TH_ERRORS
 }
 
 // forward(plan, layer, seen, q, k, v, cos, sin, params | 0, pattern | None): one new token of the patched attention forward.
 // q (B,1,H_q*D), k, v (B,1,H_kv*D): the projections as the linears return them; cos, sin (B or 1,1,D) of the same dtype;
 // pattern (H_kv,) bool, read by the launch: retrieval heads keep the parameters' retention, streaming heads 0.
 PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (n != 10) { PyErr_SetString(PyExc_TypeError, "forward() takes 10 arguments"); return nullptr; }
     const Plan* p = plan_of(a[0]);
     if (!p) return nullptr;
@@ -195,10 +202,12 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
                            static_cast<int64_t>(Hq) * D, D, &par, st);
     }
     return PyLong_FromLong(rc);
+    END_HANDLE_TH_ERRORS
 }
 
 // append(kv_bits, cache descriptor, device, layer, seen, k, v): k, v (B,H_kv,n,D) of the cache's dtype
 PyObject* append(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (n != 7) { PyErr_SetString(PyExc_TypeError, "append() takes 7 arguments"); return nullptr; }
     const int kind = static_cast<int>(PyLong_AsLong(a[0])), device = static_cast<int>(PyLong_AsLong(a[2]));
     const void* desc = as_ptr(a[1]);
@@ -223,6 +232,7 @@ PyObject* append(PyObject*, PyObject* const* a, Py_ssize_t n) {
                        : fq_append_kv_int4(c4, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), nn, st);
     }
     return PyLong_FromLong(rc);
+    END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef kMethods[] = {

@@ -40,10 +40,10 @@ def _run(body):
     assert r.returncode == 0, r.stderr[-2000:]
 
 
-@pytest.mark.parametrize("call", ["append", "step", "forward"])
-def test_tensors_on_another_gpu_are_refused(call):
-    _run(f"""
-    assert calls("cuda:1")["{call}"]() == 1          # the plan's and the cache's buffers are on cuda:0
+def test_tensors_on_another_gpu_are_refused():
+    _run("""
+    for name, call in calls("cuda:1").items():
+        assert call() == 1, name                     # the plan's and the cache's buffers are on cuda:0
     """)
 
 
@@ -58,4 +58,16 @@ def test_operators_refuse_tensors_of_two_gpus():
         assert "different GPUs" in str(e)
     else:
         raise AssertionError("accepted")
+    """)
+
+
+def test_tensors_without_storage_raise():
+    """What torch throws below the entry point becomes a Python exception (it ended the process)."""
+    _run("""
+    for name, call in calls("cuda:0").items():
+        try:
+            call()
+        except RuntimeError:
+            continue
+        raise AssertionError(name + ": accepted")
     """)
