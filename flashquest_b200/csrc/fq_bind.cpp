@@ -31,8 +31,8 @@ struct Plan {
     char* O; int64_t o_sl;          // bytes
     float* lse; int64_t lse_sl;
     char* ws; size_t ws_sl, ws_bytes;
-    char* scratch; size_t scratch_bytes;
-    char *q_rot, *k_rot, *v_rot;    // rotated q / k and cast v of the patched forward, dense, cache dtype
+    char* scratch; size_t scratch_sl, scratch_bytes;
+    char *q_rot, *k_rot, *v_rot; int64_t qr_sl, kr_sl;     // (bytes between layers) rotated q / k and cast v of the patched forward, dense, cache dtype
     float* retention;               // (n_layers, H_q): written by the patched forward from the head pattern
 };
 
@@ -84,10 +84,11 @@ struct NoGil {
 };
 
 // plan(kind, cache_desc, params, device, n_layers, scores, sc_sl, compact, cp_sl, O, o_sl_bytes, lse, lse_sl,
-//      ws, ws_sl, ws_bytes, scratch, scratch_bytes, q_rot, k_rot, v_rot, retention): addresses and sizes as integers
+//      ws, ws_sl, ws_bytes, scratch, scratch_sl, scratch_bytes, q_rot, qr_sl_bytes, k_rot, v_rot, kr_sl_bytes, retention):
+// addresses and sizes as integers.  Every buffer has a part for each layer: layers of one cache may run on different streams.
 PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 22) { PyErr_SetString(PyExc_TypeError, "plan() takes 22 arguments"); return nullptr; }
+    if (n != 25) { PyErr_SetString(PyExc_TypeError, "plan() takes 25 arguments"); return nullptr; }
     Plan* p = new Plan();
     p->kind = static_cast<int>(PyLong_AsLong(a[0]));
     if (p->kind == 3) { p->c3 = *static_cast<const fq_turbo_cache*>(as_ptr(a[1])); p->cache_dtype = p->c3.kv_dtype; }
@@ -100,9 +101,10 @@ PyObject* make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p->O = static_cast<char*>(as_ptr(a[9])); p->o_sl = PyLong_AsLongLong(a[10]);
     p->lse = static_cast<float*>(as_ptr(a[11])); p->lse_sl = PyLong_AsLongLong(a[12]);
     p->ws = static_cast<char*>(as_ptr(a[13])); p->ws_sl = PyLong_AsSize_t(a[14]); p->ws_bytes = PyLong_AsSize_t(a[15]);
-    p->scratch = static_cast<char*>(as_ptr(a[16])); p->scratch_bytes = PyLong_AsSize_t(a[17]);
-    p->q_rot = static_cast<char*>(as_ptr(a[18])); p->k_rot = static_cast<char*>(as_ptr(a[19])); p->v_rot = static_cast<char*>(as_ptr(a[20]));
-    p->retention = static_cast<float*>(as_ptr(a[21]));
+    p->scratch = static_cast<char*>(as_ptr(a[16])); p->scratch_sl = PyLong_AsSize_t(a[17]); p->scratch_bytes = PyLong_AsSize_t(a[18]);
+    p->q_rot = static_cast<char*>(as_ptr(a[19])); p->qr_sl = PyLong_AsLongLong(a[20]);
+    p->k_rot = static_cast<char*>(as_ptr(a[21])); p->v_rot = static_cast<char*>(as_ptr(a[22])); p->kr_sl = PyLong_AsLongLong(a[23]);
+    p->retention = static_cast<float*>(as_ptr(a[24]));
     if (PyErr_Occurred()) { delete p; return nullptr; }
     return PyCapsule_New(p, kPlanName, free_plan);
     END_HANDLE_TH_ERRORS
@@ -117,7 +119,7 @@ int run_layer(const Plan* p, int layer, int seen, const void* k, const void* v, 
     char* ws = p->ws + static_cast<size_t>(layer) * p->ws_sl;
     if (p->kind == 3)
         return fq_decode_layer_turbo(&p->c3, layer, seen, k, v, sb, sh, ss, n_new, q, q_dtype, q_sb, q_sh, prm, sc, cp,
-                                     p->scratch, p->scratch_bytes, O, lse, ws, p->ws_bytes, stream);
+                                     p->scratch + static_cast<size_t>(layer) * p->scratch_sl, p->scratch_bytes, O, lse, ws, p->ws_bytes, stream);
     if (p->kind == 8)
         return fq_decode_layer_int8(&p->c4, layer, seen, k, v, sb, sh, ss, n_new, q, q_dtype, q_sb, q_sh, prm, sc, cp,
                                     O, lse, ws, p->ws_bytes, stream);
@@ -194,11 +196,12 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const NoGil released;
         const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
         void* st = stream_of(p->device);
+        char *q_rot = p->q_rot + layer * p->qr_sl, *k_rot = p->k_rot + layer * p->kr_sl, *v_rot = p->v_rot + layer * p->kr_sl;
         rc = fq_rope_qkv_pattern(t[0]->data_ptr(), t[0]->stride(0), t[1]->data_ptr(), t[1]->stride(0), t[2]->data_ptr(), t[2]->stride(0), dt,
-                         t[3]->data_ptr(), cs, t[4]->data_ptr(), ss, B, Hq, Hkv, D, p->q_rot, p->k_rot, p->v_rot, p->cache_dtype,
+                         t[3]->data_ptr(), cs, t[4]->data_ptr(), ss, B, Hq, Hkv, D, q_rot, k_rot, v_rot, p->cache_dtype,
                                  pat ? static_cast<const uint8_t*>(pat->data_ptr()) : nullptr, pat ? pat->stride(0) : 0, par.retention, ret, st);
         if (rc == 0)
-            rc = run_layer(p, layer, seen, p->k_rot, p->v_rot, static_cast<int64_t>(Hkv) * D, D, D, 1, p->q_rot, p->cache_dtype,
+            rc = run_layer(p, layer, seen, k_rot, v_rot, static_cast<int64_t>(Hkv) * D, D, D, 1, q_rot, p->cache_dtype,
                            static_cast<int64_t>(Hq) * D, D, &par, st);
     }
     return PyLong_FromLong(rc);

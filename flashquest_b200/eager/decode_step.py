@@ -17,30 +17,37 @@ import torch
 from .._lib import DecodeParams, bind, check, dtype_code, lib, ptr, require_cuda, stream_ptr
 
 
+def _whole(nbytes: int) -> int:
+    """A layer's part of a workspace: whole 256-byte blocks, at least one."""
+    return max((nbytes + 255) // 256 * 256, 256)
+
+
 class _NativeSteps:
     """step() and forward_token() over the CPython module (csrc/fq_bind.cpp): one call that reads pointers and strides
     from the tensors itself.  The subclass has set the cache descriptor, the parameters and the preallocated buffers."""
     COPY_ROWS = False        # rows off a 16-byte boundary are copied before the append (a dense tensor can be off it)
 
     def _build_plan(self, kind, scores, compact, workspace, scratch=None):
-        """scores, compact, workspace: with a leading layer dimension, or shared by the layers (stride 0)."""
-        per = lambda t, nd: t.stride(0) if t.dim() == nd else 0
-        B, D, dt = self.B, self.D, self.cache.dtype
+        """scores, compact, workspace, scratch: a part for each layer, so that layers of one cache may run on different streams."""
+        B, D, L, dt = self.B, self.D, self.cache.num_layers, self.cache.dtype
         # what the patched forward's rotary embedding writes: q, k, v of the new token in the cache's dtype
-        self.q_rot = torch.empty(B, self.Hq, 1, D, dtype=dt, device=self.device)
-        self.k_rot = torch.empty(B, self.Hkv, 1, D, dtype=dt, device=self.device)
-        self.v_rot = torch.empty_like(self.k_rot)
-        self.pattern_retention = torch.zeros(self.cache.num_layers, self.Hq, dtype=torch.float32, device=self.device)
+        q_rot = torch.empty(L, B, self.Hq, 1, D, dtype=dt, device=self.device)
+        k_rot = torch.empty(L, B, self.Hkv, 1, D, dtype=dt, device=self.device)
+        v_rot = torch.empty_like(k_rot)
+        self._rot = list(zip(q_rot, k_rot, v_rot))
+        self.q_rot, self.k_rot, self.v_rot = self._rot[0]       # of the layer that forward_token has last been called for
+        self.pattern_retention = torch.zeros(L, self.Hq, dtype=torch.float32, device=self.device)
         ws_bytes = workspace.shape[-1]
         self._plan_ = bind().plan(
-            kind, ctypes.addressof(self._cdesc), ctypes.addressof(self._prm), self.device.index or 0, self.cache.num_layers,
-            scores.data_ptr(), per(scores, 4), compact.data_ptr(), per(compact, 4),
+            kind, ctypes.addressof(self._cdesc), ctypes.addressof(self._prm), self.device.index or 0, L,
+            scores.data_ptr(), scores.stride(0), compact.data_ptr(), compact.stride(0),
             self.O.data_ptr(), self.O.stride(0) * self.O.element_size(), self.lse.data_ptr(), self.lse.stride(0),
-            workspace.data_ptr(), per(workspace, 2), ws_bytes,
-            scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
-            self.q_rot.data_ptr(), self.k_rot.data_ptr(), self.v_rot.data_ptr(),
+            workspace.data_ptr(), workspace.stride(0), ws_bytes,
+            *((scratch.data_ptr(), scratch.stride(0), scratch.shape[1]) if scratch is not None else (0, 0, 0)),
+            q_rot.data_ptr(), q_rot.stride(0) * q_rot.element_size(),
+            k_rot.data_ptr(), v_rot.data_ptr(), k_rot.stride(0) * k_rot.element_size(),
             self.pattern_retention.data_ptr())
-        self._outs = [(self.O[i].unsqueeze(2), self.lse[i].unsqueeze(2)) for i in range(self.cache.num_layers)]
+        self._outs = [(self.O[i].unsqueeze(2), self.lse[i].unsqueeze(2)) for i in range(L)]
         self._step, self._forward = bind().step, bind().forward
 
     def _seen_checked(self, layer_idx, n_new):
@@ -91,6 +98,7 @@ class _NativeSteps:
             check(rc)
         self.cache._seen_tokens[layer_idx] = seen + 1
         self.launches += self.LAUNCHES + 1
+        self.q_rot, self.k_rot, self.v_rot = self._rot[layer_idx]
         return self._outs[layer_idx][0]
 
     def params_for(self, head_pattern_layer: torch.Tensor):
@@ -151,7 +159,7 @@ class QuestDecodeInt4(_NativeSteps):
             nbytes = lib().fq_sparse_decode_workspace_bytes(self.B, self.Hq, self.D, self.n_split)
         # one split-K workspace per layer: launches of different layers may overlap in a graph
         self.ws_bytes = (nbytes + 255) // 256 * 256
-        self.workspace = torch.zeros(L, max(self.ws_bytes, 256), dtype=torch.uint8, device=dev)
+        self.workspace = torch.zeros(L, _whole(nbytes), dtype=torch.uint8, device=dev)
         self.launches = 0
         # descriptors for the one-call-per-layer entry point
         self._cdesc = cache.desc()
@@ -294,7 +302,7 @@ class QuestDecodeTurbo(_NativeSteps):
     make_quest_persistent_forward (flashquest/eager/llama_persistent_patch.py:93-115,202-245) as ONE
     foreign call per layer (fq_decode_layer_turbo): append, page scores from the raw page metadata,
     top-k + compact index, rotation of Q, sparse attention in the rotated basis, rotation of O, tail
-    attention and LSE merge.  All buffers are preallocated."""
+    attention and LSE merge.  All buffers are preallocated, a part for each layer."""
     LAUNCHES = 10
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,
@@ -317,14 +325,15 @@ class QuestDecodeTurbo(_NativeSteps):
         dev = cache.K_msb.device
         self.device, self.q_dtype = dev, q_dtype
         self.sm_scale = 1.0 / math.sqrt(self.D)
-        self.scores = torch.empty(self.B, self.Hq, max(P_max, 1), dtype=torch.float32, device=dev)
-        self.compact = torch.empty(self.B, self.Hq, self.bucket, dtype=torch.int32, device=dev)
-        self.O = torch.empty(cache.num_layers, self.B, self.Hq, self.D, dtype=q_dtype, device=dev)
-        self.lse = torch.empty(cache.num_layers, self.B, self.Hq, dtype=torch.float32, device=dev)
+        L = cache.num_layers
+        self.scores = torch.empty(L, self.B, self.Hq, max(P_max, 1), dtype=torch.float32, device=dev)
+        self.compact = torch.empty(L, self.B, self.Hq, self.bucket, dtype=torch.int32, device=dev)
+        self.O = torch.empty(L, self.B, self.Hq, self.D, dtype=q_dtype, device=dev)
+        self.lse = torch.empty(L, self.B, self.Hq, dtype=torch.float32, device=dev)
         with torch.cuda.device(dev):
             self.n_split = n_split or max(1, min(lib().fq_sparse_decode_default_splits(self.B, self.Hq, self.bucket, self.page), 64))
-            self.scratch = torch.empty(lib().fq_decode_layer_turbo_scratch_bytes(self.B, self.Hq, self.D), dtype=torch.uint8, device=dev)
-            self.workspace = torch.zeros(max(lib().fq_sparse_decode_workspace_bytes(self.B, self.Hq, self.D, self.n_split), 256),
+            self.scratch = torch.empty(L, _whole(lib().fq_decode_layer_turbo_scratch_bytes(self.B, self.Hq, self.D)), dtype=torch.uint8, device=dev)
+            self.workspace = torch.zeros(L, _whole(lib().fq_sparse_decode_workspace_bytes(self.B, self.Hq, self.D, self.n_split)),
                                          dtype=torch.uint8, device=dev)
         self._cdesc = cache.desc()
         self._prm = DecodeParams(self.Hq, None, self.retention, self.k_max_static, self.num_sinks, self.window_pages,
@@ -358,13 +367,14 @@ class QuestDecodeInt8(_NativeSteps):
         dev = cache.K_uint8.device
         self.device, self.q_dtype = dev, q_dtype
         self.sm_scale = 1.0 / math.sqrt(self.D)
-        self.scores = torch.empty(self.B, self.Hq, max(P_max, 1), dtype=torch.float32, device=dev)
-        self.compact = torch.empty(self.B, self.Hq, self.bucket, dtype=torch.int32, device=dev)
-        self.O = torch.empty(cache.num_layers, self.B, self.Hq, self.D, dtype=q_dtype, device=dev)
-        self.lse = torch.empty(cache.num_layers, self.B, self.Hq, dtype=torch.float32, device=dev)
+        L = cache.num_layers
+        self.scores = torch.empty(L, self.B, self.Hq, max(P_max, 1), dtype=torch.float32, device=dev)
+        self.compact = torch.empty(L, self.B, self.Hq, self.bucket, dtype=torch.int32, device=dev)
+        self.O = torch.empty(L, self.B, self.Hq, self.D, dtype=q_dtype, device=dev)
+        self.lse = torch.empty(L, self.B, self.Hq, dtype=torch.float32, device=dev)
         # a warp should walk six pages at least, and about sixteen 128-thread CTAs per SM fill the GPU
         self.n_split = n_split or max(1, min(64, self.bucket // 24, (16 * 148) // (self.B * self.Hq)))
-        self.workspace = torch.empty(lib().fq_sparse_decode_int8_workspace_bytes(self.B, self.Hq, self.D, self.n_split),
+        self.workspace = torch.empty(L, _whole(lib().fq_sparse_decode_int8_workspace_bytes(self.B, self.Hq, self.D, self.n_split)),
                                      dtype=torch.uint8, device=dev)
         self._cdesc = cache.desc()
         self._prm = DecodeParams(self.Hq, None, self.retention, self.k_max_static, self.num_sinks, self.window_pages,

@@ -19,7 +19,7 @@ SETUP = """
     B, HQ, HKV, D = 1, 4, 2, 64
     c = _lib.Int4CacheDesc(kv_dtype=_lib.FQ_F16, L=1, B=B, Hkv=HKV, D=D, page=16, max_seq_len=64)
     prm = _lib.DecodeParams(Hq=HQ)
-    plan = mod.plan(4, ctypes.addressof(c), ctypes.addressof(prm), 0, 1, *[0] * 17)
+    plan = mod.plan(4, ctypes.addressof(c), ctypes.addressof(prm), 0, 1, *[0] * 20)
     fake = FakeTensorMode()
 
     def calls(device):

@@ -111,3 +111,41 @@ def test_int8_takes_rows_off_a_16_byte_boundary(form, n):
         out = [t.clone() for t in engine.step(f(k), f(v), q, 0)]
         results.append(out + [t.clone() for t in cache.get_views(0).values() if torch.is_tensor(t)])
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("kind", [3, 4, 8])
+def test_layers_of_one_cache_on_two_streams(kind):
+    """Every buffer between the launches of a token has a part for each layer."""
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    from flashquest_b200.eager.decode_step import QuestDecodeInt4, QuestDecodeInt8, QuestDecodeTurbo
+    cls, eng = {3: (PersistentTurboKVCache, QuestDecodeTurbo), 4: (PersistentInt4KVCache, QuestDecodeInt4), 8: (PersistentInt8KVCache, QuestDecodeInt8)}[kind]
+    L, batch, hq, hkv, d, n = 2, 8, 6, 2, 128, 4099
+    g = torch.Generator(device="cuda").manual_seed(12)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    cache = cls(batch_size=batch, num_layers=L, num_kv_heads=hkv, head_dim=d, max_seq_len=4608, page_size=16, dtype=torch.bfloat16)
+    for layer in range(L):
+        cache.update_quantized(r(batch, hkv, n, d), r(batch, hkv, n, d), layer)
+    engine = eng(cache, num_q_heads=hq, retention=0.25, num_sinks=1, window_pages=1)
+    for name in ("scores", "compact", "workspace", "scratch"):
+        buf = getattr(engine, name, None)
+        assert buf is None or (buf.shape[0] == L and buf[0].data_ptr() != buf[1].data_ptr())
+    flat = [(r(batch, 1, hq * d), r(batch, 1, hkv * d), r(batch, 1, hkv * d)) for _ in range(L)]
+    cos, sin = r(1, 1, d), r(1, 1, d)
+
+    def token(layer):
+        cache._seen_tokens[layer] = n
+        return engine.forward_token(*flat[layer], cos, sin, layer)
+    want = [token(layer).clone() for layer in range(L)]
+    rot = [[t.clone() for t in engine._rot[layer]] for layer in range(L)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(L)]
+    for _ in range(20):
+        for layer, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                token(layer)
+        torch.cuda.synchronize()
+        for layer in range(L):
+            assert torch.equal(engine.O[layer].unsqueeze(2), want[layer])
+            assert all(torch.equal(a, b) for a, b in zip(engine._rot[layer], rot[layer]))
