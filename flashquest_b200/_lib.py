@@ -201,6 +201,10 @@ def bind():
         import importlib.util
         if not os.path.exists(BIND_PATH):
             raise FlashQuestError(f"{BIND_PATH} is missing: build it with `python -m flashquest_b200.build`.")
+        from .build import bind_built_for, bind_target
+        if bind_built_for() != bind_target():          # its C++ ABI is torch's: another one would read tensors wrongly
+            raise FlashQuestError(f"{BIND_PATH} was built for {bind_built_for()}, this is {bind_target()}: "
+                                  "build it again with `python -m flashquest_b200.build`.")
         lib()
         ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)          # the module's C ABI symbols resolve against it
         spec = importlib.util.spec_from_file_location("_fq_bind", BIND_PATH)

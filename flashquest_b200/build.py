@@ -17,6 +17,7 @@ LIB = os.path.join(LIB_DIR, "libflashquest_b200.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 BIND_SRC = os.path.join(CSRC, "fq_bind.cpp")
 BIND = os.path.join(LIB_DIR, "_fq_bind.so")       # CPython module over the C ABI (see fq_bind.cpp)
+BIND_STAMP = os.path.join(LIB_DIR, "_fq_bind.built_for")       # the torch and the Python it was compiled against
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -43,9 +44,24 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def bind_target() -> str:
+    """What the CPython module depends on beside its source: torch's C++ ABI, which changes between versions, and Python's."""
+    import torch
+    return f"torch {torch.__version__} {sys.implementation.cache_tag}"
+
+
+def bind_built_for() -> str:
+    try:
+        with open(BIND_STAMP) as f:
+            return f.read()
+    except OSError:
+        return "an unknown torch"
+
+
 def build_bind(force: bool = False) -> str:
     """The CPython module: host code only, resolved against the running torch and the library beside it."""
-    if not force and not _stale(BIND, [BIND_SRC, os.path.join(INCLUDE, "flashquest_b200.h")]):
+    target = bind_target()
+    if not force and not _stale(BIND, [BIND_SRC, os.path.join(INCLUDE, "flashquest_b200.h")]) and bind_built_for() == target:
         return BIND
     import sysconfig
 
@@ -63,6 +79,8 @@ def build_bind(force: bool = False) -> str:
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for {BIND_SRC}:\n{r.stdout}\n{r.stderr}")
     os.replace(BIND + ".tmp", BIND)
+    with open(BIND_STAMP, "w") as f:
+        f.write(target)
     return BIND
 
 
