@@ -206,7 +206,6 @@ def bind():
             raise FlashQuestError(f"{BIND_PATH} was built for {bind_built_for()}, this is {bind_target()}: "
                                   "build it again with `python -m flashquest_b200.build`.")
         lib()
-        ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)          # the module's C ABI symbols resolve against it
         spec = importlib.util.spec_from_file_location("_fq_bind", BIND_PATH)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)

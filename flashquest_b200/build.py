@@ -8,6 +8,7 @@ import glob
 import os
 import subprocess
 import sys
+import threading
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
@@ -58,26 +59,34 @@ def bind_built_for() -> str:
         return "an unknown torch"
 
 
-def build_bind(force: bool = False) -> str:
-    """The CPython module: host code only, resolved against the running torch and the library beside it."""
+def _run(cmd, what):
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {what}:\n{r.stdout}\n{r.stderr}")
+
+
+def build_bind(force: bool = False, library=lambda: None) -> str:
+    """The CPython module: host code only, linked to the running torch and to the library beside it (found through its own
+    folder, so the library's symbols stay out of the process).  `library` waits for that library to be linked."""
     target = bind_target()
-    if not force and not _stale(BIND, [BIND_SRC, os.path.join(INCLUDE, "flashquest_b200.h")]) and bind_built_for() == target:
+    if not force and not _stale(BIND, [BIND_SRC, os.path.abspath(__file__), os.path.join(INCLUDE, "flashquest_b200.h")]) and bind_built_for() == target:
         return BIND
     import sysconfig
 
     import torch
     tdir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-w",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda, "include")]
     for inc in ("include", os.path.join("include", "torch", "csrc", "api", "include")):
         cmd += ["-isystem", os.path.join(tdir, inc)]
+    obj = BIND[:-3] + ".o"
+    _run(cmd + ["-c", BIND_SRC, "-o", obj], BIND_SRC)
+    library()
     tlib = os.path.join(tdir, "lib")
-    cmd += [BIND_SRC, "-o", BIND + ".tmp", "-L", tlib, f"-Wl,-rpath,{tlib}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"g++ failed for {BIND_SRC}:\n{r.stdout}\n{r.stderr}")
+    _run(["g++", "-shared", obj, "-o", BIND + ".tmp", "-L", LIB_DIR, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN",
+          "-L", tlib, f"-Wl,-rpath,{tlib}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"], BIND)
     os.replace(BIND + ".tmp", BIND)
     with open(BIND_STAMP, "w") as f:
         f.write(target)
@@ -101,18 +110,22 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError(f"nvcc failed for {src}:\n{r.stdout}\n{r.stderr}")
         return r.stderr
 
-    bind = ThreadPoolExecutor(max_workers=1).submit(build_bind, force)
-    with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
-        logs = list(ex.map(compile_one, zip(srcs, objs)))
-    if verbose:
-        for log in logs:
-            if log:
-                print(log)
-    if force or _stale(LIB, objs):
-        cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    linked = threading.Event()
+    bind = ThreadPoolExecutor(max_workers=1).submit(build_bind, force, linked.wait)
+    try:
+        with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+            logs = list(ex.map(compile_one, zip(srcs, objs)))
+        if verbose:
+            for log in logs:
+                if log:
+                    print(log)
+        if force or _stale(LIB, objs):
+            cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"]
+            r = subprocess.run(cmd, capture_output=True, text=True)
+            if r.returncode != 0:
+                raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    finally:
+        linked.set()
     bind.result()
     return LIB
 

@@ -71,3 +71,10 @@ def test_tensors_without_storage_raise():
             continue
         raise AssertionError(name + ": accepted")
     """)
+
+
+def test_library_symbols_stay_out_of_the_process():
+    _run("""
+    import ctypes
+    assert not hasattr(ctypes.CDLL(None), "fq_version")
+    """)
