@@ -63,6 +63,8 @@ def _run(cmd, what):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for {what}:\n{r.stdout}\n{r.stderr}")
+    if r.stderr:
+        print(r.stderr, file=sys.stderr)
 
 
 def build_bind(force: bool = False, library=lambda: None) -> str:
@@ -76,7 +78,7 @@ def build_bind(force: bool = False, library=lambda: None) -> str:
     import torch
     tdir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-w",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wextra",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda, "include")]
     for inc in ("include", os.path.join("include", "torch", "csrc", "api", "include")):
