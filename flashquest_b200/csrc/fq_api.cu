@@ -51,6 +51,19 @@ int* device_status_ptr() {
     return ptr;
 }
 
+int sm_count() {
+    constexpr int MAX_DEV = 64;
+    static std::atomic<int> counts[MAX_DEV];        // relaxed: concurrent host threads may store the same value
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) return 148;
+    n = counts[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+        counts[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 }  // namespace fq
 
 extern "C" const char* fq_last_error_string(void) { return fq::g_err; }

@@ -125,6 +125,9 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 // Returns nullptr (with the error string set) if the address cannot be resolved.
 int* device_status_ptr();
 
+// SMs of the current device, asked for once (148 on a B200).
+int sm_count();
+
 // ---- dtype traits ----
 template <typename T> struct Dt;
 template <> struct Dt<float> {

@@ -9,6 +9,7 @@
 // consecutive pages, so every warp load is one contiguous 512-byte run.  Each lane keeps
 // its slice of q for all NR query heads in registers; the per-page reduction is a 3-step
 // xor shuffle inside the quarter warp.
+#include "fq_score_grid.cuh"
 #include "fq_score_lane.cuh"
 
 namespace fq {
@@ -113,10 +114,10 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_early_kernel(
 // in registers; the short-lived CTAs of the kernel above start with two latencies in a row (37 us against 20 of HBM time for 134 MB).
 // 16 x 8 rows of 2048 pages 35.0 -> 24.6 us, of
 // 8191 133.9 -> 88.0 (6.1 TB/s); a ring of 4 or 6 units is no faster (25.2, 26.2).
-constexpr int SCORE_RING = 3, SCORE_STREAM_CTAS = 4 * 148;
+constexpr int SCORE_RING = 3;
 
 template <typename QT, int NR, int CH>
-__global__ void __launch_bounds__(SCORE_THREADS, NR > 3 ? 3 : 4) page_scores_stream_kernel(
+__global__ void __launch_bounds__(SCORE_THREADS, score_stream_ctas_per_sm(NR, CH)) page_scores_stream_kernel(
     const QT* __restrict__ Q, int64_t q_sb, int64_t q_sh,
     const uint16_t* __restrict__ K_scale, const uint16_t* __restrict__ K_mn,
     int64_t km_sb, int64_t km_sh, int64_t km_sp,
@@ -168,24 +169,11 @@ __global__ void __launch_bounds__(SCORE_THREADS, NR > 3 ? 3 : 4) page_scores_str
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// CTAs per (batch, kv head) row of the streaming kernel: whole waves of resident CTAs, at least 64 pages each
-static int score_stream_ctas(int rows, int P) {
-    int best = 1;
-    double best_t = 1e30;
-    for (int c = 1; c <= 64 && c * 64 <= P; ++c) {
-        const double t = (double)((rows * (int64_t)c + SCORE_STREAM_CTAS - 1) / SCORE_STREAM_CTAS) / c * (1.0 + 0.004 * c);
-        if (t < best_t) { best_t = t; best = c; }
-    }
-    return best;
-}
-
 template <typename QT, int NR>
 static void launch_scores(int CH, dim3 grid, cudaStream_t st, const void* Q, int64_t q_sb, int64_t q_sh,
                           const void* K_scale, const void* K_mn, int64_t km_sb, int64_t km_sh, int64_t km_sp,
                           int Hq, int Hkv, int P, int D, int head_off, float* scores, int64_t sc_sb, int64_t sc_sh, const DynPos& dp, float levels) {
-    // 64 pages per resident CTA and more: below that the ring never fills and the short CTAs start sooner
-    const int rows = (int)(grid.y * grid.z);
-    const int stream_ctas = (D == 128 || D == 64) && (int64_t)rows * P >= (int64_t)SCORE_STREAM_CTAS * 64 ? score_stream_ctas(rows, P) : 0;
+    const int stream_ctas = D == 128 || D == 64 ? score_stream_ctas((int)(grid.y * grid.z), P, score_stream_ctas_per_sm(NR, CH) * sm_count()) : 0;
 #define FQ_LAUNCH_SC(CHV)                                                                              \
     do {                                                                                               \
         if (stream_ctas > 0)                                                                           \
