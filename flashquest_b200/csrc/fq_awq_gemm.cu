@@ -423,7 +423,13 @@ extern "C" int fq_awq_gemm(
     // Up to 384 tiles of 128 x 128 (2.6 waves of the SMs): the split-K kernel.  Measured at 3072 x 16384: 59 us against 74 at
     // 384 rows (384 tiles), 79 against 75 at 512 (512 tiles); at 3072 x 3072: 37 against 42 at 1024 rows (192 tiles).
     int64_t tiles128 = 0;
-    for (int i = 0; i < n_proj; ++i) tiles128 += (N[i] + 127) / 128;
+    for (int i = 0; i < n_proj; ++i) {
+        FQ_CHECK_ARG(N[i] > 0 && N[i] % 128 == 0, FQ_ERR_UNSUPPORTED, "%s: N[%d]=%d must be a positive multiple of 128", fn, i, N[i]);
+        FQ_CHECK_ARG(qweight[i] && scales[i] && qzeros[i] && y[i], FQ_ERR_ARG, "%s: null tensor in projection %d", fn, i);
+        FQ_CHECK_ARG(aligned(y[i], 16) && aligned(scales[i], 16) && aligned(qweight[i], 16) && aligned(qzeros[i], 4), FQ_ERR_ALIGN,
+                     "%s: y[%d], scales[%d] and qweight[%d] must be 16-byte aligned", fn, i, i, i);
+        tiles128 += N[i] / 128;
+    }
     if (tiles128 * ((M + 127) / 128) <= 384) {
         SkinnyCall c{};
         c.x = x; c.M = M; c.K = K; c.group = group; c.n_proj = n_proj; c.interleaved = interleaved ? 1 : 0;
@@ -449,10 +455,6 @@ extern "C" int fq_awq_gemm(
     }
     int tile0 = 0;
     for (int i = 0; i < n_proj; ++i) {
-        FQ_CHECK_ARG(N[i] > 0 && N[i] % 128 == 0, FQ_ERR_UNSUPPORTED, "%s: N[%d]=%d must be a positive multiple of 128", fn, i, N[i]);
-        FQ_CHECK_ARG(qweight[i] && scales[i] && qzeros[i] && y[i], FQ_ERR_ARG, "%s: null tensor in projection %d", fn, i);
-        FQ_CHECK_ARG(aligned(y[i], 16) && aligned(scales[i], 16) && aligned(qweight[i], 16) && aligned(qzeros[i], 4), FQ_ERR_ALIGN,
-                     "%s: y[%d], scales[%d] and qweight[%d] must be 16-byte aligned", fn, i, i, i);
         p.proj[i] = GemmProj{static_cast<const __half*>(scales[i]), qzeros[i], bias ? static_cast<const __half*>(bias[i]) : nullptr,
                              static_cast<__half*>(y[i]), N[i], tile0};
         tile0 += (N[i] + GM_BN - 1) / GM_BN;
