@@ -54,15 +54,16 @@ __global__ void __launch_bounds__(256) gather_kv_f16_kernel(const fq_int4_cache 
     }
 }
 
-// y_i = x @ W_i for up to three linears sharing x: the GEMV for up to 8 rows, the tensor-core GEMM above
-static int linears(const fq_llama_model* m, const void* x, int rows, const fq_awq_linear* const* w, int n, void* const* y, void* stream) {
+// y_i = x @ W_i for up to three linears sharing x: the GEMV for up to 8 rows, the tensor-core GEMM above.  The one row behind
+// the last attention of a longer prompt stays on the GEMM with groups of 256, which the GEMV is not built for.
+static int linears(const fq_llama_model* m, const void* x, int rows, bool one_of_many, const fq_awq_linear* const* w, int n, void* const* y, void* stream) {
     const int32_t* qw[3]; const void* sc[3]; const int32_t* qz[3]; const void* bs[3]; int N[3];
     bool bias = false;
     for (int i = 0; i < n; ++i) {
         qw[i] = w[i]->qweight; sc[i] = w[i]->scales; qz[i] = w[i]->qzeros; bs[i] = w[i]->bias; N[i] = w[i]->N;
         bias |= bs[i] != nullptr;
     }
-    if (rows <= 8) {
+    if (rows <= 8 && !(one_of_many && m->group > 128)) {
         int total = 0;
         for (int i = 0; i < n; ++i) total += N[i];
         return fq_awq_gemv(x, rows, w[0]->K, m->group, n, qw, sc, qz, bias ? bs : nullptr, N, y, m->interleaved,
@@ -129,7 +130,7 @@ extern "C" int fq_llama_prefill(const fq_llama_model* m, const fq_int4_cache* c,
         {
             const fq_awq_linear* ws[3] = {&L.q, &L.k, &L.v};
             void* y[3] = {w.q, w.k, w.v};
-            if ((rc = linears(m, w.normed, S, ws, 3, y, stream)) != FQ_OK) return rc;
+            if ((rc = linears(m, w.normed, S, false, ws, 3, y, stream)) != FQ_OK) return rc;
         }
         if ((rc = fq_rope_tokens(w.q, nq, D, Hq, w.k, nkv, D, Hkv, S, D, 0, m->rope_theta, stream)) != FQ_OK) return rc;
         uint8_t* Kp = c->K_packed + l * c->pk_sl; uint8_t* Vp = c->V_packed + l * c->pk_sl;
@@ -154,20 +155,20 @@ extern "C" int fq_llama_prefill(const fq_llama_model* m, const fq_int4_cache* c,
         {
             const fq_awq_linear* ws[1] = {&L.o};
             void* y[1] = {w.delta + (size_t)first * H * 2};
-            if ((rc = linears(m, w.attn + (size_t)first * nq * 2, rows, ws, 1, y, stream)) != FQ_OK) return rc;
+            if ((rc = linears(m, w.attn + (size_t)first * nq * 2, rows, S > 8, ws, 1, y, stream)) != FQ_OK) return rc;
         }
         delta = w.delta;
         if ((rc = add_norm(L.post_norm, first, rows)) != FQ_OK) return rc;
         {
             const fq_awq_linear* ws[2] = {&L.gate, &L.up};
             void* y[2] = {w.gate, w.up};
-            if ((rc = linears(m, w.normed, rows, ws, 2, y, stream)) != FQ_OK) return rc;
+            if ((rc = linears(m, w.normed, rows, S > 8, ws, 2, y, stream)) != FQ_OK) return rc;
         }
         if ((rc = fq_swiglu(w.gate, w.up, (int64_t)rows * m->ffn, w.act, stream)) != FQ_OK) return rc;
         {
             const fq_awq_linear* ws[1] = {&L.down};
             void* y[1] = {w.delta + (size_t)first * H * 2};
-            if ((rc = linears(m, w.act, rows, ws, 1, y, stream)) != FQ_OK) return rc;
+            if ((rc = linears(m, w.act, rows, S > 8, ws, 1, y, stream)) != FQ_OK) return rc;
         }
     }
     if ((rc = add_norm(m->final_norm, S - 1, 1)) != FQ_OK) return rc;

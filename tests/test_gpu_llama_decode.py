@@ -320,3 +320,18 @@ def test_graph_replayed_decode_equals_stream_decode():
         assert torch.equal(la, b.logits), t
         assert torch.equal(ids_a, ids_b), t
     assert a.cache.get_seq_length(0) == b.cache.get_seq_length(0) == 25
+
+
+@pytest.mark.parametrize("group", [64, 128, 256])
+@pytest.mark.parametrize("S", [9, 45])
+def test_prefill_group_sizes(group, S):
+    """Every group size that the prompt's GEMM takes: the last token's linears behind the last attention are one row."""
+    from flashquest_b200.eager.llama_decode import LlamaConfig, LlamaInt4Decoder, random_llama_weights
+    cfg = LlamaConfig(hidden=256, layers=2, q_heads=4, kv_heads=2, head_dim=64, ffn=512, vocab=512, group_size=group)
+    w = random_llama_weights(cfg, "cuda", seed=5)
+    dec = LlamaInt4Decoder(cfg, w, batch_size=1, max_seq_len=64, page_size=16, retention=1.0, num_sinks=1, window_pages=1)
+    ids = torch.randint(0, cfg.vocab, (S,), generator=torch.Generator().manual_seed(11), dtype=torch.int32)
+    dec.prefill(ids.cuda())
+    want = _ref_prefill(cfg, w, ids, 16)[0].float()
+    # free-running, as in test_prefill_then_decode: the 4-bit codes of k / v may differ by a step
+    assert (dec.logits.float().cpu() - want).abs().max().item() <= 3e-2 * want.abs().max().item() + 1e-2
