@@ -1,0 +1,23 @@
+"""What the three persistent caches share: the C record of their storage that the native calls take."""
+from __future__ import annotations
+
+from transformers.cache_utils import Cache
+
+
+class DescribedCache(Cache):
+    """_storage() names the tensors whose addresses _describe() puts into the record.  Neither the
+    record nor the step objects built on it belong to a copied or saved cache (they hold addresses)."""
+    _desc = None
+    _desc_of = None
+
+    def desc(self):
+        at = tuple([t.data_ptr() for t in (self._storage()[0], self._storage()[-2])])
+        if at != self._desc_of:
+            self._desc, self._desc_of = self._describe(), at
+        return self._desc
+
+    def __getstate__(self):
+        state = dict(self.__dict__)
+        for name in ("_desc", "_desc_of", "_fq_engines"):
+            state.pop(name, None)
+        return state

@@ -11,13 +11,13 @@ from __future__ import annotations
 import ctypes
 
 import torch
-from transformers.cache_utils import Cache
 
 from .._lib import Int4CacheDesc, bind, check, dtype_code
 from ..kernel.kv_quant import quantize_kv_int4_into
+from ._described import DescribedCache
 
 
-class PersistentInt4KVCache(Cache):
+class PersistentInt4KVCache(DescribedCache):
     kv_bits = 4
 
     def __init__(self, *, batch_size: int, num_layers: int, num_kv_heads: int, head_dim: int,
@@ -50,20 +50,20 @@ class PersistentInt4KVCache(Cache):
         self.K_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self.V_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self._seen_tokens = [0] * num_layers
-        self._desc = None
 
-    def desc(self) -> Int4CacheDesc:
+    def _storage(self):
+        return (self.K_packed, self.V_packed, self.K_scale, self.K_mn,
+                self.V_scale, self.V_mn, self.K_partial, self.V_partial)
+
+    def _describe(self) -> Int4CacheDesc:
         """struct fq_int4_cache of this cache."""
-        d = self._desc
-        if d is None or d.K_packed != self.K_packed.data_ptr() or d.K_partial != self.K_partial.data_ptr():
-            d = self._desc = Int4CacheDesc(
-                self.K_packed.data_ptr(), self.V_packed.data_ptr(), *self.K_packed.stride()[:4],
-                self.K_scale.data_ptr(), self.K_mn.data_ptr(), *self.K_scale.stride()[:4],
-                self.V_scale.data_ptr(), self.V_mn.data_ptr(), *self.V_scale.stride()[:3],
-                self.K_partial.data_ptr(), self.V_partial.data_ptr(), *self.K_partial.stride()[:4],
-                dtype_code(self.K_partial), self.num_layers, self.batch_size, self.num_kv_heads, self.head_dim, self.page_size,
-                self.max_seq_len)
-        return d
+        return Int4CacheDesc(
+            self.K_packed.data_ptr(), self.V_packed.data_ptr(), *self.K_packed.stride()[:4],
+            self.K_scale.data_ptr(), self.K_mn.data_ptr(), *self.K_scale.stride()[:4],
+            self.V_scale.data_ptr(), self.V_mn.data_ptr(), *self.V_scale.stride()[:3],
+            self.K_partial.data_ptr(), self.V_partial.data_ptr(), *self.K_partial.stride()[:4],
+            dtype_code(self.K_partial), self.num_layers, self.batch_size, self.num_kv_heads, self.head_dim, self.page_size,
+            self.max_seq_len)
 
     def get_seq_length(self, layer_idx: int = 0) -> int:
         return self._seen_tokens[layer_idx]

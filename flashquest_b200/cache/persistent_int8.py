@@ -5,13 +5,13 @@ from __future__ import annotations
 import ctypes
 
 import torch
-from transformers.cache_utils import Cache
 
 from .._lib import Int4CacheDesc, check, dtype_code, lib, ptr, require_cuda, stream_ptr
 from ..kernel.kv_quant import quantize_kv_int8_into
+from ._described import DescribedCache
 
 
-class PersistentInt8KVCache(Cache):
+class PersistentInt8KVCache(DescribedCache):
     kv_bits = 8
 
     def __init__(self, *, batch_size: int, num_layers: int, num_kv_heads: int, head_dim: int,
@@ -42,19 +42,20 @@ class PersistentInt8KVCache(Cache):
 
         # the one-launch append (fq_append_kv_int8): 16-bit staging, head_dim 64 / 128, pages of 16, 32 or 64 tokens
         self._one_launch = dtype in (torch.float16, torch.bfloat16) and D in (64, 128) and page_size in (16, 32, 64)
-        self._desc = None
 
-    def desc(self) -> Int4CacheDesc:
+    def _storage(self):
+        return (self.K_uint8, self.V_uint8, self.K_scale, self.K_mn,
+                self.V_scale, self.V_mn, self.K_partial, self.V_partial)
+
+    def _describe(self) -> Int4CacheDesc:
         """struct fq_int4_cache of this cache (code rows of D bytes)."""
-        if self._desc is None or self._desc.K_packed != self.K_uint8.data_ptr() or self._desc.K_partial != self.K_partial.data_ptr():
-            self._desc = Int4CacheDesc(
-                self.K_uint8.data_ptr(), self.V_uint8.data_ptr(), *self.K_uint8.stride()[:4],
-                self.K_scale.data_ptr(), self.K_mn.data_ptr(), *self.K_scale.stride()[:4],
-                self.V_scale.data_ptr(), self.V_mn.data_ptr(), *self.V_scale.stride()[:3],
-                self.K_partial.data_ptr(), self.V_partial.data_ptr(), *self.K_partial.stride()[:4],
-                dtype_code(self.K_partial), self.num_layers, self.batch_size, self.num_kv_heads, self.head_dim, self.page_size,
-                self.max_seq_len)
-        return self._desc
+        return Int4CacheDesc(
+            self.K_uint8.data_ptr(), self.V_uint8.data_ptr(), *self.K_uint8.stride()[:4],
+            self.K_scale.data_ptr(), self.K_mn.data_ptr(), *self.K_scale.stride()[:4],
+            self.V_scale.data_ptr(), self.V_mn.data_ptr(), *self.V_scale.stride()[:3],
+            self.K_partial.data_ptr(), self.V_partial.data_ptr(), *self.K_partial.stride()[:4],
+            dtype_code(self.K_partial), self.num_layers, self.batch_size, self.num_kv_heads, self.head_dim, self.page_size,
+            self.max_seq_len)
 
     def get_seq_length(self, layer_idx: int = 0) -> int:
         return self._seen_tokens[layer_idx]

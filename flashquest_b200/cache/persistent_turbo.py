@@ -6,13 +6,13 @@ from __future__ import annotations
 import ctypes
 
 import torch
-from transformers.cache_utils import Cache
 
 from .._lib import TurboCacheDesc, bind, check, dtype_code
 from ..kernel.kv_quant import quantize_kv_int4_into, quantize_turbo_into
+from ._described import DescribedCache
 
 
-class PersistentTurboKVCache(Cache):
+class PersistentTurboKVCache(DescribedCache):
     kv_bits = 3
 
     def __init__(self, *, batch_size: int, num_layers: int, num_kv_heads: int, head_dim: int,
@@ -47,21 +47,21 @@ class PersistentTurboKVCache(Cache):
         self.K_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self.V_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self._seen_tokens = [0] * num_layers
-        self._desc = None
 
-    def desc(self) -> TurboCacheDesc:
+    def _storage(self):
+        return (self.K_msb, self.K_lsb, self.V_msb, self.V_lsb, self.K_scale_turbo,
+                self.V_scale_turbo, self.K_scale_raw, self.K_mn_raw, self.K_partial, self.V_partial)
+
+    def _describe(self) -> TurboCacheDesc:
         """struct fq_turbo_cache of this cache."""
-        d = self._desc
-        if d is None or d.K_msb != self.K_msb.data_ptr() or d.K_partial != self.K_partial.data_ptr():
-            d = self._desc = TurboCacheDesc(
-                self.K_msb.data_ptr(), self.K_lsb.data_ptr(), self.V_msb.data_ptr(), self.V_lsb.data_ptr(),
-                *self.K_msb.stride()[:4], *self.K_lsb.stride()[:4],
-                self.K_scale_turbo.data_ptr(), self.V_scale_turbo.data_ptr(), *self.K_scale_turbo.stride()[:3],
-                self.K_scale_raw.data_ptr(), self.K_mn_raw.data_ptr(), *self.K_scale_raw.stride()[:4],
-                self.K_partial.data_ptr(), self.V_partial.data_ptr(), *self.K_partial.stride()[:4],
-                dtype_code(self.K_partial), self.num_layers, self.batch_size, self.num_kv_heads, self.head_dim, self.page_size,
-                self.max_seq_len)
-        return d
+        return TurboCacheDesc(
+            self.K_msb.data_ptr(), self.K_lsb.data_ptr(), self.V_msb.data_ptr(), self.V_lsb.data_ptr(),
+            *self.K_msb.stride()[:4], *self.K_lsb.stride()[:4],
+            self.K_scale_turbo.data_ptr(), self.V_scale_turbo.data_ptr(), *self.K_scale_turbo.stride()[:3],
+            self.K_scale_raw.data_ptr(), self.K_mn_raw.data_ptr(), *self.K_scale_raw.stride()[:4],
+            self.K_partial.data_ptr(), self.V_partial.data_ptr(), *self.K_partial.stride()[:4],
+            dtype_code(self.K_partial), self.num_layers, self.batch_size, self.num_kv_heads, self.head_dim, self.page_size,
+            self.max_seq_len)
 
     def get_seq_length(self, layer_idx: int = 0) -> int:
         return self._seen_tokens[layer_idx]

@@ -1,0 +1,38 @@
+"""The native calls' record of a cache's storage holds addresses: it belongs to the cache it was made for."""
+import copy
+import io
+import pickle
+
+import pytest
+import torch
+
+
+def _cache(bits, device="cpu"):
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    return {3: PersistentTurboKVCache, 4: PersistentInt4KVCache, 8: PersistentInt8KVCache}[bits](
+        batch_size=1, num_layers=2, num_kv_heads=2, head_dim=64, max_seq_len=64, page_size=16, dtype=torch.float16, device=device)
+
+
+def _saved(cache):
+    f = io.BytesIO()
+    torch.save(cache, f)
+    f.seek(0)
+    return torch.load(f, weights_only=False)
+
+
+def _addresses(cache):
+    return {getattr(cache.desc(), name) for name, kind in cache.desc()._fields_ if getattr(kind, "__name__", "") == "c_void_p"}
+
+
+@pytest.mark.parametrize("bits", [3, 4, 8])
+@pytest.mark.parametrize("how", [copy.deepcopy, _saved, lambda c: pickle.loads(pickle.dumps(c))], ids=["deepcopy", "save", "pickle"])
+def test_copies_have_a_record_of_their_own(bits, how):
+    cache = _cache(bits)
+    cache.desc()                                     # as after the first append
+    cache._fq_engines = {"step": object()}
+    other = how(cache)
+    assert not hasattr(other, "_fq_engines") and hasattr(cache, "_fq_engines")
+    assert not (_addresses(cache) & _addresses(other))
+    assert other.K_partial.shape == cache.K_partial.shape and other._seen_tokens == cache._seen_tokens
