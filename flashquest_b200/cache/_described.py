@@ -5,13 +5,14 @@ from transformers.cache_utils import Cache
 
 
 class DescribedCache(Cache):
-    """_storage() names the tensors whose addresses _describe() puts into the record.  Neither the
-    record nor the step objects built on it belong to a copied or saved cache (they hold addresses)."""
+    """_storage() names the tensors whose addresses _describe() puts into the record.  The record is made when first asked for
+    and again whenever one of those tensors has been replaced; neither it nor the step objects built on it belong to a copied
+    or saved cache (they hold addresses)."""
     _desc = None
     _desc_of = None
 
     def desc(self):
-        at = tuple([t.data_ptr() for t in (self._storage()[0], self._storage()[-2])])
+        at = tuple([t.data_ptr() for t in self._storage()])
         if at != self._desc_of:
             self._desc, self._desc_of = self._describe(), at
         return self._desc

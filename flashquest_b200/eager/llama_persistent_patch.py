@@ -42,10 +42,11 @@ TRACE = None
 
 
 def _engine(cache, kind, num_q_heads, retention, num_sinks, window_pages):
-    """One preallocated native step object per cache and configuration, shared by all layers."""
+    """One preallocated native step object per cache and configuration, shared by all layers; a new one when the cache's storage
+    has been replaced."""
     key = (kind, num_q_heads, float(retention), int(num_sinks), int(window_pages))
     store = cache.__dict__.setdefault("_fq_engines", {})
-    if key not in store:
+    if key not in store or store[key]._cdesc is not cache.desc():
         cls = {3: QuestDecodeTurbo, 4: QuestDecodeInt4, 8: QuestDecodeInt8}[kind]
         store[key] = cls(cache, num_q_heads=num_q_heads, retention=retention, num_sinks=num_sinks,
                          window_pages=window_pages, q_dtype=cache.dtype)
@@ -109,7 +110,7 @@ def make_quest_persistent_forward(
 
     def _native(H_q):
         engine = state.get(H_q)
-        if engine is None:
+        if engine is None or engine._cdesc is not cache.desc():
             r = float(retention)
             if not (kv_bits == 3 or use_compact_kernel):
                 r = min(r, 1.0)          # the mask sequence keeps every page for a retention above 1; the other routes refuse it

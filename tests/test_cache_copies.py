@@ -36,3 +36,17 @@ def test_copies_have_a_record_of_their_own(bits, how):
     assert not hasattr(other, "_fq_engines") and hasattr(cache, "_fq_engines")
     assert not (_addresses(cache) & _addresses(other))
     assert other.K_partial.shape == cache.K_partial.shape and other._seen_tokens == cache._seen_tokens
+
+
+@pytest.mark.parametrize("bits", [3, 4, 8])
+def test_record_follows_replaced_storage(bits):
+    cache = _cache(bits)
+    names = [n for n, t in vars(cache).items() if torch.is_tensor(t)]
+    keep = []
+    for name in names:                               # one at a time: every address counts
+        before = cache.desc()
+        keep.append(getattr(cache, name))
+        setattr(cache, name, keep[-1].clone())
+        assert cache.desc() is not before and getattr(cache, name).data_ptr() in _addresses(cache)
+        assert keep[-1].data_ptr() not in _addresses(cache)
+        assert cache.desc() is cache.desc()

@@ -332,3 +332,16 @@ def test_unsupported_forms_raise_what_the_kernels_say(kv_bits, compact):
         _small(kv_bits, 16, D=256, use_compact_kernel=compact)[0]()
     with pytest.raises(RuntimeError, match="cache dtype code 0"):
         _small(kv_bits, 16, dtype=torch.float32, use_compact_kernel=compact)[0]()
+
+
+@pytest.mark.parametrize("kv_bits,page,compact", [(3, 16, False), (4, 16, False), (4, 16, True), (8, 16, False), (8, 8, False)])
+def test_storage_replaced_between_tokens(kv_bits, page, compact):
+    """A cache whose tensors have been replaced (restored from a file, say) is read where it is now."""
+    call, cache = _small(kv_bits, page, use_compact_kernel=compact)
+    want = call()
+    old = {n: t for n, t in vars(cache).items() if torch.is_tensor(t)}
+    for n, t in old.items():
+        setattr(cache, n, t.clone())
+        t.zero_()
+    assert torch.equal(call(), want)
+    assert not any(t.any() for t in old.values())                    # and nothing is written to what it was
