@@ -420,8 +420,12 @@ extern "C" int fq_awq_gemm(
     FQ_CHECK_ARG(n_proj >= 1 && n_proj <= GM_MAX_PROJ, FQ_ERR_ARG, "%s: 1..%d projections per call, got %d", fn, GM_MAX_PROJ, n_proj);
     FQ_CHECK_ARG(x && qweight && scales && qzeros && N && y, FQ_ERR_ARG, "%s: null pointer", fn);
     FQ_CHECK_ARG(aligned(x, 16), FQ_ERR_ALIGN, "%s: x must be 16-byte aligned", fn);
-    // Up to 384 tiles of 128 x 128 (2.6 waves of the SMs): the split-K kernel.  Measured at 3072 x 16384: 59 us against 74 at
-    // 384 rows (384 tiles), 79 against 75 at 512 (512 tiles); at 3072 x 3072: 37 against 42 at 1024 rows (192 tiles).
+    // Up to three waves of 128 x 128 tiles the few-row kernel, one chain of products per tile: same bits, shorter start, and a
+    // wave of it costs 1/3 to 1/2 of a 256-column tile's.  Measured, few-row / this kernel, us:
+    //   3072 -> 5120:   18.1 / 42.4 at 256 rows (80 tiles), 37.3 / 41.4 at 768 (240), 56.7 / 69.9 at 1280 (400), 74.1 / 70.0 at 1536 (480)
+    //   3072 -> 16384:  38.4 / 41.9 at 256 rows (256), 57.1 / 71.7 at 384 (384), 75.4 / 71.7 at 512 (512)
+    //   8192 -> 3072:   44.4 / 96.6 at 768 rows (144), 130 / 171 at 2048 (384)
+    //   4096 -> 6144:   72.6 / 89.1 at 1100 rows (432), 93.8 / 89.6 at 1280 (480);  14336 -> 4096: 233 / 300 at 1536 (384), 308 / 302 at 2048 (512)
     int64_t tiles128 = 0;
     for (int i = 0; i < n_proj; ++i) {
         FQ_CHECK_ARG(N[i] > 0 && N[i] % 128 == 0, FQ_ERR_UNSUPPORTED, "%s: N[%d]=%d must be a positive multiple of 128", fn, i, N[i]);
@@ -430,7 +434,8 @@ extern "C" int fq_awq_gemm(
                      "%s: y[%d], scales[%d] and qweight[%d] must be 16-byte aligned", fn, i, i, i);
         tiles128 += N[i] / 128;
     }
-    if (tiles128 * ((M + 127) / 128) <= 384) {
+    const int sms = sm_count();
+    if (tiles128 * ((M + 127) / 128) <= 3LL * sms) {
         SkinnyCall c{};
         c.x = x; c.M = M; c.K = K; c.group = group; c.n_proj = n_proj; c.interleaved = interleaved ? 1 : 0;
         for (int i = 0; i < n_proj; ++i) {
@@ -467,10 +472,7 @@ extern "C" int fq_awq_gemm(
         if (r != CUDA_SUCCESS) return fail(FQ_ERR_CUDA, "%s: tensor map for qweight[%d]: driver error %d", fn, i, (int)r);
     }
     for (int i = n_proj; i < GM_MAX_PROJ; ++i) { maps[1 + i] = maps[1]; p.proj[i] = GemmProj{nullptr, nullptr, nullptr, nullptr, 0, 1 << 30}; }
-    // one persistent CTA per SM (the shared memory of a CTA leaves room for no second one)
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    // One persistent CTA per SM (the shared memory of a CTA leaves room for no second one).
     // 256-row tiles once they fill at least one wave of the SMs, 128-row tiles (twice as many CTAs) below that
     const int mt = ((int64_t)((M + 255) / 256) * tile0 >= (int64_t)sms) ? 2 : 1;
     const int m_tiles = (M + GM_BM * mt - 1) / (GM_BM * mt);

@@ -1,4 +1,4 @@
-"""The AWQ GEMM at the edges of its row tiles and K splits (csrc/fq_awq_skinny.cu, csrc/fq_awq_gemm.cu), and the GEMV
+"""The AWQ GEMM at the edges of its row tiles (csrc/fq_awq_skinny.cu, csrc/fq_awq_gemm.cu; the two give equal bits), and the GEMV
 over its K splits and rows (csrc/fq_awq_gemv.cu), against a plain
 PyTorch product of the fp16-rounded weights, and equal to itself over repeated launches."""
 import pytest
@@ -41,6 +41,20 @@ def test_rows_and_splits(M, K, Ns, group, interleaved, bias):
         assert (y.float() - want).abs().max().item() <= 2e-3 * want.abs().max().item() + 1e-3
     for _ in range(5):
         assert all(torch.equal(a, b) for a, b in zip(got, awq_gemm_fused(x, lins)))
+
+
+@pytest.mark.parametrize("K,N,group,interleaved,bias", [(512, 512, 128, True, False), (3072, 512, 128, True, True), (1536, 512, 256, False, True)])
+def test_few_row_kernel_gives_the_bits_of_the_large_gemm(K, N, group, interleaved, bias):
+    """A row's result does not depend on the kernel that the number of rows picks: the first rows of a product of 20 000 rows
+    (256-row tiles) and of 14 336 (128-row tiles, above three waves of the few-row kernel's), alone."""
+    from flashquest_b200.kernel.fused_proj import awq_gemm_fused
+    g = torch.Generator(device="cuda").manual_seed(K)
+    lin = _linear(K, N, group, interleaved, bias, g)
+    x = torch.randn(20000, K, device="cuda", generator=g).half()
+    (large,) = awq_gemm_fused(x, (lin,))
+    assert torch.equal(awq_gemm_fused(x[:14336], (lin,))[0], large[:14336])
+    for M in (9, 16, 17, 32, 33, 64, 65, 128, 129, 300, 1000, 14000):
+        assert torch.equal(awq_gemm_fused(x[:M], (lin,))[0], large[:M]), M
 
 
 @pytest.mark.parametrize("M", [1100, 2048])
