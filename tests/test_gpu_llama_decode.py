@@ -335,3 +335,41 @@ def test_prefill_group_sizes(group, S):
     want = _ref_prefill(cfg, w, ids, 16)[0].float()
     # free-running, as in test_prefill_then_decode: the 4-bit codes of k / v may differ by a step
     assert (dec.logits.float().cpu() - want).abs().max().item() <= 3e-2 * want.abs().max().item() + 1e-2
+
+
+@pytest.mark.parametrize("B,hidden", [(1, 256), (2, 256), (3, 256), (5, 384), (8, 512)])
+def test_norm_apart_equals_the_folded_prologue(B, hidden):
+    """From three sequences on the RMSNorm in front of q/k/v and gate/up is a launch of its own: the logits of a step are those
+    of the same step with the norm folded into the GEMV, bit for bit."""
+    from flashquest_b200._lib import check, lib, ptr, stream_ptr
+    from flashquest_b200.eager.llama_decode import LlamaConfig, LlamaInt4Decoder, random_llama_weights
+    from flashquest_b200.kernel.fused_proj import awq_gemv_fused
+    cfg = LlamaConfig(hidden=hidden, layers=3, q_heads=4, kv_heads=2, head_dim=64, ffn=512, vocab=512)
+    w = random_llama_weights(cfg, "cuda", seed=9)
+    mk = lambda: LlamaInt4Decoder(cfg, w, batch_size=B, max_seq_len=64, page_size=16, retention=0.5, num_sinks=1, window_pages=1)
+    a, b = mk(), mk()
+
+    def folded(d, ids):
+        pos, x, delta = d.cache.get_seq_length(0), w.embed[ids.long()], None
+
+        def norm(**kw):
+            if delta is None:
+                return dict(kw, norm_weight=kw["norm_weight"], eps=cfg.rms_eps)
+            return dict(kw, add=delta, eps=cfg.rms_eps, return_sum=True)
+        for li, lw in enumerate(w.layers):
+            q, k, v, *s = awq_gemv_fused(x, (lw.q_proj, lw.k_proj, lw.v_proj), **norm(norm_weight=lw.input_norm),
+                                         rope=dict(mask=3, pos=pos, theta=cfg.rope_theta, head_dim=64))
+            x = s[0] if s else x
+            O, _ = d.attn.step(k.view(B, 2, 1, 64), v.view(B, 2, 1, 64), q.view(B, 4, 1, 64), li)
+            (delta,) = awq_gemv_fused(O.reshape(B, 256), (lw.o_proj,))
+            gate, up, x = awq_gemv_fused(x, (lw.gate_proj, lw.up_proj), **norm(norm_weight=lw.post_norm))
+            (delta,) = awq_gemv_fused(gate, (lw.down_proj,), swiglu_up=up)
+        normed, total = torch.empty_like(x), torch.empty_like(x)
+        st = stream_ptr(x.device)
+        check(lib().fq_add_rmsnorm(ptr(x), ptr(delta), ptr(w.final_norm), cfg.rms_eps, B, hidden, ptr(total), ptr(normed), st))
+        check(lib().fq_gemv_f16(ptr(normed), ptr(w.lm_head), B, hidden, cfg.vocab, ptr(d.logits), st))
+    ids = torch.randint(0, cfg.vocab, (20, B), generator=torch.Generator().manual_seed(B), dtype=torch.int32).cuda()
+    for t in range(20):                                            # across a page end
+        a.decode_step(ids[t])
+        folded(b, ids[t])
+        assert torch.equal(a.logits, b.logits), t

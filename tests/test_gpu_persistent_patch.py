@@ -345,3 +345,10 @@ def test_storage_replaced_between_tokens(kv_bits, page, compact):
         t.zero_()
     assert torch.equal(call(), want)
     assert not any(t.any() for t in old.values())                    # and nothing is written to what it was
+
+
+@pytest.mark.parametrize("kv_bits,page,head_dim,compact", [(4, 64, 64, False), (4, 64, 128, True), (4, 16, 128, False), (8, 64, 128, False), (8, 32, 64, False),
+                                                           (3, 64, 128, False), (3, 16, 128, False), (8, 8, 64, False), (8, 128, 128, False)])
+def test_pages_and_head_dims(kv_bits, page, head_dim, compact):
+    """The default page of 64, head_dim 128, and the INT8 pages that keep the reference's own sequence (8 and 128)."""
+    _oracle_checked_run(kv_bits, page, head_dim, compact=compact, fused=not (kv_bits == 8 and page in (8, 128)))
