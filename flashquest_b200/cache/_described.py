@@ -3,17 +3,19 @@ from __future__ import annotations
 
 from transformers.cache_utils import Cache
 
+from .._lib import bind
+
 
 class DescribedCache(Cache):
-    """_storage() names the tensors whose addresses _describe() puts into the record.  The record is made when first asked for
+    """_storage (an attrgetter) names the tensors whose addresses _describe() puts into the record.  The record is made when first asked for
     and again whenever one of those tensors has been replaced; neither it nor the step objects built on it belong to a copied
     or saved cache (they hold addresses)."""
     _desc = None
     _desc_of = None
 
     def desc(self):
-        at = tuple([t.data_ptr() for t in self._storage()])
-        if at != self._desc_of:
+        at = bind().addresses(self._storage(self), self._desc_of)      # one native call: this runs for every token and layer
+        if at is not self._desc_of:
             self._desc, self._desc_of = self._describe(), at
         return self._desc
 

@@ -9,6 +9,7 @@ constructor argument (default bf16 as in the reference).
 from __future__ import annotations
 
 import ctypes
+from operator import attrgetter
 
 import torch
 
@@ -19,6 +20,8 @@ from ._described import DescribedCache
 
 class PersistentInt4KVCache(DescribedCache):
     kv_bits = 4
+    _storage = staticmethod(attrgetter("K_packed", "V_packed", "K_scale", "K_mn",
+                                       "V_scale", "V_mn", "K_partial", "V_partial"))
 
     def __init__(self, *, batch_size: int, num_layers: int, num_kv_heads: int, head_dim: int,
                  max_seq_len: int, page_size: int = 64, device="cuda", dtype=torch.bfloat16):
@@ -50,10 +53,6 @@ class PersistentInt4KVCache(DescribedCache):
         self.K_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self.V_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self._seen_tokens = [0] * num_layers
-
-    def _storage(self):
-        return (self.K_packed, self.V_packed, self.K_scale, self.K_mn,
-                self.V_scale, self.V_mn, self.K_partial, self.V_partial)
 
     def _describe(self) -> Int4CacheDesc:
         """struct fq_int4_cache of this cache."""

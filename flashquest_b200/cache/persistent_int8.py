@@ -3,6 +3,7 @@ same constructor keywords, attributes, view keys and error behaviour."""
 from __future__ import annotations
 
 import ctypes
+from operator import attrgetter
 
 import torch
 
@@ -13,6 +14,8 @@ from ._described import DescribedCache
 
 class PersistentInt8KVCache(DescribedCache):
     kv_bits = 8
+    _storage = staticmethod(attrgetter("K_uint8", "V_uint8", "K_scale", "K_mn",
+                                       "V_scale", "V_mn", "K_partial", "V_partial"))
 
     def __init__(self, *, batch_size: int, num_layers: int, num_kv_heads: int, head_dim: int,
                  max_seq_len: int, page_size: int = 64, device="cuda", dtype=torch.bfloat16):
@@ -42,10 +45,6 @@ class PersistentInt8KVCache(DescribedCache):
 
         # the one-launch append (fq_append_kv_int8): 16-bit staging, head_dim 64 / 128, pages of 16, 32 or 64 tokens
         self._one_launch = dtype in (torch.float16, torch.bfloat16) and D in (64, 128) and page_size in (16, 32, 64)
-
-    def _storage(self):
-        return (self.K_uint8, self.V_uint8, self.K_scale, self.K_mn,
-                self.V_scale, self.V_mn, self.K_partial, self.V_partial)
 
     def _describe(self) -> Int4CacheDesc:
         """struct fq_int4_cache of this cache (code rows of D bytes)."""

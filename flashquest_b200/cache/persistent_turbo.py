@@ -4,6 +4,7 @@ and error behaviour; the append is one launch for pages of 16 tokens, three othe
 from __future__ import annotations
 
 import ctypes
+from operator import attrgetter
 
 import torch
 
@@ -14,6 +15,8 @@ from ._described import DescribedCache
 
 class PersistentTurboKVCache(DescribedCache):
     kv_bits = 3
+    _storage = staticmethod(attrgetter("K_msb", "K_lsb", "V_msb", "V_lsb", "K_scale_turbo",
+                                       "V_scale_turbo", "K_scale_raw", "K_mn_raw", "K_partial", "V_partial"))
 
     def __init__(self, *, batch_size: int, num_layers: int, num_kv_heads: int, head_dim: int,
                  max_seq_len: int, page_size: int = 64, device="cuda", dtype=torch.bfloat16):
@@ -47,10 +50,6 @@ class PersistentTurboKVCache(DescribedCache):
         self.K_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self.V_partial = torch.zeros((L, B, H, page_size, D), dtype=dtype, device=dev)
         self._seen_tokens = [0] * num_layers
-
-    def _storage(self):
-        return (self.K_msb, self.K_lsb, self.V_msb, self.V_lsb, self.K_scale_turbo,
-                self.V_scale_turbo, self.K_scale_raw, self.K_mn_raw, self.K_partial, self.V_partial)
 
     def _describe(self) -> TurboCacheDesc:
         """struct fq_turbo_cache of this cache."""

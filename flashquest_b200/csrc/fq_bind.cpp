@@ -10,6 +10,8 @@
 // has no address) becomes a Python exception.
 #include <Python.h>
 
+#include <cstring>
+
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -238,7 +240,25 @@ PyObject* append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// addresses(tensors, known): the tensors' addresses packed into bytes; `known` itself where it holds the same ones
+PyObject* addresses(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    constexpr Py_ssize_t MAX = 16;
+    if (n != 2 || !PyTuple_Check(a[0]) || PyTuple_GET_SIZE(a[0]) > MAX) { PyErr_SetString(PyExc_TypeError, "addresses() takes a tuple of up to 16 tensors and bytes"); return nullptr; }
+    const void* at[MAX];
+    const Py_ssize_t count = PyTuple_GET_SIZE(a[0]), size = count * static_cast<Py_ssize_t>(sizeof(void*));
+    for (Py_ssize_t i = 0; i < count; ++i) {
+        const at::Tensor* t = tensor_of(PyTuple_GET_ITEM(a[0], i));
+        if (!t) { PyErr_SetString(PyExc_TypeError, "addresses() takes tensors"); return nullptr; }
+        at[i] = t->data_ptr();
+    }
+    if (PyBytes_Check(a[1]) && PyBytes_GET_SIZE(a[1]) == size && std::memcmp(PyBytes_AS_STRING(a[1]), at, size) == 0) return Py_NewRef(a[1]);
+    return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(at), size);
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef kMethods[] = {
+    {"addresses", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(addresses)), METH_FASTCALL, nullptr},
     {"append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(append)), METH_FASTCALL, nullptr},
     {"plan", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(make_plan)), METH_FASTCALL, nullptr},
     {"step", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(step)), METH_FASTCALL, nullptr},

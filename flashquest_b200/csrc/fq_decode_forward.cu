@@ -16,17 +16,18 @@ __global__ void __launch_bounds__(64) rope_qkv_kernel(const TM* __restrict__ q, 
                                                       const TM* __restrict__ v, int64_t v_sb, const TM* __restrict__ cosv, int64_t c_sb,
                                                       const TM* __restrict__ sinv, int64_t s_sb, int Hq, int Hkv, int D,
                                                       TC* __restrict__ q_out, TC* __restrict__ k_out, TC* __restrict__ v_out,
-                                                      const uint8_t* __restrict__ pattern, int64_t pt_s, float retention, float* __restrict__ ret_out) {
+                                                      const uint8_t* __restrict__ pattern, int64_t pt_s, int n_rep, float retention, float* __restrict__ ret_out) {
     const int head = blockIdx.x, b = blockIdx.y, half = D / 2, i = threadIdx.x;
     pdl_wait();
     pdl_trigger();
     if (i >= half) return;
-    if (pattern != nullptr && i == 0 && b == 0 && head < Hq) ret_out[head] = pattern[(head / (Hq / Hkv)) * pt_s] ? retention : 0.0f;
     const bool is_q = head < Hq, is_v = head >= Hq + Hkv;
     const int hh = is_q ? head : is_v ? head - Hq - Hkv : head - Hq;
     const TM* src = (is_q ? q + b * q_sb : is_v ? v + b * v_sb : k + b * k_sb) + (int64_t)hh * D;
     TC* dst = is_q ? q_out + ((int64_t)b * Hq + hh) * D : (is_v ? v_out : k_out) + ((int64_t)b * Hkv + hh) * D;
     const float x1 = Dt<TM>::to_f32(src[i]), x2 = Dt<TM>::to_f32(src[i + half]);
+    const bool ret = pattern != nullptr && is_q && (i | b) == 0;
+    const uint8_t keep = ret ? pattern[head / n_rep * pt_s] : 0;              // in flight with the rest
     float a = x1, c = x2;
     if (!is_v) {
         const float c1 = Dt<TM>::to_f32(cosv[b * c_sb + i]), c2 = Dt<TM>::to_f32(cosv[b * c_sb + i + half]);
@@ -36,6 +37,7 @@ __global__ void __launch_bounds__(64) rope_qkv_kernel(const TM* __restrict__ q, 
     }
     dst[i] = from_f32<TC>(a);
     dst[i + half] = from_f32<TC>(c);
+    if (ret) ret_out[head] = keep ? retention : 0.0f;
 }
 
 template <typename TM, typename TC>
@@ -45,7 +47,7 @@ static void launch_rope_qkv(const void* q, int64_t q_sb, const void* k, int64_t 
     launch_k(PDL_QUANT, rope_qkv_kernel<TM, TC>, dim3((unsigned)(Hq + 2 * Hkv), (unsigned)B), dim3(64), 0, st,
              static_cast<const TM*>(q), q_sb, static_cast<const TM*>(k), k_sb, static_cast<const TM*>(v), v_sb,
              static_cast<const TM*>(c), c_sb, static_cast<const TM*>(s), s_sb, Hq, Hkv, D,
-             static_cast<TC*>(qo), static_cast<TC*>(ko), static_cast<TC*>(vo), pattern, pt_s, retention, ret_out);
+             static_cast<TC*>(qo), static_cast<TC*>(ko), static_cast<TC*>(vo), pattern, pt_s, Hq / Hkv, retention, ret_out);
 }
 
 }  // namespace fq

@@ -146,7 +146,11 @@ def make_quest_persistent_forward(
         if native and len(input_shape) == 2 and input_shape[1] == 1:
             engine = _native(q.shape[-1] // head_dim)
             cos, sin = position_embeddings
-            O = engine.forward_token(q, k, v, cos, sin, li, pattern=_pattern(q.device))
+            O = engine.forward_token(q, k, v, cos, sin, li, pattern=head_pattern_layer)
+            if O is None:                                  # perhaps the pattern: on the host, not bool, not (H_kv,)
+                pattern = _pattern(q.device)
+                if pattern is not head_pattern_layer:
+                    O = engine.forward_token(q, k, v, cos, sin, li, pattern=pattern)
             if O is not None:
                 if TRACE is not None:
                     TRACE(li, engine.q_rot, engine.k_rot, engine.v_rot, O)

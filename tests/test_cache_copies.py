@@ -1,10 +1,16 @@
 """The native calls' record of a cache's storage holds addresses: it belongs to the cache it was made for."""
 import copy
 import io
+import os
 import pickle
 
 import pytest
 import torch
+
+
+from flashquest_b200 import build
+
+pytestmark = pytest.mark.skipif(not os.path.exists(build.BIND), reason="library not built (python -m flashquest_b200.build)")
 
 
 def _cache(bits, device="cpu"):
