@@ -259,6 +259,8 @@ __device__ __forceinline__ void select_row(
 // rank k, its keys are ranked directly, and one scan over the warps places the output: five barriers.  Rows whose range is
 // not finite, or with more than SEL_CAND_MAX keys in the interval, go through select_row instead.  Back to
 // back, before -> now: 24 rows of 256 pages 5.9 -> 2.2 us, of 2048 7.5 -> 3.3; 384 rows of 2048 13.2 -> 6.7, of 8192 38.7 -> 20.8.
+// The limit of 8192 pages is 8 scores for each of 1024 threads, or 16 for each of 512: 64 registers a thread hold 8 of them
+// beside the search, and 1024 threads have no more.  Longer rows take the search over keys in shared memory.
 constexpr int SELR_BINS = 512, SELR_MAX_P = 8192;
 
 struct SelRegShared {

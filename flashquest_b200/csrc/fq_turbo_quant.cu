@@ -659,6 +659,8 @@ extern "C" int fq_append_kv_turbo(const fq_turbo_cache* c, int layer, int seen, 
         p.scale[0] = static_cast<uint16_t*>(c->K_scale_turbo) + layer * c->st_sl + tok0;
         p.scale[1] = static_cast<uint16_t*>(c->V_scale_turbo) + layer * c->st_sl + tok0;
         p.sc_sb = c->st_sb; p.sc_sh = c->st_sh; p.sc_ss = 1;
+        // One warp finds the extrema of 16 tokens, whose rows it brings in for the coding: a page of 16.  Larger pages would have
+        // to join those of several warps, which is not built; their K is read again by the launch at the end.
         if (page == 16) {
             p.raw_scale = Ksr; p.raw_mn = Kmr; p.km_sb = c->km_sb; p.km_sh = c->km_sh; p.km_sp = c->km_sp;
             p.n_stage = partial + n_new - n_quant;
