@@ -13,10 +13,9 @@
 //                operations, four exact subtractions (an odd nibble's factor of 16 goes with an fma) and four products per
 //                8 weights; groups of four warps take turns.  Then the accumulator, bias, fp16, 16-byte stores.
 // The K range is not split: one chain of products in k order gives the bits of the large GEMM, so a prompt's cache does not
-// depend on which kernel its length picks (tests/test_gpu_awq_rows.py).  (Split over a cluster the 16-row linears took 48 us a layer instead of 82, but a
-// last-bit difference moves 4-bit codes of the cache a few layers on.)  Bound by the chain
-// itself: 8 MMAs of 64 cycles and their waits per block of 128 k.
-// 3072 -> 5120 / 3072 / 16384 and 8192 -> 3072, 16 rows, us: large GEMM 43 / 43 / 50 / 115, here 15 / 14 / 19 / 35.
+// depend on which kernel its length picks (tests/test_gpu_awq_rows.py).  (Split over a cluster the 16-row linears took 48 us a
+// layer instead of 82, but a last-bit difference moves 4-bit codes of the cache a few layers on.)  Bound by the chain itself: 8 MMAs of 64 cycles and their waits per block of 128 k.
+// 3072 -> 5120 / 3072 / 16384 and 8192 -> 3072, 16 rows, us: large GEMM 41 / 41 / 42 / 100, here 13.5 / 13.4 / 17.7 / 33.4.
 #include "fq_awq_skinny.cuh"
 
 #include <cuda.h>

@@ -31,12 +31,11 @@ class _NativeSteps:
         """scores, compact, workspace, scratch: a part for each layer, so that layers of one cache may run on different streams."""
         B, D, L, dt = self.B, self.D, self.cache.num_layers, self.cache.dtype
         # what the patched forward's rotary embedding writes: q, k, v of the new token in the cache's dtype
-        q_rot = torch.empty(L, B, self.Hq, 1, D, dtype=dt, device=self.device)
-        k_rot = torch.empty(L, B, self.Hkv, 1, D, dtype=dt, device=self.device)
-        v_rot = torch.empty_like(k_rot)
-        self._rot = list(zip(q_rot, k_rot, v_rot))
-        self.q_rot, self.k_rot, self.v_rot = self._rot[0]       # of the layer that forward_token has last been called for
-        self.pattern_retention = torch.zeros(L, self.Hq, dtype=torch.float32, device=self.device)
+        rot = torch.empty(L, B, self.Hq + 2 * self.Hkv, 1, D, dtype=dt, device=self.device)
+        n_q, n_kv, size = B * self.Hq * D, B * self.Hkv * D, rot.element_size()
+        q_rot, sl = rot.data_ptr(), rot.stride(0) * size
+        self._rot, self._rot_layer = rot, 0                     # a layer's part: q, then k, then v, each dense
+        self.pattern_retention = torch.empty(L, self.Hq, dtype=torch.float32, device=self.device)
         ws_bytes = workspace.shape[-1]
         self._plan_ = bind().plan(
             kind, ctypes.addressof(self._cdesc), ctypes.addressof(self._prm), self.device.index or 0, L,
@@ -44,11 +43,20 @@ class _NativeSteps:
             self.O.data_ptr(), self.O.stride(0) * self.O.element_size(), self.lse.data_ptr(), self.lse.stride(0),
             workspace.data_ptr(), workspace.stride(0), ws_bytes,
             *((scratch.data_ptr(), scratch.stride(0), scratch.shape[1]) if scratch is not None else (0, 0, 0)),
-            q_rot.data_ptr(), q_rot.stride(0) * q_rot.element_size(),
-            k_rot.data_ptr(), v_rot.data_ptr(), k_rot.stride(0) * k_rot.element_size(),
+            q_rot, sl, q_rot + n_q * size, q_rot + (n_q + n_kv) * size, sl,
             self.pattern_retention.data_ptr())
         self._outs = [(self.O[i].unsqueeze(2), self.lse[i].unsqueeze(2)) for i in range(L)]
         self._step, self._forward = bind().step, bind().forward
+
+    def _rotated(self, i):
+        """q, k, v (i = 0, 1, 2) as they went into the cache, of the layer that forward_token has last been called for."""
+        n_q, n_kv = self.B * self.Hq * self.D, self.B * self.Hkv * self.D
+        at, heads = ((0, self.Hq), (n_q, self.Hkv), (n_q + n_kv, self.Hkv))[i]
+        return self._rot[self._rot_layer].view(-1)[at:at + self.B * heads * self.D].view(self.B, heads, 1, self.D)
+
+    q_rot = property(lambda self: self._rotated(0))
+    k_rot = property(lambda self: self._rotated(1))
+    v_rot = property(lambda self: self._rotated(2))
 
     def _seen_checked(self, layer_idx, n_new):
         c = self.cache
@@ -98,7 +106,7 @@ class _NativeSteps:
             check(rc)
         self.cache._seen_tokens[layer_idx] = seen + 1
         self.launches += self.LAUNCHES + 1
-        self.q_rot, self.k_rot, self.v_rot = self._rot[layer_idx]
+        self._rot_layer = layer_idx
         return self._outs[layer_idx][0]
 
     def params_for(self, head_pattern_layer: torch.Tensor):

@@ -138,7 +138,7 @@ def test_layers_of_one_cache_on_two_streams(kind):
         cache._seen_tokens[layer] = n
         return engine.forward_token(*flat[layer], cos, sin, layer)
     want = [token(layer).clone() for layer in range(L)]
-    rot = [[t.clone() for t in engine._rot[layer]] for layer in range(L)]
+    rot = engine._rot.clone()                                       # q, k, v of the rotary launch
     torch.cuda.synchronize()
     streams = [torch.cuda.Stream() for _ in range(L)]
     for _ in range(20):
@@ -148,4 +148,4 @@ def test_layers_of_one_cache_on_two_streams(kind):
         torch.cuda.synchronize()
         for layer in range(L):
             assert torch.equal(engine.O[layer].unsqueeze(2), want[layer])
-            assert all(torch.equal(a, b) for a, b in zip(engine._rot[layer], rot[layer]))
+            assert torch.equal(engine._rot[layer], rot[layer])
