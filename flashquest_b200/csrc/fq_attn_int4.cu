@@ -60,6 +60,7 @@ struct AttnParams {
     void* O; int64_t o_sb, o_sh;
     float* lse;
     int* tickets; float* partials; int n_split;
+    int ws_batch; int64_t ws_next;    // scratch in several parts: sequence b uses part b / ws_batch, ws_next bytes apart
     const int* pos; int pos_new;      // non-null: S_kv, P and tail_len are derived from *pos on the device (see DynPos)
     int pos_early;                    // *pos may be read before the dependency wait (DynPos::early)
     int* status;
@@ -615,7 +616,7 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) sparse_decode_in
     }
 
     QT* Op = static_cast<QT*>(p.O) + b * p.o_sb + hq * p.o_sh;
-    const int row = b * p.Hq + hq;
+    int row = b * p.Hq + hq;
     if (p.n_split == 1) {
         if (tid < D) Op[tid] = from_f32<QT>(l_cta > 0.f ? acc_d / l_cta : 0.f);
         if (tid == 0 && p.lse) p.lse[row] = l_cta > 0.f ? (m_cta + log2f(l_cta)) * LN2 : -INFINITY;
@@ -623,7 +624,17 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) sparse_decode_in
     }
 
     // ---------------- split-K: publish the partial, last ticket merges ----------------
-    float* part = p.partials + ((int64_t)row * p.n_split + split) * (D + 2);
+    int* tickets = p.tickets;
+    float* partials = p.partials;
+    const int lse_row = row;
+    if (p.ws_next != 0) {
+        const int in_part = b % p.ws_batch;
+        const int64_t off = (int64_t)(b / p.ws_batch) * p.ws_next;
+        tickets = reinterpret_cast<int*>(reinterpret_cast<char*>(tickets) + off);
+        partials = reinterpret_cast<float*>(reinterpret_cast<char*>(partials) + off);
+        row = in_part * p.Hq + hq;
+    }
+    float* part = partials + ((int64_t)row * p.n_split + split) * (D + 2);
     if (tid < D) part[2 + tid] = acc_d;
     if (tid == 0) { part[0] = m_cta; part[1] = l_cta; }
     __syncthreads();           // the CTA's stores are ordered before thread 0's fence below
@@ -632,14 +643,14 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) sparse_decode_in
         // one device-scope release + acquire per CTA, carried by the ticket itself (cumulative over the barrier above;
         // the barrier below hands what the last CTA acquired to its other threads)
         int t;
-        asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(t) : "l"(p.tickets + row) : "memory");
+        asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(t) : "l"(tickets + row) : "memory");
         s_ticket = t;
     }
     __syncthreads();
     if (s_ticket != p.n_split - 1) return;
     // The partials of this row are merged in split order with every load independent of the
     // others (a dependent chain of L2 round trips here would cost more than the attention).
-    const float* parts = p.partials + (int64_t)row * p.n_split * (D + 2);
+    const float* parts = partials + (int64_t)row * p.n_split * (D + 2);
     float* mw = reinterpret_cast<float*>(smem);            // [n_split] max, then weight
     float* lw = mw + p.n_split;                             // [n_split] denominators
     __shared__ float s_red[ATT_WARPS + 1];
@@ -685,8 +696,8 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) sparse_decode_in
     }
     if (tid < D) Op[tid] = from_f32<QT>(l_all > 0.f ? o_all / l_all : 0.f);
     if (tid == 0) {
-        if (p.lse) p.lse[row] = l_all > 0.f ? (m_all + log2f(l_all)) * LN2 : -INFINITY;
-        p.tickets[row] = 0;   // leave the workspace ready for the next call
+        if (p.lse) p.lse[lse_row] = l_all > 0.f ? (m_all + log2f(l_all)) * LN2 : -INFINITY;
+        tickets[row] = 0;   // leave the workspace ready for the next call
     }
 }
 
@@ -772,7 +783,8 @@ int sparse_decode_int4_launch(
     int tail_len,
     int B, int Hq, int Hkv, int S_kv, int P, int D, int page, float sm_scale,
     void* O, int64_t o_sb, int64_t o_sh, float* lse,
-    void* workspace, size_t workspace_bytes, int n_split, void* stream, const DynPos& dp, const int32_t* list_count) {
+    void* workspace, size_t workspace_bytes, int n_split, void* stream, const DynPos& dp, const int32_t* list_count,
+    const WorkspaceParts& parts) {
     const char* fn = "fq_sparse_decode_int4";
     FQ_CHECK_ARG(B > 0 && Hq > 0 && Hkv > 0 && S_kv >= 0 && P >= 0 && bucket >= 0 && tail_len >= 0, FQ_ERR_ARG, "%s: bad sizes", fn);
     FQ_CHECK_ARG(B <= 65535 && Hq <= 65535, FQ_ERR_ARG, "%s: B and H_q must be <= 65535", fn);
@@ -824,15 +836,17 @@ int sparse_decode_int4_launch(
     if (n_split > p.bucket) n_split = p.bucket > 0 ? p.bucket : 1;
     p.n_split = n_split;
     p.tickets = nullptr; p.partials = nullptr;
+    p.ws_batch = parts.batch > 0 ? parts.batch : B;
+    p.ws_next = parts.batch > 0 ? (int64_t)parts.next : 0;
     p.pos = dp.pos; p.pos_new = dp.n_new; p.pos_early = dp.early ? 1 : 0;
     p.status = device_status_ptr();
     if (p.status == nullptr) return FQ_ERR_CUDA;
     if (n_split > 1) {
-        const size_t need = fq_sparse_decode_workspace_bytes(B, Hq, D, n_split);
+        const size_t need = fq_sparse_decode_workspace_bytes(p.ws_batch, Hq, D, n_split);     // of one part
         FQ_CHECK_ARG(workspace && workspace_bytes >= need, FQ_ERR_WORKSPACE, "%s: workspace of %zu B needed, %zu given", fn, need, workspace_bytes);
         FQ_CHECK_ARG(aligned(workspace, 16), FQ_ERR_ALIGN, "%s: workspace must be 16-byte aligned", fn);
         p.tickets = static_cast<int*>(workspace);
-        p.partials = reinterpret_cast<float*>(static_cast<char*>(workspace) + (((size_t)B * Hq * 4 + 255) & ~(size_t)255));
+        p.partials = reinterpret_cast<float*>(static_cast<char*>(workspace) + (((size_t)p.ws_batch * Hq * 4 + 255) & ~(size_t)255));
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int rc;

@@ -94,6 +94,9 @@ int select_pages_launch(
     const float* retention_per_head, float retention, int k_max, int sinks, int window,
     uint8_t* mask, int64_t mk_sb, int64_t mk_sh, int32_t* compact, int64_t cp_sb, int64_t cp_sh, int bucket,
     int32_t* count, void* stream, const DynPos& dp);
+// Split-K scratch of a launch that covers several layers of a cache: every layer's sequences keep their own part, of the
+// layout a launch of that layer alone uses (its ticket words are zero between launches), `next` bytes apart.
+struct WorkspaceParts { int batch = 0; size_t next = 0; };       // batch 0: one part for the whole launch
 int sparse_decode_int4_launch(
     const void* Q, int q_dtype, int64_t q_sb, int64_t q_sh,
     const uint8_t* K_packed, int64_t kp_sb, int64_t kp_sh,
@@ -104,7 +107,8 @@ int sparse_decode_int4_launch(
     const void* K_tail, const void* V_tail, int tail_dtype, int64_t tl_sb, int64_t tl_sh, int64_t tl_ss, int tail_len,
     int B, int Hq, int Hkv, int S_kv, int P, int D, int page, float sm_scale,
     void* O, int64_t o_sb, int64_t o_sh, float* lse,
-    void* workspace, size_t workspace_bytes, int n_split, void* stream, const DynPos& dp, const int32_t* list_count = nullptr);
+    void* workspace, size_t workspace_bytes, int n_split, void* stream, const DynPos& dp, const int32_t* list_count = nullptr,
+    const WorkspaceParts& parts = WorkspaceParts{});
 
 // One layer of the graph-capturable step (append + score + select + attend with the sequence
 // length read from *pos) and the closing increment of the positions; defined in fq_decode_layer.cu.

@@ -23,14 +23,14 @@ extern "C" int fq_append_kv_int4(const fq_int4_cache* c, int layer, int seen, co
         Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, stream);
 }
 
-extern "C" int fq_decode_layer_int4(
+namespace fq {
+static int decode_layer_int4(
     const fq_int4_cache* c, int layer, int seen,
     const void* K_new, const void* V_new, int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new,
     const void* Q, int q_dtype, int64_t q_sb, int64_t q_sh,
     const fq_decode_params* prm,
     float* scores, int32_t* compact, void* O, float* lse,
-    void* workspace, size_t workspace_bytes, void* stream) {
-    using namespace fq;
+    void* workspace, size_t workspace_bytes, const WorkspaceParts& parts, void* stream) {
     const char* fn = "fq_decode_layer_int4";
     FQ_CHECK_ARG(c && prm, FQ_ERR_ARG, "%s: null descriptor", fn);
     FQ_CHECK_ARG(layer >= 0 && layer < c->L, FQ_ERR_ARG, "%s: layer_idx %d out of range [0, %d)", fn, layer, c->L);
@@ -68,14 +68,36 @@ extern "C" int fq_decode_layer_int4(
         if (rc != FQ_OK) return rc;
     }
     int n_split = prm->n_split > 0 ? prm->n_split : fq_sparse_decode_default_splits(B, Hq, prm->bucket, page);
-    return fq_sparse_decode_int4(
+    return sparse_decode_int4_launch(
         Q, q_dtype, q_sb, q_sh, Kp, c->pk_sb, c->pk_sh, Ks, Km, c->km_sb, c->km_sh, c->km_sp,
         Vp, c->pk_sb, c->pk_sh, Vs, Vm, c->vm_sb, c->vm_sh,
         compact, (int64_t)Hq * prm->bucket, prm->bucket, P > 0 ? prm->bucket : 0,
         tail ? Kt : nullptr, tail ? Vt : nullptr, c->kv_dtype, c->pt_sb, c->pt_sh, c->pt_ss, tail,
         B, Hq, Hkv, completed, P, D, page, prm->sm_scale,
-        O, (int64_t)Hq * D, D, lse, workspace, workspace_bytes, n_split, stream);
+        O, (int64_t)Hq * D, D, lse, workspace, workspace_bytes, n_split, stream, DynPos{}, nullptr, parts);
 }
+
+// The sequences of the first `n` layers as the batch of one layer.  Every stride over the layers has to be that over the
+// sequences times their number, which the dense arrays of a cache and of an engine have.
+static fq_int4_cache layers_as_batch(const fq_int4_cache* c, int n) {
+    fq_int4_cache f = *c;
+    f.L = 1; f.B = n * c->B;
+    if (c->B == 1) { f.pk_sb = c->pk_sl; f.km_sb = c->km_sl; f.vm_sb = c->vm_sl; f.pt_sb = c->pt_sl; }
+    return f;
+}
+}  // namespace fq
+
+extern "C" int fq_decode_layer_int4(
+    const fq_int4_cache* c, int layer, int seen,
+    const void* K_new, const void* V_new, int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new,
+    const void* Q, int q_dtype, int64_t q_sb, int64_t q_sh,
+    const fq_decode_params* prm,
+    float* scores, int32_t* compact, void* O, float* lse,
+    void* workspace, size_t workspace_bytes, void* stream) {
+    return fq::decode_layer_int4(c, layer, seen, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, Q, q_dtype, q_sb, q_sh, prm,
+                                 scores, compact, O, lse, workspace, workspace_bytes, fq::WorkspaceParts{}, stream);
+}
+
 
 extern "C" int fq_decode_step_int4(
     const fq_int4_cache* c, int n_layers, const int* seen,
@@ -91,6 +113,30 @@ extern "C" int fq_decode_step_int4(
     FQ_CHECK_ARG(n_layers <= 1 || ws_sl >= workspace_bytes, FQ_ERR_WORKSPACE,
                  "%s: the per-layer workspaces overlap (stride %zu B < %zu B)", fn, ws_sl, workspace_bytes);
     const size_t kv_esz = 2, q_esz = q_dtype == FQ_F32 ? 4 : 2;
+    // All layers' inputs are here and no layer waits for another: the layers of a dense cache go through the four launches
+    // together, as one batch of n_layers * B sequences.  One layer of one sequence leaves the GPU idle between dependent
+    // launches (23 us a layer for 3.4 us of HBM time).  28 layers of one sequence, 24/8 heads of 128, layer by layer ->
+    // together: 515 tokens 245 -> 27 us, 8k 520 -> 79, 32k 648 -> 245.  At 32k the metadata of all layers (235 MB) no longer stays
+    // in L2 between scoring and attention; groups that do fit were slower all the same (4 layers 353 us, 7 337, 14 256).
+    // Layers with parameters or positions of their own, or of other strides, go one by one.
+    const int B = c->B, Hq = prm->Hq;
+    bool together = n_layers > 1 && B > 0 && (int64_t)n_layers * B <= 65535 && prm_stride == 0 &&
+                    cp_sl == (int64_t)B * Hq * prm->bucket && o_sl == (int64_t)B * Hq * c->D && (!lse || lse_sl == (int64_t)B * Hq) &&
+                    c->page > 0 && sc_sl >= (int64_t)B * Hq * (c->max_seq_len / c->page);
+    if (B > 1)
+        together = together && c->pk_sl == B * c->pk_sb && c->km_sl == B * c->km_sb && c->vm_sl == B * c->vm_sb && c->pt_sl == B * c->pt_sb &&
+                   q_sl == B * q_sb && (n_new == 0 || nw_sl == B * nw_sb);
+    for (int l = 1; l < n_layers && together; ++l) together = seen[l] == seen[0];
+    if (together) {
+        const fq_int4_cache f = layers_as_batch(c, n_layers);
+        // fewer rows left to split; never more parts than a layer's scratch has been laid out for
+        fq_decode_params all = *prm;
+        if (all.n_split <= 0) all.n_split = fq_sparse_decode_default_splits(B, Hq, prm->bucket, c->page);
+        const int splits = fq_sparse_decode_default_splits(n_layers * B, Hq, prm->bucket, c->page);
+        if (splits < all.n_split) all.n_split = splits;
+        return decode_layer_int4(&f, 0, seen[0], K_new, V_new, B == 1 ? nw_sl : nw_sb, nw_sh, nw_ss, n_new, Q, q_dtype, B == 1 ? q_sl : q_sb, q_sh,
+                                 &all, scores, compact, O, lse, workspace, workspace_bytes, WorkspaceParts{B, ws_sl}, stream);
+    }
     for (int l = 0; l < n_layers; ++l) {
         const fq_decode_params* pl = reinterpret_cast<const fq_decode_params*>(reinterpret_cast<const char*>(prm) + (size_t)l * prm_stride);
         const int rc = fq_decode_layer_int4(
