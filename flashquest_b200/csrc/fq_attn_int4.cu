@@ -759,11 +759,15 @@ extern "C" int fq_sparse_decode_default_splits(int B, int Hq, int bucket, int pa
     const long slots = 148L * fq::ATT_CTAS_PER_SM;
     long n_split = slots / rows;
     if (n_split < 1) n_split = 1;
-    // One wave that leaves more than 7 % of the slots empty (e.g. 384 rows on 444 slots) finishes when the fullest
+    // A last wave that leaves more than 7 % of the slots empty (e.g. 384 rows on 444 slots, or 512) finishes when the fullest
     // SMs do while the others idle.  Three times as many, shorter CTAs are handed out as slots free up and keep every
-    // SM busy to the end -- worth it while a CTA still has 8 iterations to amortise its start and its merge over
-    // (measured at 16 x 24 rows: 113 against 121 us; at 24 rows the single full wave stays).
-    if (rows * n_split * 100 < slots * 93 && total_iters >= 3 * n_split * 8) n_split *= 3;
+    // SM busy to the end -- worth it while a CTA still has 8 iterations to amortise its start and its merge over, and 5 where
+    // more than 18 % would be empty.  Whole step, this many splits -> three times, us, retention 0.25:
+    //   8 iterations, 32k tokens: 384 rows 157 -> 149, 512 rows 204 -> 187, 672 rows 247 -> 239, 896 rows 323 -> 306
+    //   5 iterations, 16k tokens: 224 rows 82 -> 65, 312 rows 85 -> 81; 384 rows (14 % empty) 87 -> 91: stays
+    //   few rows: 24 and 64 rows (one wave, 3 and 14 % empty) are slower at any other number
+    const long waves = (rows * n_split + slots - 1) / slots, filled = 100 * rows * n_split / (waves * slots);
+    if (total_iters >= 3 * n_split * (filled < 82 ? 5 : 8) && filled < 93) n_split *= 3;
     if (n_split > total_iters) n_split = total_iters;
     if (n_split > bucket) n_split = bucket;
     if (n_split < 1) n_split = 1;
