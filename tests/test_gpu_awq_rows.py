@@ -57,6 +57,23 @@ def test_few_row_kernel_gives_the_bits_of_the_large_gemm(K, N, group, interleave
         assert torch.equal(awq_gemm_fused(x[:M], (lin,))[0], large[:M]), M
 
 
+@pytest.mark.parametrize("M", [129, 255, 256, 257, 385, 1025])
+@pytest.mark.parametrize("K,Ns,group,interleaved,bias", [(64, (9600, 128), 64, True, True), (320, (9728,), 64, False, False), (256, (128, 9600, 384, 128), 256, True, False),
+                                                         (1152, (19200,), 128, True, False)])
+def test_pair_tiles(M, K, Ns, group, interleaved, bias):
+    """Tiles of a CTA pair at their edges: rows that end in the first or the second CTA's half, projections that end in the first
+    half of their last tile, 1 to 18 k blocks, one to five tiles per pair."""
+    from flashquest_b200.kernel.fused_proj import awq_gemm_fused
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    lins = [_linear(K, N, group, interleaved, bias, g) for N in Ns]
+    x = torch.randn(M, K, device="cuda", generator=g).half()
+    got = awq_gemm_fused(x, lins)
+    for y, lin in zip(got, lins):
+        want = x.float() @ _weights(lin) + (lin.bias.float() if bias else 0)
+        assert (y.float() - want).abs().max().item() <= 2e-3 * want.abs().max().item() + 1e-3
+    assert all(torch.equal(a, b) for a, b in zip(got, awq_gemm_fused(x, lins)))
+
+
 @pytest.mark.parametrize("M", [1100, 2048])
 def test_large_tiles_repeat(M):
     """More tiles than SMs: a CTA's second tile overlaps the epilogue of its first."""
