@@ -767,7 +767,7 @@ extern "C" int fq_sparse_decode_default_splits(int B, int Hq, int bucket, int pa
     //   5 iterations, 16k tokens: 224 rows 82 -> 65, 312 rows 85 -> 81; 384 rows (14 % empty) 87 -> 91: stays
     //   few rows: 24 and 64 rows (one wave, 3 and 14 % empty) are slower at any other number
     const long waves = (rows * n_split + slots - 1) / slots, filled = 100 * rows * n_split / (waves * slots);
-    if (total_iters >= 3 * n_split * (filled < 82 ? 5 : 8) && filled < 93) n_split *= 3;
+    if (waves <= 3 && total_iters >= 3 * n_split * (filled < 82 ? 5 : 8) && filled < 93) n_split *= 3;      // four waves (1536 rows) even out by themselves
     if (n_split > total_iters) n_split = total_iters;
     if (n_split > bucket) n_split = bucket;
     if (n_split < 1) n_split = 1;
