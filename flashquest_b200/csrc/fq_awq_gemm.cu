@@ -153,7 +153,10 @@ __device__ __forceinline__ void gm_tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) 
         : "r"(taddr));
 }
 
-template <bool INTERLEAVED>
+// SWIGLU: projection 0 is the gate, 1 the up projection of the same width, and y (of projection 0) becomes
+// fp16(silu(gate)) * up of the fp16-rounded products, the arithmetic of fq_swiglu.  A tile is 128 columns of each: the first
+// CTA dequantises the gate's, the second the up projection's, and every row of both lies in one CTA's accumulators.
+template <bool INTERLEAVED, bool SWIGLU>
 __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
     const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
     const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_w3, const GemmParams p) {
@@ -203,13 +206,19 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
     // tile index -> projection, first column inside it, first row (N tiles vary fastest: neighbouring pairs share x rows)
     auto locate = [&](int tile, int& pj, int& n0, int& m0) {
         const int nt = tile % p.n_tiles;
-        pj = 0;
-#pragma unroll
-        for (int i = 1; i < GM_MAX_PROJ; ++i)
-            if (i < p.n_proj && nt >= p.proj[i].tile0) pj = i;
-        n0 = (nt - p.proj[pj].tile0) * GM_BN;
         m0 = (tile / p.n_tiles) * (2 * GM_BM);
+        if constexpr (SWIGLU) {
+            pj = rank;
+            n0 = nt * GM_CN;
+        } else {
+            pj = 0;
+#pragma unroll
+            for (int i = 1; i < GM_MAX_PROJ; ++i)
+                if (i < p.n_proj && nt >= p.proj[i].tile0) pj = i;
+            n0 = (nt - p.proj[pj].tile0) * GM_BN;
+        }
     };
+    const int w_off = SWIGLU ? 0 : rank * GM_CN;      // this CTA's first column of W inside the tile
 
     // The producer and issuer warps walk their loops as whole warps and one elected lane issues: operands that are
     // uniform over the warp then stay in uniform registers (inside a branch on lane == 0 an MMA issue took 90 cycles).
@@ -229,7 +238,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
                 const CUtensorMap* map_w = rpj == 0 ? &map_w0 : (rpj == 1 ? &map_w1 : (rpj == 2 ? &map_w2 : &map_w3));
                 if (gm_elect()) {
                     gm_mbar_expect_tx(&raw_full[rs], GM_RAW_BYTES);
-                    gm_tma_2d(sRaw + rs * GM_RAW_BYTES, map_w, (rn0 + rank * GM_CN) / 8, rk * GM_BK, &raw_full[rs]);
+                    gm_tma_2d(sRaw + rs * GM_RAW_BYTES, map_w, (rn0 + w_off) / 8, rk * GM_BK, &raw_full[rs]);
                 }
                 __syncwarp();
                 if (++rs == RS) { rs = 0; rph ^= 1u; }
@@ -302,7 +311,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
             if (tile >= total_tiles) return;
             int pj, n0, m0;
             locate(tile, pj, n0, m0);
-            const int n = n0 + rank * GM_CN + 8 * c;
+            const int n = n0 + w_off + 8 * c;
             if (n < p.proj[pj].N) {                   // a projection of 128 (mod 256) columns ends inside its last tile
                 width = p.proj[pj].N;
                 zrow = p.proj[pj].qzeros + n / 8;
@@ -389,6 +398,36 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
             if (gm_timeout(&acc_ready[set], (unsigned)use & 1u)) { failed = true; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + rank * GM_BM + lq * 32 + lane;
+            if constexpr (SWIGLU) {
+                const GemmProj &G = p.proj[0], &U = p.proj[1];
+#pragma unroll 1
+                for (int cb = 0; cb < GM_CN / 32; ++cb) {
+                    uint32_t gv[32], uv[32];
+                    const uint32_t taddr = tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(set * GM_BN + cb * 32);
+                    gm_tmem_ld32(taddr, gv);
+                    gm_tmem_ld32(taddr + GM_CN, uv);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (row < p.M) {
+                        const int n = n0 + cb * 32;
+                        __half* yrow = G.y + (int64_t)row * G.N + n;
+#pragma unroll
+                        for (int j = 0; j < 32; j += 8) {
+                            uint32_t pk[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int i = j + 2 * e;
+                                float g0 = __uint_as_float(gv[i]), g1 = __uint_as_float(gv[i + 1]), u0 = __uint_as_float(uv[i]), u1 = __uint_as_float(uv[i + 1]);
+                                if (G.bias) { g0 += __half2float(G.bias[n + i]); g1 += __half2float(G.bias[n + i + 1]); }
+                                if (U.bias) { u0 += __half2float(U.bias[n + i]); u1 += __half2float(U.bias[n + i + 1]); }
+                                const float2 f = __half22float2(__floats2half2_rn(g0, g1));
+                                const __half2 h = __hmul2(__floats2half2_rn(f.x / (1.0f + expf(-f.x)), f.y / (1.0f + expf(-f.y))), __floats2half2_rn(u0, u1));
+                                pk[e] = *reinterpret_cast<const uint32_t*>(&h);
+                            }
+                            *reinterpret_cast<uint4*>(yrow + j) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                        }
+                    }
+                }
+            } else {
 #pragma unroll 1
             for (int cb = 0; cb < GM_BN / 32; ++cb) {
                 uint32_t v[32];
@@ -412,6 +451,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
                         *reinterpret_cast<uint4*>(yrow + j) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                     }
                 }
+            }
             }
             // the set's columns have been read: hand it back to the MMA warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -446,79 +486,81 @@ static EncodeTiledFn encode_tiled_fn() {
     return reinterpret_cast<EncodeTiledFn>(fn);
 }
 
-}  // namespace fq
-
-extern "C" int fq_awq_gemm(
-    const void* x, int M, int K, int group, int n_proj,
-    const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
-    const int* N, void* const* y, int interleaved, void* stream) {
-    using namespace fq;
-    const char* fn = "fq_awq_gemm";
-    FQ_CHECK_ARG(M >= 1, FQ_ERR_ARG, "%s: M=%d", fn, M);
-    FQ_CHECK_ARG(group == 64 || group == 128 || group == 256, FQ_ERR_UNSUPPORTED, "%s: group size %d; 64, 128 and 256 are built", fn, group);
-    FQ_CHECK_ARG(K > 0 && K % group == 0, FQ_ERR_ARG, "%s: K=%d must be a multiple of the group size %d", fn, K, group);
-    FQ_CHECK_ARG(n_proj >= 1 && n_proj <= GM_MAX_PROJ, FQ_ERR_ARG, "%s: 1..%d projections per call, got %d", fn, GM_MAX_PROJ, n_proj);
-    FQ_CHECK_ARG(x && qweight && scales && qzeros && N && y, FQ_ERR_ARG, "%s: null pointer", fn);
-    FQ_CHECK_ARG(aligned(x, 16), FQ_ERR_ALIGN, "%s: x must be 16-byte aligned", fn);
-    // One wave of 128 x 128 tiles, up to three while the rows fit one tile, go to the few-row kernel, one chain of products per
-    // tile: same bits, shorter start.  From its second wave on a pair's tile of four times the size takes 1.3 of its time.
-    // Measured, few-row / this kernel, us:
-    //   3072 -> 5120:   18.8 / 26.0 at 384 rows (120 tiles), 35.7 / 26.1 at 512 (160), 54.9 / 43.2 at 1024 (320)
-    //   3072 -> 16384:  20.5 / 26.7 at 128 rows (128), 38.7 / 26.8 at 129 (256), 56.6 / 43.4 at 257 (384)
-    //   8192 -> 3072:   44.3 / 54.0 at 768 rows (144), 83.2 / 54.2 at 1024 (192);  4096 -> 6144: 24.7 / 31.1 at 384 (144), 45.5 / 31.2 at 512 (192)
-    //   4096 -> 28672:  42.6 / 54.3 at 16 rows, 49.7 / 56.0 at 128 (224 tiles, a half-empty row tile for the pair), 92.9 / 56.5 at 129 (448)
+// One wave of 128 x 128 tiles, up to three while the rows fit one tile, go to the few-row kernel, one chain of products per
+// tile: same bits, shorter start.  From its second wave on a pair's tile of four times the size takes 1.3 of its time.
+// Measured, few-row / this kernel, us:
+//   3072 -> 5120:   18.8 / 26.0 at 384 rows (120 tiles), 35.7 / 26.1 at 512 (160), 54.9 / 43.2 at 1024 (320)
+//   3072 -> 16384:  20.5 / 26.7 at 128 rows (128), 38.7 / 26.8 at 129 (256), 56.6 / 43.4 at 257 (384)
+//   8192 -> 3072:   44.3 / 54.0 at 768 rows (144), 83.2 / 54.2 at 1024 (192);  4096 -> 6144: 24.7 / 31.1 at 384 (144), 45.5 / 31.2 at 512 (192)
+//   4096 -> 28672:  42.6 / 54.3 at 16 rows, 49.7 / 56.0 at 128 (224 tiles, a half-empty row tile for the pair), 92.9 / 56.5 at 129 (448)
+static bool few_rows(const SkinnyCall& c) {
     int64_t tiles128 = 0;
-    for (int i = 0; i < n_proj; ++i) {
-        FQ_CHECK_ARG(N[i] > 0 && N[i] % 128 == 0, FQ_ERR_UNSUPPORTED, "%s: N[%d]=%d must be a positive multiple of 128", fn, i, N[i]);
-        FQ_CHECK_ARG(qweight[i] && scales[i] && qzeros[i] && y[i], FQ_ERR_ARG, "%s: null tensor in projection %d", fn, i);
-        FQ_CHECK_ARG(aligned(y[i], 16) && aligned(scales[i], 16) && aligned(qweight[i], 16) && aligned(qzeros[i], 4), FQ_ERR_ALIGN,
+    for (int i = 0; i < c.n_proj; ++i) tiles128 += c.N[i] / 128;
+    return tiles128 * ((c.M + 127) / 128) <= (int64_t)(c.M <= GM_BM ? 3 : 1) * sm_count() && awq_skinny_supported(c);
+}
+
+static int check_call(const SkinnyCall& c, const char* fn) {
+    FQ_CHECK_ARG(c.M >= 1, FQ_ERR_ARG, "%s: M=%d", fn, c.M);
+    FQ_CHECK_ARG(c.group == 64 || c.group == 128 || c.group == 256, FQ_ERR_UNSUPPORTED, "%s: group size %d; 64, 128 and 256 are built", fn, c.group);
+    FQ_CHECK_ARG(c.K > 0 && c.K % c.group == 0, FQ_ERR_ARG, "%s: K=%d must be a multiple of the group size %d", fn, c.K, c.group);
+    FQ_CHECK_ARG(aligned(c.x, 16), FQ_ERR_ALIGN, "%s: x must be 16-byte aligned", fn);
+    for (int i = 0; i < c.n_proj; ++i) {
+        FQ_CHECK_ARG(c.N[i] > 0 && c.N[i] % 128 == 0, FQ_ERR_UNSUPPORTED, "%s: N[%d]=%d must be a positive multiple of 128", fn, i, c.N[i]);
+        FQ_CHECK_ARG(c.qweight[i] && c.scales[i] && c.qzeros[i] && c.y[i], FQ_ERR_ARG, "%s: null tensor in projection %d", fn, i);
+        FQ_CHECK_ARG(aligned(c.y[i], 16) && aligned(c.scales[i], 16) && aligned(c.qweight[i], 16) && aligned(c.qzeros[i], 4), FQ_ERR_ALIGN,
                      "%s: y[%d], scales[%d] and qweight[%d] must be 16-byte aligned", fn, i, i, i);
-        tiles128 += N[i] / 128;
     }
-    const int sms = sm_count();
-    if (tiles128 * ((M + 127) / 128) <= (int64_t)(M <= GM_BM ? 3 : 1) * sms) {
-        SkinnyCall c{};
-        c.x = x; c.M = M; c.K = K; c.group = group; c.n_proj = n_proj; c.interleaved = interleaved ? 1 : 0;
-        for (int i = 0; i < n_proj; ++i) {
-            c.qweight[i] = qweight[i]; c.scales[i] = scales[i]; c.qzeros[i] = qzeros[i]; c.bias[i] = bias ? bias[i] : nullptr; c.N[i] = N[i]; c.y[i] = y[i];
-        }
-        if (awq_skinny_supported(c)) return awq_skinny_launch(c, stream, fn);
+    return FQ_OK;
+}
+
+static SkinnyCall make_call(const void* x, int M, int K, int group, int n_proj, const int32_t* const* qweight, const void* const* scales,
+                            const int32_t* const* qzeros, const void* const* bias, const int* N, void* const* y, int interleaved) {
+    SkinnyCall c{};
+    c.x = x; c.M = M; c.K = K; c.group = group; c.n_proj = n_proj; c.interleaved = interleaved ? 1 : 0;
+    for (int i = 0; i < n_proj; ++i) {
+        c.qweight[i] = qweight[i]; c.scales[i] = scales[i]; c.qzeros[i] = qzeros[i]; c.bias[i] = bias ? bias[i] : nullptr; c.N[i] = N[i]; c.y[i] = y[i];
     }
+    return c;
+}
+
+// the pair kernel on a checked call
+static int pairs_launch(const SkinnyCall& c, bool swiglu, void* stream, const char* fn) {
     EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) return fail(FQ_ERR_CUDA, "%s: the driver does not export cuTensorMapEncodeTiled", fn);
     GemmParams p{};
-    p.n_proj = n_proj; p.M = M; p.K = K; p.group = group;
+    p.n_proj = c.n_proj; p.M = c.M; p.K = c.K; p.group = c.group;
     p.status = device_status_ptr();
     if (p.status == nullptr) return FQ_ERR_CUDA;
     CUtensorMap maps[1 + GM_MAX_PROJ];
     {
-        const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
-        const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+        const cuuint64_t dims[2] = {(cuuint64_t)c.K, (cuuint64_t)c.M};
+        const cuuint64_t strides[1] = {(cuuint64_t)c.K * 2};
         const cuuint32_t box[2] = {(cuuint32_t)GM_BK, (cuuint32_t)GM_BM}, es[2] = {1, 1};
-        CUresult r = encode(&maps[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        CUresult r = encode(&maps[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(c.x), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return fail(FQ_ERR_CUDA, "%s: tensor map for x: driver error %d", fn, (int)r);
     }
     int tile0 = 0;
-    for (int i = 0; i < n_proj; ++i) {
-        p.proj[i] = GemmProj{static_cast<const __half*>(scales[i]), qzeros[i], bias ? static_cast<const __half*>(bias[i]) : nullptr,
-                             static_cast<__half*>(y[i]), N[i], tile0};
-        tile0 += (N[i] + GM_BN - 1) / GM_BN;
-        const cuuint64_t dims[2] = {(cuuint64_t)(N[i] / 8), (cuuint64_t)K};
-        const cuuint64_t strides[1] = {(cuuint64_t)(N[i] / 8) * 4};
+    for (int i = 0; i < c.n_proj; ++i) {
+        p.proj[i] = GemmProj{static_cast<const __half*>(c.scales[i]), c.qzeros[i], static_cast<const __half*>(c.bias[i]), static_cast<__half*>(c.y[i]), c.N[i], tile0};
+        tile0 += (c.N[i] + GM_BN - 1) / GM_BN;
+        const cuuint64_t dims[2] = {(cuuint64_t)(c.N[i] / 8), (cuuint64_t)c.K};
+        const cuuint64_t strides[1] = {(cuuint64_t)(c.N[i] / 8) * 4};
         const cuuint32_t box[2] = {(cuuint32_t)(GM_CN / 8), (cuuint32_t)GM_BK}, es[2] = {1, 1};
-        CUresult r = encode(&maps[1 + i], CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<int32_t*>(qweight[i]), dims, strides, box, es,
+        CUresult r = encode(&maps[1 + i], CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<int32_t*>(c.qweight[i]), dims, strides, box, es,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return fail(FQ_ERR_CUDA, "%s: tensor map for qweight[%d]: driver error %d", fn, i, (int)r);
     }
-    for (int i = n_proj; i < GM_MAX_PROJ; ++i) { maps[1 + i] = maps[1]; p.proj[i] = GemmProj{nullptr, nullptr, nullptr, nullptr, 0, 1 << 30}; }
-    const int m_tiles = (M + 2 * GM_BM - 1) / (2 * GM_BM);
-    FQ_CHECK_ARG((int64_t)m_tiles * tile0 <= 0x7fffffffLL, FQ_ERR_ARG, "%s: M=%d too large for one launch", fn, M);
+    for (int i = c.n_proj; i < GM_MAX_PROJ; ++i) { maps[1 + i] = maps[1]; p.proj[i] = GemmProj{nullptr, nullptr, nullptr, nullptr, 0, 1 << 30}; }
+    if (swiglu) tile0 = c.N[0] / GM_CN;
+    const int m_tiles = (c.M + 2 * GM_BM - 1) / (2 * GM_BM);
+    FQ_CHECK_ARG((int64_t)m_tiles * tile0 <= 0x7fffffffLL, FQ_ERR_ARG, "%s: M=%d too large for one launch", fn, c.M);
     p.n_tiles = tile0; p.m_tiles = m_tiles;
     // one persistent pair of CTAs per pair of SMs (the shared memory of a CTA leaves room for no second one)
-    const int total = m_tiles * tile0, pairs = total < sms / 2 ? total : sms / 2;
-    auto kern = interleaved ? awq_gemm_kernel<true> : awq_gemm_kernel<false>;
+    const int total = m_tiles * tile0, sms = sm_count(), pairs = total < sms / 2 ? total : sms / 2;
+    auto kern = swiglu ? (c.interleaved ? awq_gemm_kernel<true, true> : awq_gemm_kernel<false, true>)
+                       : (c.interleaved ? awq_gemm_kernel<true, false> : awq_gemm_kernel<false, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM);
     if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: cannot reserve %d B of shared memory: %s", fn, GM_SMEM, cudaGetErrorString(e));
     cudaLaunchConfig_t cfg{};
@@ -531,4 +573,41 @@ extern "C" int fq_awq_gemm(
     if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: launch failed: %s", fn, cudaGetErrorString(e));
     FQ_CHECK_LAUNCH(fn);
     return FQ_OK;
+}
+
+}  // namespace fq
+
+extern "C" int fq_awq_gemm(
+    const void* x, int M, int K, int group, int n_proj,
+    const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
+    const int* N, void* const* y, int interleaved, void* stream) {
+    using namespace fq;
+    const char* fn = "fq_awq_gemm";
+    FQ_CHECK_ARG(n_proj >= 1 && n_proj <= GM_MAX_PROJ, FQ_ERR_ARG, "%s: 1..%d projections per call, got %d", fn, GM_MAX_PROJ, n_proj);
+    FQ_CHECK_ARG(x && qweight && scales && qzeros && N && y, FQ_ERR_ARG, "%s: null pointer", fn);
+    const SkinnyCall c = make_call(x, M, K, group, n_proj, qweight, scales, qzeros, bias, N, y, interleaved);
+    const int rc = check_call(c, fn);
+    if (rc != FQ_OK) return rc;
+    return few_rows(c) ? awq_skinny_launch(c, stream, fn) : pairs_launch(c, false, stream, fn);
+}
+
+extern "C" int fq_awq_gate_up_swiglu(
+    const void* x, int M, int K, int group, const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
+    int N, void* gate, void* up, void* y, int interleaved, void* stream) {
+    using namespace fq;
+    const char* fn = "fq_awq_gate_up_swiglu";
+    FQ_CHECK_ARG(x && qweight && scales && qzeros && y, FQ_ERR_ARG, "%s: null pointer", fn);
+    const int Ns[2] = {N, N};
+    void* both[2] = {gate, up};
+    void* ys[2] = {y, y};
+    SkinnyCall c = make_call(x, M, K, group, 2, qweight, scales, qzeros, bias, Ns, ys, interleaved);
+    int rc = check_call(c, fn);
+    if (rc != FQ_OK) return rc;
+    if (!few_rows(c)) return pairs_launch(c, true, stream, fn);
+    for (int i = 0; i < 2; ++i) {
+        c.y[i] = both[i];
+        FQ_CHECK_ARG(both[i] && aligned(both[i], 16), FQ_ERR_ALIGN, "%s: gate and up must be 16-byte aligned", fn);
+    }
+    if ((rc = awq_skinny_launch(c, stream, fn)) != FQ_OK) return rc;
+    return fq_swiglu(gate, up, (int64_t)M * N, y, stream);
 }

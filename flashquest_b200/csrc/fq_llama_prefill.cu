@@ -159,12 +159,16 @@ extern "C" int fq_llama_prefill(const fq_llama_model* m, const fq_int4_cache* c,
         }
         delta = w.delta;
         if ((rc = add_norm(L.post_norm, first, rows)) != FQ_OK) return rc;
-        {
+        if (rows <= 8) {
             const fq_awq_linear* ws[2] = {&L.gate, &L.up};
             void* y[2] = {w.gate, w.up};
             if ((rc = linears(m, w.normed, rows, S > 8, ws, 2, y, stream)) != FQ_OK) return rc;
+            if ((rc = fq_swiglu(w.gate, w.up, (int64_t)rows * m->ffn, w.act, stream)) != FQ_OK) return rc;
+        } else {
+            const int32_t* qw[2] = {L.gate.qweight, L.up.qweight}; const void* sc[2] = {L.gate.scales, L.up.scales};
+            const int32_t* qz[2] = {L.gate.qzeros, L.up.qzeros}; const void* bs[2] = {L.gate.bias, L.up.bias};
+            if ((rc = fq_awq_gate_up_swiglu(w.normed, rows, H, m->group, qw, sc, qz, bs, m->ffn, w.gate, w.up, w.act, m->interleaved, stream)) != FQ_OK) return rc;
         }
-        if ((rc = fq_swiglu(w.gate, w.up, (int64_t)rows * m->ffn, w.act, stream)) != FQ_OK) return rc;
         {
             const fq_awq_linear* ws[1] = {&L.down};
             void* y[1] = {w.delta + (size_t)first * H * 2};

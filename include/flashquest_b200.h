@@ -490,6 +490,14 @@ int fq_awq_gemm(
     const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
     const int* N, void* const* y, int interleaved, void* stream);
 
+/* The gate and up projections of an MLP and fq_swiglu behind them, with the results of fq_awq_gemm and fq_swiglu:
+ * y (M,N) = fp16(silu(x @ gate)) * (x @ up).  From the sizes on where fq_awq_gemm runs its large kernel that is one launch, and
+ * gate and up are not written; below, they are two launches through the buffers gate and up (M,N).  qweight, scales, qzeros,
+ * bias: arrays of two, gate first; sizes, alignments and dtypes as for fq_awq_gemm. */
+int fq_awq_gate_up_swiglu(
+    const void* x, int M, int K, int group, const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
+    int N, void* gate, void* up, void* y, int interleaved, void* stream);
+
 /* ------------------------------------------------------------------------------------
  * One decode step of one layer on a persistent INT4 cache: append + score + select + attend.
  * Replaces, in one host call and four launches, what the reference's patched forward does

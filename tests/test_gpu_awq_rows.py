@@ -74,6 +74,27 @@ def test_pair_tiles(M, K, Ns, group, interleaved, bias):
     assert all(torch.equal(a, b) for a, b in zip(got, awq_gemm_fused(x, lins)))
 
 
+@pytest.mark.parametrize("M", [1, 100, 257, 1025])
+@pytest.mark.parametrize("K,N,group,interleaved,bias", [(128, 9600, 64, True, True), (1152, 4992, 128, False, False), (256, 19200, 256, True, False)])
+def test_gate_up_with_swiglu_equals_its_parts(M, K, N, group, interleaved, bias):
+    """One launch (and, at few rows, two) gives the bits of the projections followed by fq_swiglu."""
+    import ctypes
+    from flashquest_b200._lib import check, lib, ptr, stream_ptr
+    from flashquest_b200.kernel.fused_proj import awq_gemm_fused
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    lins = [_linear(K, N, group, interleaved, bias, g) for _ in range(2)]
+    x = torch.randn(M, K, device="cuda", generator=g).half()
+    gate, up = awq_gemm_fused(x, lins)
+    want, got = torch.empty_like(gate), torch.empty_like(gate)
+    check(lib().fq_swiglu(ptr(gate), ptr(up), gate.numel(), ptr(want), stream_ptr(x.device)))
+    VP = ctypes.c_void_p * 2
+    arr = lambda name: VP(*[ptr(getattr(lin, name)) for lin in lins])
+    buf = [torch.empty_like(gate) for _ in range(2)]
+    check(lib().fq_awq_gate_up_swiglu(ptr(x), M, K, group, arr("qweight"), arr("scales"), arr("qzeros"), arr("bias") if bias else None, N,
+                                      ptr(buf[0]), ptr(buf[1]), ptr(got), int(interleaved), stream_ptr(x.device)))
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
 @pytest.mark.parametrize("M", [1100, 2048])
 def test_large_tiles_repeat(M):
     """More tiles than SMs: a CTA's second tile overlaps the epilogue of its first."""
