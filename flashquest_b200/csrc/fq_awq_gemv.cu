@@ -38,7 +38,6 @@ constexpr int GEMV_PACKS = 32;          // int32 column packs per CTA (256 outpu
 constexpr int GEMV_TILE = GEMV_PACKS * 8;
 constexpr int GEMV_MAX_PROJ = 4;
 constexpr int GEMV_ROWS = 128;          // rows per stage = largest group size
-constexpr int GEMV_STAGE_WORDS = GEMV_ROWS * GEMV_PACKS;
 constexpr int GEMV_MAX_STAGES = 6;       // ring depth: 3 (short K ranges) or 6 (long ones: more bytes in flight per CTA)
 constexpr int GEMV_MAX_CLUSTER = 8;
 
@@ -92,9 +91,6 @@ __device__ __forceinline__ void gemv_mma_16816(float (&c)[4], uint32_t a0, uint3
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// column (inside its pack of 8) of nibble i
-__device__ __forceinline__ int gemv_nibble_col(int i, int interleaved) { return interleaved ? ((i & 3) * 2 + (i >> 2)) : i; }
-
 // Shared memory (dynamic), in this order:
 //   s_w    [STAGES][ROWS][WSTRIDE] u32    weight ring; after the main loop: row-phase partial sums, then the CTA's tile
 //   s_x    M == 1: [range] float2 (x, x) * 2^100;  M > 1: [8][range + 8] fp16 (rows past the batch are zero)
@@ -105,14 +101,23 @@ __device__ __forceinline__ int gemv_nibble_col(int i, int interleaved) { return 
 // multiplies on the tensor cores with mma.sync m16n8k16: the 16 "rows" of an A fragment are the low and the
 // high nibble of one byte position of 8 neighbouring packs (lane group g owns pack 8*blk + g), its 16 k are 16
 // weight rows, B holds the 8 activation rows; a warp owns 8 packs and every second 16-row step of the group.
-template <int M, int GEMV_STAGES>
-__global__ void __launch_bounds__(GEMV_THREADS) awq_gemv_kernel(GemvParams p) {
+//
+// FAST: groups of 128, AutoAWQ's nibble order, 16-byte rows -- all of it known to the compiler: loops without counters,
+// shared-memory offsets in the instructions, no selects.  Bound by instruction issue (8192 -> 3072 at one row: 500 instructions
+// per warp and group, 0.88 us, of which 224 multiply; weights already in L2 change nothing), so that is what the variant saves.
+// q/k/v, o, gate/up, down of the Llama-3.2-3B shape, us: one row 6.6 / 5.2 / 12.5 / 10.6 -> 6.0 / 4.7 / 11.5 / 9.8; eight rows
+// 10.0 / 7.4 / 18.0 / 17.1 -> 8.5 / 6.3 / 15.1 / 13.9.
+// (Twice the warps with half the nibbles each is slower: 12.3 against 10.2 us at two rows, the loads of words and x double.)
+template <int M, int GEMV_STAGES, bool FAST>
+__global__ void __launch_bounds__(GEMV_THREADS, 3) awq_gemv_kernel(GemvParams p) {
     constexpr bool MMA = M > 1;
+    const bool interleaved = FAST || p.interleaved, vec16 = FAST || p.vec16;
     constexpr int WSTRIDE = MMA ? GEMV_PACKS + 4 : GEMV_PACKS;     // +4 words: the fragment loads of 4 rows x 8 packs hit 32 banks
     constexpr int STAGE_WORDS = GEMV_ROWS * WSTRIDE;
     extern __shared__ __align__(16) unsigned char s_raw[];
     cg::cluster_group cluster = cg::this_cluster();
-    const int range = p.groups_per_split * p.group;
+    const int G = FAST ? 128 : p.group;
+    const int range = p.groups_per_split * G;
     const int xstride = range + 8;                                 // fp16 row stride of s_xh (M > 1)
     uint32_t* s_w = reinterpret_cast<uint32_t*>(s_raw);
     unsigned char* x_base = s_raw + (size_t)GEMV_STAGES * STAGE_WORDS * 4;
@@ -135,7 +140,6 @@ __global__ void __launch_bounds__(GEMV_THREADS) awq_gemv_kernel(GemvParams p) {
     const int g_begin = split * p.groups_per_split;
     const int g_end = min(p.n_groups, g_begin + p.groups_per_split);
     const int n_chunks = max(g_end - g_begin, 0);
-    const int G = p.group;
     const int k0 = g_begin * G, k_len = n_chunks * G;
 
     // weights of a chunk (they never change: safe to request before the previous kernel is done)
@@ -143,27 +147,33 @@ __global__ void __launch_bounds__(GEMV_THREADS) awq_gemv_kernel(GemvParams p) {
         const int g = g_begin + chunk, st = chunk % GEMV_STAGES;
         uint32_t* dst = s_w + st * STAGE_WORDS;
         const int32_t* src = pr.qweight + (int64_t)g * G * npk + pk0;
-        if (p.vec16) {
-            // 256 threads = 32 rows x 8 pieces of 16 bytes: a thread keeps its piece and walks down the rows
+        if (vec16) {
+            // 8 pieces of 16 bytes per row: a thread keeps its piece and walks down the rows
             const int r0 = tid >> 3, q = tid & 7;
             if (pk0 + q * 4 < npk) {
                 uint32_t* d = dst + r0 * WSTRIDE + q * 4;
                 const int32_t* sp = src + (int64_t)r0 * npk + q * 4;
-                for (int r = r0; r < G; r += 32, d += 32 * WSTRIDE, sp += 32 * (int64_t)npk) cp_async16(d, sp);
+                if constexpr (FAST) {
+#pragma unroll
+                    for (int i = 0; i < 128 * 8 / GEMV_THREADS; ++i) cp_async16(d + i * (GEMV_THREADS / 8) * WSTRIDE, sp + i * (GEMV_THREADS / 8) * (int64_t)npk);
+                } else {
+                    for (int r = r0; r < G; r += GEMV_THREADS / 8, d += GEMV_THREADS / 8 * WSTRIDE, sp += GEMV_THREADS / 8 * (int64_t)npk) cp_async16(d, sp);
+                }
             }
         } else {
             const int r0 = tid >> 5, q = tid & 31;
             if (pk0 + q < npk) {
                 uint32_t* d = dst + r0 * WSTRIDE + q;
                 const int32_t* sp = src + (int64_t)r0 * npk + q;
-                for (int r = r0; r < G; r += 8, d += 8 * WSTRIDE, sp += 8 * (int64_t)npk) cp_async4(d, sp);
+                for (int r = r0; r < G; r += GEMV_WARPS, d += GEMV_WARPS * WSTRIDE, sp += GEMV_WARPS * (int64_t)npk) cp_async4(d, sp);
             }
         }
     };
-    // staged input element kk (inside the CTA's K range) of row m
+    // staged input element kk (inside the CTA's K range) of row m.  M == 1: the 16 rows of a phase of a group side by side
+    auto x_at = [&](int kk) { return FAST ? (kk & ~127) + (kk & 7) * 16 + ((kk & 127) >> 3) : kk; };
     auto put_x = [&](int kk, int m, __half h) {
         if constexpr (MMA) s_xh[m * xstride + kk] = h;
-        else { const float vs = __half2float(h) * 1.2676506002282294e30f; s_xs[kk] = make_float2(vs, vs); }
+        else { const float vs = __half2float(h) * 1.2676506002282294e30f; s_xs[x_at(kk)] = make_float2(vs, vs); }
     };
 
     cluster.barrier_arrive();          // matched by the wait in front of the first access to another CTA's shared memory
@@ -212,7 +222,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) awq_gemv_kernel(GemvParams p) {
                         const float2 f = __half22float2(ah[j]);
                         ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
                         if constexpr (!MMA) {
-                            if (mine) { s_xs[kk + 2 * j] = make_float2(f.x, 0.f); s_xs[kk + 2 * j + 1] = make_float2(f.y, 0.f); }
+                            if (mine) { s_xs[x_at(kk + 2 * j)].x = f.x; s_xs[x_at(kk + 2 * j + 1)].x = f.y; }
                         }
                     }
                 }
@@ -224,7 +234,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) awq_gemv_kernel(GemvParams p) {
         for (int i = tid; i < p.M * k_len; i += GEMV_THREADS) {
             const int m = i / k_len, kk = i - m * k_len;
             float hv;
-            if constexpr (MMA) hv = __half2float(s_xh[m * xstride + kk]); else hv = s_xs[kk].x;
+            if constexpr (MMA) hv = __half2float(s_xh[m * xstride + kk]); else hv = s_xs[x_at(kk)].x;
             const __half xh = __float2half_rn(hv * s_rstd[m]);
             put_x(kk, m, __hmul(p.pro_weight[k0 + kk], xh));
         }
@@ -254,26 +264,37 @@ __global__ void __launch_bounds__(GEMV_THREADS) awq_gemv_kernel(GemvParams p) {
         }
     }
     __syncthreads();
-    // sum of x per group and row (fixed order): a warp per (group, row), lanes stride the group
-    for (int gm = warp; gm < n_chunks * M; gm += GEMV_WARPS) {
-        const int ch = gm / M, m = gm % M;
-        float s = 0.f;
-        for (int r = lane; r < G; r += 32) {
-            if constexpr (MMA) s += __half2float(s_xh[m * xstride + ch * G + r]);
-            else s += s_xs[ch * G + r].x * 7.888609052210118e-31f;            // * 2^-100 (exact)
+    // sum of x per group and row (fixed order): XQ (group, row) at a time per warp, lanes stride the group
+    constexpr int XQ = MMA ? 4 : 1;
+    for (int gm0 = XQ * warp; gm0 < n_chunks * M; gm0 += XQ * GEMV_WARPS) {
+        float s[XQ];
+#pragma unroll
+        for (int q = 0; q < XQ; ++q) {
+            const int gm = min(gm0 + q, n_chunks * M - 1), ch = gm / M, m = gm % M;
+            s[q] = 0.f;
+#pragma unroll 4
+            for (int r = lane; r < G; r += 32) {
+                if constexpr (MMA) s[q] += __half2float(s_xh[m * xstride + ch * G + r]);
+                else s[q] += s_xs[x_at(ch * G + r)].x * 7.888609052210118e-31f;      // * 2^-100 (exact)
+            }
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) s_xsum[gm] = s;
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < XQ; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+#pragma unroll
+        for (int q = 0; q < XQ; ++q)
+            if (lane == 0 && gm0 + q < n_chunks * M) s_xsum[gm0 + q] = s[q];
     }
 
     // this thread's pack: one per lane (M == 1), one per lane group of the warp's 8-pack block (M > 1)
     const int g8 = lane >> 2, t4 = lane & 3;
-    const int blk = warp & 3, kh = warp >> 2;
+    const int blk = warp & 3, kh = warp >> 2;                // M > 1; M == 1: the warp is the row phase
     const int lpk = MMA ? blk * 8 + g8 : lane;               // pack inside the tile
     const int c = pk0 + lpk;
     const bool valid = c < npk;
     constexpr int NACC = MMA ? 16 : 8;                       // M == 1: [nibble]; M > 1: [nibble][row 2*t4 + {0, 1}]
+    auto col_of = [&](int i) { return interleaved ? (i & 3) * 2 + (i >> 2) : i; };       // column (inside its pack of 8) of nibble i
     float yacc[NACC];
 #pragma unroll
     for (int j = 0; j < NACC; ++j) yacc[j] = 0.f;
@@ -298,121 +319,141 @@ __global__ void __launch_bounds__(GEMV_THREADS) awq_gemv_kernel(GemvParams p) {
         }
         const uint32_t* sw = s_w + st * STAGE_WORDS;
         // (scale and zero are first touched after the multiply loop, so their load stays in flight behind it)
-        auto scales_f32 = [&](float (&scol)[8]) {
-            const __half2* sch = reinterpret_cast<const __half2*>(&sc8);
+        auto scales_f32 = [&](float (&scol)[8]) {        // in nibble order; selects of registers, not an indexed array
+            const uint32_t w[4] = {sc8.x, sc8.y, sc8.z, sc8.w};          // columns 2j, 2j+1 of the pack in word j
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { const float2 t = __half22float2(sch[j]); scol[2 * j] = t.x; scol[2 * j + 1] = t.y; }
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t pair = interleaved ? w[i & 3] : w[i >> 1];
+                scol[i] = __half2float(__ushort_as_half((unsigned short)((interleaved ? i >> 2 : i & 1) ? pair >> 16 : pair & 0xffffu)));
+            }
         };
         if constexpr (!MMA) {
             float2 acc[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[j] = make_float2(0.f, 0.f);
-            const uint32_t* wcol = sw + lane;
-            const float2* xs = s_xs + (size_t)ch * G;
-#pragma unroll 4
-            for (int r = warp; r < G; r += GEMV_WARPS) {
-                const uint32_t w = wcol[r * WSTRIDE];
-                float2 f[4];
-                f[0] = make_float2(__uint_as_float(w & 0x0000000fu), __uint_as_float(w & 0x000000f0u));
-                f[1] = make_float2(__uint_as_float(w & 0x00000f00u), __uint_as_float(w & 0x0000f000u));
-                f[2] = make_float2(__uint_as_float(w & 0x000f0000u), __uint_as_float(w & 0x00f00000u));
-                f[3] = make_float2(__uint_as_float(w >> 24), __uint_as_float(w >> 28));
-                const float2 xx = xs[r];
+            const uint32_t* wcol = sw + lane + warp * WSTRIDE;
+            auto row = [&](uint32_t w, float2 xx) {
+                acc[0] = __ffma2_rn(make_float2(__uint_as_float(w & 0x0000000fu), __uint_as_float(w & 0x000000f0u)), xx, acc[0]);
+                acc[1] = __ffma2_rn(make_float2(__uint_as_float(w & 0x00000f00u), __uint_as_float(w & 0x0000f000u)), xx, acc[1]);
+                acc[2] = __ffma2_rn(make_float2(__uint_as_float(w & 0x000f0000u), __uint_as_float(w & 0x00f00000u)), xx, acc[2]);
+                acc[3] = __ffma2_rn(make_float2(__uint_as_float(w >> 24), __uint_as_float(w >> 28)), xx, acc[3]);
+            };
+            if constexpr (FAST) {
+                const float4* xs = reinterpret_cast<const float4*>(s_xs + (size_t)ch * 128 + warp * 16);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[j] = __ffma2_rn(f[j], xx, acc[j]);
+                for (int i = 0; i < 8; ++i) {
+                    const float4 xx = xs[i];               // rows warp + 16 i and warp + 16 i + 8
+                    row(wcol[(16 * i) * WSTRIDE], make_float2(xx.x, xx.y));
+                    row(wcol[(16 * i + 8) * WSTRIDE], make_float2(xx.z, xx.w));
+                }
+            } else {
+                const float2* xs = s_xs + (size_t)ch * G + warp;
+#pragma unroll 4
+                for (int r = 0; r < G; r += GEMV_WARPS) row(wcol[r * WSTRIDE], xs[r]);
             }
             // undo the nibble-position powers of two, then apply zero and scale of this group
-            float scol[8];
+            float scol[8], a[8];
             scales_f32(scol);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const float scv = p.interleaved ? scol[(i & 3) * 2 + (i >> 2)] : scol[i];   // a select of two registers, not an indexed array
-                // zero of nibble i, same in-place trick: (z & mask) as fp32 is zero * 2^(4i-149)
-                const float zero = i < 6 ? __uint_as_float(z & (0xfu << (4 * i))) * pow2f_i(100 - 4 * i) * pow2f_i(49)
-                                         : __uint_as_float(i == 6 ? ((z >> 24) & 15u) : (z >> 28)) * pow2f_i(100) * pow2f_i(49);
                 const float ai = (i & 1) ? acc[i >> 1].y : acc[i >> 1].x;
-                float a;
-                if (i <= 5) a = ai * pow2f_i(49 - 4 * i);
-                else if (i == 6) a = fmaf(-16.f, acc[3].y, ai) * pow2f_i(49);
-                else a = ai * pow2f_i(49);
-                // the zero term belongs to the group once, not once per row phase
-                const float zterm = warp == 0 ? zero * s_xsum[ch] : 0.f;
-                yacc[i] = fmaf(scv, a - zterm, yacc[i]);     // kept in nibble order until the columns are written
+                if (i <= 5) a[i] = ai * pow2f_i(49 - 4 * i);
+                else if (i == 6) a[i] = fmaf(-16.f, acc[3].y, ai) * pow2f_i(49);
+                else a[i] = ai * pow2f_i(49);
             }
+            if (warp == 0) {           // the zero term belongs to the group once, not once per row phase
+                const float xsum = s_xsum[ch];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) a[i] -= __fmul_rn((float)((z >> (4 * i)) & 15u), xsum);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) yacc[i] = fmaf(scol[i], a[i], yacc[i]);     // kept in nibble order until the columns are written
         } else {
             float cf[4][4];
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) cf[j][e] = 0.f;
-            const uint32_t* wp = sw + lpk;
-            const __half* xrow = s_xh + g8 * xstride + ch * G + 2 * t4;
-            for (int ks = kh; ks < G / 16; ks += 2) {
-                const int r = ks * 16 + 2 * t4;
-                const uint32_t wa = wp[r * WSTRIDE], wb = wp[(r + 1) * WSTRIDE], wc = wp[(r + 8) * WSTRIDE], wd = wp[(r + 9) * WSTRIDE];
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(xrow + ks * 16);
-                const uint32_t b1 = *reinterpret_cast<const uint32_t*>(xrow + ks * 16 + 8);
+            const uint32_t* wp = sw + lpk + (16 * kh + 2 * t4) * WSTRIDE;
+            const __half* xrow = s_xh + g8 * xstride + ch * G + 16 * kh + 2 * t4;
+            const __half2 k1024 = __float2half2_rn(1024.f), k64 = __float2half2_rn(-64.f), k16th = __float2half2_rn(0.0625f);
+            auto step = [&](const uint32_t* wr, const __half* xr) {
+                const uint32_t wa = wr[0], wb = wr[WSTRIDE], wc = wr[8 * WSTRIDE], wd = wr[9 * WSTRIDE];
+                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(xr);
+                const uint32_t b1 = *reinterpret_cast<const uint32_t*>(xr + 8);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    // byte j of the two rows side by side: halves (row r, row r+1); low nibble = nibble 2j, high = 2j+1
-                    const uint32_t sel = (uint32_t)((4 + j) << 12 | (4 + j) << 8 | j << 4 | j);
+                    // byte j of the two rows side by side: halves (row r, row r+1); low nibble h = 1024 + code, high nibble
+                    // h = 1024 + 16 code: minus 1024, and times 1/16 minus 64, both exact
+                    const uint32_t sel = (4 + j) * 0x1100u + j * 0x11u;
                     const uint32_t v1 = __byte_perm(wa, wb, sel), v2 = __byte_perm(wc, wd, sel);
-                    const __half2 k1024 = __half2half2(__ushort_as_half((unsigned short)0x6400));
-                    uint32_t a0 = (v1 & 0x000f000fu) | 0x64006400u, a1 = ((v1 >> 4) & 0x000f000fu) | 0x64006400u;
-                    uint32_t a2 = (v2 & 0x000f000fu) | 0x64006400u, a3 = ((v2 >> 4) & 0x000f000fu) | 0x64006400u;
-                    __half2 h0 = __hsub2(*reinterpret_cast<__half2*>(&a0), k1024), h1 = __hsub2(*reinterpret_cast<__half2*>(&a1), k1024);
-                    __half2 h2 = __hsub2(*reinterpret_cast<__half2*>(&a2), k1024), h3 = __hsub2(*reinterpret_cast<__half2*>(&a3), k1024);
+                    uint32_t a0 = (v1 & 0x000f000fu) | 0x64006400u, a1 = (v1 & 0x00f000f0u) | 0x64006400u;
+                    uint32_t a2 = (v2 & 0x000f000fu) | 0x64006400u, a3 = (v2 & 0x00f000f0u) | 0x64006400u;
+                    __half2 h0 = __hsub2(*reinterpret_cast<__half2*>(&a0), k1024), h1 = __hfma2(*reinterpret_cast<__half2*>(&a1), k16th, k64);
+                    __half2 h2 = __hsub2(*reinterpret_cast<__half2*>(&a2), k1024), h3 = __hfma2(*reinterpret_cast<__half2*>(&a3), k16th, k64);
                     gemv_mma_16816(cf[j], *reinterpret_cast<uint32_t*>(&h0), *reinterpret_cast<uint32_t*>(&h1),
                                    *reinterpret_cast<uint32_t*>(&h2), *reinterpret_cast<uint32_t*>(&h3), b0, b1);
                 }
+            };
+            if constexpr (FAST) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) step(wp + 32 * i * WSTRIDE, xrow + 32 * i);
+            } else {
+                for (int ks = kh; ks < G / 16; ks += 2) step(wp + 16 * (ks - kh) * WSTRIDE, xrow + 16 * (ks - kh));
             }
-            // cf[j] = {nibble 2j x rows (2t, 2t+1), nibble 2j+1 x rows (2t, 2t+1)}: sum over this warp's rows of x * code
-            const float xs0 = kh == 0 ? s_xsum[ch * M + min(2 * t4, M - 1)] : 0.f;
-            const float xs1 = kh == 0 ? s_xsum[ch * M + min(2 * t4 + 1, M - 1)] : 0.f;
+            // cf[j] = {low nibble x rows (2t, 2t+1), high nibble x rows (2t, 2t+1)} of a byte: sum over this warp's rows of x * code
             float scol[8];
             scales_f32(scol);
+            if (kh == 0) {             // the zero term belongs to the group once
+                const float xs0 = s_xsum[ch * M + min(2 * t4, M - 1)], xs1 = s_xsum[ch * M + min(2 * t4 + 1, M - 1)];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float zero = __uint_as_float(((z >> (4 * i)) & 15u) | 0x4b000000u) - 8388608.f;      // exact, one conversion less
+                    cf[i >> 1][(i & 1) * 2] = fmaf(-zero, xs0, cf[i >> 1][(i & 1) * 2]);
+                    cf[i >> 1][(i & 1) * 2 + 1] = fmaf(-zero, xs1, cf[i >> 1][(i & 1) * 2 + 1]);
+                }
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const float scv = p.interleaved ? scol[(i & 3) * 2 + (i >> 2)] : scol[i];   // a select of two registers, not an indexed array
-                const float zero = (float)((z >> (4 * i)) & 15u);
-                yacc[2 * i] = fmaf(scv, cf[i >> 1][(i & 1) * 2] - zero * xs0, yacc[2 * i]);
-                yacc[2 * i + 1] = fmaf(scv, cf[i >> 1][(i & 1) * 2 + 1] - zero * xs1, yacc[2 * i + 1]);
+                yacc[2 * i] = fmaf(scol[i], cf[i >> 1][(i & 1) * 2], yacc[2 * i]);
+                yacc[2 * i + 1] = fmaf(scol[i], cf[i >> 1][(i & 1) * 2 + 1], yacc[2 * i + 1]);
             }
         }
     }
     cp_async_wait<0>();
     // ---- the CTA's tile: add the row phases through shared memory, lay the columns out in order ----
     __syncthreads();
-    float* s_red = reinterpret_cast<float*>(s_raw);                    // row-phase partial sums
-    float* s_part = s_red + (GEMV_WARPS - 1) * 32 * NACC;              // [M][TILE] the CTA's partial tile
-    constexpr int NRED = MMA ? 4 : GEMV_WARPS - 1;                     // warps that hand their sums over
-    const int first_keep = MMA ? 4 : 1;                                // warps >= first_keep hand over (M > 1: the second k half)
-    if (warp >= first_keep) {
+    // M == 1: phases 1 .. 7 hand their sums to phase 0; M > 1: the second k half hands them to the first
+    float* s_red = reinterpret_cast<float*>(s_raw);                    // sums handed over
+    float* s_part = s_red + (MMA ? 4 : GEMV_WARPS - 1) * 32 * NACC;            // [M][TILE] the CTA's partial tile
+    const bool keep = MMA ? kh == 0 : warp == 0;
+    const int row = MMA ? blk : warp - 1;                              // of the hand-over area (M > 1: the same for both k halves)
+    if (!keep) {
 #pragma unroll
         for (int j = 0; j < NACC; j += 4)
-            *reinterpret_cast<float4*>(s_red + ((warp - first_keep) * 32 + lane) * NACC + j) = make_float4(yacc[j], yacc[j + 1], yacc[j + 2], yacc[j + 3]);
+            *reinterpret_cast<float4*>(s_red + (row * 32 + lane) * NACC + j) = make_float4(yacc[j], yacc[j + 1], yacc[j + 2], yacc[j + 3]);
     }
     __syncthreads();
     cluster.barrier_wait();            // every CTA of the cluster runs: its shared memory may be addressed
-    if (warp < first_keep) {
+    if (keep) {
         if constexpr (!MMA) {
 #pragma unroll
-            for (int k = 0; k < NRED; ++k)
+            for (int k = 0; k < GEMV_WARPS - 1; ++k)
 #pragma unroll
                 for (int j = 0; j < NACC; ++j) yacc[j] += s_red[(k * 32 + lane) * NACC + j];
             // one row: the lane's 8 columns go straight from registers into slot [split] of the first CTA
             float cv[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) cv[j] = p.interleaved ? yacc[(j >> 1) + (j & 1) * 4] : yacc[j];
+            for (int j = 0; j < 8; ++j) cv[j] = interleaved ? yacc[(j >> 1) + (j & 1) * 4] : yacc[j];
             float4* d = reinterpret_cast<float4*>(cluster.map_shared_rank(s_slot, 0) + (size_t)split * GEMV_TILE + lane * 8);
             d[0] = make_float4(cv[0], cv[1], cv[2], cv[3]);
             d[1] = make_float4(cv[4], cv[5], cv[6], cv[7]);
         } else {
 #pragma unroll
-            for (int j = 0; j < NACC; ++j) yacc[j] += s_red[(warp * 32 + lane) * NACC + j];    // warp + 4 holds the other k half of this block
+            for (int j = 0; j < NACC; ++j) yacc[j] += s_red[(row * 32 + lane) * NACC + j];    // the other k half of this block
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const int col = lpk * 8 + gemv_nibble_col(i, p.interleaved);
+                const int col = lpk * 8 + col_of(i);
                 if (2 * t4 < M) s_part[(2 * t4) * GEMV_TILE + col] = yacc[2 * i];
                 if (2 * t4 + 1 < M) s_part[(2 * t4 + 1) * GEMV_TILE + col] = yacc[2 * i + 1];
             }
@@ -569,6 +610,9 @@ extern "C" int fq_awq_gemv_fused(
         k_split *= 2;
     }
     p.k_split = k_split;
+    // Two CTAs per SM at most where two hold the launch: clusters are placed where they fit, and with room for a third some SMs
+    // got three and others one (256 CTAs of 3072 -> 16384 at 8 rows: 18.9 us, 15.1 with the room taken)
+    if ((int64_t)tiles * k_split > sm_count() && (int64_t)tiles * k_split <= 2LL * sm_count() && smem < 76 * 1024) smem = 76 * 1024;
     FQ_CHECK_ARG(((p.head_dim > 0 ? p.head_dim : 128) / 2) % (4 * (Mp == 8 ? k_split : 1)) == 0, FQ_ERR_UNSUPPORTED,
                  "%s: head_dim %d with %d-way split-K", fn, p.head_dim, k_split);
     FQ_CHECK_ARG(smem <= 226 * 1024, FQ_ERR_UNSUPPORTED, "%s: K=%d with %d rows needs %zu B of shared memory per CTA", fn, K, M, smem);
@@ -581,18 +625,23 @@ extern "C" int fq_awq_gemv_fused(
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = pdl_enabled(PDL_GEMV) ? 2 : 1;
-#define FQ_GEMV(MV, SV)                                                                                      \
+#define FQ_GEMV(MV, SV, FV)                                                                                  \
     do {                                                                                                     \
         static std::atomic<size_t> attr_smem[64];                                                            \
         int dev = 0; cudaGetDevice(&dev);                                                                    \
         if (dev < 0 || dev >= 64 || attr_smem[dev].load(std::memory_order_acquire) < smem) {                 \
-            cudaError_t e = cudaFuncSetAttribute(awq_gemv_kernel<MV, SV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            cudaError_t e = cudaFuncSetAttribute(awq_gemv_kernel<MV, SV, FV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: cannot reserve %zu B of shared memory: %s", fn, smem, cudaGetErrorString(e)); \
             if (dev >= 0 && dev < 64) attr_smem[dev].store(smem, std::memory_order_release);                 \
         }                                                                                                    \
-        cudaLaunchKernelEx(&cfg, awq_gemv_kernel<MV, SV>, p);                                                \
+        cudaLaunchKernelEx(&cfg, awq_gemv_kernel<MV, SV, FV>, p);                                            \
     } while (0)
-#define FQ_GEMV_M(MV) do { if (stages == 3) FQ_GEMV(MV, 3); else FQ_GEMV(MV, GEMV_MAX_STAGES); } while (0)
+    const bool fast = group == 128 && interleaved && vec16;
+#define FQ_GEMV_M(MV)                                                                                   \
+    do {                                                                                                \
+        if (fast) { if (stages == 3) FQ_GEMV(MV, 3, true); else FQ_GEMV(MV, GEMV_MAX_STAGES, true); }   \
+        else { if (stages == 3) FQ_GEMV(MV, 3, false); else FQ_GEMV(MV, GEMV_MAX_STAGES, false); }      \
+    } while (0)
     if (Mp == 1) FQ_GEMV_M(1);
     else if (Mp == 2) FQ_GEMV_M(2);
     else if (Mp == 4) FQ_GEMV_M(4);

@@ -124,6 +124,27 @@ def test_gemv_splits_and_tiles(M, K, Ns, interleaved, bias):
     assert all(torch.equal(a, b) for a, b in zip(got, awq_gemv_fused(x, lins)))
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("K,Ns", [(128, (32,)), (1152, (384, 96)), (8192, (512,)), (3072, (9600, 1024))])
+def test_gemv_of_known_layout_gives_the_bits_of_the_general_one(M, K, Ns):
+    """Groups of 128 in AutoAWQ's order on 16-byte rows take loops that the compiler knows the sizes of; the same weights four
+    bytes off take the general ones."""
+    from flashquest_b200.kernel.fused_proj import awq_gemv_fused
+    from flashquest_b200.quant import AWQLinear
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    lins = [_linear(K, N, 128, True, True, g) for N in Ns]
+
+    def shifted(t):
+        buf = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view_as(t)
+        return buf.copy_(t)
+    odd = [AWQLinear(shifted(lin.qweight), lin.scales, lin.qzeros, lin.bias, group_size=128, interleaved=True) for lin in lins]
+    assert all(lin.qweight.data_ptr() % 16 == 4 for lin in odd)
+    x, u = (torch.randn(M, K, device="cuda", generator=g).half() for _ in range(2))
+    for kw in ({}, dict(swiglu_up=u), dict(add=u, norm_weight=u[0], return_sum=True)):
+        for a, b in zip(awq_gemv_fused(x, lins, **kw), awq_gemv_fused(x, odd, **kw)):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
 @pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (8, 3072), (2, 8192)])
 def test_norm_equals_general_kernel(rows, H):
     """Rows 16 bytes at a time give the bits of the value-by-value kernel, which unaligned rows take."""
