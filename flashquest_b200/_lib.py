@@ -119,6 +119,7 @@ GEMV_PLAIN, GEMV_ADD_RMSNORM, GEMV_SWIGLU = 0, 1, 2
 _PROTOTYPES["fq_awq_gemv_default_splits"] = (I, [I, I, I])
 _PROTOTYPES["fq_awq_gemv"] = (I, [P, I, I, I, I, P, P, P, P, P, P, I, I, P])
 _PROTOTYPES["fq_awq_gemv_fused"] = (I, [P, I, I, I, I, P, P, P, P, P, P, I, ctypes.POINTER(GemvPrologue), ctypes.POINTER(GemvRope), I, P])
+_PROTOTYPES["fq_awq_gemv_swiglu"] = (I, [P, I, I, I, P, P, P, P, I, P, I, ctypes.POINTER(GemvPrologue), I, P])
 _PROTOTYPES["fq_awq_gate_up_swiglu"] = (I, [P, I, I, I, P, P, P, P, I, P, P, P, I, P])
 _PROTOTYPES["fq_awq_gemm"] = (I, [P, I, I, I, I, P, P, P, P, P, P, I, P])
 _PROTOTYPES["fq_wht"] = (I, [P, P, I, L, I, P])

@@ -59,6 +59,8 @@ struct GemvParams {
     const __half* pro_b; const __half* pro_weight; float eps; __half* pro_out;
     // rotary embedding
     const int* pos_dev; int pos; float theta; int head_dim;
+    // projections 0 and 1 are the gate and the up projection: a tile is 128 columns of each, y[0] = fp16(silu(gate)) * up
+    int swiglu_out;
 };
 
 __device__ __forceinline__ float pow2f_i(int n) { return __int_as_float((127 + n) << 23); }
@@ -136,21 +138,25 @@ __global__ void __launch_bounds__(GEMV_THREADS, 3) awq_gemv_kernel(GemvParams p)
         if (i < p.n_proj && tile >= p.proj[i].tile0) pi = i;
     const GemvProj pr = p.proj[pi];
     const int npk = pr.N / 8;
-    const int pk0 = (tile - pr.tile0) * GEMV_PACKS;          // first pack of the tile inside the projection
+    const int tile_packs = p.swiglu_out ? GEMV_PACKS / 2 : GEMV_PACKS;
+    const int pk0 = (tile - pr.tile0) * tile_packs;          // first pack of the tile inside the projection
     const int g_begin = split * p.groups_per_split;
     const int g_end = min(p.n_groups, g_begin + p.groups_per_split);
     const int n_chunks = max(g_end - g_begin, 0);
     const int k0 = g_begin * G, k_len = n_chunks * G;
 
     // weights of a chunk (they never change: safe to request before the previous kernel is done)
+    const int w_half = vec16 ? (tid & 7) >> 2 : (tid & 31) >> 4;         // of the tile that this thread copies from
+    const int32_t* w_src = p.swiglu_out && w_half ? p.proj[1].qweight - GEMV_PACKS / 2 : pr.qweight;
+    const int w_end = p.swiglu_out && w_half ? npk + GEMV_PACKS / 2 : npk;
     auto issue_w = [&](int chunk) {
         const int g = g_begin + chunk, st = chunk % GEMV_STAGES;
         uint32_t* dst = s_w + st * STAGE_WORDS;
-        const int32_t* src = pr.qweight + (int64_t)g * G * npk + pk0;
+        const int32_t* src = w_src + (int64_t)g * G * npk + pk0;
         if (vec16) {
             // 8 pieces of 16 bytes per row: a thread keeps its piece and walks down the rows
             const int r0 = tid >> 3, q = tid & 7;
-            if (pk0 + q * 4 < npk) {
+            if (pk0 + q * 4 < w_end) {
                 uint32_t* d = dst + r0 * WSTRIDE + q * 4;
                 const int32_t* sp = src + (int64_t)r0 * npk + q * 4;
                 if constexpr (FAST) {
@@ -162,7 +168,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 3) awq_gemv_kernel(GemvParams p)
             }
         } else {
             const int r0 = tid >> 5, q = tid & 31;
-            if (pk0 + q < npk) {
+            if (pk0 + q < w_end) {
                 uint32_t* d = dst + r0 * WSTRIDE + q;
                 const int32_t* sp = src + (int64_t)r0 * npk + q;
                 for (int r = r0; r < G; r += GEMV_WARPS, d += GEMV_WARPS * WSTRIDE, sp += GEMV_WARPS * (int64_t)npk) cp_async4(d, sp);
@@ -291,8 +297,11 @@ __global__ void __launch_bounds__(GEMV_THREADS, 3) awq_gemv_kernel(GemvParams p)
     const int g8 = lane >> 2, t4 = lane & 3;
     const int blk = warp & 3, kh = warp >> 2;                // M > 1; M == 1: the warp is the row phase
     const int lpk = MMA ? blk * 8 + g8 : lane;               // pack inside the tile
-    const int c = pk0 + lpk;
+    const bool second = p.swiglu_out && lpk >= GEMV_PACKS / 2;            // a pack of the up projection
+    const int c = pk0 + lpk - (second ? GEMV_PACKS / 2 : 0);
     const bool valid = c < npk;
+    const int32_t* qz = second ? p.proj[1].qzeros : pr.qzeros;
+    const __half* scl = second ? p.proj[1].scales : pr.scales;
     constexpr int NACC = MMA ? 16 : 8;                       // M == 1: [nibble]; M > 1: [nibble][row 2*t4 + {0, 1}]
     auto col_of = [&](int i) { return interleaved ? (i & 3) * 2 + (i >> 2) : i; };       // column (inside its pack of 8) of nibble i
     float yacc[NACC];
@@ -304,8 +313,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 3) awq_gemv_kernel(GemvParams p)
         // scale and zero of this group: issued before the wait so that they are in flight with it
         uint32_t z = 0; uint4 sc8 = make_uint4(0, 0, 0, 0);
         if (valid) {
-            z = (uint32_t)__ldg(pr.qzeros + (int64_t)g * npk + c);
-            sc8 = __ldg(reinterpret_cast<const uint4*>(pr.scales + (int64_t)g * pr.N + c * 8));
+            z = (uint32_t)__ldg(qz + (int64_t)g * npk + c);
+            sc8 = __ldg(reinterpret_cast<const uint4*>(scl + (int64_t)g * pr.N + c * 8));
         }
         // groups committed so far: chunks 0 .. max(STAGES - 1, ch + STAGES - 2); chunk ch must have landed
         if (ch == 0) cp_async_wait<GEMV_STAGES - 1>(); else cp_async_wait<GEMV_STAGES - 2>();
@@ -479,7 +488,25 @@ __global__ void __launch_bounds__(GEMV_THREADS, 3) awq_gemv_kernel(GemvParams p)
     }
     cluster.sync();                    // every partial sum has arrived at its owner
     if (!SCATTER && split != 0) return;
-    // ---- owner: add the splits in rank order, bias, rounding, rotary embedding, store ----
+    // ---- owner: add the splits in rank order, bias, rounding, rotary embedding or SwiGLU, store ----
+    if (p.swiglu_out) {
+        // gate column j and up column j lie half a tile apart, which the pieces keep
+        const int half_n = own_n / 2;
+        const __half *gb = pr.bias, *ub = p.proj[1].bias;
+        for (int i = tid; i < p.M * half_n; i += GEMV_THREADS) {
+            const int m = i / half_n, loc = i - m * half_n;
+            const int n = pk0 * 8 + (loc / pw) * period + split * pw + loc % pw;
+            if (n >= pr.N) continue;
+            const float* sl = s_slot + (size_t)m * own_n + loc;
+            float gv = 0.f, uv = 0.f;
+            for (int s = 0; s < ks_n; ++s) { gv += sl[(size_t)s * M * own_n]; uv += sl[(size_t)s * M * own_n + half_n]; }
+            if (gb) gv += __half2float(gb[n]);
+            if (ub) uv += __half2float(ub[n]);
+            const float f = __half2float(__float2half_rn(gv));
+            pr.y[(int64_t)m * pr.N + n] = __hmul(__float2half_rn(f / (1.0f + expf(-f))), __float2half_rn(uv));
+        }
+        return;
+    }
     __half* s_y = reinterpret_cast<__half*>(s_raw);                    // [M][own_n] fp16 (the ring is free)
     for (int i = tid; i < M * own_n; i += GEMV_THREADS) {
         const int m = i / own_n, loc = i - m * own_n;
@@ -534,10 +561,10 @@ extern "C" int fq_awq_gemv_default_splits(int K, int N_total, int group) {
     return ks;
 }
 
-extern "C" int fq_awq_gemv_fused(
+static int gemv_launch(
     const void* x, int M, int K, int group, int n_proj,
     const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
-    const int* N, void* const* y, int interleaved, const fq_gemv_prologue* pro, const fq_gemv_rope* rope, int k_split, void* stream) {
+    const int* N, void* const* y, int interleaved, const fq_gemv_prologue* pro, const fq_gemv_rope* rope, bool swiglu_out, int k_split, void* stream) {
     using namespace fq;
     const char* fn = "fq_awq_gemv";
     FQ_CHECK_ARG(M >= 1 && M <= 8, FQ_ERR_UNSUPPORTED, "%s: M=%d rows; the GEMV path takes 1..8 (larger M belongs to the GEMM path)", fn, M);
@@ -584,7 +611,10 @@ extern "C" int fq_awq_gemv_fused(
         if (q.rope) FQ_CHECK_ARG(N[i] % rope->head_dim == 0, FQ_ERR_ARG, "%s: N[%d]=%d is not a multiple of head_dim %d", fn, i, N[i], rope->head_dim);
         tile0 += (N[i] / 8 + GEMV_PACKS - 1) / GEMV_PACKS;
     }
+    if (swiglu_out) p.proj[1].tile0 = 1 << 30;          // both projections are the tiles of the first
     for (int i = n_proj; i < GEMV_MAX_PROJ; ++i) p.proj[i] = GemvProj{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
+    p.swiglu_out = swiglu_out ? 1 : 0;
+    if (swiglu_out) tile0 = (N[0] / 8 + GEMV_PACKS / 2 - 1) / (GEMV_PACKS / 2);
     p.tiles_total = tile0; p.vec16 = vec16;
     const int tiles = tile0;
     if (k_split > p.n_groups) {
@@ -656,5 +686,20 @@ extern "C" int fq_awq_gemv(
     const void* x, int M, int K, int group, int n_proj,
     const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
     const int* N, void* const* y, int interleaved, int k_split, void* stream) {
-    return fq_awq_gemv_fused(x, M, K, group, n_proj, qweight, scales, qzeros, bias, N, y, interleaved, nullptr, nullptr, k_split, stream);
+    return gemv_launch(x, M, K, group, n_proj, qweight, scales, qzeros, bias, N, y, interleaved, nullptr, nullptr, false, k_split, stream);
+}
+
+extern "C" int fq_awq_gemv_fused(
+    const void* x, int M, int K, int group, int n_proj,
+    const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
+    const int* N, void* const* y, int interleaved, const fq_gemv_prologue* pro, const fq_gemv_rope* rope, int k_split, void* stream) {
+    return gemv_launch(x, M, K, group, n_proj, qweight, scales, qzeros, bias, N, y, interleaved, pro, rope, false, k_split, stream);
+}
+
+extern "C" int fq_awq_gemv_swiglu(
+    const void* x, int M, int K, int group, const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
+    int N, void* y, int interleaved, const fq_gemv_prologue* pro, int k_split, void* stream) {
+    const int Ns[2] = {N, N};
+    void* ys[2] = {y, y};
+    return gemv_launch(x, M, K, group, 2, qweight, scales, qzeros, bias, Ns, ys, interleaved, pro, nullptr, true, k_split, stream);
 }

@@ -574,6 +574,7 @@ static int llama_step_impl(const fq_llama_model* m, const fq_int4_cache* cache, 
         if (out) xin = out;
         return r;
     };
+    const bool swiglu_behind = B > 1;
     for (int l = 0; l < m->n_layers; ++l) {
         const fq_llama_layer& L = m->layers[l];
         FQ_CHECK_ARG(L.q.K == H && L.q.N == nq && L.k.N == nkv && L.v.N == nkv && L.o.K == nq && L.o.N == H &&
@@ -616,23 +617,29 @@ static int llama_step_impl(const fq_llama_model* m, const fq_int4_cache* cache, 
         }
         delta = s->attn_out;
         {
-            // post_attention_layernorm -> gate/up: one launch
+            // post_attention_layernorm -> gate/up: one launch, with act_fn(gate) * up behind it from two rows on, where it would cost
+            // the down projection more: every CTA of it evaluates its range of all rows.  A token over 4k, apart / together, us:
+            // one row 1638 / 1646, two 1956 / 1949, four 2254 / 2234, eight 2546 / 2490
             const int32_t* qw[2] = {L.gate.qweight, L.up.qweight}; const void* sc[2] = {L.gate.scales, L.up.scales};
             const int32_t* qz[2] = {L.gate.qzeros, L.up.qzeros}; const void* bs[2] = {L.gate.bias, L.up.bias};
-            const int N[2] = {m->ffn, m->ffn}; void* y[2] = {s->gate, s->up};
             fq_gemv_prologue pro;
             const void* src;
             if ((rc = norm_prologue(L.post_norm, pro, &src)) != FQ_OK) return rc;
-            rc = fq_awq_gemv_fused(src, B, H, m->group, 2, qw, sc, qz, (bs[0] || bs[1]) ? bs : nullptr, N, y, m->interleaved,
-                                   &pro, nullptr, ks_gu, stream);
+            if (swiglu_behind) {
+                rc = fq_awq_gemv_swiglu(src, B, H, m->group, qw, sc, qz, (bs[0] || bs[1]) ? bs : nullptr, m->ffn, s->gate, m->interleaved,
+                                        &pro, ks_gu, stream);
+            } else {
+                const int N[2] = {m->ffn, m->ffn}; void* y[2] = {s->gate, s->up};
+                rc = fq_awq_gemv_fused(src, B, H, m->group, 2, qw, sc, qz, (bs[0] || bs[1]) ? bs : nullptr, N, y, m->interleaved,
+                                       &pro, nullptr, ks_gu, stream);
+            }
             if (rc != FQ_OK) return rc;
         }
         {
-            // act_fn(gate) * up -> down: one launch
             const int32_t* qw[1] = {L.down.qweight}; const void* sc[1] = {L.down.scales}; const int32_t* qz[1] = {L.down.qzeros};
             const void* bs[1] = {L.down.bias}; const int N[1] = {H}; void* y[1] = {s->down};
             fq_gemv_prologue pro;
-            pro.kind = FQ_GEMV_SWIGLU; pro.b = s->up; pro.weight = nullptr; pro.eps = 0.f; pro.out = nullptr;
+            pro.kind = swiglu_behind ? FQ_GEMV_PLAIN : FQ_GEMV_SWIGLU; pro.b = s->up; pro.weight = nullptr; pro.eps = 0.f; pro.out = nullptr;
             rc = fq_awq_gemv_fused(s->gate, B, m->ffn, m->group, 1, qw, sc, qz, bs[0] ? bs : nullptr, N, y, m->interleaved,
                                    &pro, nullptr, ks_dn, stream);
             if (rc != FQ_OK) return rc;

@@ -474,6 +474,12 @@ int fq_awq_gemv_fused(
     const void* x, int M, int K, int group, int n_proj,
     const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
     const int* N, void* const* y, int interleaved, const fq_gemv_prologue* pro, const fq_gemv_rope* rope, int k_split, void* stream);
+/* The gate and up projections of an MLP with SwiGLU behind them, for up to 8 rows: y (M,N) = fp16(silu(x @ gate)) * (x @ up),
+ * the bits of fq_awq_gemv_fused on both (with the same prologue and the k_split of both together) followed by fq_swiglu.
+ * qweight, scales, qzeros, bias: arrays of two, gate first. */
+int fq_awq_gemv_swiglu(
+    const void* x, int M, int K, int group, const int32_t* const* qweight, const void* const* scales, const int32_t* const* qzeros, const void* const* bias,
+    int N, void* y, int interleaved, const fq_gemv_prologue* pro, int k_split, void* stream);
 
 /* AWQ W4A16 dequant-GEMM for prefill / batched shapes (any M >= 1): the same computation as
  * fq_awq_gemv — the linears kernel/fused_proj.py:36-39,51-53 and the patched forward
@@ -677,8 +683,8 @@ int fq_argmax_f16(const void* x, int64_t rows, int N, int32_t* out, void* stream
  * around eager/llama_persistent_patch.py:164-305 (Hugging Face's LlamaDecoderLayer / LlamaMLP /
  * LlamaRMSNorm semantics) issued from native code, 8 launches per layer and no host work
  * between them.  Per layer: fq_awq_gemv_fused (add+RMSNorm -> q/k/v -> RoPE), fq_decode_layer_int4
- * (append + score + select + attend), AWQ o GEMV, fq_awq_gemv_fused (add+RMSNorm -> gate/up),
- * fq_awq_gemv_fused (SwiGLU -> down); then add+RMSNorm, fp16 lm_head GEMV, argmax.  fp16 model,
+ * (append + score + select + attend), AWQ o GEMV, fq_awq_gemv_swiglu (add+RMSNorm -> gate/up -> SwiGLU),
+ * down GEMV (one row: SwiGLU in front of down); then add+RMSNorm, fp16 lm_head GEMV, argmax.  fp16 model,
  * B <= 8 sequences.
  * All pointers inside the structs are device pointers except `layers` (host array). */
 typedef struct fq_awq_linear {
@@ -702,7 +708,7 @@ typedef struct fq_llama_scratch {
     void *resid0, *resid1, *normed;                /* (B, hidden) fp16 */
     void *q, *k, *v;                               /* (B, q_heads*D), (B, kv_heads*D) x2 fp16 */
     void *attn_out, *down;                         /* (B, hidden) fp16 */
-    void *gate, *up;                               /* (B, ffn) fp16 */
+    void *gate, *up;                               /* (B, ffn) fp16; from two rows on gate holds silu(gate) * up */
     void* logits; int32_t* next_ids;               /* (B, vocab) fp16, (B) */
     float* scores; int64_t sc_sl;                  /* per layer (B,Hq,P_max) fp32, layer stride in elements */
     int32_t* compact; int64_t cp_sl;               /* per layer (B,Hq,bucket) */

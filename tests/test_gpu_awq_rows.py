@@ -145,6 +145,33 @@ def test_gemv_of_known_layout_gives_the_bits_of_the_general_one(M, K, Ns):
             assert torch.equal(a.view(torch.int16), b.view(torch.int16))
 
 
+@pytest.mark.parametrize("M", [1, 2, 4, 7, 8])
+@pytest.mark.parametrize("K,N,group,interleaved,bias", [(128, 128, 128, True, True), (3072, 8192, 128, True, False), (1152, 352, 128, True, True),
+                                                        (320, 264, 64, False, True), (1024, 1000, 32, True, False)])
+def test_gemv_with_swiglu_behind_equals_its_parts(M, K, N, group, interleaved, bias):
+    """Tiles of gate and up columns side by side give the bits of the two projections followed by fq_swiglu, with and without
+    the norm in front, at every split."""
+    import ctypes
+    from flashquest_b200._lib import GEMV_ADD_RMSNORM, GemvPrologue, check, lib, ptr, stream_ptr
+    from flashquest_b200.kernel.fused_proj import awq_gemv_fused
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    lins = [_linear(K, N, group, interleaved, bias, g) for _ in range(2)]
+    x, b = (torch.randn(M, K, device="cuda", generator=g).half() for _ in range(2))
+    w = torch.rand(K, device="cuda", generator=g).half()
+    VP = ctypes.c_void_p * 2
+    arr = lambda name: VP(*[ptr(getattr(lin, name)) for lin in lins])
+    for k_split in (1, 2, 8, lib().fq_awq_gemv_default_splits(K, 2 * N, group)):
+        for norm in (False, True):
+            gate, up = awq_gemv_fused(x, lins, k_split=k_split, **(dict(add=b, norm_weight=w, return_sum=True) if norm else {}))[:2]
+            want, got, total = torch.empty_like(gate), torch.empty_like(gate), torch.empty_like(x)
+            check(lib().fq_swiglu(ptr(gate), ptr(up), gate.numel(), ptr(want), stream_ptr(x.device)))
+            pro = GemvPrologue(GEMV_ADD_RMSNORM, ptr(b), ptr(w), 1e-5, ptr(total)) if norm else None
+            check(lib().fq_awq_gemv_swiglu(ptr(x), M, K, group, arr("qweight"), arr("scales"), arr("qzeros"), arr("bias") if bias else None, N,
+                                           ptr(got), int(interleaved), ctypes.byref(pro) if norm else None, k_split, stream_ptr(x.device)))
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16)), (k_split, norm)
+            assert not norm or torch.equal(total, x + b)
+
+
 @pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (8, 3072), (2, 8192)])
 def test_norm_equals_general_kernel(rows, H):
     """Rows 16 bytes at a time give the bits of the value-by-value kernel, which unaligned rows take."""
