@@ -640,9 +640,14 @@ static int gemv_launch(
         k_split *= 2;
     }
     p.k_split = k_split;
-    // Two CTAs per SM at most where two hold the launch: clusters are placed where they fit, and with room for a third some SMs
-    // got three and others one (256 CTAs of 3072 -> 16384 at 8 rows: 18.9 us, 15.1 with the room taken)
-    if ((int64_t)tiles * k_split > sm_count() && (int64_t)tiles * k_split <= 2LL * sm_count() && smem < 76 * 1024) smem = 76 * 1024;
+    // No more CTAs per SM than an even spread of the launch needs: clusters, started early beside the kernel in front, are placed
+    // where they fit, and with room for more some SMs got two or three and others none.  The request for shared memory takes the
+    // room.  One per SM up to one CTA per SM, and then alone (115 KB, which lets the kernel in front share the SM, is 0.5 to 1 %
+    // slower than 170); two per SM up to two.  A token over 4k, room for as many as fit -> this: one row 1640 -> 1550 us, four
+    // 2160 -> 1948, eight 2469 -> 2219; over 32k one row 1885 -> 1790.  256 CTAs of 3072 -> 16384 alone, eight rows: 18.9 -> 15.1
+    const int64_t ctas = (int64_t)tiles * k_split;
+    const size_t room = ctas <= sm_count() ? 170 * 1024 : ctas <= 2LL * sm_count() ? 112 * 1024 : 0;
+    if (smem < room) smem = room;
     FQ_CHECK_ARG(((p.head_dim > 0 ? p.head_dim : 128) / 2) % (4 * (Mp == 8 ? k_split : 1)) == 0, FQ_ERR_UNSUPPORTED,
                  "%s: head_dim %d with %d-way split-K", fn, p.head_dim, k_split);
     FQ_CHECK_ARG(smem <= 226 * 1024, FQ_ERR_UNSUPPORTED, "%s: K=%d with %d rows needs %zu B of shared memory per CTA", fn, K, M, smem);
