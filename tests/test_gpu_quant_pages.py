@@ -99,3 +99,27 @@ def test_rope_of_the_patched_forward_matches_hugging_face(model, stage, D):
     # one staged token: its value is the output
     assert torch.allclose(O.float(), want_v.float().repeat_interleave(Hq // Hkv, 1), atol=1e-3)
     assert cache.get_seq_length() == 1
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_values_that_are_not_numbers(bits, dtype):
+    """Infinities and NaNs in K and V: the codes of the channels and tokens that have them, and of their neighbours."""
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    D, S, page = 128, 64, 16
+    outs = []
+    for first in (0, 1):                        # whole pages at once, and (one token first) the general kernel's last pages
+        K, V = _data(1, 2, S, D, dtype, 5), _data(1, 2, S, D, dtype, 6)
+        for x in (K, V):
+            x[0, 0, 17, 5], x[0, 0, 33, 70], x[0, 1, 18, 9] = float("inf"), float("-inf"), float("nan")
+        cache = (PersistentInt4KVCache if bits == 4 else PersistentInt8KVCache)(
+            batch_size=1, num_layers=1, num_kv_heads=2, head_dim=D, max_seq_len=S, page_size=page, dtype=dtype)
+        if first:
+            for t in range(S):
+                cache.update_quantized(K[:, :, t:t + 1].cuda(), V[:, :, t:t + 1].cuda(), 0)
+        else:
+            cache.update_quantized(K.cuda(), V.cuda(), 0)
+        outs.append(cache)
+    for name in (("K_packed", "V_packed") if bits == 4 else ("K_uint8", "V_uint8")):
+        assert torch.equal(getattr(outs[0], name), getattr(outs[1], name)), name
