@@ -34,6 +34,7 @@ struct TurboAttnParams {
     float sm_scale;
     void* O; int64_t o_sb, o_sh; float* lse;
     int* tickets; float* partials; int n_split;
+    uint32_t m_mul[4], l_mul[2];      // 1 << (12 - 2 j); 1 << 8, 1 << 4: unknown to the compiler (see pair_at)
     int fast;            // planes are token-contiguous and 16-byte aligned: 16-byte async copies
 };
 
@@ -236,11 +237,12 @@ __global__ void __launch_bounds__(TQ_THREADS, 3) sparse_decode_turbo_kernel(Turb
             }
         }
     };
-    // codebook pair of channels (2j, 2j+1) of this lane from the raw plane bytes: mask, then shift-and-add
+    // codebook pair of channels (2j, 2j+1) of this lane from the raw plane bytes: mask, then multiply-and-add by powers of two that
+    // the compiler cannot turn into shifts: the integer pipe is the busier one (245.0 -> 242.0 us for 16 x 32k)
     auto pair_at = [&](uint32_t M, uint32_t L, int j) -> float2 {
-        const uint32_t a = lut_addr + ((M & (3u << (2 * j))) << (12 - 2 * j));
-        const uint32_t b = j < 2 ? ((L & (15u << (4 * j))) << (8 - 4 * j)) : j == 2 ? (L & 0x0f00u) : ((L >> 4) & 0x0f00u);
-        return tq_lds_f2(a + b);
+        const uint32_t a = (M & (3u << (2 * j))) * p.m_mul[j] + lut_addr;
+        const uint32_t l = L & (15u << (4 * j));
+        return tq_lds_f2(j < 2 ? l * p.l_mul[j] + a : j == 2 ? l + a : (l >> 4) + a);
     };
 
     float m_run = -INFINITY, l_run = 0.f;
@@ -450,6 +452,8 @@ extern "C" int fq_sparse_decode_turbo(
         FQ_CHECK_ARG((int64_t)P * page >= S_kv, FQ_ERR_ARG, "%s: %d pages of %d tokens do not cover S_kv=%d", fn, P, page, S_kv);
     }
     TurboAttnParams p;
+    for (int j = 0; j < 4; ++j) p.m_mul[j] = 1u << (12 - 2 * j);
+    p.l_mul[0] = 1u << 8; p.l_mul[1] = 1u << 4;
     p.Q = Q_rot; p.q_sb = q_sb; p.q_sh = q_sh;
     p.K_msb = K_msb; p.K_lsb = K_lsb; p.V_msb = V_msb; p.V_lsb = V_lsb;
     p.km_sb = km_sb; p.km_sh = km_sh; p.km_ss = km_ss; p.kl_sb = kl_sb; p.kl_sh = kl_sh; p.kl_ss = kl_ss;
