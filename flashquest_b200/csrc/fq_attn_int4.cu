@@ -300,6 +300,14 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) sparse_decode_in
 #pragma unroll
     for (int j = 0; j < DPL / 2; ++j) acc[j] = make_float2(0.f, 0.f);
     bool timed_out = false;
+    constexpr int TD = D / 32;
+    float tm[ATT_WARPS], tl[ATT_WARPS], tacc[ATT_WARPS][TD];       // states over the staged tokens (the producer warp's)
+#pragma unroll
+    for (int w = 0; w < ATT_WARPS; ++w) {
+        tm[w] = -INFINITY; tl[w] = 0.f;
+#pragma unroll
+        for (int j = 0; j < TD; ++j) tacc[w][j] = 0.f;
+    }
 
     if (is_producer) {
         // =========================== producer warp ===========================
@@ -340,6 +348,57 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) sparse_decode_in
             timed_out = __any_sync(0xffffffffu, timed_out);
         }
         if (timed_out && lane == 0) atomicExch(p.status, FQ_ERR_TIMEOUT);
+
+        // ---- tail: dense attention over the staged (unquantised) tokens, by the CTA of split 0, while the consumers work on the
+        // last units.  Behind them, in the consumer warps, its loads stood in the way of every row's last ticket (0.7 us).
+        // Four states, state w takes tail tokens w, w + 4, ...; lane owns D/32 channels.
+        const int dyn_tail = DYN ? (pos_v + p.pos_new) % p.page : p.tail_len;
+        if (split == 0 && dyn_tail > 0 && !timed_out) {
+            float qt[TD];
+            const QT* qp = static_cast<const QT*>(p.Q) + b * p.q_sb + hq * p.q_sh + TD * lane;
+#pragma unroll
+            for (int j = 0; j < TD; ++j) qt[j] = Dt<QT>::to_f32(qp[j]) * (p.sm_scale * LOG2E);
+            const int64_t head = b * p.tl_sb + hkv * p.tl_sh + TD * lane;
+            for (int t0 = 0; t0 < dyn_tail; t0 += ATT_WARPS) {
+                float kv[ATT_WARPS][TD], vv[ATT_WARPS][TD], sdt[ATT_WARPS];
+#pragma unroll
+                for (int w = 0; w < ATT_WARPS; ++w) {
+                    const int64_t ro = head + (int64_t)min(t0 + w, dyn_tail - 1) * p.tl_ss;
+#pragma unroll
+                    for (int j = 0; j < TD; ++j) {
+                        if (p.tail_dtype == FQ_BF16) {
+                            kv[w][j] = ld_as_f32<__nv_bfloat16>(p.K_tail, ro + j);
+                            vv[w][j] = ld_as_f32<__nv_bfloat16>(p.V_tail, ro + j);
+                        } else {
+                            kv[w][j] = ld_as_f32<__half>(p.K_tail, ro + j);
+                            vv[w][j] = ld_as_f32<__half>(p.V_tail, ro + j);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int w = 0; w < ATT_WARPS; ++w) {
+                    sdt[w] = 0.f;
+#pragma unroll
+                    for (int j = 0; j < TD; ++j) sdt[w] = fmaf(qt[j], kv[w][j], sdt[w]);
+                }
+#pragma unroll
+                for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+                    for (int w = 0; w < ATT_WARPS; ++w) sdt[w] += __shfl_xor_sync(0xffffffffu, sdt[w], off);
+#pragma unroll
+                for (int w = 0; w < ATT_WARPS; ++w) {
+                    if (t0 + w < dyn_tail) {
+                        const float mnew = fmaxf(tm[w], sdt[w]);
+                        const float al = ex2(tm[w] - mnew);
+                        const float pr = ex2(sdt[w] - mnew);
+                        tl[w] = tl[w] * al + pr;
+#pragma unroll
+                        for (int j = 0; j < TD; ++j) tacc[w][j] = fmaf(pr, vv[w][j], tacc[w][j] * al);
+                        tm[w] = mnew;
+                    }
+                }
+            }
+        }
     } else {
         // =========================== consumer warps ===========================
         UnitCtx<DPL, TPL> ctx_cur, ctx_nxt;     // metadata of the unit in hand and of the next one
@@ -539,46 +598,6 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) sparse_decode_in
         l_part = l_q;
     }
 
-    // ---------------- tail: dense attention over the staged (unquantised) tokens ----------------
-    // Done by the CTA of split 0; warp w takes tail tokens w, w+WARPS, ...; lane owns D/32 channels.
-    constexpr int TD = D / 32;
-    float tm = -INFINITY, tl = 0.f, tacc[TD];
-#pragma unroll
-    for (int j = 0; j < TD; ++j) tacc[j] = 0.f;
-    const int dyn_tail = DYN ? (pos_v + p.pos_new) % p.page : p.tail_len;
-    if (split == 0 && dyn_tail > 0 && !is_producer) {
-        float qt[TD];
-        const QT* qp = static_cast<const QT*>(p.Q) + b * p.q_sb + hq * p.q_sh + TD * lane;
-#pragma unroll
-        for (int j = 0; j < TD; ++j) qt[j] = Dt<QT>::to_f32(qp[j]) * (p.sm_scale * LOG2E);
-        for (int t = warp; t < dyn_tail; t += ATT_WARPS) {
-            const int64_t ro = b * p.tl_sb + hkv * p.tl_sh + (int64_t)t * p.tl_ss + TD * lane;
-            float kv[TD], vv[TD];
-#pragma unroll
-            for (int j = 0; j < TD; ++j) {
-                if (p.tail_dtype == FQ_BF16) {
-                    kv[j] = ld_as_f32<__nv_bfloat16>(p.K_tail, ro + j);
-                    vv[j] = ld_as_f32<__nv_bfloat16>(p.V_tail, ro + j);
-                } else {
-                    kv[j] = ld_as_f32<__half>(p.K_tail, ro + j);
-                    vv[j] = ld_as_f32<__half>(p.V_tail, ro + j);
-                }
-            }
-            float sdt = 0.f;
-#pragma unroll
-            for (int j = 0; j < TD; ++j) sdt = fmaf(qt[j], kv[j], sdt);
-#pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) sdt += __shfl_xor_sync(0xffffffffu, sdt, off);
-            const float mnew = fmaxf(tm, sdt);
-            const float al = ex2(tm - mnew);
-            const float pr = ex2(sdt - mnew);
-            tl = tl * al + pr;
-#pragma unroll
-            for (int j = 0; j < TD; ++j) tacc[j] = fmaf(pr, vv[j], tacc[j] * al);
-            tm = mnew;
-        }
-    }
-
     // ---------------- CTA merge of all states through shared memory ----------------
     __syncthreads();   // every warp is done with the staging area (st_acc aliases it)
     if (!is_producer) {
@@ -586,10 +605,14 @@ __global__ void __launch_bounds__(ATT_THREADS, ATT_CTAS_PER_SM) sparse_decode_in
         if (l == 0) { st_m[sid] = m_run; st_l[sid] = l_part; }
 #pragma unroll
         for (int j = 0; j < DPL; ++j) st_acc[sid * D + DPL * l + j] = o[j];
-        const int tsid = ATT_WARPS * 4 + warp;
-        if (lane == 0) { st_m[tsid] = tm; st_l[tsid] = tl; }
+    } else {
 #pragma unroll
-        for (int j = 0; j < TD; ++j) st_acc[tsid * D + TD * lane + j] = tacc[j];
+        for (int w = 0; w < ATT_WARPS; ++w) {
+            const int tsid = ATT_WARPS * 4 + w;
+            if (lane == 0) { st_m[tsid] = tm[w]; st_l[tsid] = tl[w]; }
+#pragma unroll
+            for (int j = 0; j < TD; ++j) st_acc[tsid * D + TD * lane + j] = tacc[w][j];
+        }
     }
     __syncthreads();
     // warp 0 turns the per-state maxima into merge weights once; then thread d sums channel d
