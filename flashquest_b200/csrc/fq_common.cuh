@@ -68,6 +68,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // selection and attention, which always follow the append launch; the append itself reads after its wait.
 struct DynPos { const int* pos = nullptr; int n_new = 0; int page = 1; int max_tokens = 0; bool early = false; };
 
+struct QuantParams;      // fq_append.cuh
+
 // Launch functions behind the public entry points of the same names, with the position record explicit.
 int quantize_kv_int4_launch(
     const void* K_head, const void* V_head, int64_t hd_sb, int64_t hd_sh, int64_t hd_ss, int n_head,
@@ -81,7 +83,14 @@ int page_scores_int4_launch(
     const void* Q, int q_dtype, int64_t q_sb, int64_t q_sh,
     const void* K_scale, const void* K_mn, int64_t km_sb, int64_t km_sh, int64_t km_sp,
     int B, int Hq, int Hkv, int P, int D, float* scores, int64_t sc_sb, int64_t sc_sh, void* stream, const DynPos& dp,
-    float levels = 15.0f);
+    float levels = 15.0f, const QuantParams* append = nullptr, int append_dtype = 0);
+bool page_scores_take_append(int q_dtype, int B, int Hq, int Hkv, int P, int D);
+// The append of a decode step as page_scores_int4_launch takes it along.  Rows staged behind `seen` tokens, no page completed
+// (pos null), or anything that n_new < page tokens can do, read from *pos.  false: the append's own launch is needed.
+bool append_stage_params(QuantParams& q, void* K_partial, void* V_partial, int64_t pt_sb, int64_t pt_sh, int64_t pt_ss, const void* K_new, const void* V_new,
+                         int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int dtype, int B, int H, int D, int page, int seen, int n_new);
+bool append_dyn_params(QuantParams& q, const fq_int4_cache* c, int layer, const int* pos, const void* K_new, const void* V_new,
+                       int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new);
 bool score_select_fusable(int Hq, int Hkv, int P, int D);
 int score_select_launch(
     const void* Q, int q_dtype, int64_t q_sb, int64_t q_sh,

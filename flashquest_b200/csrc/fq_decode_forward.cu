@@ -2,6 +2,7 @@
 // (flashquest/eager/llama_persistent_patch.py:164-245): the rotary embedding of q and k with Hugging Face's
 // roundings, the cast to the cache's dtype, and the decode layer of the INT8 cache (append, page scores, selection,
 // attention with the staged tail in the same softmax) as one host call.
+#include "fq_append.cuh"
 #include "fq_quant_pages.cuh"
 
 namespace fq {
@@ -10,7 +11,7 @@ namespace fq {
 // dtype TC; v is only cast.  One CTA per (head, batch), a thread per channel pair (i, i + D/2).  Latency-bound: it
 // replaces eleven element-wise launches of a few hundred values each.
 // `pattern` (one byte per KV head, not 0: a retrieval head) is turned into the retention of every query head here, at each
-// call: the caller's tensor may have changed since the last one.  The selection, three launches on, reads the result.
+// call: the caller's tensor may have changed since the last one.  The selection, two launches on or three, reads the result.
 template <typename TM, typename TC>
 __global__ void __launch_bounds__(64) rope_qkv_kernel(const TM* __restrict__ q, int64_t q_sb, const TM* __restrict__ k, int64_t k_sb,
                                                       const TM* __restrict__ v, int64_t v_sb, const TM* __restrict__ cosv, int64_t c_sb,
@@ -118,23 +119,28 @@ extern "C" int fq_decode_layer_int8(
     FQ_CHECK_ARG(layer >= 0 && layer < c->L, FQ_ERR_ARG, "%s: layer_idx %d out of range [0, %d)", fn, layer, c->L);
     const int page = c->page, D = c->D, B = c->B, Hkv = c->Hkv, Hq = prm->Hq;
     int rc;
-    if (n_new > 0) {
+    const int now = seen + n_new, tail = now % page, completed = now - tail, P = completed / page;
+    char* Kt = static_cast<char*>(c->K_partial) + layer * c->pt_sl * 2;
+    char* Vt = static_cast<char*>(c->V_partial) + layer * c->pt_sl * 2;
+    // tokens that complete no page are staged in the launch of the scores
+    QuantParams staged;
+    const bool along = seen >= 0 && now <= c->max_seq_len && (page == 16 || page == 32 || page == 64) && page_scores_take_append(q_dtype, B, Hq, Hkv, P, D) &&
+                       append_stage_params(staged, Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, K_new, V_new, nw_sb, nw_sh, nw_ss, c->kv_dtype, B, Hkv, D, page, seen, n_new);
+    if (n_new > 0 && !along) {
         rc = fq_append_kv_int8(c, layer, seen, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, stream);
         if (rc != FQ_OK) return rc;
     }
-    const int now = seen + n_new, tail = now % page, completed = now - tail, P = completed / page;
     const uint16_t* Ks = static_cast<const uint16_t*>(c->K_scale) + layer * c->km_sl;
     const uint16_t* Km = static_cast<const uint16_t*>(c->K_mn) + layer * c->km_sl;
     if (P > 0) {
-        rc = fq_page_scores_int8(Q, q_dtype, q_sb, q_sh, Ks, Km, c->km_sb, c->km_sh, c->km_sp, B, Hq, Hkv, P, D, scores, (int64_t)Hq * P, P, stream);
+        rc = page_scores_int4_launch(Q, q_dtype, q_sb, q_sh, Ks, Km, c->km_sb, c->km_sh, c->km_sp, B, Hq, Hkv, P, D, scores, (int64_t)Hq * P, P, stream,
+                                     DynPos{}, 255.0f, along ? &staged : nullptr, c->kv_dtype);
         if (rc != FQ_OK) return rc;
         rc = fq_select_pages(scores, (int64_t)Hq * P, P, B, Hq, P, prm->retention_per_head, prm->retention,
                              prm->k_max_static < P ? prm->k_max_static : P, prm->sinks, prm->window, nullptr, 0, 0,
                              compact, (int64_t)Hq * prm->bucket, prm->bucket, prm->bucket, nullptr, stream);
         if (rc != FQ_OK) return rc;
     }
-    const char* Kt = static_cast<const char*>(c->K_partial) + layer * c->pt_sl * 2;
-    const char* Vt = static_cast<const char*>(c->V_partial) + layer * c->pt_sl * 2;
     return fq_sparse_decode_int8(
         Q, q_dtype, q_sb, q_sh, c->K_packed + layer * c->pk_sl, c->V_packed + layer * c->pk_sl, c->pk_sb, c->pk_sh, c->pk_ss,
         Ks, Km, c->km_sb, c->km_sh, c->km_sp, static_cast<const uint16_t*>(c->V_scale) + layer * c->vm_sl,

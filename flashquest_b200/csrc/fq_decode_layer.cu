@@ -2,7 +2,7 @@
 // INT4 cache: pack-on-append, page scores, top-k + compact index, sparse attention with the
 // staged tail.  No device code of its own; it exists so that a caller pays one foreign call
 // per layer instead of four plus the slicing arithmetic.
-#include "fq_common.cuh"
+#include "fq_append.cuh"
 
 extern "C" int fq_append_kv_int4(const fq_int4_cache* c, int layer, int seen, const void* K_new, const void* V_new,
                                  int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new, void* stream) {
@@ -49,17 +49,21 @@ static int decode_layer_int4(
     char* Vt = static_cast<char*>(c->V_partial) + layer * c->pt_sl * esz;
 
     int rc;
-    if (n_new > 0) {
-        rc = fq_append_kv_int4(c, layer, seen, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, stream);
-        if (rc != FQ_OK) return rc;
-    }
     const int now = seen + n_new;
     const int tail = now % page;
     const int completed = now - tail;
     const int P = completed / page;
+    // tokens that complete no page are staged in the launch of the scores
+    QuantParams staged;
+    const bool along = page_scores_take_append(q_dtype, B, Hq, Hkv, P, D) &&
+                       append_stage_params(staged, Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, K_new, V_new, nw_sb, nw_sh, nw_ss, c->kv_dtype, B, Hkv, D, page, seen, n_new);
+    if (n_new > 0 && !along) {
+        rc = fq_append_kv_int4(c, layer, seen, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, stream);
+        if (rc != FQ_OK) return rc;
+    }
     if (P > 0) {
-        rc = fq_page_scores_int4(Q, q_dtype, q_sb, q_sh, Ks, Km, c->km_sb, c->km_sh, c->km_sp,
-                                 B, Hq, Hkv, P, D, scores, (int64_t)Hq * P, P, stream);
+        rc = page_scores_int4_launch(Q, q_dtype, q_sb, q_sh, Ks, Km, c->km_sb, c->km_sh, c->km_sp,
+                                     B, Hq, Hkv, P, D, scores, (int64_t)Hq * P, P, stream, DynPos{}, 15.0f, along ? &staged : nullptr, c->kv_dtype);
         if (rc != FQ_OK) return rc;
         const int k_max = prm->k_max_static < P ? prm->k_max_static : P;
         rc = fq_select_pages(scores, (int64_t)Hq * P, P, B, Hq, P, prm->retention_per_head, prm->retention,
@@ -186,14 +190,16 @@ int decode_layer_int4_dyn(const fq_int4_cache* c, int l, const int* pos, const v
     DynPos dp_early = dp;          // scores, selection and attention come at least two launches after any writer of *pos
     dp_early.early = true;
     int rc = FQ_OK;
-    if (append)
+    QuantParams now;
+    const bool along = append && page_scores_take_append(q_dtype, B, Hq, Hkv, P_max, D) && append_dyn_params(now, c, l, pos, Kn, Vn, nw_sb, nw_sh, nw_ss, n_new);
+    if (append && !along)
         rc = quantize_kv_int4_launch(Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, page - n_new, Kn, Vn, nw_sb, nw_sh, nw_ss, n_new,
                                      c->kv_dtype, B, Hkv, D, page, page,
                                      Kp, Vp, c->pk_sb, c->pk_sh, c->pk_ss, Ks, Km, c->km_sb, c->km_sh, c->km_sp,
                                      Vs, Vm, c->vm_sb, c->vm_sh, 1, Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, stream, dp);
     if (rc != FQ_OK) return rc;
     rc = page_scores_int4_launch(Ql, q_dtype, q_sb, q_sh, Ks, Km, c->km_sb, c->km_sh, c->km_sp, B, Hq, Hkv, P_max, D,
-                                 sc, (int64_t)Hq * P_max, P_max, stream, dp_early);
+                                 sc, (int64_t)Hq * P_max, P_max, stream, dp_early, 15.0f, along ? &now : nullptr, c->kv_dtype);
     if (rc != FQ_OK) return rc;
     rc = select_pages_launch(sc, (int64_t)Hq * P_max, P_max, B, Hq, P_max, pl->retention_per_head, pl->retention,
                              pl->k_max_static < P_max ? pl->k_max_static : P_max, pl->sinks, pl->window, nullptr, 0, 0,

@@ -3,7 +3,7 @@
 // metadata, top-k + compact index, rotation of Q, sparse attention over the selected planes in
 // the rotated basis, rotation of O back, tail attention over the staged tokens and the LSE merge.
 // No device code of its own: it exists so that a caller pays one foreign call per layer.
-#include "fq_common.cuh"
+#include "fq_append.cuh"
 
 extern "C" size_t fq_decode_layer_turbo_scratch_bytes(int B, int Hq, int D) {
     if (B <= 0 || Hq <= 0 || D <= 0) return 0;
@@ -40,14 +40,18 @@ extern "C" int fq_decode_layer_turbo(
     char* Kt = static_cast<char*>(c->K_partial) + layer * c->pt_sl * esz;
     char* Vt = static_cast<char*>(c->V_partial) + layer * c->pt_sl * esz;
     int rc;
-    if (n_new > 0) {
-        rc = fq_append_kv_turbo(c, layer, seen, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, stream);
-        if (rc != FQ_OK) return rc;
-    }
     const int now = seen + n_new;
     const int tail = now % page;
     const int completed = now - tail;
     const int P = completed / page;
+    // tokens that complete no page are staged in the launch of the scores
+    QuantParams staged;
+    const bool along = page_scores_take_append(q_dtype, B, Hq, Hkv, P, D) &&
+                       append_stage_params(staged, Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, K_new, V_new, nw_sb, nw_sh, nw_ss, c->kv_dtype, B, Hkv, D, page, seen, n_new);
+    if (n_new > 0 && !along) {
+        rc = fq_append_kv_turbo(c, layer, seen, K_new, V_new, nw_sb, nw_sh, nw_ss, n_new, stream);
+        if (rc != FQ_OK) return rc;
+    }
     const int64_t rows = (int64_t)B * Hq;
     char* sb = static_cast<char*>(scratch);
     void* Q_rot = sb;
@@ -56,7 +60,8 @@ extern "C" int fq_decode_layer_turbo(
     float* lse_parts = reinterpret_cast<float*>(sb + ((rows * D * 8 + 255) & ~(int64_t)255));
     const bool sparse = P > 0, both = sparse && tail > 0;
     if (sparse) {
-        rc = fq_page_scores_int4(Q, q_dtype, q_sb, q_sh, Ksr, Kmr, c->km_sb, c->km_sh, c->km_sp, B, Hq, Hkv, P, D, scores, (int64_t)Hq * P, P, stream);
+        rc = page_scores_int4_launch(Q, q_dtype, q_sb, q_sh, Ksr, Kmr, c->km_sb, c->km_sh, c->km_sp, B, Hq, Hkv, P, D, scores, (int64_t)Hq * P, P, stream,
+                                     DynPos{}, 15.0f, along ? &staged : nullptr, c->kv_dtype);
         if (rc != FQ_OK) return rc;
         const int k_max = prm->k_max_static < P ? prm->k_max_static : P;
         rc = fq_select_pages(scores, (int64_t)Hq * P, P, B, Hq, P, prm->retention_per_head, prm->retention, k_max, prm->sinks, prm->window,

@@ -9,6 +9,7 @@
 // consecutive pages, so every warp load is one contiguous 512-byte run.  Each lane keeps
 // its slice of q for all NR query heads in registers; the per-page reduction is a 3-step
 // xor shuffle inside the quarter warp.
+#include "fq_append.cuh"
 #include "fq_score_grid.cuh"
 #include "fq_score_lane.cuh"
 
@@ -17,17 +18,105 @@ namespace fq {
 constexpr int SCORE_THREADS = 128;            // 16 pages per CTA iteration
 constexpr int SCORE_PAGES_PER_CTA = 32;       // 2 iterations per CTA
 
+// What a decode step appends in the launch of its page scores, by one extra CTA per (batch, kv head).  A launch of its own for 4 KB
+// per head took 1.9 to 2.5 us of every layer.  Two forms: rows to stage behind a known number of tokens, no page completed; and,
+// with the position read on the device, whatever the position asks for.  There, pages completed before do not wait for the
+// append, and the score of a page completed now is the same CTA's work.
+struct NoAppend {};
+struct StageAppend {
+    const uint16_t *K_new, *V_new; int64_t nw_sb, nw_sh, nw_ss;
+    uint16_t *K_stage, *V_stage; int64_t st_sb, st_sh, st_ss;      // row 0 of the new tokens, unless the position is read on the device
+    int n;
+};
+struct DynAppend { StageAppend st; QuantParams q; int bf16; };
+
+// rows of n tokens, K and V, 16 bytes per thread and pass; before() runs between the loads and the stores and returns the first row
+template <typename F>
+__device__ __forceinline__ void stage_rows(const StageAppend& a, int b, int h, int chunks, F&& before) {
+    const int i = threadIdx.x, per = a.n * chunks;
+    auto src = [&](int j) {
+        const int r = (j % per) / chunks, c = j % chunks;
+        return reinterpret_cast<const uint4*>((j < per ? a.K_new : a.V_new) + b * a.nw_sb + h * a.nw_sh + r * a.nw_ss + 8 * c);
+    };
+    uint4 first_v = make_uint4(0, 0, 0, 0);
+    if (i < 2 * per) first_v = *src(i);
+    const int row0 = before();
+    if (row0 < 0) return;
+    for (int j = i; j < 2 * per; j += SCORE_THREADS) {
+        const uint4 v = j == i ? first_v : *src(j);
+        const int r = row0 + (j % per) / chunks, c = j % chunks;
+        *reinterpret_cast<uint4*>((j < per ? a.K_stage : a.V_stage) + b * a.st_sb + h * a.st_sh + r * a.st_ss + 8 * c) = v;
+    }
+}
+
+// the append that completes a page: one step in `page`
+__device__ __noinline__ void append_page(const DynAppend& a, int b, int h) {
+    QuantParams p = a.q;
+    if (!quant_locate(p)) return;                              // full: nothing is written (the host checks its own count)
+    if (a.bf16) quant_int4_cta<__nv_bfloat16>(p, b, h, 0);
+    else quant_int4_cta<__half>(p, b, h, 0);
+}
+
+template <typename QT, int NR, int CH>
+__device__ __forceinline__ void append_and_score(const DynAppend& a, const QT* __restrict__ Q, int64_t q_sb, int64_t q_sh, int b, int hkv, int n_rep, int head_off,
+                                                 int P, int D, float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, float levels, const int* pos, int pos_early) {
+    int seen = 0;
+    if (pos_early) seen = __ldcg(pos);
+    pdl_wait();
+    pdl_trigger();
+    if (!pos_early) seen = *pos;
+    const int page_len = a.q.page, partial = seen % page_len;
+    const bool completes = partial + a.q.n_new >= page_len;
+    stage_rows(a.st, b, hkv, D >> 3, [&]() { return completes || seen < 0 || seen + a.q.n_new > a.q.max_tokens ? -1 : partial; });
+    if (!completes) return;
+    append_page(a, b, hkv);
+    const int page = seen / page_len;                          // completed by this append
+    if (page >= P) return;
+    __syncthreads();                                           // the metadata row is written; read it behind L1, which may hold older bytes
+    if (threadIdx.x >= 32) return;
+    const int l = threadIdx.x & 7, n_chunks = D >> 3, nr = min(NR, n_rep - head_off);
+    uint4 m4[CH], s4[CH];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+        const int chunk = l + 8 * c;
+        m4[c] = s4[c] = make_uint4(0, 0, 0, 0);
+        if (chunk < n_chunks) {
+            const int64_t at = b * a.q.km_sb + hkv * a.q.km_sh + (int64_t)page * a.q.km_sp + 8 * chunk;
+            m4[c] = __ldcg(reinterpret_cast<const uint4*>(a.q.K_mn + at));
+            s4[c] = __ldcg(reinterpret_cast<const uint4*>(a.q.K_scale + at));
+        }
+    }
+    float q[NR][CH][8];
+    score_load_q<QT, NR, CH>(Q + b * q_sb, q_sh, hkv * n_rep + head_off, nr, l, n_chunks, q);
+    const float v = score_page<NR, CH>(q, m4, s4, l, levels);
+    if (threadIdx.x < nr) scores[b * sc_sb + (hkv * n_rep + head_off + l) * sc_sh + page] = v;
+}
+
 // NR = query heads handled per pass (<= 4), CH = 8-channel chunks per lane (D = 64*CH, or
 // D = 32 with CH = 1 where lanes 4..7 hold no chunk).
-template <typename QT, int NR, int CH>
+template <typename QT, int NR, int CH, typename APPEND>
 __global__ void __launch_bounds__(SCORE_THREADS) page_scores_kernel(
     const QT* __restrict__ Q, int64_t q_sb, int64_t q_sh,
     const uint16_t* __restrict__ K_scale, const uint16_t* __restrict__ K_mn,
     int64_t km_sb, int64_t km_sh, int64_t km_sp,
     int Hq, int Hkv, int P, int D, int head_off,
-    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, const int* __restrict__ pos, int pos_new, int pos_page, int pos_early, float levels) {
+    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, const int* __restrict__ pos, int pos_new, int pos_page, int pos_early, float levels,
+    const __grid_constant__ APPEND app) {
     const int b = blockIdx.z, hkv = blockIdx.y;
     const int n_rep = Hq / Hkv;
+    if constexpr (std::is_same_v<APPEND, StageAppend>) {
+        if (blockIdx.x == gridDim.x - 1) {
+            pdl_wait();
+            pdl_trigger();
+            stage_rows(app, b, hkv, D >> 3, []() { return 0; });
+            return;
+        }
+    } else if constexpr (std::is_same_v<APPEND, DynAppend>) {
+        if (blockIdx.x == gridDim.x - 1) {
+            append_and_score<QT, NR, CH>(app, Q, q_sb, q_sh, b, hkv, n_rep, head_off, P, D, scores, sc_sb, sc_sh, levels, pos, pos_early);
+            return;
+        }
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int l = lane & 7, qw = lane >> 3;
     const int n_chunks = D >> 3;
@@ -38,7 +127,8 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_kernel(
     pdl_trigger();
     if (pos) {
         if (!pos_early) pos_v = *pos;
-        P = min(P, (pos_v + pos_new) / pos_page);          // completed pages after this step's append
+        // completed pages after this step's append; before it where that is made here
+        P = min(P, (pos_v + (std::is_same_v<APPEND, DynAppend> ? 0 : pos_new)) / pos_page);
     }
 
     // Metadata loads of every page this quarter warp will score are issued first, the q loads
@@ -66,15 +156,23 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_kernel(
 // page_scores_kernel for the decode step, where the position may be read before the dependency wait
 // (DynPos::early): the rows of the pages completed before this step -- nothing in flight writes them -- are
 // requested before the wait as well, so the CTA spends the end of the previous kernel fetching instead of waiting.
-template <typename QT, int NR, int CH>
+template <typename QT, int NR, int CH, typename APPEND>
 __global__ void __launch_bounds__(SCORE_THREADS) page_scores_early_kernel(
     const QT* __restrict__ Q, int64_t q_sb, int64_t q_sh,
     const uint16_t* __restrict__ K_scale, const uint16_t* __restrict__ K_mn,
     int64_t km_sb, int64_t km_sh, int64_t km_sp,
     int Hq, int Hkv, int P, int D, int head_off,
-    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, const int* __restrict__ pos, int pos_new, int pos_page, float levels) {
+    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, const int* __restrict__ pos, int pos_new, int pos_page, float levels,
+    const __grid_constant__ APPEND app) {
     const int b = blockIdx.z, hkv = blockIdx.y;
     const int n_rep = Hq / Hkv;
+    constexpr bool ALONG = std::is_same_v<APPEND, DynAppend>;
+    if constexpr (ALONG) {
+        if (blockIdx.x == gridDim.x - 1) {
+            append_and_score<QT, NR, CH>(app, Q, q_sb, q_sh, b, hkv, n_rep, head_off, P, D, scores, sc_sb, sc_sh, levels, pos, 1);
+            return;
+        }
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int l = lane & 7, qw = lane >> 3;
     const int n_chunks = D >> 3;
@@ -93,7 +191,7 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_early_kernel(
     }
     pdl_wait();        // Q and the newest metadata row come from the kernels before this one
     pdl_trigger();
-    P = min(P, (pos_v + pos_new) / pos_page);              // completed pages after this step's append
+    P = ALONG ? P_old : min(P, (pos_v + pos_new) / pos_page);          // completed pages after this step's append
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
         const int p = p_base + it * 16 + warp * 4 + qw;
@@ -169,40 +267,64 @@ __global__ void __launch_bounds__(SCORE_THREADS, score_stream_ctas_per_sm(NR, CH
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+static int stream_ctas(int nr, int D, int rows, int P) {
+    const int CH = D <= 64 ? 1 : D / 64, NR = nr > 4 ? 4 : nr;
+    return D == 128 || D == 64 ? score_stream_ctas(rows, P, score_stream_ctas_per_sm(NR, CH) * sm_count()) : 0;
+}
+
+// Whether the launch of these scores can take the step's append along: the short-lived CTAs' kernels, 64 or 128 channels.  Streaming
+// CTAs stay for as long as their pages last, and there the append is 1 to 2 % of the step.
+bool page_scores_take_append(int q_dtype, int B, int Hq, int Hkv, int P, int D) {
+    return (q_dtype == FQ_F16 || q_dtype == FQ_BF16) && (D == 64 || D == 128) && P > 0 && Hkv > 0 && Hq % Hkv == 0 && stream_ctas(Hq / Hkv, D, B * Hkv, P) == 0;
+}
+
 template <typename QT, int NR>
 static void launch_scores(int CH, dim3 grid, cudaStream_t st, const void* Q, int64_t q_sb, int64_t q_sh,
                           const void* K_scale, const void* K_mn, int64_t km_sb, int64_t km_sh, int64_t km_sp,
-                          int Hq, int Hkv, int P, int D, int head_off, float* scores, int64_t sc_sb, int64_t sc_sh, const DynPos& dp, float levels) {
-    const int stream_ctas = D == 128 || D == 64 ? score_stream_ctas((int)(grid.y * grid.z), P, score_stream_ctas_per_sm(NR, CH) * sm_count()) : 0;
-#define FQ_LAUNCH_SC(CHV)                                                                              \
-    do {                                                                                               \
-        if (stream_ctas > 0)                                                                           \
-            launch_k(PDL_SCORES, page_scores_stream_kernel<QT, NR, (CHV > 2 ? 2 : CHV)>, dim3((unsigned)stream_ctas, grid.y, grid.z), dim3(SCORE_THREADS), 0, st, \
-                     static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale),     \
-                     static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P, head_off, scores, sc_sb, sc_sh, \
-                     dp.pos, dp.n_new, dp.page, levels);                                               \
-        else if (dp.pos != nullptr && dp.early)                                                             \
-            launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV>, grid, dim3(SCORE_THREADS), 0, st,              \
-                     static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale),     \
-                     static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P, D, head_off, scores, sc_sb, sc_sh, \
-                     dp.pos, dp.n_new, dp.page, levels);                                               \
-        else                                                                                           \
-            launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV>, grid, dim3(SCORE_THREADS), 0, st,    \
-                     static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale),     \
-                     static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P, D, head_off, scores, sc_sb, sc_sh, \
-                     dp.pos, dp.n_new, dp.page, 0, levels);                                            \
+                          int Hq, int Hkv, int P, int D, int head_off, float* scores, int64_t sc_sb, int64_t sc_sh, const DynPos& dp, float levels,
+                          const DynAppend* app) {
+    const int ctas = stream_ctas(NR, D, (int)(grid.y * grid.z), P);
+    const NoAppend none{};
+    const bool early = dp.pos != nullptr && dp.early;
+#define FQ_SC_ARGS static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale), static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P, D, \
+                   head_off, scores, sc_sb, sc_sh, dp.pos, dp.n_new, dp.page
+#define FQ_LAUNCH_SC(CHV)                                                                                                                                                  \
+    do {                                                                                                                                                                   \
+        if (ctas > 0)                                                                                                                                                      \
+            launch_k(PDL_SCORES, page_scores_stream_kernel<QT, NR, (CHV > 2 ? 2 : CHV)>, dim3((unsigned)ctas, grid.y, grid.z), dim3(SCORE_THREADS), 0, st,                 \
+                     static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale), static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P,    \
+                     head_off, scores, sc_sb, sc_sh, dp.pos, dp.n_new, dp.page, levels);                                                                                   \
+        else if (early) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, none);                    \
+        else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, 0, levels, none);                                  \
     } while (0)
+    if constexpr (sizeof(QT) == 2) {
+        if (app) {
+            ++grid.x;
+#define FQ_LAUNCH_AP(CHV)                                                                                                                                                  \
+    do {                                                                                                                                                                   \
+        if (early) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, *app);                          \
+        else if (dp.pos) launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, 0, levels, *app);                   \
+        else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, StageAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, 0, levels, app->st);                         \
+    } while (0)
+            if (CH == 1) FQ_LAUNCH_AP(1);
+            else FQ_LAUNCH_AP(2);
+#undef FQ_LAUNCH_AP
+            return;
+        }
+    }
     if (CH == 1) FQ_LAUNCH_SC(1);
     else if (CH == 2) FQ_LAUNCH_SC(2);
     else FQ_LAUNCH_SC(4);
 #undef FQ_LAUNCH_SC
+#undef FQ_SC_ARGS
 }
 
 template <typename QT>
 static void launch_scores_nr(int nr, int CH, dim3 grid, cudaStream_t st, const void* Q, int64_t q_sb, int64_t q_sh,
                              const void* K_scale, const void* K_mn, int64_t km_sb, int64_t km_sh, int64_t km_sp,
-                             int Hq, int Hkv, int P, int D, int head_off, float* scores, int64_t sc_sb, int64_t sc_sh, const DynPos& dp, float levels) {
-#define FQ_ARGS CH, grid, st, Q, q_sb, q_sh, K_scale, K_mn, km_sb, km_sh, km_sp, Hq, Hkv, P, D, head_off, scores, sc_sb, sc_sh, dp, levels
+                             int Hq, int Hkv, int P, int D, int head_off, float* scores, int64_t sc_sb, int64_t sc_sh, const DynPos& dp, float levels,
+                             const DynAppend* app) {
+#define FQ_ARGS CH, grid, st, Q, q_sb, q_sh, K_scale, K_mn, km_sb, km_sh, km_sp, Hq, Hkv, P, D, head_off, scores, sc_sb, sc_sh, dp, levels, app
     if (nr == 1) launch_scores<QT, 1>(FQ_ARGS);
     else if (nr == 2) launch_scores<QT, 2>(FQ_ARGS);
     else if (nr == 3) launch_scores<QT, 3>(FQ_ARGS);
@@ -214,7 +336,7 @@ int page_scores_int4_launch(
     const void* Q, int q_dtype, int64_t q_sb, int64_t q_sh,
     const void* K_scale, const void* K_mn, int64_t km_sb, int64_t km_sh, int64_t km_sp,
     int B, int Hq, int Hkv, int P, int D,
-    float* scores, int64_t sc_sb, int64_t sc_sh, void* stream, const DynPos& dp, float levels) {
+    float* scores, int64_t sc_sb, int64_t sc_sh, void* stream, const DynPos& dp, float levels, const QuantParams* append, int append_dtype) {
     const char* fn = levels == 255.0f ? "fq_page_scores_int8" : "fq_page_scores_int4";
     FQ_CHECK_ARG(B > 0 && Hq > 0 && Hkv > 0 && P >= 0, FQ_ERR_ARG, "%s: bad sizes", fn);
     FQ_CHECK_ARG(Hq % Hkv == 0, FQ_ERR_ARG, "%s: H_q=%d must be divisible by H_kv=%d", fn, Hq, Hkv);
@@ -230,10 +352,21 @@ int page_scores_int4_launch(
     const int CH = D <= 64 ? 1 : D / 64;
     dim3 grid((unsigned)((P + SCORE_PAGES_PER_CTA - 1) / SCORE_PAGES_PER_CTA), (unsigned)Hkv, (unsigned)B);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // query heads of a group are served four at a time (one pass over the metadata per four)
+    DynAppend app{};
+    if (append) {
+        FQ_CHECK_ARG(page_scores_take_append(q_dtype, B, Hq, Hkv, P, D) && (append_dtype == FQ_F16 || append_dtype == FQ_BF16) && append->n_layers == 1, FQ_ERR_ARG,
+                     "%s: an append that this launch does not take", fn);
+        const QuantParams& q = *append;
+        app.q = q; app.bf16 = append_dtype == FQ_BF16;
+        const int64_t first = q.pos ? 0 : q.n_head * q.st_ss;
+        app.st = StageAppend{static_cast<const uint16_t*>(q.K_new), static_cast<const uint16_t*>(q.V_new), q.nw_sb, q.nw_sh, q.nw_ss,
+                             static_cast<uint16_t*>(q.stage_K) + first, static_cast<uint16_t*>(q.stage_V) + first, q.st_sb, q.st_sh, q.st_ss, q.n_new};
+    }
+    // query heads of a group are served four at a time (one pass over the metadata per four); the first pass appends, the others
+    // find the page completed
     for (int off = 0; off < n_rep; off += 4) {
         const int nr = n_rep - off < 4 ? n_rep - off : 4;
-#define FQ_ARGS nr, CH, grid, st, Q, q_sb, q_sh, K_scale, K_mn, km_sb, km_sh, km_sp, Hq, Hkv, P, D, off, scores, sc_sb, sc_sh, dp, levels
+#define FQ_ARGS nr, CH, grid, st, Q, q_sb, q_sh, K_scale, K_mn, km_sb, km_sh, km_sp, Hq, Hkv, P, D, off, scores, sc_sb, sc_sh, dp, levels, append && off == 0 ? &app : nullptr
         if (q_dtype == FQ_F32) launch_scores_nr<float>(FQ_ARGS);
         else if (q_dtype == FQ_F16) launch_scores_nr<__half>(FQ_ARGS);
         else launch_scores_nr<__nv_bfloat16>(FQ_ARGS);

@@ -122,7 +122,7 @@ class _NativeSteps:
 
 
 class QuestDecodeInt4(_NativeSteps):
-    LAUNCHES = 4
+    LAUNCHES = 3          # one more where the append completes a page
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4,
                  window_pages: int = 2, head_pattern_layer: torch.Tensor | None = None,
@@ -206,7 +206,7 @@ class QuestDecodeInt4(_NativeSteps):
             ptr(self.workspace), self.workspace.stride(0), self.workspace.shape[1], stream_ptr(self.device)))
         for li in range(Ln):
             c._seen_tokens[li] += n_new
-        self.launches += 4 * Ln
+        self.launches += self.LAUNCHES       # all layers together where they are of equal length
         return self.O.unsqueeze(3), self.lse.unsqueeze(3)
 
     def capture_step_graph(self, k_new: torch.Tensor, v_new: torch.Tensor, q: torch.Tensor, before=None, after=None):
@@ -311,7 +311,7 @@ class QuestDecodeTurbo(_NativeSteps):
     foreign call per layer (fq_decode_layer_turbo): append, page scores from the raw page metadata,
     top-k + compact index, rotation of Q, sparse attention in the rotated basis, rotation of O, tail
     attention and LSE merge.  All buffers are preallocated, a part for each layer."""
-    LAUNCHES = 10
+    LAUNCHES = 7
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,
                  q_dtype=torch.bfloat16, n_split: int | None = None):
@@ -354,7 +354,7 @@ class QuestDecodeInt8(_NativeSteps):
     """Decode-branch dispatcher for the persistent INT8 cache: the kv_bits == 8 route of make_quest_persistent_forward
     (flashquest/eager/llama_persistent_patch.py:202-245) as ONE foreign call per layer (fq_decode_layer_int8): append, page
     scores, top-k with compact index, attention with the staged tail in the same softmax."""
-    LAUNCHES = 5
+    LAUNCHES = 4
     COPY_ROWS = True
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,

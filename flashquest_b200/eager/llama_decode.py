@@ -157,7 +157,7 @@ class LlamaInt4Decoder:
                                          seen, ptr(x), self.B, ctypes.byref(self._scratch), stream_ptr(self.dev)))
         for li in range(n_l):
             c._seen_tokens[li] += 1
-        self.launches += 8 * n_l + 3
+        self.launches += 7 * n_l + 3
         return self.next_ids
 
     def prefill(self, token_ids: torch.Tensor) -> torch.Tensor:
@@ -186,7 +186,7 @@ class LlamaInt4Decoder:
                                      ptr(ws), nbytes, ptr(self.logits), ptr(self.next_ids), stream_ptr(self.dev)))
         for li in range(c.layers):
             cache._seen_tokens[li] = S
-        self.launches += 11 * c.layers + 3
+        self.launches += 10 * c.layers + 3
         return self.next_ids
 
     # -- thin wrappers over the C ABI ------------------------------------------------------
@@ -231,7 +231,7 @@ class LlamaInt4Decoder:
             graph.replay()
             for li in range(n_l):
                 c._seen_tokens[li] += 1
-            self.launches += 8 * n_l + 4
+            self.launches += 7 * n_l + 4
             return ids
 
         replay.graph, replay.ids, replay.pos = graph, ids, pos

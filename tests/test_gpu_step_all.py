@@ -70,3 +70,35 @@ def test_layers_together_equal_layers_alone(B, Ln, Hq, Hkv, D, page, seen, n, fo
         else:
             a, b = a[:, :, :, :ca._seen_tokens[0] - done], b[:, :, :, :ca._seen_tokens[0] - done]
         assert bit_equal(a, b), name
+
+
+@pytest.mark.parametrize("bits", [3, 4, 8])
+@pytest.mark.parametrize("B,Hq,Hkv,D,page,seen,n", [(1, 24, 8, 128, 16, 40, 1), (2, 32, 8, 64, 64, 130, 1), (3, 6, 2, 128, 16, 160, 15),
+                                                    (1, 12, 2, 128, 32, 66, 7), (2, 8, 8, 64, 16, 31, 1), (1, 24, 8, 128, 64, 127, 64)])
+def test_rows_staged_with_the_scores(bits, B, Hq, Hkv, D, page, seen, n):
+    """A step whose tokens complete no page stages them in the launch of the scores (the last two complete one, in a launch of
+    their own): the staged rows, and what the same step gives after an append by itself."""
+    from flashquest_b200.cache.persistent_int4 import PersistentInt4KVCache
+    from flashquest_b200.cache.persistent_int8 import PersistentInt8KVCache
+    from flashquest_b200.cache.persistent_turbo import PersistentTurboKVCache
+    from flashquest_b200.eager.decode_step import QuestDecodeInt4, QuestDecodeInt8, QuestDecodeTurbo
+    C, E = {3: (PersistentTurboKVCache, QuestDecodeTurbo), 4: (PersistentInt4KVCache, QuestDecodeInt4), 8: (PersistentInt8KVCache, QuestDecodeInt8)}[bits]
+    k0, v0 = (make_kv(i, (B, Hkv, seen, D), torch.float16).cuda() for i in (1, 2))
+    k, v = (make_kv(i, (B, Hkv, 2 * n, D), torch.float16).cuda()[:, :, ::2] for i in (3, 4))
+    q = make_q(5, (B, Hq, 1, D), torch.float16).cuda()
+    outs = []
+    for along in (True, False):
+        cache = C(batch_size=B, num_layers=2, num_kv_heads=Hkv, head_dim=D, max_seq_len=(seen + n) // page * page + 2 * page, page_size=page,
+                  device="cuda", dtype=torch.float16)
+        step = E(cache, num_q_heads=Hq, retention=0.5, num_sinks=1, window_pages=1, q_dtype=torch.float16)
+        cache.update_quantized(k0, v0, 1)
+        if along:
+            O, lse = step.step(k, v, q, 1)
+        else:
+            cache.update_quantized(k, v, 1)
+            O, lse = step.step(k[:, :, :0], v[:, :, :0], q, 1)
+        left = (seen + n) % page
+        outs.append((O.clone(), lse.clone(), cache.K_partial[1, :, :, :left].clone(), cache.V_partial[1, :, :, :left].clone()))
+        if left and left >= n:
+            assert bit_equal(outs[-1][2][:, :, left - n:], k) and bit_equal(outs[-1][3][:, :, left - n:], v)
+    assert all(bit_equal(a, b) for a, b in zip(*outs))
