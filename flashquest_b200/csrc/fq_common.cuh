@@ -119,6 +119,17 @@ int sparse_decode_int4_launch(
     void* workspace, size_t workspace_bytes, int n_split, void* stream, const DynPos& dp, const int32_t* list_count = nullptr,
     const WorkspaceParts& parts = WorkspaceParts{});
 
+int sparse_decode_turbo_launch(
+    const void* Q, int q_dtype, int64_t q_sb, int64_t q_sh,
+    const uint8_t* K_msb, int64_t km_sb, int64_t km_sh, int64_t km_ss, const uint8_t* K_lsb, int64_t kl_sb, int64_t kl_sh, int64_t kl_ss,
+    const void* K_scale, int64_t ks_sb, int64_t ks_sh,
+    const uint8_t* V_msb, int64_t vm_sb, int64_t vm_sh, int64_t vm_ss, const uint8_t* V_lsb, int64_t vl_sb, int64_t vl_sh, int64_t vl_ss,
+    const void* V_scale, int64_t vs_sb, int64_t vs_sh, const int32_t* compact, int64_t cp_sb, int64_t cp_sh, int bucket,
+    int B, int Hq, int Hkv, int S_kv, int P, int D, int page, float sm_scale,
+    void* O_rot, int64_t o_sb, int64_t o_sh, float* lse, void* workspace, size_t workspace_bytes, int n_split, void* stream, bool rotate_q);
+int turbo_finish_launch(const void* O_rot, const float* lse_rot, const void* Q, int q_dtype, const void* K_tail, const void* V_tail, int tail_dtype,
+                        int64_t tl_sb, int64_t tl_sh, int64_t tl_ss, int tail_len, int B, int Hq, int Hkv, int D, float sm_scale, void* O, float* lse, void* stream);
+
 // One layer of the graph-capturable step (append + score + select + attend with the sequence
 // length read from *pos) and the closing increment of the positions; defined in fq_decode_layer.cu.
 int decode_layer_int4_dyn(const fq_int4_cache* c, int layer, const int* pos, const void* K_new, const void* V_new,

@@ -54,9 +54,7 @@ extern "C" int fq_decode_layer_turbo(
     }
     const int64_t rows = (int64_t)B * Hq;
     char* sb = static_cast<char*>(scratch);
-    void* Q_rot = sb;
     void* O_rot = sb + rows * D * 2;
-    char* O_parts = sb + rows * D * 4;
     float* lse_parts = reinterpret_cast<float*>(sb + ((rows * D * 8 + 255) & ~(int64_t)255));
     const bool sparse = P > 0, both = sparse && tail > 0;
     if (sparse) {
@@ -67,27 +65,22 @@ extern "C" int fq_decode_layer_turbo(
         rc = fq_select_pages(scores, (int64_t)Hq * P, P, B, Hq, P, prm->retention_per_head, prm->retention, k_max, prm->sinks, prm->window,
                              nullptr, 0, 0, compact, (int64_t)Hq * prm->bucket, prm->bucket, prm->bucket, nullptr, stream);
         if (rc != FQ_OK) return rc;
-        if ((rc = fq_wht(Q, Q_rot, q_dtype, rows, D, stream)) != FQ_OK) return rc;
         int n_split = prm->n_split > 0 ? prm->n_split : fq_sparse_decode_default_splits(B, Hq, prm->bucket, page);
         if (n_split > 64) n_split = 64;
-        rc = fq_sparse_decode_turbo(Q_rot, q_dtype, (int64_t)Hq * D, D,
+        // Q is rotated by the attention's own CTAs
+        rc = sparse_decode_turbo_launch(Q, q_dtype, (int64_t)Hq * D, D,
                                     Kms, c->ms_sb, c->ms_sh, c->ms_ss, Kls, c->ls_sb, c->ls_sh, c->ls_ss, Kst, c->st_sb, c->st_sh,
                                     Vms, c->ms_sb, c->ms_sh, c->ms_ss, Vls, c->ls_sb, c->ls_sh, c->ls_ss, Vst, c->st_sb, c->st_sh,
                                     compact, (int64_t)Hq * prm->bucket, prm->bucket, prm->bucket,
                                     B, Hq, Hkv, completed, P, D, page, prm->sm_scale,
-                                    O_rot, (int64_t)Hq * D, D, both ? lse_parts : lse, workspace, workspace_bytes, n_split, stream);
+                                    O_rot, (int64_t)Hq * D, D, both ? lse_parts : lse, workspace, workspace_bytes, n_split, stream, true);
         if (rc != FQ_OK) return rc;
-        if ((rc = fq_wht(O_rot, both ? static_cast<void*>(O_parts) : O, q_dtype, rows, D, stream)) != FQ_OK) return rc;
+        if (both)
+            return turbo_finish_launch(O_rot, lse_parts, Q, q_dtype, Kt, Vt, c->kv_dtype, c->pt_sb, c->pt_sh, c->pt_ss, tail, B, Hq, Hkv, D, prm->sm_scale, O, lse, stream);
+        return fq_wht(O_rot, O, q_dtype, rows, D, stream);
     }
-    if (tail > 0 || !sparse) {
-        // dense attention over the staged tokens: the tail-only case of the INT4 kernel (no pages)
-        rc = fq_sparse_decode_int4(Q, q_dtype, q_sb, q_sh, nullptr, 0, 0, nullptr, nullptr, 0, 0, 0, nullptr, 0, 0, nullptr, nullptr, 0, 0,
-                                   nullptr, 0, 0, 0, tail ? Kt : nullptr, tail ? Vt : nullptr, c->kv_dtype, c->pt_sb, c->pt_sh, c->pt_ss, tail,
-                                   B, Hq, Hkv, 0, 0, D, page < 16 ? 16 : page, prm->sm_scale,
-                                   both ? static_cast<void*>(O_parts + rows * D * 2) : O, (int64_t)Hq * D, D, both ? lse_parts + rows : lse,
-                                   nullptr, 0, 1, stream);
-        if (rc != FQ_OK) return rc;
-    }
-    if (both) return fq_lse_merge(O_parts, lse_parts, q_dtype, 2, rows, D, O, lse, stream);
-    return FQ_OK;
+    // no page yet: dense attention over the staged tokens, the tail-only case of the INT4 kernel
+    return fq_sparse_decode_int4(Q, q_dtype, q_sb, q_sh, nullptr, 0, 0, nullptr, nullptr, 0, 0, 0, nullptr, 0, 0, nullptr, nullptr, 0, 0,
+                                 nullptr, 0, 0, 0, tail ? Kt : nullptr, tail ? Vt : nullptr, c->kv_dtype, c->pt_sb, c->pt_sh, c->pt_ss, tail,
+                                 B, Hq, Hkv, 0, 0, D, page < 16 ? 16 : page, prm->sm_scale, O, (int64_t)Hq * D, D, lse, nullptr, 0, 1, stream);
 }

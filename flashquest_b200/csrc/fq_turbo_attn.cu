@@ -15,6 +15,7 @@
 #include <atomic>
 
 #include "fq_common.cuh"
+#include "fq_wht.cuh"
 
 namespace fq {
 
@@ -25,7 +26,8 @@ constexpr float TQ_LOG2E = 1.4426950408889634f;
 constexpr float TQ_LN2 = 0.6931471805599453f;
 
 struct TurboAttnParams {
-    const void* Q; int64_t q_sb, q_sh;                     // rotated Q (B,Hq,D)
+    const void* Q; int64_t q_sb, q_sh;                     // Q (B,Hq,D): rotated, or to be rotated here
+    int rotate_q;                                          // (in front of the dependency wait: Q is older than the kernel before)
     const uint8_t *K_msb, *K_lsb, *V_msb, *V_lsb;
     int64_t km_sb, km_sh, km_ss, kl_sb, kl_sh, kl_ss, vm_sb, vm_sh, vm_ss, vl_sb, vl_sh, vl_ss;
     const uint16_t *K_scale, *V_scale; int64_t ks_sb, ks_sh, vs_sb, vs_sh;   // (B,Hkv,S) bf16, token stride 1
@@ -119,6 +121,15 @@ __global__ void __launch_bounds__(TQ_THREADS, 3) sparse_decode_turbo_kernel(Turb
             s_lut[i] = make_float2(va, vb);
         }
     }
+    __shared__ QT s_q[D];
+    if (p.rotate_q && warp == TQ_WARPS - 1) {
+        constexpr int EPL = D / 32;
+        float v[EPL];
+        load_row<QT, EPL>(static_cast<const QT*>(p.Q) + b * p.q_sb + hq * p.q_sh, lane, D, v);
+        wht_lanes<QT, EPL>(v, lane, D);
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) s_q[lane * EPL + j] = from_f32<QT>(v[j]);
+    }
     __syncthreads();
     pdl_wait();        // the rotated Q and the page list come from the kernels before this one
     pdl_trigger();
@@ -126,7 +137,7 @@ __global__ void __launch_bounds__(TQ_THREADS, 3) sparse_decode_turbo_kernel(Turb
 
     float2 q2[4];      // this lane's 8 channels of q * sm_scale * log2(e)
     {
-        const QT* qp = static_cast<const QT*>(p.Q) + b * p.q_sb + hq * p.q_sh + 8 * c;
+        const QT* qp = p.rotate_q ? s_q + 8 * c : static_cast<const QT*>(p.Q) + b * p.q_sb + hq * p.q_sh + 8 * c;
         const float sc = p.sm_scale * TQ_LOG2E;
 #pragma unroll
         for (int j = 0; j < 4; ++j) q2[j] = make_float2(Dt<QT>::to_f32(qp[2 * j]) * sc, Dt<QT>::to_f32(qp[2 * j + 1]) * sc);
@@ -394,6 +405,128 @@ __global__ void __launch_bounds__(TQ_THREADS, 3) sparse_decode_turbo_kernel(Turb
     }
 }
 
+// What follows the attention over the rotated pages in a decode step with staged tokens: the rotation of O back, the dense attention
+// over the staged tokens and the LSE merge of the two, in one launch with the arithmetic of the three (fq_wht, the tail-only
+// fq_sparse_decode_int4 and fq_lse_merge, 13 us of 245 for 16 x 32k and a third of a step over 500 tokens).  One warp per row; the staged
+// tokens are older than the kernel before and are attended while it runs.
+struct TurboFinishParams {
+    const void *O_rot; const float* lse_rot;               // (rows, D) dense, (rows)
+    const void* Q; const void *K_tail, *V_tail; int tail_dtype; int64_t tl_sb, tl_sh, tl_ss; int tail_len;
+    int64_t rows; int Hq, n_rep;
+    float sm_scale;
+    void* O; float* lse;
+};
+
+template <typename T, int D>
+__global__ void __launch_bounds__(128) turbo_finish_kernel(TurboFinishParams p) {
+    constexpr int EPL = D / 32, NS = 4;                    // four states, state w takes staged tokens w, w + 4, ...
+    const int lane = threadIdx.x & 31;
+    const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    const bool live = r < p.rows;
+    float o2[EPL], lse2 = -INFINITY;
+    if (live) {
+        const int b = (int)(r / p.Hq), hq = (int)(r % p.Hq);
+        float q[EPL], tm[NS], tl[NS], tacc[NS][EPL];
+        const T* qp = static_cast<const T*>(p.Q) + r * D + EPL * lane;
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) q[j] = Dt<T>::to_f32(qp[j]) * (p.sm_scale * TQ_LOG2E);
+#pragma unroll
+        for (int w = 0; w < NS; ++w) {
+            tm[w] = -INFINITY; tl[w] = 0.f;
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) tacc[w][j] = 0.f;
+        }
+        const int64_t head = b * p.tl_sb + (hq / p.n_rep) * p.tl_sh + EPL * lane;
+        for (int t0 = 0; t0 < p.tail_len; t0 += NS) {
+            float kv[NS][EPL], vv[NS][EPL], s[NS];
+#pragma unroll
+            for (int w = 0; w < NS; ++w) {
+                const int64_t ro = head + (int64_t)min(t0 + w, p.tail_len - 1) * p.tl_ss;
+                s[w] = 0.f;
+#pragma unroll
+                for (int j = 0; j < EPL; ++j) {
+                    if (p.tail_dtype == FQ_BF16) {
+                        kv[w][j] = Dt<__nv_bfloat16>::to_f32(static_cast<const __nv_bfloat16*>(p.K_tail)[ro + j]);
+                        vv[w][j] = Dt<__nv_bfloat16>::to_f32(static_cast<const __nv_bfloat16*>(p.V_tail)[ro + j]);
+                    } else {
+                        kv[w][j] = Dt<__half>::to_f32(static_cast<const __half*>(p.K_tail)[ro + j]);
+                        vv[w][j] = Dt<__half>::to_f32(static_cast<const __half*>(p.V_tail)[ro + j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int w = 0; w < NS; ++w)
+#pragma unroll
+                for (int j = 0; j < EPL; ++j) s[w] = fmaf(q[j], kv[w][j], s[w]);
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+                for (int w = 0; w < NS; ++w) s[w] += __shfl_xor_sync(0xffffffffu, s[w], off);
+#pragma unroll
+            for (int w = 0; w < NS; ++w) {
+                if (t0 + w < p.tail_len) {
+                    const float mnew = fmaxf(tm[w], s[w]);
+                    const float al = tq_ex2(tm[w] - mnew), pr = tq_ex2(s[w] - mnew);
+                    tl[w] = tl[w] * al + pr;
+#pragma unroll
+                    for (int j = 0; j < EPL; ++j) tacc[w][j] = fmaf(pr, vv[w][j], tacc[w][j] * al);
+                    tm[w] = mnew;
+                }
+            }
+        }
+        float mx = tm[0], wl[NS], wg[NS];
+#pragma unroll
+        for (int w = 1; w < NS; ++w) mx = fmaxf(mx, tm[w]);
+#pragma unroll
+        for (int w = 0; w < NS; ++w) { wg[w] = mx == -INFINITY ? 0.f : tq_ex2(tm[w] - mx); wl[w] = tl[w] * wg[w]; }
+        const float l = (wl[0] + wl[2]) + (wl[1] + wl[3]);
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+            float a = 0.f;
+#pragma unroll
+            for (int w = 0; w < NS; ++w) a = fmaf(tacc[w][j], wg[w], a);
+            o2[j] = Dt<T>::rn(l > 0.f ? a / l : 0.f);
+        }
+        lse2 = l > 0.f ? (mx + log2f(l)) * TQ_LN2 : -INFINITY;
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (!live) return;
+    float o1[EPL];
+    load_row<T, EPL>(static_cast<const T*>(p.O_rot) + r * D, lane, D, o1);
+    const float lse1 = p.lse_rot[r];
+    wht_lanes<T, EPL>(o1, lane, D);
+    T* O = static_cast<T*>(p.O) + r * D + EPL * lane;
+    const float m = fmaxf(lse1, lse2);
+    if (m == -INFINITY) {
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) O[j] = from_f32<T>(0.f);
+        if (lane == 0 && p.lse) p.lse[r] = -INFINITY;
+        return;
+    }
+    const float w1 = expf(lse1 - m), w2 = expf(lse2 - m);
+    float wsum = 0.f;
+    wsum += w1; wsum += w2;
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) {
+        float a = 0.f;
+        a = fmaf(w1, o1[j], a);
+        a = fmaf(w2, o2[j], a);
+        O[j] = from_f32<T>(a / wsum);
+    }
+    if (lane == 0 && p.lse) p.lse[r] = m + logf(wsum);
+}
+
+int turbo_finish_launch(const void* O_rot, const float* lse_rot, const void* Q, int q_dtype, const void* K_tail, const void* V_tail, int tail_dtype,
+                        int64_t tl_sb, int64_t tl_sh, int64_t tl_ss, int tail_len, int B, int Hq, int Hkv, int D, float sm_scale, void* O, float* lse, void* stream) {
+    TurboFinishParams p{O_rot, lse_rot, Q, K_tail, V_tail, tail_dtype, tl_sb, tl_sh, tl_ss, tail_len, (int64_t)B * Hq, Hq, Hq / Hkv, sm_scale, O, lse};
+    void (*kern)(TurboFinishParams) = q_dtype == FQ_F16 ? (D == 128 ? turbo_finish_kernel<__half, 128> : turbo_finish_kernel<__half, 64>)
+                                                        : (D == 128 ? turbo_finish_kernel<__nv_bfloat16, 128> : turbo_finish_kernel<__nv_bfloat16, 64>);
+    launch_k(PDL_ATTN, kern, dim3((unsigned)((p.rows + 3) / 4)), dim3(128), 0, static_cast<cudaStream_t>(stream), p);
+    FQ_CHECK_LAUNCH("fq_decode_layer_turbo");
+    return FQ_OK;
+}
+
 // _merge_two_attentions (eager/llama_persistent_patch.py:50-61) for n parts:
 // O = sum_i exp(lse_i - m) O_i / sum_i exp(lse_i - m), lse = m + log(sum).  One warp per row.
 template <typename T>
@@ -424,7 +557,8 @@ __global__ void __launch_bounds__(128) lse_merge_kernel(const T* __restrict__ O_
 
 }  // namespace fq
 
-extern "C" int fq_sparse_decode_turbo(
+namespace fq {
+int sparse_decode_turbo_launch(
     const void* Q_rot, int q_dtype, int64_t q_sb, int64_t q_sh,
     const uint8_t* K_msb, int64_t km_sb, int64_t km_sh, int64_t km_ss,
     const uint8_t* K_lsb, int64_t kl_sb, int64_t kl_sh, int64_t kl_ss,
@@ -435,8 +569,7 @@ extern "C" int fq_sparse_decode_turbo(
     const int32_t* compact, int64_t cp_sb, int64_t cp_sh, int bucket,
     int B, int Hq, int Hkv, int S_kv, int P, int D, int page, float sm_scale,
     void* O_rot, int64_t o_sb, int64_t o_sh, float* lse,
-    void* workspace, size_t workspace_bytes, int n_split, void* stream) {
-    using namespace fq;
+    void* workspace, size_t workspace_bytes, int n_split, void* stream, bool rotate_q) {
     const char* fn = "fq_sparse_decode_turbo";
     FQ_CHECK_ARG(B > 0 && Hq > 0 && Hkv > 0 && S_kv >= 0 && P >= 0 && bucket >= 0, FQ_ERR_ARG, "%s: bad sizes", fn);
     FQ_CHECK_ARG(B <= 65535 && Hq <= 65535, FQ_ERR_ARG, "%s: B and H_q must be <= 65535", fn);
@@ -454,6 +587,7 @@ extern "C" int fq_sparse_decode_turbo(
     TurboAttnParams p;
     for (int j = 0; j < 4; ++j) p.m_mul[j] = 1u << (12 - 2 * j);
     p.l_mul[0] = 1u << 8; p.l_mul[1] = 1u << 4;
+    p.rotate_q = rotate_q ? 1 : 0;
     p.Q = Q_rot; p.q_sb = q_sb; p.q_sh = q_sh;
     p.K_msb = K_msb; p.K_lsb = K_lsb; p.V_msb = V_msb; p.V_lsb = V_lsb;
     p.km_sb = km_sb; p.km_sh = km_sh; p.km_ss = km_ss; p.kl_sb = kl_sb; p.kl_sh = kl_sh; p.kl_ss = kl_ss;
@@ -499,6 +633,25 @@ extern "C" int fq_sparse_decode_turbo(
     launch_k(PDL_ATTN, kern, grid, dim3(TQ_THREADS), smem, st, p);
     FQ_CHECK_LAUNCH(fn);
     return FQ_OK;
+}
+
+}  // namespace fq
+
+extern "C" int fq_sparse_decode_turbo(
+    const void* Q_rot, int q_dtype, int64_t q_sb, int64_t q_sh,
+    const uint8_t* K_msb, int64_t km_sb, int64_t km_sh, int64_t km_ss,
+    const uint8_t* K_lsb, int64_t kl_sb, int64_t kl_sh, int64_t kl_ss,
+    const void* K_scale, int64_t ks_sb, int64_t ks_sh,
+    const uint8_t* V_msb, int64_t vm_sb, int64_t vm_sh, int64_t vm_ss,
+    const uint8_t* V_lsb, int64_t vl_sb, int64_t vl_sh, int64_t vl_ss,
+    const void* V_scale, int64_t vs_sb, int64_t vs_sh,
+    const int32_t* compact, int64_t cp_sb, int64_t cp_sh, int bucket,
+    int B, int Hq, int Hkv, int S_kv, int P, int D, int page, float sm_scale,
+    void* O_rot, int64_t o_sb, int64_t o_sh, float* lse,
+    void* workspace, size_t workspace_bytes, int n_split, void* stream) {
+    return fq::sparse_decode_turbo_launch(Q_rot, q_dtype, q_sb, q_sh, K_msb, km_sb, km_sh, km_ss, K_lsb, kl_sb, kl_sh, kl_ss, K_scale, ks_sb, ks_sh,
+                                          V_msb, vm_sb, vm_sh, vm_ss, V_lsb, vl_sb, vl_sh, vl_ss, V_scale, vs_sb, vs_sh, compact, cp_sb, cp_sh, bucket,
+                                          B, Hq, Hkv, S_kv, P, D, page, sm_scale, O_rot, o_sb, o_sh, lse, workspace, workspace_bytes, n_split, stream, false);
 }
 
 extern "C" int fq_lse_merge(const void* O_parts, const float* lse_parts, int dtype, int n, int64_t rows, int D,

@@ -311,7 +311,7 @@ class QuestDecodeTurbo(_NativeSteps):
     foreign call per layer (fq_decode_layer_turbo): append, page scores from the raw page metadata,
     top-k + compact index, rotation of Q, sparse attention in the rotated basis, rotation of O, tail
     attention and LSE merge.  All buffers are preallocated, a part for each layer."""
-    LAUNCHES = 7
+    LAUNCHES = 4
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,
                  q_dtype=torch.bfloat16, n_split: int | None = None):
