@@ -268,13 +268,22 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int l = lane & 7, qw = lane >> 3;
     const float c = p.sm_scale * I8_LOG2E;
+    // Codes as fp32 operands with one integer instruction each: a byte masked in place and read as an fp32 (sub)normal is
+    // code * 2^(8 k - 149) for byte k = 0..2, a shift brings byte 3 to the bottom.  The power of two goes into the multiplier, which
+    // 2^80 keeps away from both ends of the range (scales up to 1e14).  A conversion by byte permute and subtraction and one FMA per
+    // code instead: 44 us for 4 x 20k tokens of 24/8 heads; this 40 (waiting for its loads most of the time).
+    auto up = [](int k) { return __int_as_float((127 + (k < 3 ? 80 - 8 * k : 80)) << 23); };           // 2^80 / 2^(8 k)
+    auto down = [](int k) { return __int_as_float((127 - (k < 3 ? 80 - 8 * k : 80)) << 23); };         // its reciprocal
+    auto home = [](int k) { return __int_as_float((127 + (k < 3 ? 69 - 8 * k : 69)) << 23); };         // 2^149 / 2^80 / 2^(8 k): a sum over codes
+    pdl_wait();        // the page list comes from the kernel before
     pdl_trigger();     // the merge may become resident
-    float q[DPL];
+    float q[DPL];      // times up()
 #pragma unroll
-    for (int j = 0; j < DPL; ++j) q[j] = i8_ld(p.Q, p.q_dtype, b * p.q_sb + hq * p.q_sh + DPL * l + j) * c;
-    float m = -INFINITY, lsum = 0.f, mnacc = 0.f, acc[DPL];
+    for (int j = 0; j < DPL; ++j) q[j] = i8_ld(p.Q, p.q_dtype, b * p.q_sb + hq * p.q_sh + DPL * l + j) * c * up(j & 3);
+    float m = -INFINITY, lsum = 0.f, mnacc = 0.f;
+    float2 acc[DPL / 2];
 #pragma unroll
-    for (int j = 0; j < DPL; ++j) acc[j] = 0.f;
+    for (int j = 0; j < DPL / 2; ++j) acc[j] = make_float2(0.f, 0.f);
     auto quarter_sum = [](float v) {
         v += __shfl_xor_sync(0xffffffffu, v, 4);
         v += __shfl_xor_sync(0xffffffffu, v, 2);
@@ -286,10 +295,8 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
         v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
         return v;
     };
-    // byte k of w as fp32: the byte becomes the low mantissa byte of 2^23 (one byte permute), which is then subtracted
-    auto code_f32 = [](uint32_t w, int k) -> float {
-        return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7540u | (unsigned)k)) - 8388608.0f;
-    };
+    auto low2 = [](uint32_t w) { return make_float2(__uint_as_float(w & 0xffu), __uint_as_float(w & 0xff00u)); };
+    auto high2 = [](uint32_t w) { return make_float2(__uint_as_float(w & 0xff0000u), __uint_as_float(w >> 24)); };
     auto load_codes = [&](const uint8_t* row, uint32_t (&w)[NW]) {
         if constexpr (NW == 4) { const uint4 u = *reinterpret_cast<const uint4*>(row); w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w; }
         else { const uint2 u = *reinterpret_cast<const uint2*>(row); w[0] = u.x; w[1] = u.y; }
@@ -314,7 +321,7 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 qs[8 * c8 + j] = q[8 * c8 + j] * sc8[j];
-                qmn = fmaf(q[8 * c8 + j], mn8[j], qmn);
+                qmn = fmaf(q[8 * c8 + j], mn8[j] * down(j & 3), qmn);
             }
         }
         qmn = quarter_sum(qmn);
@@ -333,13 +340,14 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
             float mx = -INFINITY;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                float a = 0.f;
+                float2 a = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int w = 0; w < NW; ++w)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) a = fmaf(qs[4 * w + k], code_f32(kw[u][w], k), a);
-                a = quarter_sum(a);
-                sc[u] = t0 + qw + 4 * u < t_end ? a + qmn : -INFINITY;
+                for (int w = 0; w < NW; ++w) {
+                    a = __ffma2_rn(low2(kw[u][w]), make_float2(qs[4 * w], qs[4 * w + 1]), a);
+                    a = __ffma2_rn(high2(kw[u][w]), make_float2(qs[4 * w + 2], qs[4 * w + 3]), a);
+                }
+                const float dot = quarter_sum(a.x + a.y);
+                sc[u] = t0 + qw + 4 * u < t_end ? fmaf(dot, home(0), qmn) : -INFINITY;
                 mx = fmaxf(mx, sc[u]);
             }
             mx = warp_max4(mx);
@@ -347,21 +355,26 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
             const float al = i8_ex2(m - m_new);
             lsum *= al; mnacc *= al;
 #pragma unroll
-            for (int j = 0; j < DPL; ++j) acc[j] *= al;
+            for (int j = 0; j < DPL / 2; ++j) acc[j] = __fmul2_rn(acc[j], make_float2(al, al));
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const float pr = i8_ex2(sc[u] - m_new);        // 0 past the end
-                const float ps = pr * vs[u];
+                const float ps = pr * vs[u] * up(0);
+                const float2 ps2 = make_float2(ps, ps);
                 lsum += pr;
                 mnacc = fmaf(pr, vm[u], mnacc);
 #pragma unroll
-                for (int w = 0; w < NW; ++w)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) acc[4 * w + k] = fmaf(ps, code_f32(vw[u][w], k), acc[4 * w + k]);
+                for (int w = 0; w < NW; ++w) {
+                    acc[2 * w] = __ffma2_rn(low2(vw[u][w]), ps2, acc[2 * w]);
+                    acc[2 * w + 1] = __ffma2_rn(high2(vw[u][w]), ps2, acc[2 * w + 1]);
+                }
             }
             m = m_new;
         }
     }
+    float out[DPL];
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) out[j] = ((j & 1) ? acc[j / 2].y : acc[j / 2].x) * home(j & 3);
     // the staged (unquantised) tail belongs to split 0: a quarter warp per token
     if (split == 0) {
         for (int t0 = 4 * warp; t0 < p.tail_len; t0 += 16) {       // warp-uniform trip count
@@ -370,7 +383,7 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
             const int64_t ro = b * p.tl_sb + hkv * p.tl_sh + (int64_t)(live ? t : 0) * p.tl_ss + DPL * l;
             float a = 0.f;
 #pragma unroll
-            for (int j = 0; j < DPL; ++j) a = fmaf(q[j], i8_ld(p.K_tail, p.tail_dtype, ro + j), a);
+            for (int j = 0; j < DPL; ++j) a = fmaf(q[j] * down(j & 3), i8_ld(p.K_tail, p.tail_dtype, ro + j), a);
             a = quarter_sum(a);
             const float s = live ? a : -INFINITY;
             const float m_new = fmaxf(m, warp_max4(s));        // finite: token t0 is live
@@ -378,7 +391,7 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
             lsum = lsum * al + pr;
             mnacc *= al;
 #pragma unroll
-            for (int j = 0; j < DPL; ++j) acc[j] = fmaf(pr, live ? i8_ld(p.V_tail, p.tail_dtype, ro + j) : 0.f, acc[j] * al);
+            for (int j = 0; j < DPL; ++j) out[j] = fmaf(pr, live ? i8_ld(p.V_tail, p.tail_dtype, ro + j) : 0.f, out[j] * al);
             m = m_new;
         }
     }
@@ -388,12 +401,12 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
         lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
         mnacc += __shfl_xor_sync(0xffffffffu, mnacc, off);
 #pragma unroll
-        for (int j = 0; j < DPL; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
+        for (int j = 0; j < DPL; ++j) out[j] += __shfl_xor_sync(0xffffffffu, out[j], off);
     }
     if (lane == 0) { s_m[warp] = m; s_l[warp] = lsum; }
     if (qw == 0) {
 #pragma unroll
-        for (int j = 0; j < DPL; ++j) s_acc[warp][DPL * l + j] = acc[j] + mnacc;
+        for (int j = 0; j < DPL; ++j) s_acc[warp][DPL * l + j] = out[j] + mnacc;
     }
     __syncthreads();
     float mx = fmaxf(fmaxf(s_m[0], s_m[1]), fmaxf(s_m[2], s_m[3]));
@@ -573,8 +586,8 @@ extern "C" int fq_sparse_decode_int8_counted(
     // (An ordinary launch: one wave of CTAs that started early would settle unevenly around the selection's, 59 against 53 us for
     // a step of 4 x 20k.  The merge behind it starts early.)
     if (vec16) {
-        if (D == 128) sparse_decode_int8_q_kernel<128><<<grid, 128, 0, st>>>(p);
-        else sparse_decode_int8_q_kernel<64><<<grid, 128, 0, st>>>(p);
+        if (D == 128) launch_k(PDL_ATTN, sparse_decode_int8_q_kernel<128>, grid, dim3(128), 0, st, p);
+        else launch_k(PDL_ATTN, sparse_decode_int8_q_kernel<64>, grid, dim3(128), 0, st, p);
     } else {
         if (D == 128) sparse_decode_int8_kernel<128><<<grid, 128, 0, st>>>(p);
         else sparse_decode_int8_kernel<64><<<grid, 128, 0, st>>>(p);
