@@ -246,6 +246,10 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
                 if (r >= RS) { ++r; break; }                        // steady state: one raw request per x request
             }
             if (failed) break;
+            if (g == 0) {          // x is the previous kernel's; the weights never change and are on their way
+                pdl_wait();
+                pdl_trigger();
+            }
             if (xk == 0) locate(xt, xpj, xn0, xm0);
             if (gm_timeout(&x_empty[xs], xph)) { failed = true; break; }
             if (gm_elect()) {
@@ -389,6 +393,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
     } else {
         // =========================== epilogue ===========================
         const int lq = warp & 3;                      // the TMEM lane quarter this warp may read
+        pdl_wait();                                   // y may have been read by the kernel before
         int it = 0;
         for (int tile = pair; tile < total_tiles && !failed; tile += pairs, ++it) {
             int pj, n0, m0;
@@ -565,10 +570,12 @@ static int pairs_launch(const SkinnyCall& c, bool swiglu, void* stream, const ch
     if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: cannot reserve %d B of shared memory: %s", fn, GM_SMEM, cudaGetErrorString(e));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(2 * pairs)); cfg.blockDim = dim3(GM_THREADS); cfg.dynamicSmemBytes = GM_SMEM; cfg.stream = static_cast<cudaStream_t>(stream);
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-    cfg.attrs = &at; cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = pdl_enabled(PDL_GEMV) ? 2 : 1;
     e = cudaLaunchKernelEx(&cfg, kern, maps[0], maps[1], maps[2], maps[3], maps[4], p);
     if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: launch failed: %s", fn, cudaGetErrorString(e));
     FQ_CHECK_LAUNCH(fn);
