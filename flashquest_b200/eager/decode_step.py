@@ -4,7 +4,7 @@ Host-side counterpart of the decode branch of make_quest_persistent_forward
 (flashquest/eager/llama_persistent_patch.py:202-245): static k_max / BUCKET_MAX computed
 once (:77-85), per-head retention from a head pattern (:214-219), page scores from the
 metadata, top-k + compact index, sparse attention over the selected pages, and the staged
-tail merged in the same softmax.  Three kernel launches per layer, no allocation per step
+tail merged in the same softmax.  Three kernel launches per layer (the first one also appends), no allocation per step
 (all outputs preallocated), so a whole multi-layer step can be captured in a CUDA graph.
 """
 from __future__ import annotations
@@ -15,6 +15,7 @@ import math
 import torch
 
 from .._lib import DecodeParams, bind, check, dtype_code, lib, ptr, require_cuda, stream_ptr
+from ..kernel.sparse_fwd import int8_splits
 
 
 def _whole(nbytes: int) -> int:
@@ -179,7 +180,8 @@ class QuestDecodeInt4(_NativeSteps):
     def step_all(self, k_new: torch.Tensor, v_new: torch.Tensor, q: torch.Tensor):
         """step() for every layer in ONE foreign call (fq_decode_step_int4): k_new, v_new
         (L,B,H_kv,n,D) in the cache's dtype, q (L,B,H_q,1,D).  For callers that hold all layers'
-        projections at once (stacked independent layers); returns (O (L,B,H_q,1,D), lse (L,B,H_q,1))."""
+        projections at once (stacked independent layers): layers of one length go through the launches as one batch, whose attention
+        may merge fewer parts than a layer's own.  Returns (O (L,B,H_q,1,D), lse (L,B,H_q,1))."""
         c = self.cache
         Ln = c.num_layers
         n_new = k_new.shape[3]
@@ -380,8 +382,7 @@ class QuestDecodeInt8(_NativeSteps):
         self.compact = torch.empty(L, self.B, self.Hq, self.bucket, dtype=torch.int32, device=dev)
         self.O = torch.empty(L, self.B, self.Hq, self.D, dtype=q_dtype, device=dev)
         self.lse = torch.empty(L, self.B, self.Hq, dtype=torch.float32, device=dev)
-        # a warp should walk six pages at least, and about sixteen 128-thread CTAs per SM fill the GPU
-        self.n_split = n_split or max(1, min(64, self.bucket // 24, (16 * 148) // (self.B * self.Hq)))
+        self.n_split = n_split or int8_splits(self.B * self.Hq, self.bucket * self.page)
         self.workspace = torch.empty(L, _whole(lib().fq_sparse_decode_int8_workspace_bytes(self.B, self.Hq, self.D, self.n_split)),
                                      dtype=torch.uint8, device=dev)
         self._cdesc = cache.desc()

@@ -12,6 +12,23 @@ from ..eager.selection import build_compact_selection
 _SUPPORTED_HEAD_DIMS = (64, 128)
 
 
+def int8_splits(rows: int, tokens: int) -> int:
+    """Parts that the attention over `tokens` tokens of each of `rows` (sequence, query head) rows is split into: whole waves
+    of the four CTAs that fit an SM, as few as fill their last one to 0.85, and no part below 160 tokens (40 a warp), where
+    the merge costs more than it gives.  List, attention and merge with sixteen CTAs per SM and 96 list entries a part (24 of
+    a tight list), whatever the page size -> this rule, us, a quarter of the pages selected: 96 rows of 20k tokens in pages of
+    64 59 -> 42 (3 -> 6 parts; 8: 53), 24 rows of 8k 53 -> 16 (1 -> 12), 320 rows 74 -> 61 (1 -> 5), 432 rows 84 -> 77 (1 -> 4);
+    pages of 16, 384 rows of 32k 268 -> 254 (6 -> 3), 24 rows 34.1 -> 32.5 (21 -> 24; 32: 42), 96 rows of 8k 30 -> 28."""
+    slots, best, fill = 4 * 148, 1, 0.0
+    for waves in range(1, 5):
+        n = waves * slots // max(rows, 1)
+        if n * rows > fill * waves * slots:
+            best, fill = n, n * rows / (waves * slots)
+        if fill >= 0.85:
+            break
+    return max(1, min(64, best, tokens // 160))
+
+
 def flash_attn_sparse_fwd(Q, K_uint8, K_scale, K_mn, V_uint8, V_scale, V_mn, *, selection_mask, page_size: int = 64,
                           sm_scale=None, return_lse: bool = True, K_partial=None, V_partial=None, n_split=None):
     """Decode-only sparse forward with INT8 KV (kernel/sparse_fwd.py:140).
@@ -61,10 +78,7 @@ def flash_attn_sparse_fwd(Q, K_uint8, K_scale, K_mn, V_uint8, V_scale, V_mn, *, 
     O = torch.empty(B, H_q, D, dtype=Q.dtype, device=dev)
     L = torch.empty(B, H_q, dtype=torch.float32, device=dev) if return_lse else None
     if n_split is None:
-        # a warp should walk at least six to eight pages (the list made from a mask is as wide as the page count and
-        # about a quarter of it is real: one split per 96 entries at most), and about sixteen 128-thread CTAs per SM
-        # are enough to fill the GPU (measured at 2048 pages: 16-24 splits best at batch 1, 4-8 at batch 16)
-        n_split = max(1, min(64, bucket // 96, max(1, (16 * 148) // max(B * H_q, 1))))
+        n_split = int8_splits(B * H_q, bucket * int(page_size) // 4)      # a mask's list is as wide as the page count, about a quarter of it is real
     with torch.cuda.device(dev):
         ws = torch.empty(lib().fq_sparse_decode_int8_workspace_bytes(B, H_q, D, n_split), dtype=torch.uint8, device=dev)
         check(lib().fq_sparse_decode_int8_counted(

@@ -109,6 +109,18 @@ def test_attention_matches_oracle(dtype, B, Hq, Hkv, S, D, page):
     assert _lib.lib().fq_device_status() == 0
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,S,page,parts", [(1, 24, 8, 8192, 64, 12), (4, 24, 8, 2560, 64, 4), (1, 2, 1, 600, 16, 1), (1, 3, 1, 45056, 128, 64),
+                                                   (27, 16, 8, 2560, 64, 4)])
+def test_default_parts_match_oracle(B, Hq, Hkv, S, page, parts):
+    # whole waves of CTAs, 160 tokens a part at least, 64 parts at most; the bound is the attention's own
+    from flashquest_b200.kernel.sparse_fwd import flash_attn_sparse_fwd, int8_splits
+    assert int8_splits(B * Hq, S // 4) == parts
+    Q, kv, mask = _att_case(31, B, Hq, Hkv, S, 128, page, torch.bfloat16, retention=0.25)
+    Ow, lw = oracle.sparse_attn_int8(Q, *kv, selection_mask=mask, page_size=page)
+    O, lse = flash_attn_sparse_fwd(Q.cuda(), *[t.cuda() for t in kv], selection_mask=mask.cuda(), page_size=page)
+    _close(O, lse, Ow, lw, torch.bfloat16)
+
+
 @pytest.mark.parametrize("S_kv", [64, 96, 100, 128, 192, 1023])
 def test_partial_last_page(S_kv):
     # the reference's edge grid: S_kv not a multiple of the page size, every page selected
