@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
     // Codes as fp32 operands with one integer instruction each: a byte masked in place and read as an fp32 (sub)normal is
     // code * 2^(8 k - 149) for byte k = 0..2, a shift brings byte 3 to the bottom.  The power of two goes into the multiplier, which
     // 2^80 keeps away from both ends of the range (scales up to 1e14).  A conversion by byte permute and subtraction and one FMA per
-    // code instead: 44 us for 4 x 20k tokens of 24/8 heads; this 40 (waiting for its loads most of the time).
+    // code instead: 44 us for 4 x 20k tokens of 24/8 heads; this 40, both waiting for their loads most of the time.
     auto up = [](int k) { return __int_as_float((127 + (k < 3 ? 80 - 8 * k : 80)) << 23); };           // 2^80 / 2^(8 k)
     auto down = [](int k) { return __int_as_float((127 - (k < 3 ? 80 - 8 * k : 80)) << 23); };         // its reciprocal
     auto home = [](int k) { return __int_as_float((127 + (k < 3 ? 69 - 8 * k : 69)) << 23); };         // 2^149 / 2^80 / 2^(8 k): a sum over codes
@@ -308,27 +308,26 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
     const uint16_t* Vmn = p.V_mn + b * p.vm_sb + hkv * p.vm_sh;
     int n_list = p.bucket;
     if (p.list_count) n_list = max(0, min(n_list, __ldg(p.list_count + b * p.Hq + hq)));
-    for (int e = split + p.n_split * warp; e < n_list; e += p.n_split * 4) {
-        const int pg = list[e];
+    int e = split + p.n_split * warp, next = e < n_list ? list[e] : -1;
+    for (; e < n_list; e += p.n_split * 4) {
+        const int pg = next;             // the entry after it is requested a page ahead
+        if (e + p.n_split * 4 < n_list) next = list[e + p.n_split * 4];
         if (pg < 0 || pg >= p.P || pg * p.page >= p.S_kv) continue;
+        // Bound by the wait for loads (58 % of the warps' time) at the 16 warps that the registers leave an SM.  The list entry is
+        // requested a page ahead, the page's metadata and its first 16 tokens together, one round trip instead of three in a row:
+        // 16 x 32k tokens in pages of 16 225 -> 166 us, 4 x 20k in pages of 64 34.6 -> 32.3.  K codes a step ahead as well: 174 (or
+        // spilled); codes prefetched into L2 a page ahead without this: 229.
         const int64_t mo = b * p.km_sb + hkv * p.km_sh + (int64_t)pg * p.km_sp + DPL * l;
-        float qs[DPL], qmn = 0.f;
+        const int t_end = min((pg + 1) * p.page, p.S_kv);
+        uint4 scr[DPL / 8], mnr[DPL / 8];
 #pragma unroll
         for (int c8 = 0; c8 < DPL / 8; ++c8) {
-            float sc8[8], mn8[8];
-            load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(p.K_scale + mo) + 8 * c8, sc8);
-            load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(p.K_mn + mo) + 8 * c8, mn8);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                qs[8 * c8 + j] = q[8 * c8 + j] * sc8[j];
-                qmn = fmaf(q[8 * c8 + j], mn8[j] * down(j & 3), qmn);
-            }
+            scr[c8] = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.K_scale) + mo + 8 * c8);
+            mnr[c8] = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.K_mn) + mo + 8 * c8);
         }
-        qmn = quarter_sum(qmn);
-        const int t_end = min((pg + 1) * p.page, p.S_kv);
-        for (int t0 = pg * p.page; t0 < t_end; t0 += 16) {
-            uint32_t kw[4][NW], vw[4][NW];
-            float vs[4], vm[4], sc[4];
+        uint32_t kw[4][NW], vw[4][NW];
+        float vs[4], vm[4];
+        auto load_tokens = [&](int t0) {
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int t = min(t0 + qw + 4 * u, t_end - 1);      // past the end: a repeat of the last token, masked below
@@ -337,6 +336,22 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
                 vs[u] = bf16_lo(Vsc[t]);
                 vm[u] = bf16_lo(Vmn[t]);
             }
+        };
+        load_tokens(pg * p.page);
+        float qs[DPL], qmn = 0.f;
+#pragma unroll
+        for (int c8 = 0; c8 < DPL / 8; ++c8) {
+            const uint32_t sw[4] = {scr[c8].x, scr[c8].y, scr[c8].z, scr[c8].w}, mw[4] = {mnr[c8].x, mnr[c8].y, mnr[c8].z, mnr[c8].w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float sc = j & 1 ? bf16_hi(sw[j / 2]) : bf16_lo(sw[j / 2]), mn = j & 1 ? bf16_hi(mw[j / 2]) : bf16_lo(mw[j / 2]);
+                qs[8 * c8 + j] = q[8 * c8 + j] * sc;
+                qmn = fmaf(q[8 * c8 + j], mn * down(j & 3), qmn);
+            }
+        }
+        qmn = quarter_sum(qmn);
+        for (int t0 = pg * p.page;;) {
+            float sc[4];
             float mx = -INFINITY;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -370,6 +385,9 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
                 }
             }
             m = m_new;
+            t0 += 16;
+            if (t0 >= t_end) break;
+            load_tokens(t0);
         }
     }
     float out[DPL];

@@ -17,8 +17,8 @@ def int8_splits(rows: int, tokens: int) -> int:
     of the four CTAs that fit an SM, as few as fill their last one to 0.85, and no part below 160 tokens (40 a warp), where
     the merge costs more than it gives.  List, attention and merge with sixteen CTAs per SM and 96 list entries a part (24 of
     a tight list), whatever the page size -> this rule, us, a quarter of the pages selected: 96 rows of 20k tokens in pages of
-    64 59 -> 42 (3 -> 6 parts; 8: 53), 24 rows of 8k 53 -> 16 (1 -> 12), 320 rows 74 -> 61 (1 -> 5), 432 rows 84 -> 77 (1 -> 4);
-    pages of 16, 384 rows of 32k 268 -> 254 (6 -> 3), 24 rows 34.1 -> 32.5 (21 -> 24; 32: 42), 96 rows of 8k 30 -> 28."""
+    64 43 -> 34 (3 -> 6 parts; 8: 42), 24 rows of 8k 38 -> 14.5 (1 -> 12), 320 rows 55 -> 47 (1 -> 5), 432 rows 60 -> 59 (1 -> 4);
+    pages of 16, 384 rows of 32k 170 -> 169 (6 -> 3), 24 rows 26.4 -> 25.8 (21 -> 24; 32: 31), 96 rows of 8k 22.7 -> 21.3."""
     slots, best, fill = 4 * 148, 1, 0.0
     for waves in range(1, 5):
         n = waves * slots // max(rows, 1)
