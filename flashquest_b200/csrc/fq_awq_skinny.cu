@@ -1,8 +1,9 @@
-// AWQ W4A16 linears for 9 .. a few hundred rows on tcgen05: short prompts.
+// AWQ W4A16 linears for 9 .. a few hundred rows on tcgen05: short prompts (up to one wave of tiles, or three while one tile
+// holds all rows; beyond, the large GEMM in fq_awq_gemm.cu).
 //
 // y[M,N] = x[M,K] @ W with W in AutoAWQ's GEMM format.  The work is reading the weights (0.5 byte each) once; the grid of
-// 256-column tiles of the large GEMM leaves most SMs idle at few rows (12 of 148 for 3072 columns) and its three or four
-// stages wait for the TMA latency.  Here a CTA owns 128 columns and up to 128 rows, and every kind of data has a ring as deep
+// 256-column tiles of the large GEMM leaves most SMs idle at few rows (24 of 148 for 3072 columns) and its stages wait
+// for the TMA latency.  Here a CTA owns 128 columns and up to 128 rows, and every kind of data has a ring as deep
 // as its latency asks:
 //   warp 0       raw weight tiles (128 k x 128 columns = 8 KiB) by TMA, the first ones before the dependency wait (weights
 //                never change); scales and zeros by bulk copies

@@ -630,7 +630,10 @@ int fq_decode_layer_turbo(
  * (elements), workspace stride ws_sl (bytes; each layer needs its own split-K workspace).
  * seen[layer] (host array) is the number of tokens already in that layer; params is one
  * struct for all layers (params_stride 0) or an array of structs params_stride bytes apart.
- * Stops at the first failing layer and returns its error. */
+ * Layers of one length, with one params struct, in dense arrays (each layer stride is B times the batch stride) go through the
+ * launches together, as one batch of n_layers * B sequences: the attention may then be split into fewer parts than for one
+ * layer, and O and lse differ in their last bits.  Others go one by one; the call stops at the first failing layer and returns
+ * its error. */
 int fq_decode_step_int4(
     const fq_int4_cache* cache, int n_layers, const int* seen,
     const void* K_new, const void* V_new, int64_t nw_sl, int64_t nw_sb, int64_t nw_sh, int64_t nw_ss, int n_new,
@@ -681,9 +684,9 @@ int fq_argmax_f16(const void* x, int64_t rows, int N, int32_t* out, void* stream
 /* ------------------------------------------------------------------------------------
  * One greedy decode step of a Llama-shaped model in ONE foreign call: the decoder-layer loop
  * around eager/llama_persistent_patch.py:164-305 (Hugging Face's LlamaDecoderLayer / LlamaMLP /
- * LlamaRMSNorm semantics) issued from native code, 8 launches per layer and no host work
+ * LlamaRMSNorm semantics) issued from native code, 7 launches per layer and no host work
  * between them.  Per layer: fq_awq_gemv_fused (add+RMSNorm -> q/k/v -> RoPE), fq_decode_layer_int4
- * (append + score + select + attend), AWQ o GEMV, fq_awq_gemv_swiglu (add+RMSNorm -> gate/up -> SwiGLU),
+ * (append and score, select, attend), AWQ o GEMV, fq_awq_gemv_swiglu (add+RMSNorm -> gate/up -> SwiGLU),
  * down GEMV (one row: SwiGLU in front of down); then add+RMSNorm, fp16 lm_head GEMV, argmax.  fp16 model,
  * B <= 8 sequences.
  * All pointers inside the structs are device pointers except `layers` (host array). */
