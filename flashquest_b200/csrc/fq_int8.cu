@@ -130,18 +130,16 @@ __device__ __forceinline__ float i8_ld(const void* p, int dtype, int64_t i) {
     return dtype == FQ_F16 ? __half2float(static_cast<const __half*>(p)[i]) : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
 }
 
-// Grid (n_split, Hq, B), 4 warps.  A warp takes pages of the row's compact list (entry index = split + n_split * (warp +
-// 4 * i)); lane owns CPL = D/32 consecutive channels of every token.  Each CTA writes a normalised partial (O, lse).
+// Any alignment of the rows, any scales that fp32 holds the products of.  Grid (n_split, Hq, B), 4 warps.  A warp takes pages
+// of the row's compact list (entry index = split + n_split * (warp + 4 * i)); lane owns CPL = D/32 consecutive channels of every
+// token.  Each CTA writes a normalised partial (O, lse).
 template <int D>
-__global__ void __launch_bounds__(128) sparse_decode_int8_kernel(Int8AttnParams p) {
+__device__ __forceinline__ void int8_cta_any(const Int8AttnParams& p, float (&s_m)[4], float (&s_l)[4], float (&s_acc)[4][D]) {
     constexpr int CPL = D / 32;
-    __shared__ float s_m[4], s_l[4];
-    __shared__ float s_acc[4][D];
     const int split = blockIdx.x, hq = blockIdx.y, b = blockIdx.z;
     const int hkv = hq / (p.Hq / p.Hkv);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float c = p.sm_scale * I8_LOG2E;
-    pdl_trigger();     // the merge may become resident
     float q[CPL];
 #pragma unroll
     for (int j = 0; j < CPL; ++j) q[j] = i8_ld(p.Q, p.q_dtype, b * p.q_sb + hq * p.q_sh + CPL * lane + j) * c;
@@ -252,6 +250,14 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_kernel(Int8AttnParams 
     if (d == 0) p.part_lse[(int64_t)split * rows + row] = lsum > 0.f ? (mx + log2f(lsum)) * I8_LN2 : -INFINITY;
 }
 
+template <int D>
+__global__ void __launch_bounds__(128) sparse_decode_int8_kernel(Int8AttnParams p) {
+    __shared__ float s_m[4], s_l[4];
+    __shared__ float s_acc[4][D];
+    pdl_trigger();     // the merge may become resident
+    int8_cta_any<D>(p, s_m, s_l, s_acc);
+}
+
 // The same computation for 16-byte aligned code and metadata rows.  Eight lanes (a quarter warp) own one token: lane l
 // holds D/8 consecutive channels (one 16-byte load of codes at head_dim 128), so a page of 16 tokens is four tokens per
 // quarter warp, their loads in flight together, a 3-step shuffle reduction per logit and ONE online-softmax update per
@@ -269,8 +275,10 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
     const int l = lane & 7, qw = lane >> 3;
     const float c = p.sm_scale * I8_LOG2E;
     // Codes as fp32 operands with one integer instruction each: a byte masked in place and read as an fp32 (sub)normal is
-    // code * 2^(8 k - 149) for byte k = 0..2, a shift brings byte 3 to the bottom.  The power of two goes into the multiplier, which
-    // 2^80 keeps away from both ends of the range (scales up to 1e14).  A conversion by byte permute and subtraction and one FMA per
+    // code * 2^(8 k - 149) for byte k = 0..2, a shift brings byte 3 to the bottom.  The power of two goes into the multiplier; 2^80 of
+    // it leaves both ends of fp32 free for scales that caches hold in earnest.  A multiplier that it makes infinite (q times scale, or a V
+    // scale, from 2^48 on: bf16 caches can) and results so small that products have lost bits below 2^-149 (a V scale under 1e-11) are
+    // recognised, and the CTA starts again in the general form.  A conversion by byte permute and subtraction and one FMA per
     // code instead: 44 us for 4 x 20k tokens of 24/8 heads; this 40, both waiting for their loads most of the time.
     auto up = [](int k) { return __int_as_float((127 + (k < 3 ? 80 - 8 * k : 80)) << 23); };           // 2^80 / 2^(8 k)
     auto down = [](int k) { return __int_as_float((127 - (k < 3 ? 80 - 8 * k : 80)) << 23); };         // its reciprocal
@@ -280,6 +288,9 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
     float q[DPL];      // times up()
 #pragma unroll
     for (int j = 0; j < DPL; ++j) q[j] = i8_ld(p.Q, p.q_dtype, b * p.q_sb + hq * p.q_sh + DPL * l + j) * c * up(j & 3);
+    float unfit = 0.f;                   // NaN once a multiplier was infinite
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) unfit = fmaf(q[j], 0.f, unfit);
     float m = -INFINITY, lsum = 0.f, mnacc = 0.f;
     float2 acc[DPL / 2];
 #pragma unroll
@@ -362,6 +373,7 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
                     a = __ffma2_rn(high2(kw[u][w]), make_float2(qs[4 * w + 2], qs[4 * w + 3]), a);
                 }
                 const float dot = quarter_sum(a.x + a.y);
+                if (u == 0) unfit = fmaf(dot, 0.f, unfit);         // an infinite multiplier shows in every dot product of the page, 0 * inf too
                 sc[u] = t0 + qw + 4 * u < t_end ? fmaf(dot, home(0), qmn) : -INFINITY;
                 mx = fmaxf(mx, sc[u]);
             }
@@ -393,6 +405,16 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
     float out[DPL];
 #pragma unroll
     for (int j = 0; j < DPL; ++j) out[j] = ((j & 1) ? acc[j / 2].y : acc[j / 2].x) * home(j & 3);
+    // bits lost below 2^-149 are worth tokens * 2^-80 at most, nothing against a largest channel of 2^-30 or more (the packed caches'
+    // V scales are 1e-6 at least, so only a warp that met no V code but 0 comes out smaller)
+    bool again;
+    {
+        float big = 0.f;
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) { big = fmaxf(big, fabsf(out[j])); unfit = fmaf(out[j], 0.f, unfit); }
+        big = warp_max(big);
+        again = !(unfit == 0.f) || (lsum > 0.f && big < 9.3e-10f);
+    }
     // the staged (unquantised) tail belongs to split 0: a quarter warp per token
     if (split == 0) {
         for (int t0 = 4 * warp; t0 < p.tail_len; t0 += 16) {       // warp-uniform trip count
@@ -426,7 +448,7 @@ __global__ void __launch_bounds__(128) sparse_decode_int8_q_kernel(Int8AttnParam
 #pragma unroll
         for (int j = 0; j < DPL; ++j) s_acc[warp][DPL * l + j] = out[j] + mnacc;
     }
-    __syncthreads();
+    if (__syncthreads_or(again)) { int8_cta_any<D>(p, s_m, s_l, s_acc); return; }
     float mx = fmaxf(fmaxf(s_m[0], s_m[1]), fmaxf(s_m[2], s_m[3]));
     float ltot = 0.f, o = 0.f;
     const int d = threadIdx.x;

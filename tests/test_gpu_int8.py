@@ -226,3 +226,30 @@ def test_attention_with_rows_that_are_not_16_byte_aligned(D):
     O2, lse2 = flash_attn_sparse_fwd(Q.cuda(), *dev, selection_mask=mask.cuda(), page_size=page)
     _close(O2, lse2, Ow, lw, dtype)
     assert _lib.lib().fq_device_status() == 0
+
+
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("q,ks,vs", [(1.0, 1e-6, 1e-6), (1.0, 1e16, 1.0), (1e16, 1e-18, 1.0), (1.0, 1e-2, 1e16), (1.0, 1e-2, 1e-26), (1e16, 1e-18, 1e30)])
+def test_scales_of_any_size(D, q, ks, vs):
+    """Scales that the power of two in the 16-byte form's multipliers would make infinite, or whose products it would lose, give
+    what the general form gives.  Bound of a logit: 2^-16 of the sum of its absolute products (D roundings of 2^-24 and those of
+    the metadata products are less); where logits are that far apart one token has all the weight.  O against the largest |V|."""
+    from flashquest_b200.kernel.sparse_fwd import flash_attn_sparse_fwd
+    B, Hq, Hkv, S, page, dtype = 2, 4, 2, 656, 16, torch.bfloat16
+    Q, kv, mask = _att_case(35, B, Hq, Hkv, S, D, page, dtype)
+    g = torch.Generator().manual_seed(36)
+    Ks, Vs = kv[1], kv[4]
+    kv = (kv[0], (ks * (1 + torch.rand(Ks.shape, generator=g))).to(dtype), (-150 * ks * (1 + torch.rand(Ks.shape, generator=g))).to(dtype),
+          kv[3], (vs * (1 + torch.rand(Vs.shape, generator=g))).to(dtype), (-150 * vs * (1 + torch.rand(Vs.shape, generator=g))).to(dtype))
+    Q = (q * Q.float()).to(dtype)
+    Ow, lw = oracle.sparse_attn_int8(Q, *kv, selection_mask=mask, page_size=page)
+    dev = [t.cuda() for t in kv]
+    wide = [torch.zeros(B, Hkv, S, D + 4, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    wide[0][..., :D], wide[1][..., :D] = dev[0], dev[3]
+    logit_tol = 2 ** -16 * Q.float().abs().sum(-1).max() * 512 * ks * 2 / D ** 0.5 + LSE_TOL
+    for K, V in ((dev[0], dev[3]), (wide[0][..., :D], wide[1][..., :D])):
+        for n_split in (None, 1):
+            O, lse = flash_attn_sparse_fwd(Q.cuda(), K, dev[1], dev[2], V, dev[4], dev[5], selection_mask=mask.cuda(), page_size=page, n_split=n_split)
+            assert (lse.cpu() - lw).abs().max() <= logit_tol
+            err = (O.float().cpu() - Ow).abs()
+            assert (err <= O_TOL * 512 * vs + 2 ** -8 * Ow.abs()).all(), float((err / vs).max())
