@@ -373,3 +373,31 @@ def test_norm_apart_equals_the_folded_prologue(B, hidden):
         a.decode_step(ids[t])
         folded(b, ids[t])
         assert torch.equal(a.logits, b.logits), t
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim", [(8, 1, 64), (10, 2, 128), (16, 2, 64)])
+def test_more_than_four_query_heads_per_kv_head(q_heads, kv_heads, head_dim):
+    """The scores of a group go in several launches, of which the first appends: across a page end the later ones find the completed
+    page.  By graph (position on the device) and from the host: equal logits, and the scores of all heads those of the oracle."""
+    from flashquest_b200.eager.llama_decode import LlamaConfig, LlamaInt4Decoder, random_llama_weights
+    cfg = LlamaConfig(hidden=256, layers=2, q_heads=q_heads, kv_heads=kv_heads, head_dim=head_dim, ffn=512, vocab=512)
+    w = random_llama_weights(cfg, "cuda", seed=6)
+    mk = lambda: LlamaInt4Decoder(cfg, w, batch_size=2, max_seq_len=96, page_size=16, retention=0.5, num_sinks=1, window_pages=1)
+    a, b = mk(), mk()
+    ids = torch.tensor([7, 123], dtype=torch.int32, device="cuda")
+    for d in (a, b):
+        x = ids
+        for _ in range(14):
+            x = d.decode_step(x).clone()
+    replay = a.capture_decode_graph(x)
+    for t in range(15, 52):                               # cached tokens behind the step
+        replay()
+        x = b.decode_step(x).clone()
+        assert torch.equal(a.logits, b.logits), t
+        P, v = t // 16, b.cache.get_views(cfg.layers - 1)
+        if P == 0:
+            continue
+        q = b._nat["q"].view(2, q_heads, 1, head_dim)      # the last layer's
+        want = oracle.page_scores_int4_fast(q.cpu(), v["K_scale"].cpu(), v["K_mn"].cpu()).view(2, q_heads, P)
+        assert torch.equal(a.attn.scores[-1, :, :, :P].cpu(), want), t
+        assert torch.equal(b.attn.scores[-1].view(-1)[:2 * q_heads * P].view(2, q_heads, P).cpu(), want), t
