@@ -191,7 +191,7 @@ int decode_layer_int4_dyn(const fq_int4_cache* c, int l, const int* pos, const v
     dp_early.early = true;
     int rc = FQ_OK;
     QuantParams now;
-    const bool along = append && page_scores_take_append(q_dtype, B, Hq, Hkv, P_max, D) && append_dyn_params(now, c, l, pos, Kn, Vn, nw_sb, nw_sh, nw_ss, n_new);
+    const bool along = append && q_dtype == FQ_F16 && c->kv_dtype == FQ_F16 && page_scores_take_append(q_dtype, B, Hq, Hkv, P_max, D) && append_dyn_params(now, c, l, pos, Kn, Vn, nw_sb, nw_sh, nw_ss, n_new);
     if (append && !along)
         rc = quantize_kv_int4_launch(Kt, Vt, c->pt_sb, c->pt_sh, c->pt_ss, page - n_new, Kn, Vn, nw_sb, nw_sh, nw_ss, n_new,
                                      c->kv_dtype, B, Hkv, D, page, page,

@@ -21,14 +21,14 @@ constexpr int SCORE_PAGES_PER_CTA = 32;       // 2 iterations per CTA
 // What a decode step appends in the launch of its page scores, by one extra CTA per (batch, kv head).  A launch of its own for 4 KB
 // per head took 1.9 to 2.5 us of every layer.  Two forms: rows to stage behind a known number of tokens, no page completed; and,
 // with the position read on the device, whatever the position asks for.  There, pages completed before do not wait for the
-// append, and the score of a page completed now is the same CTA's work.
+// append, and the score of a page completed now is the same CTA's work.  That form is the Llama step's, in fp16 throughout.
 struct NoAppend {};
 struct StageAppend {
     const uint16_t *K_new, *V_new; int64_t nw_sb, nw_sh, nw_ss;
     uint16_t *K_stage, *V_stage; int64_t st_sb, st_sh, st_ss;      // row 0 of the new tokens, unless the position is read on the device
     int n;
 };
-struct DynAppend { StageAppend st; QuantParams q; int bf16; };
+struct DynAppend { StageAppend st; QuantParams q; };
 
 // rows of n tokens, K and V, 16 bytes per thread and pass; before() runs between the loads and the stores and returns the first row
 template <typename F>
@@ -53,18 +53,15 @@ __device__ __forceinline__ void stage_rows(const StageAppend& a, int b, int h, i
 __device__ __noinline__ void append_page(const DynAppend& a, int b, int h) {
     QuantParams p = a.q;
     if (!quant_locate(p)) return;                              // full: nothing is written (the host checks its own count)
-    if (a.bf16) quant_int4_cta<__nv_bfloat16>(p, b, h, 0);
-    else quant_int4_cta<__half>(p, b, h, 0);
+    quant_int4_cta<__half>(p, b, h, 0);
 }
 
 template <typename QT, int NR, int CH>
 __device__ __forceinline__ void append_and_score(const DynAppend& a, const QT* __restrict__ Q, int64_t q_sb, int64_t q_sh, int b, int hkv, int n_rep, int head_off,
-                                                 int P, int D, float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, float levels, const int* pos, int pos_early) {
-    int seen = 0;
-    if (pos_early) seen = __ldcg(pos);
+                                                 int P, int D, float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, float levels, const int* pos) {
+    const int seen = __ldcg(pos);
     pdl_wait();
     pdl_trigger();
-    if (!pos_early) seen = *pos;
     const int page_len = a.q.page, partial = seen % page_len;
     const bool completes = partial + a.q.n_new >= page_len;
     stage_rows(a.st, b, hkv, D >> 3, [&]() { return completes || seen < 0 || seen + a.q.n_new > a.q.max_tokens ? -1 : partial; });
@@ -100,7 +97,7 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_kernel(
     const uint16_t* __restrict__ K_scale, const uint16_t* __restrict__ K_mn,
     int64_t km_sb, int64_t km_sh, int64_t km_sp,
     int Hq, int Hkv, int P, int D, int head_off,
-    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, const int* __restrict__ pos, int pos_new, int pos_page, int pos_early, float levels,
+    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, float levels,
     const __grid_constant__ APPEND app) {
     const int b = blockIdx.z, hkv = blockIdx.y;
     const int n_rep = Hq / Hkv;
@@ -111,25 +108,13 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_kernel(
             stage_rows(app, b, hkv, D >> 3, []() { return 0; });
             return;
         }
-    } else if constexpr (std::is_same_v<APPEND, DynAppend>) {
-        if (blockIdx.x == gridDim.x - 1) {
-            append_and_score<QT, NR, CH>(app, Q, q_sb, q_sh, b, hkv, n_rep, head_off, P, D, scores, sc_sb, sc_sh, levels, pos, pos_early);
-            return;
-        }
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int l = lane & 7, qw = lane >> 3;
     const int n_chunks = D >> 3;
     const int nr = min(NR, n_rep - head_off);   // heads actually present in this pass
-    int pos_v = 0;
-    if (pos && pos_early) pos_v = __ldcg(pos);             // in flight during the wait (see DynPos::early)
     pdl_wait();        // Q and the newest metadata row come from the kernels before this one
     pdl_trigger();
-    if (pos) {
-        if (!pos_early) pos_v = *pos;
-        // completed pages after this step's append; before it where that is made here
-        P = min(P, (pos_v + (std::is_same_v<APPEND, DynAppend> ? 0 : pos_new)) / pos_page);
-    }
 
     // Metadata loads of every page this quarter warp will score are issued first, the q loads
     // after them, so the two global-memory latencies overlap instead of adding up.
@@ -169,7 +154,7 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_early_kernel(
     constexpr bool ALONG = std::is_same_v<APPEND, DynAppend>;
     if constexpr (ALONG) {
         if (blockIdx.x == gridDim.x - 1) {
-            append_and_score<QT, NR, CH>(app, Q, q_sb, q_sh, b, hkv, n_rep, head_off, P, D, scores, sc_sb, sc_sh, levels, pos, 1);
+            append_and_score<QT, NR, CH>(app, Q, q_sb, q_sh, b, hkv, n_rep, head_off, P, D, scores, sc_sb, sc_sh, levels, pos);
             return;
         }
     }
@@ -191,7 +176,7 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_early_kernel(
     }
     pdl_wait();        // Q and the newest metadata row come from the kernels before this one
     pdl_trigger();
-    P = ALONG ? P_old : min(P, (pos_v + pos_new) / pos_page);          // completed pages after this step's append
+    P = ALONG ? P_old : min(P, (pos_v + pos_new) / pos_page);          // completed pages after this step's append; before it where that is made here
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
         const int p = p_base + it * 16 + warp * 4 + qw;
@@ -285,30 +270,29 @@ static void launch_scores(int CH, dim3 grid, cudaStream_t st, const void* Q, int
                           const DynAppend* app) {
     const int ctas = stream_ctas(NR, D, (int)(grid.y * grid.z), P);
     const NoAppend none{};
-    const bool early = dp.pos != nullptr && dp.early;
 #define FQ_SC_ARGS static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale), static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P, D, \
-                   head_off, scores, sc_sb, sc_sh, dp.pos, dp.n_new, dp.page
+                   head_off, scores, sc_sb, sc_sh
 #define FQ_LAUNCH_SC(CHV)                                                                                                                                                  \
     do {                                                                                                                                                                   \
         if (ctas > 0)                                                                                                                                                      \
             launch_k(PDL_SCORES, page_scores_stream_kernel<QT, NR, (CHV > 2 ? 2 : CHV)>, dim3((unsigned)ctas, grid.y, grid.z), dim3(SCORE_THREADS), 0, st,                 \
                      static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale), static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P,    \
                      head_off, scores, sc_sb, sc_sh, dp.pos, dp.n_new, dp.page, levels);                                                                                   \
-        else if (early) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, none);                    \
-        else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, 0, levels, none);                                  \
+        else if (dp.pos) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, dp.pos, dp.n_new, dp.page, levels, none); \
+        else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, none);                                     \
     } while (0)
     if constexpr (sizeof(QT) == 2) {
         if (app) {
             ++grid.x;
-#define FQ_LAUNCH_AP(CHV)                                                                                                                                                  \
-    do {                                                                                                                                                                   \
-        if (early) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, *app);                          \
-        else if (dp.pos) launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, 0, levels, *app);                   \
-        else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, StageAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, 0, levels, app->st);                         \
-    } while (0)
-            if (CH == 1) FQ_LAUNCH_AP(1);
-            else FQ_LAUNCH_AP(2);
-#undef FQ_LAUNCH_AP
+            if constexpr (std::is_same_v<QT, __half>) {
+                if (dp.pos) {
+                    if (CH == 1) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, 1, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, dp.pos, dp.n_new, dp.page, levels, *app);
+                    else launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, 2, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, dp.pos, dp.n_new, dp.page, levels, *app);
+                    return;
+                }
+            }
+            if (CH == 1) launch_k(PDL_SCORES, page_scores_kernel<QT, NR, 1, StageAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, app->st);
+            else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, 2, StageAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, app->st);
             return;
         }
     }
@@ -352,12 +336,13 @@ int page_scores_int4_launch(
     const int CH = D <= 64 ? 1 : D / 64;
     dim3 grid((unsigned)((P + SCORE_PAGES_PER_CTA - 1) / SCORE_PAGES_PER_CTA), (unsigned)Hkv, (unsigned)B);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    FQ_CHECK_ARG(!dp.pos || dp.early, FQ_ERR_ARG, "%s: a device position that the kernels may not read early", fn);
     DynAppend app{};
     if (append) {
-        FQ_CHECK_ARG(page_scores_take_append(q_dtype, B, Hq, Hkv, P, D) && (append_dtype == FQ_F16 || append_dtype == FQ_BF16) && append->n_layers == 1, FQ_ERR_ARG,
-                     "%s: an append that this launch does not take", fn);
+        FQ_CHECK_ARG(page_scores_take_append(q_dtype, B, Hq, Hkv, P, D) && (append_dtype == FQ_F16 || append_dtype == FQ_BF16) && append->n_layers == 1 &&
+                     append->pos == dp.pos && (!dp.pos || (q_dtype == FQ_F16 && append_dtype == FQ_F16)), FQ_ERR_ARG, "%s: an append that this launch does not take", fn);
         const QuantParams& q = *append;
-        app.q = q; app.bf16 = append_dtype == FQ_BF16;
+        app.q = q;
         const int64_t first = q.pos ? 0 : q.n_head * q.st_ss;
         app.st = StageAppend{static_cast<const uint16_t*>(q.K_new), static_cast<const uint16_t*>(q.V_new), q.nw_sb, q.nw_sh, q.nw_ss,
                              static_cast<uint16_t*>(q.stage_K) + first, static_cast<uint16_t*>(q.stage_V) + first, q.st_sb, q.st_sh, q.st_ss, q.n_new};
