@@ -5,7 +5,8 @@
 // flight to fill it (67 M elements of a 32k-token layer against 172 MB, 26 us at the measured copy rate), so the work per
 // element is what this kernel removes:
 //  * a warp owns 16 tokens of K or of V and keeps them in registers (32 per lane, packed): one read of the input, 8 loads of
-//    16 bytes in flight per lane, no second pass.  K and V in one warp needed 120 registers, 16 warps per SM; apart 24 fit;
+//    16 bytes in flight per lane, no second pass.  K and V in one warp needed 120 registers, 16 warps per SM; apart 24 to 28 fit
+//    (quant_pages_ctas);
 //  * minima and maxima on packed pairs; the page's other tiles (page 32 / 64) join through shared memory;
 //  * a code is the quotient by one residual step (two for V, whose scales are fp32) from the approximate reciprocal, which rounds
 //    like the IEEE one (fq_exact_div.cuh), two elements per instruction, rounded by adding 1.5 * 2^23.  Redoing the elements near
@@ -87,9 +88,15 @@ __device__ __forceinline__ uint2 encode8(const uint32_t (&w)[4], const float2 (&
     return out;
 }
 
+// CTAs of four warps per SM that the registers are cut for: six have 80 a thread, seven 72.  One layer of 32k tokens, 8 heads, L2
+// flushed in between, six against seven: 8-bit bf16 of 128 channels 51.2 -> 49.2 us although 100 bytes spill, of 64 channels (no spills) 35.6 -> 33.6,
+// fp16 of 64 channels 33.6 both; 8-bit fp16 of 128 channels spills 340 bytes at 72, 51.2 -> 53.2.  4-bit codes need the 80.
+template <typename T, int D, int BITS>
+constexpr int quant_pages_ctas() { return BITS == 8 && !(std::is_same_v<T, __half> && D == 128) ? 7 : 6; }
+
 // 16 tokens of one (b, h) per warp.  A lane owns 8 channels (one 16-byte load) of every RPI-th token.
 template <typename T, int D, int BITS, int NT>      // NT: 16-token tiles per page
-__global__ void __launch_bounds__(128, BITS == 8 ? 7 : 6) quant_pages_kernel(QuantPagesParams p) {
+__global__ void __launch_bounds__(128, quant_pages_ctas<T, D, BITS>()) quant_pages_kernel(QuantPagesParams p) {
     constexpr int LPT = D / 8;            // lanes per token
     constexpr int RPI = 32 / LPT;         // tokens per load instruction
     constexpr int NI = 16 / RPI;          // loads per lane for a tile (8 at D 128, 4 at D 64)
