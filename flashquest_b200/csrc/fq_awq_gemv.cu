@@ -40,6 +40,7 @@ constexpr int GEMV_MAX_PROJ = 4;
 constexpr int GEMV_ROWS = 128;          // rows per stage = largest group size
 constexpr int GEMV_MAX_STAGES = 6;       // ring depth: 3 (short K ranges) or 6 (long ones: more bytes in flight per CTA)
 constexpr int GEMV_MAX_CLUSTER = 8;
+constexpr size_t GEMV_SMEM_MAX = 226 * 1024;
 
 struct GemvProj {
     const int32_t* qweight; const __half* scales; const int32_t* qzeros; const __half* bias; __half* y;
@@ -636,7 +637,7 @@ static int gemv_launch(
         smem = stages * stage_bytes + fixed;
         // the deep ring only while two CTAs still fit on an SM
         if (smem > 113 * 1024 && stages > 3) { stages = 3; smem = stages * stage_bytes + fixed; }
-        if (smem <= 226 * 1024 || k_split >= GEMV_MAX_CLUSTER || k_split * 2 > p.n_groups) break;
+        if (smem <= GEMV_SMEM_MAX || k_split >= GEMV_MAX_CLUSTER || k_split * 2 > p.n_groups) break;
         k_split *= 2;
     }
     p.k_split = k_split;
@@ -650,7 +651,7 @@ static int gemv_launch(
     if (smem < room) smem = room;
     FQ_CHECK_ARG(((p.head_dim > 0 ? p.head_dim : 128) / 2) % (4 * (Mp == 8 ? k_split : 1)) == 0, FQ_ERR_UNSUPPORTED,
                  "%s: head_dim %d with %d-way split-K", fn, p.head_dim, k_split);
-    FQ_CHECK_ARG(smem <= 226 * 1024, FQ_ERR_UNSUPPORTED, "%s: K=%d with %d rows needs %zu B of shared memory per CTA", fn, K, M, smem);
+    FQ_CHECK_ARG(smem <= GEMV_SMEM_MAX, FQ_ERR_UNSUPPORTED, "%s: K=%d with %d rows needs %zu B of shared memory per CTA", fn, K, M, smem);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)tiles, (unsigned)k_split); cfg.blockDim = dim3(GEMV_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
@@ -662,13 +663,8 @@ static int gemv_launch(
     cfg.attrs = at; cfg.numAttrs = pdl_enabled(PDL_GEMV) ? 2 : 1;
 #define FQ_GEMV(MV, SV, FV)                                                                                  \
     do {                                                                                                     \
-        static std::atomic<size_t> attr_smem[64];                                                            \
-        int dev = 0; cudaGetDevice(&dev);                                                                    \
-        if (dev < 0 || dev >= 64 || attr_smem[dev].load(std::memory_order_acquire) < smem) {                 \
-            cudaError_t e = cudaFuncSetAttribute(awq_gemv_kernel<MV, SV, FV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-            if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: cannot reserve %zu B of shared memory: %s", fn, smem, cudaGetErrorString(e)); \
-            if (dev >= 0 && dev < 64) attr_smem[dev].store(smem, std::memory_order_release);                 \
-        }                                                                                                    \
+        cudaError_t e = allow_smem<awq_gemv_kernel<MV, SV, FV>>(GEMV_SMEM_MAX);                              \
+        if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: cannot reserve %zu B of shared memory: %s", fn, smem, cudaGetErrorString(e)); \
         cudaLaunchKernelEx(&cfg, awq_gemv_kernel<MV, SV, FV>, p);                                            \
     } while (0)
     const bool fast = group == 128 && interleaved && vec16;

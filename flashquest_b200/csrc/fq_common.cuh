@@ -142,6 +142,21 @@ int quant_append_layers_dyn(const fq_int4_cache* c, int n_layers, const int* pos
 int rope_launch(void* q, int64_t q_sb, int64_t q_sh, int Hq, void* k, int64_t k_sb, int64_t k_sh, int Hkv, int B, int D, int pos,
                 float theta, void* stream, const int* pos_dev, int pos_step);
 
+// Lets a kernel ask for up to `bytes` of dynamic shared memory, the most that any call of it does.  The limit belongs to the
+// function, not to the launch: set to what one call needs, it could be lowered between another thread's setting and launch.
+template <auto KERNEL>
+inline cudaError_t allow_smem(size_t bytes) {
+    static std::atomic<uint64_t> done{0};            // one bit per device; concurrent threads may repeat the same setting
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 // Device-side status word of the current device: kernels that wait (mbarrier) record a

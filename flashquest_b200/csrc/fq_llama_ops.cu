@@ -426,7 +426,8 @@ static int add_rmsnorm_launch(const void* a, const void* b, const void* weight, 
                               void* sum_out, void* y, bool piecewise, void* stream) {
     const char* fn = "fq_add_rmsnorm";
     FQ_CHECK_ARG(a && weight && y && rows >= 0 && H > 0, FQ_ERR_ARG, "%s: bad arguments", fn);
-    FQ_CHECK_ARG((size_t)H * 2 <= 96 * 1024, FQ_ERR_UNSUPPORTED, "%s: hidden size %d too large", fn, H);
+    constexpr size_t NORM_SMEM_MAX = 96 * 1024;
+    FQ_CHECK_ARG((size_t)H * 2 <= NORM_SMEM_MAX, FQ_ERR_UNSUPPORTED, "%s: hidden size %d too large", fn, H);
     if (rows == 0) return FQ_OK;
     if (H % 8 == 0 && H <= 8 * NORM_THREADS * NORM_CHUNKS && aligned(a, 16) && aligned(b, 16) && aligned(weight, 16) && aligned(sum_out, 16) && aligned(y, 16)) {
         launch_k(PDL_GEMV, piecewise ? add_rmsnorm_vec_kernel<false> : add_rmsnorm_vec_kernel<true>, dim3((unsigned)rows), dim3(NORM_THREADS), 0, static_cast<cudaStream_t>(stream),
@@ -437,7 +438,7 @@ static int add_rmsnorm_launch(const void* a, const void* b, const void* weight, 
     }
     const size_t smem = (size_t)H * 2;
     if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(add_rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem<add_rmsnorm_kernel>(NORM_SMEM_MAX);
         if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: %s", fn, cudaGetErrorString(e));
     }
     launch_k(PDL_GEMV, add_rmsnorm_kernel, dim3((unsigned)rows), dim3(NORM_THREADS), smem, static_cast<cudaStream_t>(stream),
@@ -518,10 +519,11 @@ extern "C" int fq_gemv_f16(const void* x, const void* W, int M, int K, int N, vo
     FQ_CHECK_ARG(M >= 1 && M <= 8, FQ_ERR_UNSUPPORTED, "%s: M=%d rows; 1..8 are built", fn, M);
     FQ_CHECK_ARG(K % 8 == 0 && aligned(W, 16) && aligned(x, 2), FQ_ERR_ALIGN, "%s: K must be a multiple of 8 and W 16-byte aligned", fn);
     cudaStream_t st0 = static_cast<cudaStream_t>(stream);
-    if (K % 32 == 0 && aligned(x, 16) && (size_t)8 * (K + GEMVM_XPAD) * 2 <= 100 * 1024) {
+    constexpr size_t MMA_SMEM_MAX = 100 * 1024, SMEM_MAX = 200 * 1024;
+    if (K % 32 == 0 && aligned(x, 16) && (size_t)8 * (K + GEMVM_XPAD) * 2 <= MMA_SMEM_MAX) {
         const size_t smem_m = (size_t)8 * (K + GEMVM_XPAD) * 2;
         if (smem_m > 40 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(gemv_f16_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_m);
+            cudaError_t e = allow_smem<gemv_f16_mma_kernel>(MMA_SMEM_MAX);
             if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: %s", fn, cudaGetErrorString(e));
         }
         const int tiles = (N + GEMVM_ROWS - 1) / GEMVM_ROWS;
@@ -532,13 +534,13 @@ extern "C" int fq_gemv_f16(const void* x, const void* W, int M, int K, int N, vo
     }
     const int Mp = M <= 1 ? 1 : (M <= 2 ? 2 : (M <= 4 ? 4 : 8));
     const size_t smem = (size_t)Mp * K * 4;
-    FQ_CHECK_ARG(smem <= 200 * 1024, FQ_ERR_UNSUPPORTED, "%s: M x K = %d x %d does not fit in shared memory", fn, M, K);
+    FQ_CHECK_ARG(smem <= SMEM_MAX, FQ_ERR_UNSUPPORTED, "%s: M x K = %d x %d does not fit in shared memory", fn, M, K);
     dim3 grid((unsigned)((N + GEMVH_WARPS - 1) / GEMVH_WARPS));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define FQ_GH(MV)                                                                                                  \
     do {                                                                                                           \
         if (smem > 40 * 1024) {                                                                                    \
-            cudaError_t e = cudaFuncSetAttribute(gemv_f16_kernel<MV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            cudaError_t e = allow_smem<gemv_f16_kernel<MV>>(SMEM_MAX);                                             \
             if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: %s", fn, cudaGetErrorString(e));                   \
         }                                                                                                          \
         launch_k(PDL_GEMV, gemv_f16_kernel<MV>, grid, dim3(GEMVH_WARPS * 32), smem, st, static_cast<const __half*>(x), \

@@ -474,6 +474,7 @@ constexpr int FUSED_THREADS = 512;
 constexpr int FUSED_CLUSTER = 8;
 constexpr int FUSED_MAX_P = 16384;
 constexpr int FUSED_QW = FUSED_THREADS / 8; // quarter warps per CTA = pages scored per pass
+constexpr size_t FUSED_SMEM_MAX = FUSED_MAX_P * 4 + 2 * (2 * FUSED_QW) * 4 * 128;      // scores of a row, two rounds of metadata
 
 struct ScoreSelectParams {
     const void* Q; int64_t q_sb, q_sh;
@@ -672,7 +673,7 @@ int select_pages_launch(
     } else if (P <= SEL_SMEM_MAX_P) {
         const size_t smem = (size_t)P * 4;
         if (smem > 36 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(select_pages_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaError_t e = allow_smem<select_pages_kernel<true>>(SEL_SMEM_MAX_P * 4);
             if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: cannot reserve %zu B of shared memory: %s", fn, smem, cudaGetErrorString(e));
         }
         launch_k(PDL_SELECT_LONG, select_pages_kernel<true>, grid, dim3(select_threads(P)), smem, st,
@@ -700,7 +701,7 @@ static cudaError_t launch_score_select(int CH, const ScoreSelectParams& p, dim3 
 #define FQ_SS(CHV)                                                                                                   \
     do {                                                                                                             \
         if (smem > 36 * 1024) {                                                                                      \
-            cudaError_t e = cudaFuncSetAttribute(score_select_kernel<QT, NR, CHV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            cudaError_t e = allow_smem<score_select_kernel<QT, NR, CHV>>(FUSED_SMEM_MAX);                            \
             if (e != cudaSuccess) return e;                                                                          \
         }                                                                                                            \
         return cudaLaunchKernelEx(&cfg, score_select_kernel<QT, NR, CHV>, p);                                        \
