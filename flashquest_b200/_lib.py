@@ -25,6 +25,7 @@ I, L, P, F, Z = c_int, c_int64, c_void_p, c_float, c_size_t
 _PROTOTYPES = {
     "fq_last_error_string": (ctypes.c_char_p, []),
     "fq_version": (ctypes.c_char_p, []),
+    "fq_launches": (ctypes.c_ulonglong, []),
     "fq_device_status": (I, []),
     "fq_quantize_kv_int4": (I, [P, P, L, L, L, I, P, P, L, L, L, I, I, I, I, I, I, I,
                                 P, P, L, L, L, P, P, L, L, L, P, P, L, L, L, P, P, L, L, L, P]),

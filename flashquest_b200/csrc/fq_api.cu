@@ -24,6 +24,10 @@ int fail(int code, const char* fmt, ...) {
     return code;
 }
 
+static thread_local unsigned long long g_launches = 0;
+
+void count_launch() { ++g_launches; }
+
 __device__ int g_fq_status = 0;
 
 // The address is looked up once per device and remembered (relaxed atomics: concurrent host
@@ -67,6 +71,8 @@ int sm_count() {
 }  // namespace fq
 
 extern "C" const char* fq_last_error_string(void) { return fq::g_err; }
+
+extern "C" unsigned long long fq_launches(void) { return fq::g_launches; }
 
 extern "C" const char* fq_version(void) { return "flashquest_b200 0.1 (sm_100a)"; }
 

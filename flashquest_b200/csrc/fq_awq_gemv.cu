@@ -665,6 +665,7 @@ static int gemv_launch(
     do {                                                                                                     \
         cudaError_t e = allow_smem<awq_gemv_kernel<MV, SV, FV>>(GEMV_SMEM_MAX);                              \
         if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: cannot reserve %zu B of shared memory: %s", fn, smem, cudaGetErrorString(e)); \
+        count_launch();                                                                                      \
         cudaLaunchKernelEx(&cfg, awq_gemv_kernel<MV, SV, FV>, p);                                            \
     } while (0)
     const bool fast = group == 128 && interleaved && vec16;

@@ -369,6 +369,7 @@ static int sk_launch(const SkinnyCall& c, SkParams& p, const CUtensorMap* maps, 
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at; cfg.numAttrs = 1;
+    count_launch();
     cudaError_t e = cudaLaunchKernelEx(&cfg, awq_skinny_kernel<IL, TN>, maps[0], maps[1], maps[2], maps[3], maps[4], p);
     if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "%s: launch failed: %s", fn, cudaGetErrorString(e));
     FQ_CHECK_LAUNCH(fn);

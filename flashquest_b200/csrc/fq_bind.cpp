@@ -10,6 +10,7 @@
 // has no address) becomes a Python exception.
 #include <Python.h>
 
+#include <atomic>
 #include <cstring>
 
 #include <ATen/core/Tensor.h>
@@ -36,6 +37,7 @@ struct Plan {
     char* scratch; size_t scratch_sl, scratch_bytes;
     char *q_rot, *k_rot, *v_rot; int64_t qr_sl, kr_sl;     // (bytes between layers) rotated q / k and cast v of the patched forward, dense, cache dtype
     float* retention;               // (n_layers, H_q): written by the patched forward from the head pattern
+    std::atomic<unsigned long long> launches{0};           // kernels that step() and forward() have launched
 };
 
 const char* kPlanName = "flashquest_b200.plan";
@@ -83,6 +85,13 @@ void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream(static_cast
 struct NoGil {
     PyThreadState* state = PyEval_SaveThread();
     ~NoGil() { PyEval_RestoreThread(state); }
+};
+
+struct CountLaunches {
+    Plan* plan;
+    const unsigned long long before = fq_launches();
+    explicit CountLaunches(Plan* p) : plan(p) {}
+    ~CountLaunches() { plan->launches.fetch_add(fq_launches() - before, std::memory_order_relaxed); }
 };
 
 // plan(kind, cache_desc, params, device, n_layers, scores, sc_sl, compact, cp_sl, O, o_sl_bytes, lse, lse_sl,
@@ -133,7 +142,7 @@ int run_layer(const Plan* p, int layer, int seen, const void* k, const void* v, 
 PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 7) { PyErr_SetString(PyExc_TypeError, "step() takes 7 arguments"); return nullptr; }
-    const Plan* p = plan_of(a[0]);
+    Plan* p = plan_of(a[0]);
     if (!p) return nullptr;
     const int layer = static_cast<int>(PyLong_AsLong(a[1])), seen = static_cast<int>(PyLong_AsLong(a[2]));
     const at::Tensor *k = tensor_of(a[3]), *v = tensor_of(a[4]), *q = tensor_of(a[5]);
@@ -156,6 +165,7 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     {
         const NoGil released;
         const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
+        const CountLaunches counted(p);
         rc = run_layer(p, layer, seen, k->data_ptr(), v->data_ptr(), k->stride(0), k->stride(1), k->stride(2), static_cast<int>(k->size(2)),
                        q->data_ptr(), dtype_of(*q), q_sb, q_sh, &par, stream_of(p->device));
     }
@@ -169,7 +179,7 @@ PyObject* step(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 10) { PyErr_SetString(PyExc_TypeError, "forward() takes 10 arguments"); return nullptr; }
-    const Plan* p = plan_of(a[0]);
+    Plan* p = plan_of(a[0]);
     if (!p) return nullptr;
     const int layer = static_cast<int>(PyLong_AsLong(a[1])), seen = static_cast<int>(PyLong_AsLong(a[2]));
     const at::Tensor* t[5];
@@ -197,6 +207,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     {
         const NoGil released;
         const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(p->device));
+        const CountLaunches counted(p);
         void* st = stream_of(p->device);
         char *q_rot = p->q_rot + layer * p->qr_sl, *k_rot = p->k_rot + layer * p->kr_sl, *v_rot = p->v_rot + layer * p->kr_sl;
         rc = fq_rope_qkv_pattern(t[0]->data_ptr(), t[0]->stride(0), t[1]->data_ptr(), t[1]->stride(0), t[2]->data_ptr(), t[2]->stride(0), dt,
@@ -257,7 +268,15 @@ PyObject* addresses(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// launches() of the calling thread, launches(plan) of the plan's calls
+PyObject* launches(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n == 0) return PyLong_FromUnsignedLongLong(fq_launches());
+    const Plan* p = plan_of(a[0]);
+    return p ? PyLong_FromUnsignedLongLong(p->launches.load(std::memory_order_relaxed)) : nullptr;
+}
+
 PyMethodDef kMethods[] = {
+    {"launches", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(launches)), METH_FASTCALL, nullptr},
     {"addresses", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(addresses)), METH_FASTCALL, nullptr},
     {"append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(append)), METH_FASTCALL, nullptr},
     {"plan", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(make_plan)), METH_FASTCALL, nullptr},

@@ -16,6 +16,9 @@ namespace fq {
 void set_error(const char* fmt, ...);
 int fail(int code, const char* fmt, ...);
 
+// Kernels launched through the library by this thread (fq_launches): called once beside every launch.
+void count_launch();
+
 #define FQ_CHECK_ARG(cond, code, ...)              \
     do {                                           \
         if (!(cond)) return fq::fail((code), __VA_ARGS__); \
@@ -48,6 +51,7 @@ inline cudaError_t launch_k(int kind, void (*kernel)(KP...), dim3 grid, dim3 blo
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at; cfg.numAttrs = pdl_enabled(kind) ? 1 : 0;
+    count_launch();
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
 }
 
@@ -65,7 +69,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // `early`: the kernel may read *pos BEFORE its dependency wait, overlapping the load with the wait.  Safe only for a
 // kernel at least two launches behind the one that last wrote *pos: a dependent launch starts no earlier than its
 // predecessor's own wait has returned, i.e. after the writer has completed.  The decode layer sets it for scores,
-// selection and attention, which always follow the append launch; the append itself reads after its wait.
+// selection and attention, which follow the append launch, or the q/k/v projections where the append rides in the launch of the
+// scores; an append launch of its own reads after its wait.
 struct DynPos { const int* pos = nullptr; int n_new = 0; int page = 1; int max_tokens = 0; bool early = false; };
 
 struct QuantParams;      // fq_append.cuh

@@ -210,6 +210,7 @@ extern "C" int fq_ctx_select_attend(
     const int n = G * k_c;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     FQ_CHECK_ARG(rows <= 0x7fffffff, FQ_ERR_ARG, "%s: too many rows", fn);
+    count_launch();
     ctx_pack_candidates_kernel<<<(unsigned)rows, 256, 0, st>>>(gathered, G, rows, k_c, s.cand_scores, s.cand_ids);
     FQ_CHECK_LAUNCH(fn);
     // global top-k over the candidates (every page that can be among the global top k is among them)
@@ -217,6 +218,7 @@ extern "C" int fq_ctx_select_attend(
                              s.win, (int64_t)Hq * n, n, nullptr, 0, 0, 0, nullptr, stream);
     if (rc != FQ_OK) return rc;
     if (P_local > 0) {
+        count_launch();
         ctx_scatter_winners_kernel<<<(unsigned)rows, 256, 0, st>>>(s.win, s.cand_ids, n, lo, hi, P_global, sinks, window, s.mask);
         FQ_CHECK_LAUNCH(fn);
         rc = fq_build_compact(s.mask, P_local, rows, P_local, s.compact, bucket_local, bucket_local, stream);

@@ -513,11 +513,13 @@ static void launch_quant_int8(const void* K, const void* V, int64_t in_sb, int64
                               uint16_t* Vs, uint16_t* Vm, int64_t vm_sb, int64_t vm_sh, cudaStream_t st) {
     if (K) {
         const int64_t warps = (int64_t)B * H * ((S + page - 1) / page);
+        count_launch();
         quant_k_int8_kernel<T><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(static_cast<const T*>(K), in_sb, in_sh, in_ss, B, H, S, D, page,
                                                                           Kc, c_sb, c_sh, c_ss, Ks, Km, km_sb, km_sh, km_sp);
     }
     if (V) {
         const int64_t warps = (int64_t)B * H * S;
+        count_launch();
         quant_v_int8_kernel<T><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(static_cast<const T*>(V), in_sb, in_sh, in_ss, B, H, S, D,
                                                                           Vc, c_sb, c_sh, c_ss, Vs, Vm, vm_sb, vm_sh);
     }
@@ -567,6 +569,7 @@ extern "C" int fq_dequantize_int8(
     FQ_CHECK_ARG(codes && scale && mn && out, FQ_ERR_ARG, "%s: null pointer", fn);
     const int64_t total = (int64_t)B * H * S * D;
     const int64_t want = (total + 255) / 256;
+    count_launch();
     dequant_int8_kernel<<<(unsigned)(want < 148 * 16 ? want : 148 * 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         codes, c_sb, c_sh, c_ss, static_cast<const uint16_t*>(scale), static_cast<const uint16_t*>(mn), m_sb, m_sh, m_s2, per_page,
         B, H, S, D, page, static_cast<uint16_t*>(out), o_sb, o_sh, o_ss);
@@ -629,6 +632,7 @@ extern "C" int fq_sparse_decode_int8_counted(
         if (D == 128) launch_k(PDL_ATTN, sparse_decode_int8_q_kernel<128>, grid, dim3(128), 0, st, p);
         else launch_k(PDL_ATTN, sparse_decode_int8_q_kernel<64>, grid, dim3(128), 0, st, p);
     } else {
+        count_launch();
         if (D == 128) sparse_decode_int8_kernel<128><<<grid, 128, 0, st>>>(p);
         else sparse_decode_int8_kernel<64><<<grid, 128, 0, st>>>(p);
     }

@@ -569,6 +569,7 @@ extern "C" int fq_argmax_f16(const void* x, int64_t rows, int N, int32_t* out, v
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = 2;
+    count_launch();
     cudaLaunchKernelEx(&cfg, argmax_f16_kernel, static_cast<const __half*>(x), N, out);
     FQ_CHECK_LAUNCH(fn);
     return FQ_OK;

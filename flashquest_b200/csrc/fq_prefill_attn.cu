@@ -215,6 +215,7 @@ static int launch_prefill(const PrefillParams& p, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(FQ_ERR_CUDA, "fq_prefill_attention: cannot reserve %zu B of shared memory: %s", smem, cudaGetErrorString(e));
     dim3 grid((unsigned)((p.Sq + PF_BM - 1) / PF_BM), (unsigned)p.Hq, (unsigned)p.B);
+    count_launch();
     kern<<<grid, PF_THREADS, smem, st>>>(p);
     return FQ_OK;
 }

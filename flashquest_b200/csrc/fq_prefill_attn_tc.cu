@@ -453,6 +453,7 @@ bool prefill_attention_tc_launch(const void* Q, int64_t q_sb, int64_t q_sh, int6
     cudaError_t e = cudaFuncSetAttribute(prefill_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM);
     if (e != cudaSuccess) { *rc = fail(FQ_ERR_CUDA, "fq_prefill_attention: cannot reserve %d B of shared memory: %s", PT_SMEM, cudaGetErrorString(e)); return true; }
     dim3 grid((unsigned)((Sq + PT_BM - 1) / PT_BM), (unsigned)Hq, (unsigned)B);
+    count_launch();
     prefill_attn_tc_kernel<<<grid, PT_THREADS, PT_SMEM, st>>>(mq, mk, mv, p);
     return true;
 }

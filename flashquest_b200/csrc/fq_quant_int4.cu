@@ -254,6 +254,7 @@ extern "C" int fq_dequantize_int4(
     const int64_t total = (int64_t)B * H * S * (D / 8);
     const int64_t want = (total + 255) / 256;
     const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
+    count_launch();
     dequant_int4_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         packed, pk_sb, pk_sh, pk_ss, static_cast<const uint16_t*>(scale), static_cast<const uint16_t*>(mn),
         m_sb, m_sh, m_s2, per_page, B, H, S, D, page, static_cast<uint16_t*>(out), o_sb, o_sh, o_ss);

@@ -704,6 +704,7 @@ static cudaError_t launch_score_select(int CH, const ScoreSelectParams& p, dim3 
             cudaError_t e = allow_smem<score_select_kernel<QT, NR, CHV>>(FUSED_SMEM_MAX);                            \
             if (e != cudaSuccess) return e;                                                                          \
         }                                                                                                            \
+        count_launch();                                                                                              \
         return cudaLaunchKernelEx(&cfg, score_select_kernel<QT, NR, CHV>, p);                                        \
     } while (0)
     if (CH == 1) FQ_SS(1);
@@ -791,6 +792,7 @@ extern "C" int fq_build_compact_counted(const uint8_t* mask, int64_t mk_sr, int6
     FQ_CHECK_ARG(rows >= 0 && P >= 0 && compact && (mask || P == 0 || rows == 0), FQ_ERR_ARG, "%s: bad arguments", fn);
     if (rows == 0) return FQ_OK;
     FQ_CHECK_ARG(rows <= 0x7fffffffLL, FQ_ERR_ARG, "%s: too many rows", fn);
+    count_launch();
     build_compact_kernel<<<(unsigned)rows, select_threads(P), 0, static_cast<cudaStream_t>(stream)>>>(
         mask, mk_sr, P, compact, cp_sr, bucket, count);
     FQ_CHECK_LAUNCH(fn);

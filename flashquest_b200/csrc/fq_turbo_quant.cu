@@ -401,6 +401,7 @@ static bool turbo_launch128(const TurboParams& p, int dtype, int B, int H, cudaS
     const int iters = tiles > 148 * 24 ? 2 : 1;
     const int per_cta = TQ_WARPS * TQ_TOK * iters;
     dim3 grid((unsigned)((p.n_quant + per_cta - 1) / per_cta), (unsigned)H, (unsigned)(B * p.n_streams));
+    count_launch();
     if (dtype == FQ_F16) turbo_quant128_kernel<__half><<<grid, TQ_WARPS * 32, 0, st>>>(p, iters, in16, out16);
     else turbo_quant128_kernel<__nv_bfloat16><<<grid, TQ_WARPS * 32, 0, st>>>(p, iters, in16, out16);
     return true;
@@ -460,6 +461,7 @@ static int launch_wht(const void* x, void* out, int64_t n_rows, int D, cudaStrea
 template <typename T>
 static void launch_turbo(const TurboParams& p, dim3 grid, cudaStream_t st) {
     const int epl = p.D >= 32 ? p.D / 32 : 1;
+    count_launch();
 #define FQ_T(E) turbo_quant_kernel<T, E><<<grid, 128, 0, st>>>(p)
     switch (epl) {
         case 1: FQ_T(1); break;
@@ -588,6 +590,7 @@ extern "C" int fq_dequantize_turbo(
     dim3 grid((unsigned)((S + 3) / 4), (unsigned)H, (unsigned)B);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int epl = D >= 32 ? D / 32 : 1;
+    count_launch();
 #define FQ_D(E) turbo_dequant_kernel<E><<<grid, 128, 0, st>>>(msb, ms_sb, ms_sh, ms_ss, lsb, ls_sb, ls_sh, ls_ss, \
         static_cast<const uint16_t*>(scale), sc_sb, sc_sh, sc_ss, S, D, static_cast<uint16_t*>(out), o_sb, o_sh, o_ss)
     switch (epl) {

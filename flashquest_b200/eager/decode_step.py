@@ -4,8 +4,9 @@ Host-side counterpart of the decode branch of make_quest_persistent_forward
 (flashquest/eager/llama_persistent_patch.py:202-245): static k_max / BUCKET_MAX computed
 once (:77-85), per-head retention from a head pattern (:214-219), page scores from the
 metadata, top-k + compact index, sparse attention over the selected pages, and the staged
-tail merged in the same softmax.  Three kernel launches per layer (the first one also appends), no allocation per step
-(all outputs preallocated), so a whole multi-layer step can be captured in a CUDA graph.
+tail merged in the same softmax.  Three kernel launches per layer (the first one also appends, where that
+completes no page), no allocation per step (all outputs preallocated), so a whole multi-layer step can be
+captured in a CUDA graph.
 """
 from __future__ import annotations
 
@@ -48,6 +49,16 @@ class _NativeSteps:
             self.pattern_retention.data_ptr())
         self._outs = [(self.O[i].unsqueeze(2), self.lse[i].unsqueeze(2)) for i in range(L)]
         self._step, self._forward = bind().step, bind().forward
+        self._launched = 0
+
+    @property
+    def launches(self) -> int:
+        """Kernels that this object's calls have launched."""
+        return self._launched + bind().launches(self._plan_)
+
+    @launches.setter
+    def launches(self, value: int):
+        self._launched += value - self.launches
 
     def _rotated(self, i):
         """q, k, v (i = 0, 1, 2) as they went into the cache, of the layer that forward_token has last been called for."""
@@ -91,7 +102,6 @@ class _NativeSteps:
         if rc:
             check(rc)
         self.cache._seen_tokens[layer_idx] = seen + n_new
-        self.launches += self.LAUNCHES
         return self._outs[layer_idx]
 
     def forward_token(self, q, k, v, cos, sin, layer_idx: int, prm=None, pattern=None):
@@ -106,7 +116,6 @@ class _NativeSteps:
         if rc:
             check(rc)
         self.cache._seen_tokens[layer_idx] = seen + 1
-        self.launches += self.LAUNCHES + 1
         self._rot_layer = layer_idx
         return self._outs[layer_idx][0]
 
@@ -123,8 +132,6 @@ class _NativeSteps:
 
 
 class QuestDecodeInt4(_NativeSteps):
-    LAUNCHES = 3          # one more where the append completes a page
-
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4,
                  window_pages: int = 2, head_pattern_layer: torch.Tensor | None = None,
                  q_dtype=torch.bfloat16, n_split: int | None = None):
@@ -169,7 +176,6 @@ class QuestDecodeInt4(_NativeSteps):
         # one split-K workspace per layer: launches of different layers may overlap in a graph
         self.ws_bytes = (nbytes + 255) // 256 * 256
         self.workspace = torch.zeros(L, _whole(nbytes), dtype=torch.uint8, device=dev)
-        self.launches = 0
         # descriptors for the one-call-per-layer entry point
         self._cdesc = cache.desc()
         self._prm = DecodeParams(
@@ -199,6 +205,7 @@ class QuestDecodeInt4(_NativeSteps):
         if q4.stride(3) != 1:
             q4 = q4.contiguous()
         seen = (ctypes.c_int * Ln)(*c._seen_tokens[:Ln])
+        before = bind().launches()
         check(lib().fq_decode_step_int4(
             ctypes.byref(self._cdesc), Ln, seen,
             ptr(k_new), ptr(v_new), k_new.stride(0), k_new.stride(1), k_new.stride(2), k_new.stride(3), n_new,
@@ -206,9 +213,9 @@ class QuestDecodeInt4(_NativeSteps):
             ptr(self.scores), self.scores.stride(0), ptr(self.compact), self.compact.stride(0),
             ptr(self.O), self.O.stride(0), ptr(self.lse), self.lse.stride(0),
             ptr(self.workspace), self.workspace.stride(0), self.workspace.shape[1], stream_ptr(self.device)))
+        self._launched += bind().launches() - before
         for li in range(Ln):
             c._seen_tokens[li] += n_new
-        self.launches += self.LAUNCHES       # all layers together where they are of equal length
         return self.O.unsqueeze(3), self.lse.unsqueeze(3)
 
     def capture_step_graph(self, k_new: torch.Tensor, v_new: torch.Tensor, q: torch.Tensor, before=None, after=None):
@@ -245,7 +252,9 @@ class QuestDecodeInt4(_NativeSteps):
         with torch.cuda.graph(graph, capture_error_mode="thread_local"):
             if before is not None:
                 before()
+            first = bind().launches()
             launch()
+            launches = bind().launches() - first
             if after is not None:
                 after()
 
@@ -255,7 +264,7 @@ class QuestDecodeInt4(_NativeSteps):
                 raise RuntimeError(f"PersistentInt4KVCache: seen+new={seen + n_new} exceeds max_seq_len={c.max_seq_len}")
             graph.replay()
             c._seen_tokens[:Ln] = [t + n_new for t in c._seen_tokens[:Ln]]
-            self.launches += 3 * Ln + 2          # one append for all layers, 3 per layer, the position update
+            self._launched += launches
             return self.O.unsqueeze(3), self.lse.unsqueeze(3)
 
         replay.graph, replay.pos = graph, pos
@@ -264,6 +273,7 @@ class QuestDecodeInt4(_NativeSteps):
     def attend(self, q: torch.Tensor, layer_idx: int):
         """q (B,H_q,1,D) or (B,H_q,D), the cache's dtype family (fp16/bf16).  Returns views
         (O (B,H_q,1,D), lse (B,H_q,1)) of preallocated per-layer buffers."""
+        before = bind().launches()
         c = self.cache
         seen = c._seen_tokens[layer_idx]
         page = self.page
@@ -287,7 +297,6 @@ class QuestDecodeInt4(_NativeSteps):
                 ptr(self.retention_per_q), self.retention, min(self.k_max_static, P), self.num_sinks,
                 self.window_pages, None, 0, 0, ptr(compact), compact.stride(0), compact.stride(1), self.bucket,
                 None, st))
-            self.launches += 2
         Kp, Vp, Vs, Vm = c.K_packed[li], c.V_packed[li], c.V_scale[li], c.V_mn[li]
         Kt, Vt = c.K_partial[li], c.V_partial[li]
         O, lse = self.O[li], self.lse[li]
@@ -303,7 +312,7 @@ class QuestDecodeInt4(_NativeSteps):
             self.B, self.Hq, self.Hkv, completed, P, self.D, page, self.sm_scale,
             ptr(O), O.stride(0), O.stride(1), ptr(lse),
             ptr(self.workspace[li]), self.workspace.shape[1], self.n_split, st))
-        self.launches += 1
+        self._launched += bind().launches() - before
         return O.unsqueeze(2), lse.unsqueeze(2)
 
 
@@ -313,7 +322,6 @@ class QuestDecodeTurbo(_NativeSteps):
     foreign call per layer (fq_decode_layer_turbo): append, page scores from the raw page metadata,
     top-k + compact index, rotation of Q, sparse attention in the rotated basis, rotation of O, tail
     attention and LSE merge.  All buffers are preallocated, a part for each layer."""
-    LAUNCHES = 4
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,
                  q_dtype=torch.bfloat16, n_split: int | None = None):
@@ -348,7 +356,6 @@ class QuestDecodeTurbo(_NativeSteps):
         self._cdesc = cache.desc()
         self._prm = DecodeParams(self.Hq, None, self.retention, self.k_max_static, self.num_sinks, self.window_pages,
                                  self.bucket, self.sm_scale, self.n_split)
-        self.launches = 0
         self._build_plan(3, self.scores, self.compact, self.workspace, self.scratch)
 
 
@@ -356,7 +363,6 @@ class QuestDecodeInt8(_NativeSteps):
     """Decode-branch dispatcher for the persistent INT8 cache: the kv_bits == 8 route of make_quest_persistent_forward
     (flashquest/eager/llama_persistent_patch.py:202-245) as ONE foreign call per layer (fq_decode_layer_int8): append, page
     scores, top-k with compact index, attention with the staged tail in the same softmax."""
-    LAUNCHES = 4
     COPY_ROWS = True
 
     def __init__(self, cache, *, num_q_heads: int, retention: float = 0.20, num_sinks: int = 4, window_pages: int = 2,
@@ -388,5 +394,4 @@ class QuestDecodeInt8(_NativeSteps):
         self._cdesc = cache.desc()
         self._prm = DecodeParams(self.Hq, None, self.retention, self.k_max_static, self.num_sinks, self.window_pages,
                                  self.bucket, self.sm_scale, self.n_split)
-        self.launches = 0
         self._build_plan(8, self.scores, self.compact, self.workspace)

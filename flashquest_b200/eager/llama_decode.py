@@ -21,7 +21,7 @@ import ctypes
 
 import torch
 
-from .._lib import (AwqLinearDesc, LlamaLayerDesc, LlamaModelDesc, LlamaScratchDesc, check, lib, ptr, stream_ptr)
+from .._lib import (AwqLinearDesc, LlamaLayerDesc, LlamaModelDesc, LlamaScratchDesc, bind, check, lib, ptr, stream_ptr)
 from ..cache.persistent_int4 import PersistentInt4KVCache
 from ..kernel.fused_proj import awq_gemv_fused
 from ..quant import AWQLinear
@@ -116,7 +116,7 @@ class LlamaInt4Decoder:
         self.normed, self.act = mk(batch_size, H), mk(batch_size, cfg.ffn)
         self.logits = mk(batch_size, cfg.vocab)
         self.next_ids = torch.empty(batch_size, dtype=torch.int32, device=self.dev)
-        self.launches = 0
+        self.launches = 0                                        # kernels launched, besides those of self.attn's own calls
         self._build_native()
 
     def _build_native(self):
@@ -153,11 +153,12 @@ class LlamaInt4Decoder:
         seen = (ctypes.c_int * n_l)(*c._seen_tokens[:n_l])
         if c._seen_tokens[0] + 1 > c.max_seq_len:
             raise RuntimeError(f"PersistentInt4KVCache: seen+new={c._seen_tokens[0] + 1} exceeds max_seq_len={c.max_seq_len}")
+        before = bind().launches()
         check(lib().fq_llama_decode_step(ctypes.byref(self._model), ctypes.byref(self.attn._cdesc), ctypes.byref(self.attn._prm),
                                          seen, ptr(x), self.B, ctypes.byref(self._scratch), stream_ptr(self.dev)))
         for li in range(n_l):
             c._seen_tokens[li] += 1
-        self.launches += 7 * n_l + 3
+        self.launches += bind().launches() - before
         return self.next_ids
 
     def prefill(self, token_ids: torch.Tensor) -> torch.Tensor:
@@ -182,24 +183,23 @@ class LlamaInt4Decoder:
         x = self.w.embed[token_ids.to(self.dev).long()]          # (S, H) gather: plumbing
         nbytes = lib().fq_llama_prefill_workspace_bytes(ctypes.byref(self._model), S)
         ws = torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
+        before = bind().launches()
         check(lib().fq_llama_prefill(ctypes.byref(self._model), ctypes.byref(self.attn._cdesc), ptr(x), S, self.attn.sm_scale,
                                      ptr(ws), nbytes, ptr(self.logits), ptr(self.next_ids), stream_ptr(self.dev)))
         for li in range(c.layers):
             cache._seen_tokens[li] = S
-        self.launches += 10 * c.layers + 3
+        self.launches += bind().launches() - before
         return self.next_ids
 
     # -- thin wrappers over the C ABI ------------------------------------------------------
     def _add_rmsnorm(self, a, b, weight, sum_out, y):
         check(lib().fq_add_rmsnorm(ptr(a), ptr(b), ptr(weight), self.cfg.rms_eps, a.shape[0], a.shape[1],
                                    ptr(sum_out), ptr(y), stream_ptr(self.dev)))
-        self.launches += 1
 
     def _rope(self, q, k, pos):
         c = self.cfg
         check(lib().fq_rope(ptr(q), q.stride(0), q.stride(1), c.q_heads, ptr(k), k.stride(0), k.stride(1), c.kv_heads,
                             self.B, c.head_dim, int(pos), c.rope_theta, stream_ptr(self.dev)))
-        self.launches += 1
 
     def capture_decode_graph(self, token_ids: torch.Tensor):
         """CUDA graph of one greedy step that feeds itself: embedding gather of the ids buffer, the
@@ -220,9 +220,11 @@ class LlamaInt4Decoder:
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, capture_error_mode="thread_local"):
             x = self.w.embed[ids.long()]
+            before = bind().launches()
             check(lib().fq_llama_decode_step_dev(ctypes.byref(self._model), ctypes.byref(self.attn._cdesc),
                                                  ctypes.byref(self.attn._prm), ptr(pos), ptr(x), self.B,
                                                  ctypes.byref(self._scratch), stream_ptr(self.dev)))
+            launches = bind().launches() - before
             ids.copy_(self.next_ids)
 
         def replay():
@@ -231,7 +233,7 @@ class LlamaInt4Decoder:
             graph.replay()
             for li in range(n_l):
                 c._seen_tokens[li] += 1
-            self.launches += 7 * n_l + 4
+            self.launches += launches
             return ids
 
         replay.graph, replay.ids, replay.pos = graph, ids, pos
@@ -244,6 +246,7 @@ class LlamaInt4Decoder:
         c, w, B = self.cfg, self.w, self.B
         L = lib()
         st = stream_ptr(self.dev)
+        before, before_attn = bind().launches(), self.attn.launches
         pos = self.cache.get_seq_length(0)
         x = w.embed[token_ids.long()]                            # (B, H) gather: plumbing
         flip = 0
@@ -276,9 +279,8 @@ class LlamaInt4Decoder:
             check(L.fq_swiglu(ptr(gate), ptr(up), gate.numel(), ptr(self.act), st))
             (down,) = awq_gemv_fused(self.act.view(B, 1, -1), (lw.down_proj,))
             delta = down.view(B, -1)
-            self.launches += 5
         x = add_norm(x, delta, w.final_norm)
         check(L.fq_gemv_f16(ptr(self.normed), ptr(w.lm_head), B, c.hidden, c.vocab, ptr(self.logits), st))
         check(L.fq_argmax_f16(ptr(self.logits), B, c.vocab, ptr(self.next_ids), st))
-        self.launches += 2
+        self.launches += bind().launches() - before - (self.attn.launches - before_attn)
         return self.next_ids

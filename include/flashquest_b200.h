@@ -41,6 +41,9 @@ extern "C" {
 const char* fq_last_error_string(void);
 const char* fq_version(void);
 
+/* How many kernels the calls of this thread have launched (captured ones count once, at their capture). */
+unsigned long long fq_launches(void);
+
 /* Reads and clears the device-side status word of the current device (synchronises the
  * device).  0 = no kernel reported a problem; FQ_ERR_TIMEOUT = a bounded wait on an
  * asynchronous copy ran out and the kernel returned early. */
