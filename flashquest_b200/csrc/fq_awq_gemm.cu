@@ -13,12 +13,12 @@
 //   warp 1       : in the first CTA, one lane issues tcgen05.mma (M 256, N 256, K 16, fp16 x fp16 -> fp32 in TMEM),
 //                  four per step, commits the stages back to both producers and the accumulator set to both epilogues;
 //                  in both, the warp owns the tensor-memory allocation (512 columns);
-//   warps 2..9   : dequantise the raw tile to fp16 in shared memory, (code - zero) * scale rounded
+//   warps 2..13  : three groups that take turns dequantise the raw tile to fp16 in shared memory, (code - zero) * scale rounded
 //                  once to fp16 like the reference's GEMM kernels, written N-contiguous in the
 //                  canonical MN-major 128-byte-swizzle layout (AWQ's nibble order makes every
 //                  masked word a pair of neighbouring columns, so a 32-bit word of codes becomes one
 //                  16-byte store);
-//   warps 10..13 : epilogue — drain an accumulator set (tcgen05.ld, lane quarter = warp id mod 4),
+//   warps 14..17 : epilogue — drain an accumulator set (tcgen05.ld, lane quarter = warp id mod 4),
 //                  add the bias, convert to fp16, store y, hand the set back.
 // Stages and accumulator sets are handed over through mbarriers (TMA bytes -> dequantised ->
 // consumed; multiplied -> drained), those the first CTA's MMA warp waits for with arrivals from both CTAs; every wait is
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) awq_gemm_kernel(
         }
     } else if (warp < 2 + GM_DEQ_WARPS) {
         // =========================== dequantise ===========================
-        // two groups of four warps alternate: one block is converted while the other's is multiplied
+        // three groups of four warps take turns: two blocks are converted while a third is multiplied
         const int grp = (warp - 2) / GM_DEQ_GROUP;
         const int t = (tid - 64) % (GM_DEQ_GROUP * 32);
         const int c = t & 15;                         // int32 column of the raw tile = 8 of this CTA's output columns

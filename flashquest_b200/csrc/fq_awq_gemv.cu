@@ -111,6 +111,8 @@ __device__ __forceinline__ void gemv_mma_16816(float (&c)[4], uint32_t a0, uint3
 // q/k/v, o, gate/up, down of the Llama-3.2-3B shape, us: one row 6.6 / 5.2 / 12.5 / 10.6 -> 6.0 / 4.7 / 11.5 / 9.8; eight rows
 // 10.0 / 7.4 / 18.0 / 17.1 -> 8.5 / 6.3 / 15.1 / 13.9.
 // (Twice the warps with half the nibbles each is slower: 12.3 against 10.2 us at two rows, the loads of words and x double.)
+// Registers are cut for three CTAs per SM, which launches of more than two per SM with the short ring have; those that `room`
+// spreads over the SMs by one or two leave them unused.
 template <int M, int GEMV_STAGES, bool FAST>
 __global__ void __launch_bounds__(GEMV_THREADS, 3) awq_gemv_kernel(GemvParams p) {
     constexpr bool MMA = M > 1;
@@ -550,7 +552,9 @@ extern "C" int fq_awq_gemv_default_splits(int K, int N_total, int group) {
     if (K <= 0 || N_total <= 0 || group <= 0) return 1;
     const int n_groups = K / group;
     const int tiles = (N_total / 8 + fq::GEMV_PACKS - 1) / fq::GEMV_PACKS;
-    int want = (3 * 148 + tiles - 1) / tiles;       // about three CTAs per SM
+    // as many splits as three CTAs per SM allow, at most a cluster's eight (2048 -> 11264: 352 CTAs; the Llama-3.2-3B shapes end
+    // below that, with 160, 96, 256 and 96, and are spread by `room` in gemv_launch)
+    int want = (3 * 148 + tiles - 1) / tiles;
     if (want > fq::GEMV_MAX_CLUSTER) want = fq::GEMV_MAX_CLUSTER;
     if (want > n_groups) want = n_groups;
     if (want < 1) want = 1;

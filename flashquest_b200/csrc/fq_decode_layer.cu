@@ -120,8 +120,9 @@ extern "C" int fq_decode_step_int4(
     // All layers' inputs are here and no layer waits for another: the layers of a dense cache go through the four launches
     // together, as one batch of n_layers * B sequences.  One layer of one sequence leaves the GPU idle between dependent
     // launches (23 us a layer for 3.4 us of HBM time).  28 layers of one sequence, 24/8 heads of 128, layer by layer ->
-    // together: 515 tokens 245 -> 27 us, 8k 520 -> 79, 32k 648 -> 245.  At 32k the metadata of all layers (235 MB) no longer stays
-    // in L2 between scoring and attention; groups that do fit were slower all the same (4 layers 353 us, 7 337, 14 256).
+    // together: 515 tokens 245 -> 18 us, 8k 520 -> 73, 32k 648 -> 235.  At 32k the metadata of all layers (235 MB) no longer stays
+    // in L2 between scoring and attention; groups that do fit were slower all the same (4 layers 353 us, 7 337, 14 256, all 28
+    // with the attention of that time 245).
     // Layers with parameters or positions of their own, or of other strides, go one by one.
     const int B = c->B, Hq = prm->Hq;
     bool together = n_layers > 1 && B > 0 && (int64_t)n_layers * B <= 65535 && prm_stride == 0 &&

@@ -626,8 +626,9 @@ extern "C" int fq_sparse_decode_int8_counted(
     // 16-byte aligned code and metadata rows: the quarter-warp-per-token kernel
     const bool vec16 = have_pages && aligned(K_uint8, 16) && aligned(V_uint8, 16) && kv_sb % 16 == 0 && kv_sh % 16 == 0 && kv_ss % 16 == 0 &&
                        aligned(K_scale, 16) && aligned(K_mn, 16) && km_sb % 8 == 0 && km_sh % 8 == 0 && km_sp % 8 == 0;
-    // (An ordinary launch: one wave of CTAs that started early would settle unevenly around the selection's, 59 against 53 us for
-    // a step of 4 x 20k.  The merge behind it starts early.)
+    // Attention and merge start early.  A whole INT8 step with an ordinary launch of the attention against this, us: 4 x 20k in pages
+    // of 64 41.4 and 39.8, 16 x 32k in pages of 16 195.0 and 192.5, one sequence of 4k 17.0 and 15.5.  (The unaligned form reads its
+    // list without a wait and is an ordinary launch.)
     if (vec16) {
         if (D == 128) launch_k(PDL_ATTN, sparse_decode_int8_q_kernel<128>, grid, dim3(128), 0, st, p);
         else launch_k(PDL_ATTN, sparse_decode_int8_q_kernel<64>, grid, dim3(128), 0, st, p);

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(TQ_THREADS, 3) sparse_decode_turbo_kernel(Turb
         for (int j = 0; j < EPL; ++j) s_q[lane * EPL + j] = from_f32<QT>(v[j]);
     }
     __syncthreads();
-    pdl_wait();        // the rotated Q and the page list come from the kernels before this one
+    pdl_wait();        // the page list, and Q where it comes rotated, are the kernels' before this one
     pdl_trigger();
     const uint32_t lut_addr = (uint32_t)__cvta_generic_to_shared(s_lut) + lane * 8;      // this lane's column of the table
 

@@ -257,6 +257,8 @@ int fq_prefill_attention(
  *   fq_sparse_decode_workspace_bytes(...) bytes whose first B*Hq*4 bytes were zeroed once
  *   (the kernel leaves them zero again); concurrent calls must not share a workspace.
  * D in {64,128}; page in {8,16,32,64,128}.  Page rows must be 16-byte aligned.
+ * Range: |Q| * sm_scale * log2(e), that times K_scale, and V_scale must stay below 2^28 (2.7e8), where the kernel's
+ * multipliers become infinite.  fp16 Q, K and V cannot reach it at sm_scale = 1/sqrt(D); bf16 values of 1e9 can.
  */
 size_t fq_sparse_decode_workspace_bytes(int B, int Hq, int D, int n_split);
 int fq_sparse_decode_default_splits(int B, int Hq, int bucket, int page);
