@@ -106,8 +106,9 @@ __device__ __forceinline__ void gemv_mma_16816(float (&c)[4], uint32_t a0, uint3
 // weight rows, B holds the 8 activation rows; a warp owns 8 packs and every second 16-row step of the group.
 //
 // FAST: groups of 128, AutoAWQ's nibble order, 16-byte rows -- all of it known to the compiler: loops without counters,
-// shared-memory offsets in the instructions, no selects.  Bound by instruction issue (8192 -> 3072 at one row: 500 instructions
-// per warp and group, 0.88 us, of which 224 multiply; weights already in L2 change nothing), so that is what the variant saves.
+// shared-memory offsets in the instructions, no selects.  Bound by its instructions at two warps per scheduler (8192 -> 3072 at one row: 500 instructions
+// per warp and group, of which 224 multiply, 0.88 us, 58 % of the slots with loads from shared memory to wait for; weights
+// already in L2 change nothing), so that is what the variant saves.
 // q/k/v, o, gate/up, down of the Llama-3.2-3B shape, us: one row 6.6 / 5.2 / 12.5 / 10.6 -> 6.0 / 4.7 / 11.5 / 9.8; eight rows
 // 10.0 / 7.4 / 18.0 / 17.1 -> 8.5 / 6.3 / 15.1 / 13.9.
 // (Twice the warps with half the nibbles each is slower: 12.3 against 10.2 us at two rows, the loads of words and x double.)
