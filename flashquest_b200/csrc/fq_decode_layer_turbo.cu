@@ -8,7 +8,7 @@
 extern "C" size_t fq_decode_layer_turbo_scratch_bytes(int B, int Hq, int D) {
     if (B <= 0 || Hq <= 0 || D <= 0) return 0;
     const size_t rows = (size_t)B * Hq;
-    return ((rows * D * 2 * 4 + 255) & ~(size_t)255) + rows * 2 * 4;     // Q_rot, O_rot, two O parts (16-bit) | two lse parts
+    return ((rows * D * 2 + 255) & ~(size_t)255) + rows * 4;     // O in the rotated basis (16-bit) | lse of its part
 }
 
 extern "C" int fq_decode_layer_turbo(
@@ -54,8 +54,8 @@ extern "C" int fq_decode_layer_turbo(
     }
     const int64_t rows = (int64_t)B * Hq;
     char* sb = static_cast<char*>(scratch);
-    void* O_rot = sb + rows * D * 2;
-    float* lse_parts = reinterpret_cast<float*>(sb + ((rows * D * 8 + 255) & ~(int64_t)255));
+    void* O_rot = sb;
+    float* lse_rot = reinterpret_cast<float*>(sb + ((rows * D * 2 + 255) & ~(int64_t)255));
     const bool sparse = P > 0, both = sparse && tail > 0;
     if (sparse) {
         rc = page_scores_int4_launch(Q, q_dtype, q_sb, q_sh, Ksr, Kmr, c->km_sb, c->km_sh, c->km_sp, B, Hq, Hkv, P, D, scores, (int64_t)Hq * P, P, stream,
@@ -73,10 +73,10 @@ extern "C" int fq_decode_layer_turbo(
                                     Vms, c->ms_sb, c->ms_sh, c->ms_ss, Vls, c->ls_sb, c->ls_sh, c->ls_ss, Vst, c->st_sb, c->st_sh,
                                     compact, (int64_t)Hq * prm->bucket, prm->bucket, prm->bucket,
                                     B, Hq, Hkv, completed, P, D, page, prm->sm_scale,
-                                    O_rot, (int64_t)Hq * D, D, both ? lse_parts : lse, workspace, workspace_bytes, n_split, stream, true);
+                                    O_rot, (int64_t)Hq * D, D, both ? lse_rot : lse, workspace, workspace_bytes, n_split, stream, true);
         if (rc != FQ_OK) return rc;
         if (both)
-            return turbo_finish_launch(O_rot, lse_parts, Q, q_dtype, Kt, Vt, c->kv_dtype, c->pt_sb, c->pt_sh, c->pt_ss, tail, B, Hq, Hkv, D, prm->sm_scale, O, lse, stream);
+            return turbo_finish_launch(O_rot, lse_rot, Q, q_dtype, Kt, Vt, c->kv_dtype, c->pt_sb, c->pt_sh, c->pt_ss, tail, B, Hq, Hkv, D, prm->sm_scale, O, lse, stream);
         return fq_wht(O_rot, O, q_dtype, rows, D, stream);
     }
     // no page yet: dense attention over the staged tokens, the tail-only case of the INT4 kernel

@@ -601,7 +601,7 @@ int fq_rope_qkv_pattern(const void* q, int64_t q_sb, const void* k, int64_t k_sb
  * like fq_int4_cache does for the INT4 cache; both msb planes share one set of strides, both lsb
  * planes another, both token scales a third.  Q and O are dense (B,Hq,D) in the RAW basis;
  * scores (B,Hq,P) and compact (B,Hq,bucket) are scratch; `scratch` holds
- * fq_decode_layer_turbo_scratch_bytes(B,Hq,D) bytes (rotated Q and O, the two partial results);
+ * fq_decode_layer_turbo_scratch_bytes(B,Hq,D) bytes (O and lse of the pages, in the rotated basis);
  * workspace / n_split as for fq_sparse_decode_turbo.  page must be a multiple of 16. */
 typedef struct fq_turbo_cache {
     uint8_t* K_msb; uint8_t* K_lsb; uint8_t* V_msb; uint8_t* V_lsb;   /* (L,B,H,S,D/8) and (L,B,H,S,D/4) u8 */
