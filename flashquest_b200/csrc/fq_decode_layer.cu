@@ -188,7 +188,9 @@ int decode_layer_int4_dyn(const fq_int4_cache* c, int l, const int* pos, const v
     char* Kt = static_cast<char*>(c->K_partial) + l * c->pt_sl * kv_esz;
     char* Vt = static_cast<char*>(c->V_partial) + l * c->pt_sl * kv_esz;
     // host-side sizes are the maxima (they size grids and pass validation); the kernels read *pos
-    DynPos dp_early = dp;          // scores, selection and attention come at least two launches after any writer of *pos
+    // Scores, selection and attention come at least two launches after any writer of *pos: with the append along, where the scores
+    // are the first launch here, the caller has one that waits (the Llama step's q/k/v projections) between the writer and this call.
+    DynPos dp_early = dp;
     dp_early.early = true;
     int rc = FQ_OK;
     QuantParams now;

@@ -401,3 +401,36 @@ def test_more_than_four_query_heads_per_kv_head(q_heads, kv_heads, head_dim):
         want = oracle.page_scores_int4_fast(q.cpu(), v["K_scale"].cpu(), v["K_mn"].cpu()).view(2, q_heads, P)
         assert torch.equal(a.attn.scores[-1, :, :, :P].cpu(), want), t
         assert torch.equal(b.attn.scores[-1].view(-1)[:2 * q_heads * P].view(2, q_heads, P).cpu(), want), t
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim,page,S", [(24, 8, 128, 16, 1019), (12, 2, 128, 16, 539), (16, 2, 64, 64, 2170)])
+def test_graph_equals_host_past_the_first_scoring_cta(q_heads, kv_heads, head_dim, page, S):
+    """A page that a graph's step completes, beyond the 32 pages of one scoring CTA: packed and scored by the CTA that appends, with no
+    window page to put it into the selection whatever its score.  Logits and page scores are those of the host's step, bit for
+    bit, and the scores the oracle's."""
+    from flashquest_b200.eager.llama_decode import LlamaConfig, LlamaInt4Decoder, random_llama_weights
+    cfg = LlamaConfig(hidden=256, layers=2, q_heads=q_heads, kv_heads=kv_heads, head_dim=head_dim, ffn=512, vocab=512)
+    w = random_llama_weights(cfg, "cuda", seed=7)
+    mk = lambda: LlamaInt4Decoder(cfg, w, batch_size=1, max_seq_len=(S // page + 4) * page, page_size=page, retention=0.3, num_sinks=1, window_pages=0)
+    a, b = mk(), mk()
+    prompt = torch.randint(0, cfg.vocab, (S,), generator=torch.Generator().manual_seed(S), dtype=torch.int32).cuda()
+    x = a.prefill(prompt).clone()
+    assert torch.equal(x, b.prefill(prompt))
+    for d in (a, b):                                   # the first call outside a capture
+        y = d.decode_step(x).clone()
+    x = y
+    replay = a.capture_decode_graph(x)
+    ends = 0
+    for t in range(S + 2, S + 2 + (page + 12 if page < 64 else 24)):                     # cached tokens behind the step
+        replay()
+        x = b.decode_step(x).clone()
+        assert torch.equal(a.logits, b.logits), t
+        P, v = t // page, b.cache.get_views(cfg.layers - 1)
+        assert P > 32
+        mine, host = a.attn.scores[-1, 0, :, :P], b.attn.scores[-1].view(-1)[:q_heads * P].view(q_heads, P)
+        assert torch.equal(mine, host), t
+        if t % page == 0:
+            ends += 1
+            q = b._nat["q"].view(1, q_heads, 1, head_dim)                                  # the last layer's
+            assert torch.equal(mine.cpu(), oracle.page_scores_int4_fast(q.cpu(), v["K_scale"].cpu(), v["K_mn"].cpu()).view(q_heads, P)), t
+    assert ends >= 1
