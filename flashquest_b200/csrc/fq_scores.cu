@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_kernel(
     const uint16_t* __restrict__ K_scale, const uint16_t* __restrict__ K_mn,
     int64_t km_sb, int64_t km_sh, int64_t km_sp,
     int Hq, int Hkv, int P, int D, int head_off,
-    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, float levels,
+    float* __restrict__ scores, int64_t sc_sb, int64_t sc_sh, const int* __restrict__ pos, int pos_new, int pos_page, int pos_early, float levels,
     const __grid_constant__ APPEND app) {
     const int b = blockIdx.z, hkv = blockIdx.y;
     const int n_rep = Hq / Hkv;
@@ -113,8 +113,17 @@ __global__ void __launch_bounds__(SCORE_THREADS) page_scores_kernel(
     const int l = lane & 7, qw = lane >> 3;
     const int n_chunks = D >> 3;
     const int nr = min(NR, n_rep - head_off);   // heads actually present in this pass
+    // A position on the device of either kind (DynPos); the decode steps take the kernel below for theirs.  Calls without one pass
+    // both branches by, and the code in front of the wait and behind it stays apart: with neither branch the compiler lays the set-up
+    // out behind the wait, and 28 layers of 2049 pages (scores, selection, attention) take 575 us instead of 563, with the second alone 573.
+    int pos_v = 0;
+    if (pos && pos_early) pos_v = __ldcg(pos);             // in flight during the wait
     pdl_wait();        // Q and the newest metadata row come from the kernels before this one
     pdl_trigger();
+    if (pos) {
+        if (!pos_early) pos_v = *pos;
+        P = min(P, (pos_v + pos_new) / pos_page);          // completed pages after this step's append
+    }
 
     // Metadata loads of every page this quarter warp will score are issued first, the q loads
     // after them, so the two global-memory latencies overlap instead of adding up.
@@ -271,28 +280,28 @@ static void launch_scores(int CH, dim3 grid, cudaStream_t st, const void* Q, int
     const int ctas = stream_ctas(NR, D, (int)(grid.y * grid.z), P);
     const NoAppend none{};
 #define FQ_SC_ARGS static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale), static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P, D, \
-                   head_off, scores, sc_sb, sc_sh
+                   head_off, scores, sc_sb, sc_sh, dp.pos, dp.n_new, dp.page
 #define FQ_LAUNCH_SC(CHV)                                                                                                                                                  \
     do {                                                                                                                                                                   \
         if (ctas > 0)                                                                                                                                                      \
             launch_k(PDL_SCORES, page_scores_stream_kernel<QT, NR, (CHV > 2 ? 2 : CHV)>, dim3((unsigned)ctas, grid.y, grid.z), dim3(SCORE_THREADS), 0, st,                 \
                      static_cast<const QT*>(Q), q_sb, q_sh, static_cast<const uint16_t*>(K_scale), static_cast<const uint16_t*>(K_mn), km_sb, km_sh, km_sp, Hq, Hkv, P,    \
                      head_off, scores, sc_sb, sc_sh, dp.pos, dp.n_new, dp.page, levels);                                                                                   \
-        else if (dp.pos) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, dp.pos, dp.n_new, dp.page, levels, none); \
-        else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, none);                                     \
+        else if (dp.pos && dp.early) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, none);       \
+        else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, CHV, NoAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, dp.early ? 1 : 0, levels, none);                   \
     } while (0)
     if constexpr (sizeof(QT) == 2) {
         if (app) {
             ++grid.x;
             if constexpr (std::is_same_v<QT, __half>) {
                 if (dp.pos) {
-                    if (CH == 1) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, 1, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, dp.pos, dp.n_new, dp.page, levels, *app);
-                    else launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, 2, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, dp.pos, dp.n_new, dp.page, levels, *app);
+                    if (CH == 1) launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, 1, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, *app);
+                    else launch_k(PDL_SCORES, page_scores_early_kernel<QT, NR, 2, DynAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, *app);
                     return;
                 }
             }
-            if (CH == 1) launch_k(PDL_SCORES, page_scores_kernel<QT, NR, 1, StageAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, app->st);
-            else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, 2, StageAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, levels, app->st);
+            if (CH == 1) launch_k(PDL_SCORES, page_scores_kernel<QT, NR, 1, StageAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, 0, levels, app->st);
+            else launch_k(PDL_SCORES, page_scores_kernel<QT, NR, 2, StageAppend>, grid, dim3(SCORE_THREADS), 0, st, FQ_SC_ARGS, 0, levels, app->st);
             return;
         }
     }
@@ -336,11 +345,10 @@ int page_scores_int4_launch(
     const int CH = D <= 64 ? 1 : D / 64;
     dim3 grid((unsigned)((P + SCORE_PAGES_PER_CTA - 1) / SCORE_PAGES_PER_CTA), (unsigned)Hkv, (unsigned)B);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    FQ_CHECK_ARG(!dp.pos || dp.early, FQ_ERR_ARG, "%s: a device position that the kernels may not read early", fn);
     DynAppend app{};
     if (append) {
         FQ_CHECK_ARG(page_scores_take_append(q_dtype, B, Hq, Hkv, P, D) && (append_dtype == FQ_F16 || append_dtype == FQ_BF16) && append->n_layers == 1 &&
-                     append->pos == dp.pos && (!dp.pos || (q_dtype == FQ_F16 && append_dtype == FQ_F16)), FQ_ERR_ARG, "%s: an append that this launch does not take", fn);
+                     append->pos == dp.pos && (!dp.pos || (dp.early && q_dtype == FQ_F16 && append_dtype == FQ_F16)), FQ_ERR_ARG, "%s: an append that this launch does not take", fn);
         const QuantParams& q = *append;
         app.q = q;
         const int64_t first = q.pos ? 0 : q.n_head * q.st_ss;
